@@ -266,6 +266,11 @@ class QuantizedWeight:
             self.context._ck("wf_weight_free", self.context._lib.wf_weight_free(self.context.handle, h))
 
 
+def _address(a: np.ndarray) -> int:
+    """a.ctypes.data without building a ctypes object (1 us of a 20 us call)."""
+    return a.__array_interface__["data"][0]
+
+
 class CudaOpKernel:
     def execute(self, op, inputs: List) -> List:
         raise NotImplementedError
@@ -329,7 +334,7 @@ class QuantizedLinearKernel(CudaOpKernel):
             return [out]
         x = np.ascontiguousarray(lhs.data)
         y = np.empty((m, n), np.float32)
-        ctx._ck("wf_qlinear", lib.wf_qlinear(ctx.handle, rhs.handle, x.ctypes.data, dt, 0, m, y.ctypes.data, 0, self.stream))
+        ctx._ck("wf_qlinear", lib.wf_qlinear(ctx.handle, rhs.handle, _address(x), dt, 0, m, _address(y), 0, self.stream))
         return [Tensor(y, "f32")]
 
 

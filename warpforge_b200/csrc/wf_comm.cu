@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(GATHER_THREADS) gather_small_kernel(float* __r
             }
             __nanosleep(40);
         }
-        if (gave_up) atomicOr(status, STATUS_PEER_WAIT_TIMEOUT);
+        if (gave_up) report_status(status, STATUS_PEER_WAIT_TIMEOUT);
     }
     // the last CTA out counts the gather
     __syncthreads();
@@ -266,7 +266,7 @@ __global__ void gather_wait_done_kernel(GatherPeers peers, const unsigned int* e
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
         if (!t0) t0 = now;
         if (now - t0 > wait_ns || (*reinterpret_cast<volatile int*>(status) & STATUS_PEER_WAIT_TIMEOUT)) {
-            atomicOr(status, STATUS_PEER_WAIT_TIMEOUT);
+            report_status(status, STATUS_PEER_WAIT_TIMEOUT);
             return;
         }
         __nanosleep(100);
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(GATHER_THREADS) gather_large_kernel(float* __r
     }
     __syncthreads();
     if (failed) {
-        if (threadIdx.x == 0) atomicOr(status, STATUS_PEER_WAIT_TIMEOUT);
+        if (threadIdx.x == 0) report_status(status, STATUS_PEER_WAIT_TIMEOUT);
     } else {
         // strips of `rows` floats: strip c belongs to token c / world and to the rank (c % world + rank) % world, so
         // that the CTAs of all ranks read from all peers at once
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(32) gather_bulk_kernel(float* __restrict__ y, 
     }
     failed = __any_sync(0xFFFFFFFFu, failed);
     if (failed) {
-        if (lane == 0) atomicOr(status, STATUS_PEER_WAIT_TIMEOUT);
+        if (lane == 0) report_status(status, STATUS_PEER_WAIT_TIMEOUT);
     } else if (lane == 0) {
         asm volatile("fence.proxy.async;" ::: "memory");  // what the flags ordered is read by the copy engine from here on
         const int64_t n = (int64_t)world * rows;
@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(32) gather_bulk_kernel(float* __restrict__ y, 
         }
         asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         if (aborted) {
-            atomicOr(status, STATUS_GEMV_FIXUP_TIMEOUT);
+            report_status(status, STATUS_GEMV_FIXUP_TIMEOUT);
             drain_after_abort();
         }
     }
@@ -650,15 +650,17 @@ int wf_comm_destroy(int64_t ctx, int64_t comm) {
     cudaDeviceSynchronize();
     if (k->peer_ok) {
         // The peers may still be reading this rank's block of the last large gather: wait for their "done".  A peer
-        // that has gone lets this wait run out; that is no failure of any call of this context, so the status word
+        // that has gone lets this wait run out; that is no failure of any call of this context, so the status
         // is put back afterwards.
-        int before = 0;
+        int before = 0, before_host[STATUS_BITS];
         cudaMemcpy(&before, c->d_status, sizeof before, cudaMemcpyDeviceToHost);
+        for (int b = 0; b < STATUS_BITS; b++) before_host[b] = c->h_status[b];
         GatherPeers peers;
         for (int r = 0; r < WF_MAX_GATHER_RANKS; r++) peers.land[r] = k->land[r];
         gather_wait_done_kernel<<<1, 32, 0, c->stream>>>(peers, k->d_epoch, c->d_status, k->world, k->rank, k->wait_ns);
         cudaDeviceSynchronize();
         cudaMemcpy(c->d_status, &before, sizeof before, cudaMemcpyHostToDevice);
+        for (int b = 0; b < STATUS_BITS; b++) c->h_status[b] = before_host[b];
     }
     release_peer_landing(k);
     nccl().CommDestroy(k->comm);

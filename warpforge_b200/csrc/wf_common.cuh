@@ -17,11 +17,29 @@ constexpr uint32_t CTX_MAGIC = 0x57464358;     // "WFCX"
 constexpr uint32_t WEIGHT_MAGIC = 0x57465754;  // "WFWT"
 constexpr uint32_t COMM_MAGIC = 0x5746434D;    // "WFCM"
 
-// Device-side status bits, OR-ed into Context::d_status by kernels that give up a wait.
+// Device-side status bits, reported through Context::d_status by kernels that give up a wait (report_status).
 constexpr int STATUS_GEMV_FIXUP_TIMEOUT = 1;
 constexpr int STATUS_GEMM_PIPE_TIMEOUT = 2;
 constexpr int STATUS_PEER_WAIT_TIMEOUT = 4;
 constexpr int STATUS_BAD_INDEX = 8;  // an embedding index outside the table
+
+// The status block: `bits` collects what kernels report (and is what running kernels look at); `host` is the device
+// address of one int per bit in pinned host memory, set with it, so that the host learns the outcome of a stream it
+// has waited for from its own memory.  Copying the bits back instead cost every synchronising call about 10 us.
+struct StatusBlock {
+    int bits;
+    int pad;
+    int* host;
+};
+constexpr int STATUS_BITS = 4;
+#ifdef __CUDACC__
+__device__ __forceinline__ void report_status(int* status, int bit) {
+    StatusBlock* b = reinterpret_cast<StatusBlock*>(status);
+    atomicOr(&b->bits, bit);
+    *reinterpret_cast<volatile int*>(b->host + (31 - __clz(bit))) = 1;
+    __threadfence_system();
+}
+#endif
 
 struct Context;
 
@@ -57,7 +75,8 @@ struct Context {
     int sm_count = 0;
     int cc_major = 0, cc_minor = 0;
     cudaStream_t stream = nullptr;  // the context's own compute stream
-    int* d_status = nullptr;
+    int* d_status = nullptr;            // StatusBlock in device memory
+    volatile int* h_status = nullptr;   // its host words, pinned
     int salt = 0;                            // instrumentation level, 2 = kernel timing stamps
     unsigned long long* d_timing = nullptr;  // [sm_count][8]
     std::mutex mu;  // guards against concurrent use (try_lock -> WF_ERR_BUSY)
@@ -73,6 +92,7 @@ struct Context {
     std::unordered_map<cudaStream_t, GemvScratch> gemv_scratch;
     // pinned staging for host-pointer calls
     void* h_stage = nullptr;
+    void* h_stage_dev = nullptr;  // its address on the device
     int64_t h_stage_bytes = 0;
     void* d_stage = nullptr;
     int64_t d_stage_bytes = 0;
@@ -91,7 +111,7 @@ struct Context {
 
 int set_error(Context* c, int status, const char* fmt, ...);
 int cuda_status(Context* c, cudaError_t e, const char* what);
-// Reads and clears the device status word after the stream has been waited for: WF_OK, or the failure a
+// Reads and clears the status after the stream has been waited for: WF_OK, or the failure a
 // kernel recorded there (a bounded wait that ran out, an index outside a table).
 int read_device_status(Context* c);
 // WF_OK, or WF_ERR_RECORDING when `s` is being recorded into a graph: the caller is about to allocate (or

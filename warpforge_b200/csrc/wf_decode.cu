@@ -141,7 +141,7 @@ struct ProgRun {
                     __nanosleep(20);
                 } while (++spins < GEMV_FIXUP_SPINS && !*failed);
                 if (v.y != want_tag) {
-                    atomicOr(P.status, STATUS_PEER_WAIT_TIMEOUT);
+                    report_status(P.status, STATUS_PEER_WAIT_TIMEOUT);
                     *failed = 1;
                     return;
                 }
@@ -173,7 +173,7 @@ struct ProgRun {
             if (!*failed) {
                 while (ld_acquire_gpu(&P.sync->arrive) < want && ++spins < PROG_BARRIER_SPINS) __nanosleep(50);
                 if (spins >= PROG_BARRIER_SPINS) {
-                    atomicOr(P.status, STATUS_PEER_WAIT_TIMEOUT);
+                    report_status(P.status, STATUS_PEER_WAIT_TIMEOUT);
                     *failed = 1;
                 }
             }
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_program_kernel(const Pro
         stamp();
     }
     if (failed) {
-        if (lane == 0) atomicOr(P.status, STATUS_GEMV_FIXUP_TIMEOUT);
+        if (lane == 0) report_status(P.status, STATUS_GEMV_FIXUP_TIMEOUT);
         *run.failed = 1;
         drain_after_abort();
     }
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_program_kernel(const 
         stamp();
     }
     if (failed) {
-        if (lane == 0) atomicOr(P.status, STATUS_GEMV_FIXUP_TIMEOUT);
+        if (lane == 0) report_status(P.status, STATUS_GEMV_FIXUP_TIMEOUT);
         *run.failed = 1;
     }
     run.leave();

@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_kernel(const GemmParams 
     const uint32_t tmem_base = *tmem_slot;
 
     auto fail = [&]() {
-        atomicOr(p.status, STATUS_GEMM_PIPE_TIMEOUT);
+        report_status(p.status, STATUS_GEMM_PIPE_TIMEOUT);
         *abort_flag = 1;
     };
 

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvPara
                    emit_row);
     stamp(4);
     if (*abort_flag) {  // a wait ran out somewhere in this CTA
-        if (lane == 0) atomicOr(p.status, STATUS_GEMV_FIXUP_TIMEOUT);
+        if (lane == 0) report_status(p.status, STATUS_GEMV_FIXUP_TIMEOUT);
     }
     stamp(5);
 }

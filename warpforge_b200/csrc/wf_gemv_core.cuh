@@ -930,7 +930,7 @@ __device__ __forceinline__ void publish_piece(uint2* slot, const float (&v)[(ELE
         if (i >= ELEMS) continue;
         int spins = 0;  // the slot's previous content must have been taken before it is overwritten
         while (ld_slot(slot + i).y != 0u && ++spins < GEMV_FIXUP_SPINS) __nanosleep(32);
-        if (spins >= GEMV_FIXUP_SPINS) atomicOr(status, STATUS_GEMV_FIXUP_TIMEOUT);
+        if (spins >= GEMV_FIXUP_SPINS) report_status(status, STATUS_GEMV_FIXUP_TIMEOUT);
         st_slot(slot + i, make_uint2(__float_as_uint(v[u]), 1u));
     }
 }
@@ -961,7 +961,7 @@ __device__ __forceinline__ void collect_pieces(uint2* slots, float (&v)[(ELEMS +
                 e[u] = ld_slot(sp);
             }
             if (e[u].y == 0u) {
-                atomicOr(status, STATUS_GEMV_FIXUP_TIMEOUT);
+                report_status(status, STATUS_GEMV_FIXUP_TIMEOUT);
                 gave_up = true;
             } else {
                 v[u] += __uint_as_float(e[u].x);

@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNPar
     __syncthreads();
     stamp(1);
     if (*reinterpret_cast<volatile int*>(smem + 8)) {  // the copies did not land in time: y would be garbage
-        if (threadIdx.x == 0) atomicOr(p.status, STATUS_GEMV_FIXUP_TIMEOUT);
+        if (threadIdx.x == 0) report_status(p.status, STATUS_GEMV_FIXUP_TIMEOUT);
         drain_after_abort();
         return;
     }

@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(256) embedding_kernel(const int64_t* __restric
     for (int64_t r = blockIdx.x; r < count; r += gridDim.x) {
         const int64_t idx = (int64_t)(int)indices[r];  // `(int) indexData.getAtIndex(JAVA_LONG, i)`
         const bool ok = idx >= 0 && idx < vocab;
-        if (!ok && threadIdx.x == 0) atomicOr(status, STATUS_BAD_INDEX);
+        if (!ok && threadIdx.x == 0) report_status(status, STATUS_BAD_INDEX);
         const float* src = table + (size_t)(ok ? idx : 0) * dim;
         float* dst = y + (size_t)r * dim;
         if (vec) {

@@ -58,7 +58,8 @@ int ensure_stage(Context* c, int64_t host_bytes, int64_t dev_bytes) {
         if (c->h_stage) cudaFreeHost(c->h_stage);
         c->h_stage = nullptr;
         c->h_stage_bytes = 0;
-        WF_CUDA(c, cudaMallocHost(&c->h_stage, (size_t)host_bytes));
+        WF_CUDA(c, cudaHostAlloc(&c->h_stage, (size_t)host_bytes, cudaHostAllocMapped));
+        WF_CUDA(c, cudaHostGetDevicePointer(&c->h_stage_dev, c->h_stage, 0));
         c->h_stage_bytes = host_bytes;
     }
     if (dev_bytes > c->d_stage_bytes) {
@@ -69,6 +70,30 @@ int ensure_stage(Context* c, int64_t host_bytes, int64_t dev_bytes) {
         c->d_stage_bytes = dev_bytes;
     }
     return WF_OK;
+}
+
+// Host operands of one call up to this size skip the copy engine: a kernel reads the activations out of the pinned
+// staging buffer, and the projection's own kernel writes its rows into it.  A copy-engine transfer costs about 5 us of
+// hand-overs between the engines on either side whatever its size; stores over the link cost 24 bytes of header per
+// 32 bytes of rows, so beyond this size the engine is the better carrier again.  One fp32 token through a Q8_0
+// [4096 x 4096] weight, Backend.execute: 49.9 us with copies and a status copy, 28.6 us without.
+constexpr int64_t HOST_DIRECT_BYTES = 128 << 10;
+
+__global__ void __launch_bounds__(256) fetch_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, int n) {
+    // nothing on the stream touches the staging buffers here (every call that used them was waited for), so the
+    // projection behind may be placed at once and request its weights under this kernel
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < n) {
+        uint4 v;
+        asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src + i));
+        dst[i] = v;
+    }
+}
+static cudaError_t fetch_from_host(void* d_dst, const void* h_src_dev, int64_t bytes, cudaStream_t s) {
+    const int n = (int)((bytes + 15) / 16);  // the staging buffers are 256-byte granular
+    fetch_kernel<<<(n + 255) / 256, 256, 0, s>>>(static_cast<const uint4*>(h_src_dev), static_cast<uint4*>(d_dst), n);
+    return cudaGetLastError();
 }
 
 // Host blocks (pageable memory, e.g. a mapped file) -> tiled device layout as a three-stage pipeline over
@@ -195,13 +220,19 @@ int wf_init(int device, int64_t* ctx) {
     c->cc_minor = prop.minor;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&c->d_status, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(c->d_status, 0, sizeof(int));
+    StatusBlock block{0, 0, nullptr};
+    if (e == cudaSuccess) e = cudaHostAlloc((void**)&c->h_status, STATUS_BITS * sizeof(int), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&block.host, (void*)c->h_status, 0);
+    if (e == cudaSuccess) e = cudaMalloc(&c->d_status, sizeof block);
+    if (e == cudaSuccess) e = cudaMemcpy(c->d_status, &block, sizeof block, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         if (c->stream) cudaStreamDestroy(c->stream);
+        if (c->h_status) cudaFreeHost((void*)c->h_status);
+        if (c->d_status) cudaFree(c->d_status);
         delete c;
         return WF_ERR_CUDA_BASE + (int)e;
     }
+    for (int b = 0; b < STATUS_BITS; b++) c->h_status[b] = 0;
     {
         std::lock_guard<std::mutex> lk(g_registry_mu);
         g_contexts.insert(c);
@@ -245,6 +276,7 @@ int wf_destroy(int64_t ctx) {
     if (c->d_gemm_partial) cudaFree(c->d_gemm_partial);
     if (c->d_gemm_ready) cudaFree(c->d_gemm_ready);
     cudaFree(c->d_status);
+    cudaFreeHost((void*)c->h_status);
     if (c->d_timing) cudaFree(c->d_timing);
     cudaStreamDestroy(c->stream);
     c->magic = 0;
@@ -298,9 +330,11 @@ int wf_stream_destroy(int64_t ctx, int64_t stream) {
 namespace wf {
 int read_device_status(Context* c) {
     int st = 0;
-    WF_CUDA(c, cudaMemcpy(&st, c->d_status, sizeof st, cudaMemcpyDeviceToHost));
+    for (int b = 0; b < STATUS_BITS; b++)
+        if (c->h_status[b] != 0) st |= 1 << b;
     if (st != 0) {
-        WF_CUDA(c, cudaMemset(c->d_status, 0, sizeof st));
+        for (int b = 0; b < STATUS_BITS; b++) c->h_status[b] = 0;
+        WF_CUDA(c, cudaMemset(c->d_status, 0, sizeof(int)));
         if (st == STATUS_BAD_INDEX) return set_error(c, WF_ERR_INDEX, "an embedding index was outside the table (its row was written as zeros)");
         return set_error(c, WF_ERR_DEVICE_WAIT, "a device-side bounded wait expired (status bits 0x%x)", st);
     }
@@ -510,26 +544,26 @@ int wf_qlinear(int64_t ctx, int64_t weight, const void* x, int x_dtype, int x_on
     const int64_t xb = m * w->g.k * (x_dtype == WF_DTYPE_F32 ? 4 : 2), yb = m * w->g.rows * 4;
     const void* d_x = x;
     float* d_y = static_cast<float*>(y);
+    const int64_t yo = (xb + 255) & ~255LL;  // x and y in the staging buffers
+    const bool y_direct = !y_on_device && yb <= HOST_DIRECT_BYTES;
     if (!x_on_device || !y_on_device) {
         // host operands: pinned staging, copies on the same stream, result waited for
-        const int64_t xo = 0, yo = (xb + 255) & ~255LL;
         int rc = ensure_stage(c, yo + yb, yo + yb);
         if (rc != WF_OK) return rc;
         if (!x_on_device) {
-            memcpy(static_cast<uint8_t*>(c->h_stage) + xo, x, (size_t)xb);
-            WF_CUDA(c, cudaMemcpyAsync(static_cast<uint8_t*>(c->d_stage) + xo, static_cast<uint8_t*>(c->h_stage) + xo,
-                                       (size_t)xb, cudaMemcpyHostToDevice, s));
-            d_x = static_cast<uint8_t*>(c->d_stage) + xo;
+            memcpy(c->h_stage, x, (size_t)xb);
+            if (xb <= HOST_DIRECT_BYTES) WF_CUDA(c, fetch_from_host(c->d_stage, c->h_stage_dev, xb, s));
+            else WF_CUDA(c, cudaMemcpyAsync(c->d_stage, c->h_stage, (size_t)xb, cudaMemcpyHostToDevice, s));
+            d_x = c->d_stage;
         }
-        if (!y_on_device) d_y = reinterpret_cast<float*>(static_cast<uint8_t*>(c->d_stage) + yo);
+        if (!y_on_device) d_y = reinterpret_cast<float*>(static_cast<uint8_t*>(y_direct ? c->h_stage_dev : c->d_stage) + yo);
     }
     GemvCall call{w, d_x, x_dtype, m, d_y, w->g.rows, 0};
     // many tokens: tensor-core GEMM; a few tokens: the HBM-bound GEMV
     int rc = gemm_supported(*w, x_dtype, m, call.d_x) ? gemm_launch(c, call, s) : gemv_launch(c, call, s);
     if (rc != WF_OK) return rc;
     if (!y_on_device) {
-        const int64_t yo = (xb + 255) & ~255LL;
-        WF_CUDA(c, cudaMemcpyAsync(static_cast<uint8_t*>(c->h_stage) + yo, d_y, (size_t)yb, cudaMemcpyDeviceToHost, s));
+        if (!y_direct) WF_CUDA(c, cudaMemcpyAsync(static_cast<uint8_t*>(c->h_stage) + yo, d_y, (size_t)yb, cudaMemcpyDeviceToHost, s));
         WF_CUDA(c, cudaStreamSynchronize(s));
         memcpy(y, static_cast<uint8_t*>(c->h_stage) + yo, (size_t)yb);
         return read_device_status(c);  // the result is in the caller's hands: a wait that ran out must not pass as success

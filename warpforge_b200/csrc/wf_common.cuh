@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <map>
 #include <mutex>
 #include <string>
 #include <unordered_map>
@@ -41,6 +42,8 @@ __device__ __forceinline__ void report_status(int* status, int bit) {
 }
 #endif
 
+constexpr int UPLOAD_RING = 6;  // pinned chunks
+
 struct Context;
 
 struct Weight {
@@ -51,6 +54,7 @@ struct Weight {
     int64_t row0 = 0;        // first global row of this shard
     int64_t total_rows = 0;  // rows of the unsharded tensor
     uint8_t* d_tiles = nullptr;
+    int64_t tiles_held = 0;  // bytes allocated at d_tiles (a reused buffer may be larger than g.bytes())
     int programs = 0;        // live programs whose op lists point at d_tiles
     // how the several-token decode kernel cuts this weight, per activation dtype (bf16 / fp32) and column count:
     // {slices, k-tiles per slice, team size, uses partial sums}, slices = -1 until first asked for (0: no cut fits)
@@ -89,6 +93,8 @@ struct Context {
     std::unordered_map<int64_t, int64_t> allocs;  // device ptr -> bytes
     std::vector<void*> host_allocs;
     std::vector<Weight*> weights;
+    std::multimap<int64_t, uint8_t*> spare_tiles;  // tile buffers of freed weights by size, at most SPARE_TILES_BYTES in all
+    int64_t spare_tiles_bytes = 0;
     std::unordered_map<cudaStream_t, GemvScratch> gemv_scratch;
     // pinned staging for host-pointer calls
     void* h_stage = nullptr;
@@ -96,10 +102,11 @@ struct Context {
     int64_t h_stage_bytes = 0;
     void* d_stage = nullptr;
     int64_t d_stage_bytes = 0;
-    void* h_upload = nullptr;  // two pinned chunks the weight upload streams a host tensor through
+    void* h_upload = nullptr;  // ring of pinned chunks the weight upload streams a host tensor through
     void* d_upload = nullptr;  // their landing place on the device, read by the repack kernel
     int64_t upload_chunk_bytes = 0;
-    cudaEvent_t upload_done[2] = {nullptr, nullptr};
+    cudaStream_t upload_stream = nullptr;
+    cudaEvent_t upload_done[UPLOAD_RING] = {}, upload_repacked[UPLOAD_RING] = {};  // chunk transferred / its tiles written
     void* d_x16 = nullptr;  // fp16 copy of the activations for the tensor-core GEMM
     int64_t x16_bytes = 0;
     float* d_gemm_partial = nullptr;       // [sm_count][512][128] pieces of tiles cut by a share boundary
@@ -121,6 +128,8 @@ int refuse_allocation_while_recording(Context* c, cudaStream_t s, const char* wh
 Context* get_context(int64_t h);
 Weight* get_weight(Context* c, int64_t h);
 cudaStream_t resolve_stream(Context* c, int64_t stream);
+cudaError_t take_tiles(Context* c, int64_t bytes, uint8_t** tiles, int64_t* held);
+void release_spare_tiles(Context* c);
 int ensure_stage(Context* c, int64_t host_bytes, int64_t dev_bytes);
 // validated shard upload + repack shared by wf_weight_upload and wf_gguf_upload; takes the context lock
 int weight_upload(Context* c, int qtype, const void* blocks, int64_t n_rows, int64_t k, int shard_rank, int shard_world,

@@ -12,6 +12,10 @@
 #include <thread>
 #include <unordered_set>
 
+#if defined(__x86_64__)
+#include <emmintrin.h>
+#endif
+
 #include "wf_common.cuh"
 
 namespace wf {
@@ -96,16 +100,80 @@ static cudaError_t fetch_from_host(void* d_dst, const void* h_src_dev, int64_t b
     return cudaGetLastError();
 }
 
+// Tile buffers of freed weights are kept for the next upload of about the same size: cudaMalloc and cudaFree of a
+// large buffer take 0.3 ms each, as much as 18 MB of blocks on the link, and far more when other processes of the
+// machine use the driver.  Bounded, emptied when an allocation of the context fails and when it is destroyed.
+// A buffer enters the pool after the device has been synchronised (wf_weight_free), so it is idle for every stream.
+constexpr int64_t SPARE_TILES_BYTES = 256 << 20;
+
+cudaError_t take_tiles(Context* c, int64_t bytes, uint8_t** tiles, int64_t* held) {
+    auto it = c->spare_tiles.lower_bound(bytes);
+    if (it != c->spare_tiles.end() && it->first <= bytes + bytes / 8 + (1 << 16)) {
+        *held = it->first;
+        *tiles = it->second;
+        c->spare_tiles_bytes -= it->first;
+        c->spare_tiles.erase(it);
+        return cudaSuccess;
+    }
+    *held = bytes;
+    cudaError_t e = cudaMalloc(tiles, (size_t)bytes);
+    if (e == cudaErrorMemoryAllocation && !c->spare_tiles.empty()) {
+        cudaGetLastError();
+        release_spare_tiles(c);
+        e = cudaMalloc(tiles, (size_t)bytes);
+    }
+    return e;
+}
+
+void release_spare_tiles(Context* c) {
+    for (auto& kv : c->spare_tiles) cudaFree(kv.second);
+    c->spare_tiles.clear();
+    c->spare_tiles_bytes = 0;
+}
+
+static void give_back_tiles(Context* c, uint8_t* tiles, int64_t held) {
+    if (held + c->spare_tiles_bytes > SPARE_TILES_BYTES) {
+        cudaFree(tiles);
+        return;
+    }
+    c->spare_tiles.emplace(held, tiles);
+    c->spare_tiles_bytes += held;
+}
+
 // Host blocks (pageable memory, e.g. a mapped file) -> tiled device layout as a three-stage pipeline over
-// chunks of whole 16-row tiles: helper threads copy chunk i+1 into one of two pinned buffers while the DMA
+// chunks of whole 16-row tiles: helper threads copy later chunks into a ring of pinned buffers while the DMA
 // of chunk i runs and the repack kernel of chunk i-1 writes its tiles.  A plain cudaMemcpyAsync from
 // pageable memory stages through one driver thread and runs several times slower; the scratch on the
-// device is two chunks, not a second copy of the tensor.
-constexpr int64_t UPLOAD_CHUNK = 8 << 20;
-constexpr int UPLOAD_THREADS = 4;
+// device is the ring, not a second copy of the tensor.
+// The link (55 GB/s) bounds it: the chunk at hand is cut into small pieces that all helpers take in turn, and the
+// chunks are short, so that the link starts early and the last transfer and repack are short as well.  A core copies
+// 12 GB/s around the caches; more helpers than it takes to feed the link only cost their start (66 MB of Q4_0: 2.8 ms
+// with two, 1.43 ms with four, 1.64 ms with twelve; 3.2 ms with 8 MB chunks, four helpers copying through the caches,
+// transfers and repacks on one stream and a cudaMalloc / cudaFree per tensor).
+constexpr int64_t UPLOAD_CHUNK = 2 << 20, UPLOAD_PIECE = 128 << 10;
+constexpr int UPLOAD_MAX_THREADS = 4;
+
+// Copy into pinned memory that the link reads next and the host never does: stores around the caches where the
+// instruction set has them.  Lines left modified in the caches of several cores have to be fetched from there by the
+// transfer: the more helpers, the slower it ran (9.4 MB: 0.55 ms with two, 1.3 ms with twelve).
+static void copy_to_pinned(uint8_t* dst, const uint8_t* src, size_t n) {
+#if defined(__x86_64__)
+    for (; n >= 64; n -= 64, src += 64, dst += 64) {  // dst is 64-byte aligned: pieces start at multiples of 128 KB
+        const __m128i a = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src)), b = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src) + 1);
+        const __m128i e = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src) + 2), f = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src) + 3);
+        _mm_stream_si128(reinterpret_cast<__m128i*>(dst), a);
+        _mm_stream_si128(reinterpret_cast<__m128i*>(dst) + 1, b);
+        _mm_stream_si128(reinterpret_cast<__m128i*>(dst) + 2, e);
+        _mm_stream_si128(reinterpret_cast<__m128i*>(dst) + 3, f);
+    }
+    _mm_sfence();
+#endif
+    memcpy(dst, src, n);
+}
 
 static cudaError_t upload_and_repack(Context* c, int qtype, const uint8_t* src, int64_t rows, int64_t k, int64_t row_bytes,
-                                     uint8_t* d_tiles, int64_t tile_row_bytes, int q4_0_order, cudaStream_t s) {
+                                     uint8_t** d_tiles, int64_t* held, int64_t tiles_bytes, int64_t tile_row_bytes, int q4_0_order,
+                                     cudaStream_t s) {
     const int64_t chunk_rows = std::max<int64_t>(TILE_ROWS, UPLOAD_CHUNK / row_bytes / TILE_ROWS * TILE_ROWS);
     const int64_t chunk_bytes = (chunk_rows * row_bytes + 255) & ~255LL;
     const int nchunks = (int)((rows + chunk_rows - 1) / chunk_rows);
@@ -115,51 +183,73 @@ static cudaError_t upload_and_repack(Context* c, int qtype, const uint8_t* src, 
         if (c->d_upload) cudaFree(c->d_upload);
         c->h_upload = c->d_upload = nullptr;
         c->upload_chunk_bytes = 0;
-        e = cudaMallocHost(&c->h_upload, (size_t)(2 * chunk_bytes));
-        if (e == cudaSuccess) e = cudaMalloc(&c->d_upload, (size_t)(2 * chunk_bytes));
+        e = cudaMallocHost(&c->h_upload, (size_t)(UPLOAD_RING * chunk_bytes));
+        if (e == cudaSuccess) e = cudaMalloc(&c->d_upload, (size_t)(UPLOAD_RING * chunk_bytes));
         if (e != cudaSuccess) return e;
         c->upload_chunk_bytes = chunk_bytes;
     }
-    for (int i = 0; i < 2; i++)
+    if (!c->upload_stream && (e = cudaStreamCreateWithFlags(&c->upload_stream, cudaStreamNonBlocking)) != cudaSuccess) return e;
+    for (int i = 0; i < UPLOAD_RING; i++) {
         if (!c->upload_done[i] && (e = cudaEventCreateWithFlags(&c->upload_done[i], cudaEventDisableTiming)) != cudaSuccess) return e;
+        if (!c->upload_repacked[i] && (e = cudaEventCreateWithFlags(&c->upload_repacked[i], cudaEventDisableTiming)) != cudaSuccess) return e;
+    }
     uint8_t* const pinned = static_cast<uint8_t*>(c->h_upload);
     auto chunk_size = [&](int i) { return std::min(chunk_rows, rows - i * chunk_rows) * row_bytes; };
 
-    // released: chunks [0, released) may be written into their pinned buffer; filled[i]: helpers done with chunk i
-    const int helpers_n = rows * row_bytes > (1 << 20) ? UPLOAD_THREADS : 0;
-    std::atomic<int> released{2};
+    // Pieces are taken in order from one counter; released: chunks [0, released) may be written into their pinned
+    // buffer; left[i]: pieces of chunk i not copied yet.
+    const int pieces = (int)((chunk_bytes + UPLOAD_PIECE - 1) / UPLOAD_PIECE);
+    std::atomic<int> released{UPLOAD_RING};
+    std::atomic<int64_t> next{0};
     std::atomic<bool> stop{false};
-    std::vector<std::atomic<int>> filled((size_t)nchunks);
-    for (auto& f : filled) f.store(0);
+    std::vector<std::atomic<int>> left((size_t)nchunks);
+    for (auto& f : left) f.store(pieces);
+    auto copy_pieces = [&]() {
+        for (;;) {
+            const int64_t item = next.fetch_add(1, std::memory_order_relaxed);
+            const int i = (int)(item / pieces);
+            if (i >= nchunks) return;
+            while (released.load(std::memory_order_acquire) <= i && !stop.load(std::memory_order_relaxed)) std::this_thread::yield();
+            if (stop.load(std::memory_order_relaxed)) return;
+            const int64_t n = chunk_size(i), lo = std::min(n, item % pieces * UPLOAD_PIECE), hi = std::min(n, lo + UPLOAD_PIECE);
+            if (hi > lo) copy_to_pinned(pinned + (i % UPLOAD_RING) * chunk_bytes + lo, src + i * chunk_rows * row_bytes + lo, (size_t)(hi - lo));
+            left[(size_t)i].fetch_sub(1, std::memory_order_release);
+        }
+    };
+    // one helper per half megabyte at most: starting a thread costs about what copying that much does
+    const int helpers_n = (int)std::min<int64_t>(rows * row_bytes >> 19, UPLOAD_MAX_THREADS);
     std::vector<std::thread> helpers;
-    for (int t = 0; t < helpers_n; t++)
-        helpers.emplace_back([&, t] {
-            for (int i = 0; i < nchunks; i++) {
-                while (released.load(std::memory_order_acquire) <= i && !stop.load()) std::this_thread::yield();
-                if (stop.load()) return;
-                const int64_t n = chunk_size(i), part = (n / helpers_n + 4095) & ~4095LL;
-                const int64_t lo = std::min(n, t * part), hi = std::min(n, (t + 1) * part);
-                if (hi > lo) memcpy(pinned + (i & 1) * chunk_bytes + lo, src + i * chunk_rows * row_bytes + lo, (size_t)(hi - lo));
-                filled[(size_t)i].fetch_add(1, std::memory_order_release);
+    for (int t = 0; t < helpers_n; t++) helpers.emplace_back(copy_pieces);
+    if (helpers_n == 0) copy_pieces();  // less than half a megabyte is one chunk
+
+    // the tiles are allocated while the helpers fill the ring
+    e = take_tiles(c, tiles_bytes, d_tiles, held);
+    if (e == cudaSuccess) e = cudaMemsetAsync(*d_tiles, 0, (size_t)tiles_bytes, s);
+    int sent = 0;  // chunks whose DMA has left their pinned buffer
+    auto give_back = [&](int upto) {  // release the buffers of chunks below `upto` that have been sent
+        while (sent < upto) {
+            if (cudaEventQuery(c->upload_done[sent % UPLOAD_RING]) != cudaSuccess) {
+                cudaGetLastError();  // "not ready" is no error
+                return;
             }
-        });
+            released.store(++sent + UPLOAD_RING, std::memory_order_release);
+        }
+    };
     for (int i = 0; i < nchunks && e == cudaSuccess; i++) {
         const int64_t n = chunk_size(i), r0 = i * chunk_rows;
-        uint8_t* h = pinned + (i & 1) * chunk_bytes;
-        uint8_t* d = static_cast<uint8_t*>(c->d_upload) + (i & 1) * chunk_bytes;
-        if (helpers_n == 0) {
-            if (i >= 2) e = cudaEventSynchronize(c->upload_done[i & 1]);
-            memcpy(h, src + r0 * row_bytes, (size_t)n);
-        } else {
-            while (filled[(size_t)i].load(std::memory_order_acquire) < helpers_n) std::this_thread::yield();
+        uint8_t* h = pinned + (i % UPLOAD_RING) * chunk_bytes;
+        uint8_t* d = static_cast<uint8_t*>(c->d_upload) + (i % UPLOAD_RING) * chunk_bytes;
+        while (left[(size_t)i].load(std::memory_order_acquire) > 0) {
+            give_back(i);
+            std::this_thread::yield();
         }
-        if (e == cudaSuccess) e = cudaMemcpyAsync(d, h, (size_t)n, cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = cudaEventRecord(c->upload_done[i & 1], s);
-        if (e == cudaSuccess) e = launch_repack(qtype, d, d_tiles + r0 / TILE_ROWS * tile_row_bytes, n / row_bytes, k, q4_0_order, s);
-        if (helpers_n && i >= 1 && e == cudaSuccess) {  // the DMA of chunk i-1 has left its pinned buffer: chunk i+1 may fill it
-            e = cudaEventSynchronize(c->upload_done[(i - 1) & 1]);
-            released.store(i + 2, std::memory_order_release);
-        }
+        // transfers on a stream of their own, so that the link does not wait for the repack kernels
+        if (i >= UPLOAD_RING) e = cudaStreamWaitEvent(c->upload_stream, c->upload_repacked[i % UPLOAD_RING], 0);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(d, h, (size_t)n, cudaMemcpyHostToDevice, c->upload_stream);
+        if (e == cudaSuccess) e = cudaEventRecord(c->upload_done[i % UPLOAD_RING], c->upload_stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, c->upload_done[i % UPLOAD_RING], 0);
+        if (e == cudaSuccess) e = launch_repack(qtype, d, *d_tiles + r0 / TILE_ROWS * tile_row_bytes, n / row_bytes, k, q4_0_order, s);
+        if (e == cudaSuccess) e = cudaEventRecord(c->upload_repacked[i % UPLOAD_RING], s);
     }
     stop.store(e != cudaSuccess);
     for (std::thread& h : helpers) h.join();
@@ -256,6 +346,7 @@ int wf_destroy(int64_t ctx) {
         w->magic = 0;
         delete w;
     }
+    release_spare_tiles(c);
     for (auto& kv : c->allocs) cudaFree(reinterpret_cast<void*>(kv.first));
     for (void* h : c->host_allocs) cudaFreeHost(h);
     for (auto& kv : c->gemv_scratch) {
@@ -271,6 +362,9 @@ int wf_destroy(int64_t ctx) {
     if (c->d_upload) cudaFree(c->d_upload);
     for (cudaEvent_t e : c->upload_done)
         if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : c->upload_repacked)
+        if (e) cudaEventDestroy(e);
+    if (c->upload_stream) cudaStreamDestroy(c->upload_stream);
     if (c->d_stage) cudaFree(c->d_stage);
     if (c->d_x16) cudaFree(c->d_x16);
     if (c->d_gemm_partial) cudaFree(c->d_gemm_partial);
@@ -365,7 +459,13 @@ int wf_malloc(int64_t ctx, int64_t bytes, int64_t* dptr) {
     WF_ENTER(ctx);
     if (!dptr || bytes < 0) return WF_ERR_INVALID_ARGUMENT;
     void* p = nullptr;
-    WF_CUDA(c, cudaMalloc(&p, (size_t)std::max<int64_t>(bytes, 1)));
+    cudaError_t e = cudaMalloc(&p, (size_t)std::max<int64_t>(bytes, 1));
+    if (e == cudaErrorMemoryAllocation && !c->spare_tiles.empty()) {
+        cudaGetLastError();
+        release_spare_tiles(c);
+        e = cudaMalloc(&p, (size_t)std::max<int64_t>(bytes, 1));
+    }
+    if (e != cudaSuccess) return cuda_status(c, e, "cudaMalloc");
     c->allocs[reinterpret_cast<int64_t>(p)] = bytes;
     *dptr = reinterpret_cast<int64_t>(p);
     return WF_OK;
@@ -457,11 +557,8 @@ int weight_upload(Context* c, int qtype, const void* blocks, int64_t n_rows, int
     w->g.rt_alloc = (w->g.rt + 7) / 8 * 8;
     w->row0 = row0;
     w->total_rows = n_rows;
-    cudaError_t e = cudaMalloc(&w->d_tiles, (size_t)w->g.bytes());
-    if (e == cudaSuccess) e = cudaMemsetAsync(w->d_tiles, 0, (size_t)w->g.bytes(), c->stream);
-    if (e == cudaSuccess)
-        e = upload_and_repack(c, qtype, static_cast<const uint8_t*>(blocks) + row0 * row_bytes, rows, k, row_bytes, w->d_tiles,
-                              w->g.kt * (int64_t)tile_bytes(w->g.qtype), q4_0_order, c->stream);
+    cudaError_t e = upload_and_repack(c, qtype, static_cast<const uint8_t*>(blocks) + row0 * row_bytes, rows, k, row_bytes, &w->d_tiles,
+                                      &w->tiles_held, w->g.bytes(), w->g.kt * (int64_t)tile_bytes(w->g.qtype), q4_0_order, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         if (w->d_tiles) cudaFree(w->d_tiles);
@@ -484,8 +581,8 @@ int wf_weight_free(int64_t ctx, int64_t weight) {
     if (w->programs > 0)
         return set_error(c, WF_ERR_IN_USE, "weight is referenced by %d live program(s): destroy them first", w->programs);
     c->weights.erase(std::find(c->weights.begin(), c->weights.end(), w));
-    WF_CUDA(c, cudaStreamSynchronize(c->stream));
-    cudaFree(w->d_tiles);
+    WF_CUDA(c, cudaDeviceSynchronize());  // kernels of any stream may still read the tiles
+    give_back_tiles(c, w->d_tiles, w->tiles_held);
     w->magic = 0;
     delete w;
     return WF_OK;

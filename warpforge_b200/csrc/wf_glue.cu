@@ -12,37 +12,47 @@
 // double, so results agree to rounding of the reduction (about 1e-7 relative), not bit for bit.
 //
 // All of them are HBM-bound: one read and one write of the tensor.  Row operations keep the row in
-// registers between the reduction and the normalisation (one CTA per row, up to 8192 columns; longer
-// rows are read again from L2), element operations move 16 bytes per thread per step.
+// registers between the reduction and the normalisation (up to 16384 columns; longer
+// rows are read again from L2), element operations move 16 bytes per thread and load.
+#include <algorithm>
+#include <type_traits>
+
 #include "wf_common.cuh"
 
 namespace wf {
 
-constexpr int ROW_THREADS = 256;
-constexpr int ROW_VEC = 8;  // float4 per thread held in registers: rows up to 256 * 8 * 4 = 8192 columns
+// A row operation gives each row to a group of T threads that hold it in registers, 16 floats each: a warp for rows
+// up to 512 columns (eight rows per CTA, no barrier anywhere), a CTA of 64 - 1024 threads beyond (rows up to 16384).
+// Bound by HBM as long as enough rows are in flight per SM to cover one row's chain of load, reductions and store, so
+// the group fits the row: 256 threads with room for 32 floats each left three quarters of their registers idle on a
+// row of 2048, and 64 floats per lane of a warp per row takes so many registers that softmax had 8 warps per SM.
+constexpr int ROW_CTA = 256;  // threads of a CTA whose warps take a row each
 
-// `red` is private to one reduction (each call site passes its own array), so one barrier is enough
-__device__ __forceinline__ double block_sum(double v, double* red) {
+// Sum over the group's T threads, in double; every thread gets it.  `red` (T / 32 doubles, unused for a warp) is private
+// to one reduction, so one barrier is enough.
+template <int T> __device__ __forceinline__ double group_sum(double v, double* red) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    if (T == 32) return v;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) red[warp] = v;
     __syncthreads();
     double t = 0.0;
 #pragma unroll
-    for (int w = 0; w < ROW_THREADS / 32; w++) t += red[w];
+    for (int w = 0; w < T / 32; w++) t += red[w];
     return t;
 }
 
-__device__ __forceinline__ float block_max(float v, float* red) {
+template <int T> __device__ __forceinline__ float group_max(float v, float* red) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+    if (T == 32) return v;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) red[warp] = v;
     __syncthreads();
     float t = red[0];
 #pragma unroll
-    for (int w = 1; w < ROW_THREADS / 32; w++) t = fmaxf(t, red[w]);
+    for (int w = 1; w < T / 32; w++) t = fmaxf(t, red[w]);
     return t;
 }
 
@@ -104,126 +114,195 @@ __device__ __forceinline__ float exp_as_host(float x, const double* tab) {
 template <> __device__ __forceinline__ float exp_sel<true>(float x, const double* tab) { return exp_as_host(x, tab); }
 template <> __device__ __forceinline__ float exp_sel<false>(float x, const double*) { return expf(x); }
 
-// A row held by one CTA: float4 pieces in registers when the row is 16-byte addressable and short
-// enough, otherwise element loops over global memory.  `f(i, x)` visits every element.
-struct RowView {
+// A row held by a group of T threads, 4 V floats each.  16-byte pieces where the row is 16-byte addressable (VEC), single
+// floats with neighbouring threads on neighbouring elements otherwise; V == 0: the row does not fit and is visited in
+// global memory.
+template <int T, int V> struct Row {
     const float* x;
-    int n;
+    int n, t;
     bool vec;
-    float4 r[ROW_VEC];
-    __device__ RowView(const float* row, int n_) : x(row), n(n_) {
-        vec = (n % 4 == 0) && n <= ROW_THREADS * ROW_VEC * 4 && (reinterpret_cast<uintptr_t>(row) % 16 == 0);
+    float r[V > 0 ? 4 * V : 1];
+    // element index of r[4 j + e]
+    __device__ __forceinline__ int at(int j, int e) const { return vec ? (j * T + t) * 4 + e : (4 * j + e) * T + t; }
+    __device__ __forceinline__ Row(const float* row, int n_) : x(row), n(n_), t(T == 32 ? (int)(threadIdx.x & 31) : (int)threadIdx.x) {
+        vec = (n % 4 == 0) && (reinterpret_cast<uintptr_t>(row) % 16 == 0);
+        if (V == 0) return;
         if (vec) {
 #pragma unroll
-            for (int j = 0; j < ROW_VEC; j++) {
-                const int i = (j * ROW_THREADS + threadIdx.x) * 4;
-                r[j] = i < n ? __ldcs(reinterpret_cast<const float4*>(x + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int j = 0; j < V; j++) {
+                const int i = at(j, 0);
+                const float4 v = i < n ? __ldcs(reinterpret_cast<const float4*>(x + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                r[4 * j] = v.x, r[4 * j + 1] = v.y, r[4 * j + 2] = v.z, r[4 * j + 3] = v.w;
             }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4 * V; j++) r[j] = j * T + t < n ? __ldcs(x + j * T + t) : 0.f;
         }
     }
-    // x[i] <- h(x[i]) where the row is held in registers (the caller falls back to recomputing otherwise)
-    template <class H> __device__ __forceinline__ void map_registers(H h) {
+    // the sum of f(x[i]) over the row: fp32 over eight elements of a thread (32 where the row is walked in global
+    // memory), double from there on
+    template <class F> __device__ __forceinline__ double sum(F f, double* red) const {
+        double total = 0.0;
+        if (V > 0) {
 #pragma unroll
-        for (int j = 0; j < ROW_VEC; j++)
-            if ((j * ROW_THREADS + (int)threadIdx.x) * 4 < n) r[j] = make_float4(h(r[j].x), h(r[j].y), h(r[j].z), h(r[j].w));
+            for (int j0 = 0; j0 < V; j0 += 2) {
+                float part = 0.f;
+#pragma unroll
+                for (int j = j0; j < j0 + 2 && j < V; j++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+                        if (at(j, e) < n) part = __fadd_rn(part, f(r[4 * j + e]));
+                total += (double)part;
+            }
+        } else {
+            for (int i0 = t; i0 < n; i0 += 32 * T) {
+                float part = 0.f;
+                for (int i = i0; i < min(n, i0 + 32 * T); i += T) part = __fadd_rn(part, f(x[i]));
+                total += (double)part;
+            }
+        }
+        return group_sum<T>(total, red);
+    }
+    // x[i] <- h(x[i]) where the row is held in registers
+    template <class H> __device__ __forceinline__ void map(H h) {
+#pragma unroll
+        for (int j = 0; j < V; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (at(j, e) < n) r[4 * j + e] = h(r[4 * j + e]);
     }
     template <class F> __device__ __forceinline__ void for_each(F f) const {
-        if (vec) {
+        if (V > 0) {
 #pragma unroll
-            for (int j = 0; j < ROW_VEC; j++) {
-                const int i = (j * ROW_THREADS + threadIdx.x) * 4;
-                if (i < n) {
-                    f(i, r[j].x);
-                    f(i + 1, r[j].y);
-                    f(i + 2, r[j].z);
-                    f(i + 3, r[j].w);
+            for (int j = 0; j < V; j++)
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    if (at(j, e) < n) f(r[4 * j + e]);
+        } else {
+            for (int i = t; i < n; i += T) f(x[i]);
+        }
+    }
+    // y[i] = g(x[i], a[i], b[i]); a and b may be null (1 and 0 are passed for them, and g knows)
+    template <class G> __device__ __forceinline__ void write(float* y, const float* a, const float* b, G g) const {
+        if (V > 0) {
+            const bool wide = vec && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % 16) == 0;
+#pragma unroll
+            for (int j = 0; j < V; j++) {
+                if (wide) {
+                    const int i = at(j, 0);
+                    if (i >= n) continue;
+                    const float4 p = a ? __ldg(reinterpret_cast<const float4*>(a + i)) : make_float4(1.f, 1.f, 1.f, 1.f);
+                    const float4 q = b ? __ldg(reinterpret_cast<const float4*>(b + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    __stcs(reinterpret_cast<float4*>(y + i), make_float4(g(r[4 * j], p.x, q.x), g(r[4 * j + 1], p.y, q.y), g(r[4 * j + 2], p.z, q.z), g(r[4 * j + 3], p.w, q.w)));
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const int i = at(j, e);
+                        if (i < n) __stcs(y + i, g(r[4 * j + e], a ? __ldg(a + i) : 1.f, b ? __ldg(b + i) : 0.f));
+                    }
                 }
             }
         } else {
-            for (int i = threadIdx.x; i < n; i += ROW_THREADS) f(i, x[i]);
-        }
-    }
-    // y[i] = g(i, x[i]); 16-byte stores on the register path
-    template <class G> __device__ __forceinline__ void write(float* y, G g) const {
-        if (vec && reinterpret_cast<uintptr_t>(y) % 16 == 0) {
-#pragma unroll
-            for (int j = 0; j < ROW_VEC; j++) {
-                const int i = (j * ROW_THREADS + threadIdx.x) * 4;
-                if (i < n) __stcs(reinterpret_cast<float4*>(y + i), make_float4(g(i, r[j].x), g(i + 1, r[j].y), g(i + 2, r[j].z), g(i + 3, r[j].w)));
-            }
-        } else {
-            for_each([&](int i, float v) { y[i] = g(i, v); });
+            for (int i = t; i < n; i += T) y[i] = g(x[i], a ? __ldg(a + i) : 1.f, b ? __ldg(b + i) : 0.f);
         }
     }
 };
 
+// row of this thread's group, -1 for a group without one
+template <int T> __device__ __forceinline__ int64_t row_of_group(int64_t rows) {
+    const int64_t r = T == 32 ? (int64_t)blockIdx.x * (ROW_CTA / 32) + (threadIdx.x >> 5) : (int64_t)blockIdx.x;
+    return r < rows ? r : -1;
+}
+
 // CustomCallKernel.java:368-412: rms = (float) sqrt(sumSq / n + eps); y = x * (1 / rms) [* gamma]
-__global__ void __launch_bounds__(ROW_THREADS) rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
-                                                               float* __restrict__ y, int n, float eps) {
-    __shared__ double red[ROW_THREADS / 32];
-    const RowView row(x + (size_t)blockIdx.x * n, n);
-    float part = 0.f;
-    row.for_each([&](int, float v) { part = __fadd_rn(part, __fmul_rn(v, v)); });
-    const float sum_sq = (float)block_sum((double)part, red);
+template <int T, int V>
+__global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
+                                                                         float* __restrict__ y, int64_t rows, int n, float eps) {
+    __shared__ double red[T / 32];
+    const int64_t r = row_of_group<T>(rows);
+    if (r < 0) return;
+    const Row<T, V> row(x + (size_t)r * n, n);
+    const float sum_sq = (float)row.sum([](float v) { return __fmul_rn(v, v); }, red);
     const float rms = (float)sqrt((double)__fadd_rn(__fdiv_rn(sum_sq, (float)n), eps));
     const float inv = __fdiv_rn(1.0f, rms);
-    row.write(y + (size_t)blockIdx.x * n, [&](int i, float v) {
+    row.write(y + (size_t)r * n, gamma, nullptr, [&](float v, float gm, float) {
         const float t = __fmul_rn(v, inv);
-        return gamma ? __fmul_rn(t, gamma[i]) : t;
+        return gamma ? __fmul_rn(t, gm) : t;
     });
 }
 
 // CustomCallKernel.java:109-171: mean, then the variance of (x - mean), invStd = 1 / (float) sqrt(var + eps)
-__global__ void __launch_bounds__(ROW_THREADS) layer_norm_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
-                                                                 const float* __restrict__ beta, float* __restrict__ y, int n,
-                                                                 float eps) {
-    __shared__ double red[ROW_THREADS / 32], red2[ROW_THREADS / 32];
-    const RowView row(x + (size_t)blockIdx.x * n, n);
-    float part = 0.f;
-    row.for_each([&](int, float v) { part = __fadd_rn(part, v); });
-    const float mean = __fdiv_rn((float)block_sum((double)part, red), (float)n);
-    part = 0.f;
-    row.for_each([&](int, float v) {
-        const float d = __fsub_rn(v, mean);
-        part = __fadd_rn(part, __fmul_rn(d, d));
-    });
-    const float var = __fdiv_rn((float)block_sum((double)part, red2), (float)n);
+template <int T, int V>
+__global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) layer_norm_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
+                                                                           const float* __restrict__ beta, float* __restrict__ y,
+                                                                           int64_t rows, int n, float eps) {
+    __shared__ double red[T / 32], red2[T / 32];
+    const int64_t r = row_of_group<T>(rows);
+    if (r < 0) return;
+    const Row<T, V> row(x + (size_t)r * n, n);
+    const float mean = __fdiv_rn((float)row.sum([](float v) { return v; }, red), (float)n);
+    const float var = __fdiv_rn((float)row.sum(
+                                    [&](float v) {
+                                        const float d = __fsub_rn(v, mean);
+                                        return __fmul_rn(d, d);
+                                    },
+                                    red2),
+                                (float)n);
     const float inv = __fdiv_rn(1.0f, (float)sqrt((double)__fadd_rn(var, eps)));
-    row.write(y + (size_t)blockIdx.x * n, [&](int i, float v) {
+    row.write(y + (size_t)r * n, gamma, beta, [&](float v, float gm, float bt) {
         float t = __fmul_rn(__fsub_rn(v, mean), inv);
-        if (gamma) t = __fmul_rn(t, gamma[i]);
-        if (beta) t = __fadd_rn(t, beta[i]);
+        if (gamma) t = __fmul_rn(t, gm);
+        if (beta) t = __fadd_rn(t, bt);
         return t;
     });
 }
 
 // CustomCallKernel.java:173-224, over the last dimension: (float) exp(x - max) / sum
-template <bool EXACT>
-__global__ void __launch_bounds__(ROW_THREADS) softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int n) {
-    __shared__ double red[ROW_THREADS / 32];
-    __shared__ float redf[ROW_THREADS / 32];
+template <int T, int V, bool EXACT>
+__global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int64_t rows, int n) {
+    __shared__ double red[T / 32];
+    __shared__ float redf[T / 32];
     __shared__ double tab[32];
     if (EXACT) load_exp_table(tab);
-    RowView row(x + (size_t)blockIdx.x * n, n);
+    const int64_t r = row_of_group<T>(rows);
+    if (r < 0) return;
+    Row<T, V> row(x + (size_t)r * n, n);
     float mx = -INFINITY;
-    row.for_each([&](int, float v) { mx = v > mx ? v : mx; });  // `if (val > maxVal)`: a NaN never becomes the maximum
-    mx = block_max(mx, redf);
-    float part = 0.f;
-    if (row.vec) {  // the exponentials replace the row in registers: one exp per element
-        row.map_registers([&](float v) { return exp_sel<EXACT>(__fsub_rn(v, mx), tab); });
-        row.for_each([&](int, float e) { part = __fadd_rn(part, e); });
-        const float sum = (float)block_sum((double)part, red);
-        row.write(y + (size_t)blockIdx.x * n, [&](int, float e) { return __fdiv_rn(e, sum); });
+    row.for_each([&](float v) { mx = v > mx ? v : mx; });  // `if (val > maxVal)`: a NaN never becomes the maximum
+    mx = group_max<T>(mx, redf);
+    auto ex = [&](float v) { return exp_sel<EXACT>(__fsub_rn(v, mx), tab); };
+    if (V > 0) {  // the exponentials replace the row in registers: one exp per element
+        row.map(ex);
+        // e / sum, sum in [1, n]: the quotient estimate e * rn(1 / sum) corrected by its exact residual (Markstein, "Computation
+        // of elementary functions on the IBM RISC System/6000", 1990) is the correctly rounded quotient wherever it is a
+        // normal float -- three operations instead of a division per element
+        const float sum = (float)row.sum([](float e) { return e; }, red), inv = __frcp_rn(sum);
+        row.write(y + (size_t)r * n, nullptr, nullptr, [&](float e, float, float) {
+            const float q = __fmul_rn(e, inv);
+            return __fmaf_rn(__fmaf_rn(-q, sum, e), inv, q);
+        });
     } else {
-        row.for_each([&](int, float v) { part = __fadd_rn(part, exp_sel<EXACT>(__fsub_rn(v, mx), tab)); });
-        const float sum = (float)block_sum((double)part, red);
-        row.write(y + (size_t)blockIdx.x * n, [&](int, float v) { return __fdiv_rn(exp_sel<EXACT>(__fsub_rn(v, mx), tab), sum); });
+        const float sum = (float)row.sum(ex, red);
+        row.write(y + (size_t)r * n, nullptr, nullptr, [&](float v, float, float) { return __fdiv_rn(ex(v), sum); });
     }
+}
+
+// The group for rows of n columns: f(threads, floats / 4 per thread, CTAs).
+template <class F> static void with_row_group(int64_t rows, int64_t n, F&& f) {
+    const unsigned packed = (unsigned)((rows + ROW_CTA / 32 - 1) / (ROW_CTA / 32)), each = (unsigned)rows;
+    using std::integral_constant;
+    if (n <= 512) f(integral_constant<int, 32>{}, integral_constant<int, 4>{}, packed);
+    else if (n <= 1024) f(integral_constant<int, 64>{}, integral_constant<int, 4>{}, each);
+    else if (n <= 2048) f(integral_constant<int, 128>{}, integral_constant<int, 4>{}, each);
+    else if (n <= 4096) f(integral_constant<int, 256>{}, integral_constant<int, 4>{}, each);
+    else if (n <= 8192) f(integral_constant<int, 512>{}, integral_constant<int, 4>{}, each);
+    else if (n <= 16384) f(integral_constant<int, 1024>{}, integral_constant<int, 4>{}, each);
+    else f(integral_constant<int, 512>{}, integral_constant<int, 0>{}, each);
 }
 
 // ---- element operations: 16 bytes per thread per step, grid sized to the SM count
 template <bool EXACT> __device__ __forceinline__ float silu_as_host(float x, const double* tab) {  // CustomCallKernel.java:273-275
-    const float sigmoid = __fdiv_rn(1.0f, __fadd_rn(1.0f, exp_sel<EXACT>(-x, tab)));
+    const float sigmoid = __frcp_rn(__fadd_rn(1.0f, exp_sel<EXACT>(-x, tab)));
     return __fmul_rn(x, sigmoid);
 }
 
@@ -245,21 +324,43 @@ template <int OP, bool EXACT> __device__ __forceinline__ float el(float a, float
     return __fadd_rn(a, b);
 }
 
+// Several pieces of every operand are requested before the first one is used -- with one at a time add ran at 88 %, swiglu at
+// 82 % of HBM speed on 134 MB tensors.  Two operands: four pieces, 64 bytes of each; one operand: two, since silu is
+// bound by issue slots as much as by bytes and wants the warps.  EL_CTAS CTAs per SM, all resident.
+template <int OP, bool EXACT> struct ElShape {
+    static constexpr bool UNARY = OP == EL_SILU || OP == EL_GELU;
+    static constexpr int UNROLL = UNARY || EXACT ? 2 : 4, CTAS = UNARY || EXACT ? 6 : OP == EL_SWIGLU ? 3 : 4;  // what the registers allow
+};
 template <int OP, bool EXACT>
-__global__ void __launch_bounds__(256) elementwise_kernel(const float* __restrict__ a, const float* __restrict__ b,
-                                                          float* __restrict__ y, int64_t n, int vec) {
+__global__ void __launch_bounds__(256, (ElShape<OP, EXACT>::CTAS)) elementwise_kernel(const float* __restrict__ a, const float* __restrict__ b,
+                                                                                      float* __restrict__ y, int64_t n, int vec) {
+    constexpr bool UNARY = ElShape<OP, EXACT>::UNARY;
+    constexpr int EL_UNROLL = ElShape<OP, EXACT>::UNROLL;
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
     __shared__ double tab[32];
     if (OP != EL_ADD && OP != EL_GELU && EXACT) load_exp_table(tab);
     if (vec) {
-        for (int64_t i = tid; i < n / 4; i += step) {
-            const float4 u = __ldcs(reinterpret_cast<const float4*>(a) + i);
-            const float4 v = (OP == EL_SILU || OP == EL_GELU) ? u : __ldcs(reinterpret_cast<const float4*>(b) + i);
-            __stcs(reinterpret_cast<float4*>(y) + i, make_float4(el<OP, EXACT>(u.x, v.x, tab), el<OP, EXACT>(u.y, v.y, tab), el<OP, EXACT>(u.z, v.z, tab), el<OP, EXACT>(u.w, v.w, tab)));
+        const int64_t n4 = n / 4;
+        for (int64_t i0 = tid; i0 < n4; i0 += EL_UNROLL * step) {
+            float4 u[EL_UNROLL], v[EL_UNROLL];
+#pragma unroll
+            for (int j = 0; j < EL_UNROLL; j++) {
+                const int64_t i = i0 + j * step;
+                if (i < n4) {
+                    u[j] = __ldcs(reinterpret_cast<const float4*>(a) + i);
+                    if (!UNARY) v[j] = __ldcs(reinterpret_cast<const float4*>(b) + i);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < EL_UNROLL; j++) {
+                const int64_t i = i0 + j * step;
+                const float4 p = u[j], q = UNARY ? u[j] : v[j];
+                if (i < n4) __stcs(reinterpret_cast<float4*>(y) + i, make_float4(el<OP, EXACT>(p.x, q.x, tab), el<OP, EXACT>(p.y, q.y, tab), el<OP, EXACT>(p.z, q.z, tab), el<OP, EXACT>(p.w, q.w, tab)));
+            }
         }
-        for (int64_t i = n / 4 * 4 + tid; i < n; i += step) y[i] = el<OP, EXACT>(a[i], (OP == EL_SILU || OP == EL_GELU) ? 0.f : b[i], tab);
+        for (int64_t i = n4 * 4 + tid; i < n; i += step) y[i] = el<OP, EXACT>(a[i], UNARY ? 0.f : b[i], tab);
     } else {
-        for (int64_t i = tid; i < n; i += step) y[i] = el<OP, EXACT>(a[i], (OP == EL_SILU || OP == EL_GELU) ? 0.f : b[i], tab);
+        for (int64_t i = tid; i < n; i += step) y[i] = el<OP, EXACT>(a[i], UNARY ? 0.f : b[i], tab);
     }
 }
 
@@ -328,8 +429,19 @@ __global__ void __launch_bounds__(256) embedding_kernel(const int64_t* __restric
         const float* src = table + (size_t)(ok ? idx : 0) * dim;
         float* dst = y + (size_t)r * dim;
         if (vec) {
-            for (int i = threadIdx.x; i < dim / 4; i += blockDim.x)
-                reinterpret_cast<float4*>(dst)[i] = ok ? __ldg(reinterpret_cast<const float4*>(src) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int i0 = threadIdx.x; i0 < dim / 4; i0 += 4 * blockDim.x) {  // four pieces of the row in flight per thread
+                float4 v[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int i = i0 + j * blockDim.x;
+                    v[j] = ok && i < dim / 4 ? __ldg(reinterpret_cast<const float4*>(src) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int i = i0 + j * blockDim.x;
+                    if (i < dim / 4) reinterpret_cast<float4*>(dst)[i] = v[j];
+                }
+            }
         } else {
             for (int i = threadIdx.x; i < dim; i += blockDim.x) dst[i] = ok ? src[i] : 0.f;
         }
@@ -339,9 +451,11 @@ __global__ void __launch_bounds__(256) embedding_kernel(const int64_t* __restric
 static bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 static bool aligned4(const void* p) { return reinterpret_cast<uintptr_t>(p) % 4 == 0; }
 
-static int element_grid(Context* c, int64_t n) {
-    const int64_t want = (n / 4 + 255) / 256;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)c->sm_count * 8));
+template <int OP, bool EXACT>
+static void launch_element(Context* c, const float* a, const float* b, float* y, int64_t n, int vec, cudaStream_t s) {
+    const int64_t want = (n / 4 + 255) / 256, most = (int64_t)c->sm_count * ElShape<OP, EXACT>::CTAS;
+    const int grid = (int)std::max<int64_t>(1, std::min(want, most));
+    elementwise_kernel<OP, EXACT><<<grid, 256, 0, s>>>(a, b, y, n, vec);
 }
 
 }  // namespace wf
@@ -385,8 +499,11 @@ int wf_rms_norm(int64_t ctx, int64_t x_dev, int64_t gamma_dev, int64_t y_dev, in
     GLUE_ENTER(ctx);
     int rc = check_rows(c, "rms_norm", x_dev, y_dev, rows, n);
     if (rc != WF_OK || rows == 0) return rc;
-    rms_norm_kernel<<<(unsigned)rows, ROW_THREADS, 0, s>>>(reinterpret_cast<const float*>(x_dev), reinterpret_cast<const float*>(gamma_dev),
-                                                          reinterpret_cast<float*>(y_dev), (int)n, eps);
+    with_row_group(rows, n, [&](auto t, auto v, unsigned grid) {
+        constexpr int T = decltype(t)::value, V = decltype(v)::value;
+        rms_norm_kernel<T, V><<<grid, T == 32 ? ROW_CTA : T, 0, s>>>(reinterpret_cast<const float*>(x_dev), reinterpret_cast<const float*>(gamma_dev),
+                                                                    reinterpret_cast<float*>(y_dev), rows, (int)n, eps);
+    });
     return launched(c, "rms_norm");
 }
 
@@ -395,8 +512,12 @@ int wf_layer_norm(int64_t ctx, int64_t x_dev, int64_t gamma_dev, int64_t beta_de
     GLUE_ENTER(ctx);
     int rc = check_rows(c, "layer_norm", x_dev, y_dev, rows, n);
     if (rc != WF_OK || rows == 0) return rc;
-    layer_norm_kernel<<<(unsigned)rows, ROW_THREADS, 0, s>>>(reinterpret_cast<const float*>(x_dev), reinterpret_cast<const float*>(gamma_dev),
-                                                            reinterpret_cast<const float*>(beta_dev), reinterpret_cast<float*>(y_dev), (int)n, eps);
+    with_row_group(rows, n, [&](auto t, auto v, unsigned grid) {
+        constexpr int T = decltype(t)::value, V = decltype(v)::value;
+        layer_norm_kernel<T, V><<<grid, T == 32 ? ROW_CTA : T, 0, s>>>(
+            reinterpret_cast<const float*>(x_dev), reinterpret_cast<const float*>(gamma_dev), reinterpret_cast<const float*>(beta_dev),
+            reinterpret_cast<float*>(y_dev), rows, (int)n, eps);
+    });
     return launched(c, "layer_norm");
 }
 
@@ -404,10 +525,13 @@ int wf_softmax(int64_t ctx, int64_t x_dev, int64_t y_dev, int64_t rows, int64_t 
     GLUE_ENTER(ctx);
     int rc = check_rows(c, "softmax", x_dev, y_dev, rows, n);
     if (rc != WF_OK || rows == 0) return rc;
-    if (c->glue_exact)
-        softmax_kernel<true><<<(unsigned)rows, ROW_THREADS, 0, s>>>(reinterpret_cast<const float*>(x_dev), reinterpret_cast<float*>(y_dev), (int)n);
-    else
-        softmax_kernel<false><<<(unsigned)rows, ROW_THREADS, 0, s>>>(reinterpret_cast<const float*>(x_dev), reinterpret_cast<float*>(y_dev), (int)n);
+    with_row_group(rows, n, [&](auto t, auto v, unsigned grid) {
+        constexpr int T = decltype(t)::value, V = decltype(v)::value;
+        const float* x = reinterpret_cast<const float*>(x_dev);
+        float* y = reinterpret_cast<float*>(y_dev);
+        if (c->glue_exact) softmax_kernel<T, V, true><<<grid, T == 32 ? ROW_CTA : T, 0, s>>>(x, y, rows, (int)n);
+        else softmax_kernel<T, V, false><<<grid, T == 32 ? ROW_CTA : T, 0, s>>>(x, y, rows, (int)n);
+    });
     return launched(c, "softmax");
 }
 
@@ -422,13 +546,12 @@ static int elementwise(int64_t ctx, int op, const char* what, int64_t a_dev, int
     const int vec = aligned16(a) && aligned16(y) && (unary || aligned16(b));
     const float *fa = static_cast<const float*>(a), *fb = static_cast<const float*>(b);
     float* fy = reinterpret_cast<float*>(y_dev);
-    const int grid = element_grid(c, count);
-    if (op == EL_GELU) elementwise_kernel<EL_GELU, false><<<grid, 256, 0, s>>>(fa, fb, fy, count, vec);
-    else if (op == EL_SILU && c->glue_exact) elementwise_kernel<EL_SILU, true><<<grid, 256, 0, s>>>(fa, fb, fy, count, vec);
-    else if (op == EL_SILU) elementwise_kernel<EL_SILU, false><<<grid, 256, 0, s>>>(fa, fb, fy, count, vec);
-    else if (op == EL_SWIGLU && c->glue_exact) elementwise_kernel<EL_SWIGLU, true><<<grid, 256, 0, s>>>(fa, fb, fy, count, vec);
-    else if (op == EL_SWIGLU) elementwise_kernel<EL_SWIGLU, false><<<grid, 256, 0, s>>>(fa, fb, fy, count, vec);
-    else elementwise_kernel<EL_ADD, false><<<grid, 256, 0, s>>>(fa, fb, fy, count, vec);
+    if (op == EL_GELU) launch_element<EL_GELU, false>(c, fa, fb, fy, count, vec, s);
+    else if (op == EL_SILU && c->glue_exact) launch_element<EL_SILU, true>(c, fa, fb, fy, count, vec, s);
+    else if (op == EL_SILU) launch_element<EL_SILU, false>(c, fa, fb, fy, count, vec, s);
+    else if (op == EL_SWIGLU && c->glue_exact) launch_element<EL_SWIGLU, true>(c, fa, fb, fy, count, vec, s);
+    else if (op == EL_SWIGLU) launch_element<EL_SWIGLU, false>(c, fa, fb, fy, count, vec, s);
+    else launch_element<EL_ADD, false>(c, fa, fb, fy, count, vec, s);
     return launched(c, what);
 }
 

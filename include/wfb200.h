@@ -195,9 +195,8 @@ int wf_embedding(int64_t ctx, int64_t indices_dev, int64_t table_dev, int64_t y_
  * and the call returns after the result is in `y`.  With device pointers the call only
  * enqueues work on `stream`; with a host pointer it waits for the result and reports a bounded
  * device-side wait that ran out as WF_ERR_DEVICE_WAIT, like wf_stream_sync.  Up to 32 bf16 tokens
- * (10 fp32 tokens) per launch run on the memory-bound decode kernels; more bf16 tokens run on the
- * tensor-core GEMM, whose activation copy and tile-piece scratch belong to the context: many-token
- * calls of one context must not overlap on different streams. */
+ * (10 fp32 tokens) per launch run on the memory-bound decode kernels; more tokens run on the tensor-core GEMM,
+ * which keeps its activation copy and tile-piece scratch per stream. */
 int wf_qlinear(int64_t ctx, int64_t weight, const void* x, int x_dtype, int x_on_device, int64_t m, void* y,
                int y_on_device, int64_t stream);
 

@@ -1,0 +1,87 @@
+"""The tensor-core kernels at the edges of their tiles: CTA pairs (256 rows x 512 tokens, from 129 tokens and a dozen tiles
+on) and K-splitting clusters (128 rows x 128 tokens; ranks with no tokens of their own to finish, several tiles per
+cluster), K that ends inside a stage of 64, and fp32 tokens.
+
+bf16 tokens: the bars of test_gpu_gemm.py.  fp32 tokens: products are exact to 2^-22 and an accumulator takes at most 32
+steps between two drains, each cutting the partial sum off at its 24th bit: 32 x 2^-23 = 3.8e-6 of the result at
+the very most, in the 2-norm against float64."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from warpforge_b200 import quant as Q
+
+pytestmark = pytest.mark.gpu
+
+QT = {"q4_0": O.Q4_0, "q4_1": O.Q4_1, "q5_0": O.Q5_0, "q8_0": O.Q8_0, "q4_k": O.Q4_K}
+
+
+@pytest.fixture(scope="module")
+def backend():
+    from warpforge_b200.backend import NvidiaBackend
+
+    b = NvidiaBackend(0)
+    yield b
+    b.close()
+
+
+def _run(backend, oracle, name, rows, k, x, tensor):
+    """Two calls (the second finds the scratch of the first) and the exact product."""
+    from warpforge_b200.backend import DotGeneralOp, LINEAR_DIMS
+
+    qt = Q.QuantizationType[name.upper()]
+    blocks = Q.synth_weight(qt, rows, k, rows + k + len(x))
+    w = backend.upload_weight(qt, blocks, rows, k)
+    got = [backend.execute(DotGeneralOp(LINEAR_DIMS, (len(x), rows)), [tensor, w])[0].data for _ in range(2)]
+    w.close()
+    assert np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
+    wf = oracle.dequant(QT[name], blocks, rows * k).reshape(rows, k).astype(np.float64)
+    return got[0], x.astype(np.float64) @ wf.T
+
+
+@pytest.mark.parametrize("name", sorted(QT))
+@pytest.mark.parametrize("rows,k,m", [
+    (130, 352, 33), (1000, 1120, 80), (700, 5152, 77), (2500, 672, 128),  # clusters; K ends inside a stage
+    (3000, 544, 129), (3072, 1024, 257), (2900, 288, 513), (1600, 2080, 1100),  # pairs; 129 tokens: one half, 257: the next begins
+    (300, 800, 300), (128, 4128, 600),  # few tiles: clusters on several token tiles
+])
+def test_bf16_tokens(backend, oracle, name, rows, k, m):
+    from warpforge_b200.backend import Tensor
+
+    if name == "q4_k":
+        k = max(256, k // 256 * 256)
+    xb = Q.synth_activation_bf16(m, k, rows + m)
+    got, want = _run(backend, oracle, name, rows, k, Q.bf16_bits_to_float(xb), Tensor.from_bf16_bits(xb))
+    d = got - want
+    assert np.max(np.abs(d)) <= 1e-3 * np.max(np.abs(want))
+    assert np.linalg.norm(d) <= 3e-4 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("name", sorted(QT))
+@pytest.mark.parametrize("rows,k,m", [(100, 96, 11), (257, 2080, 24), (1000, 4000, 96), (640, 1024, 97), (2100, 544, 200)])
+def test_fp32_tokens(backend, oracle, name, rows, k, m):
+    from warpforge_b200.backend import Tensor
+
+    if name == "q4_k":
+        k = max(256, k // 256 * 256)
+    x = Q.synth_activation_f32(m, k, rows + m)
+    x[1] *= 1e20  # a scale of its own per token
+    got, want = _run(backend, oracle, name, rows, k, x, Tensor.from_float_array(x))
+    for rows_of in (slice(1, 2), np.r_[0, 2:m]):
+        assert np.linalg.norm((got - want)[rows_of]) <= 3.8e-6 * np.linalg.norm(want[rows_of])
+
+
+def test_fp32_tokens_keep_fp32s_range(backend, oracle):
+    """Weights beyond fp16's range (a scale of 20000): the many-token kernel cannot hold them, the call still answers."""
+    from warpforge_b200.backend import DotGeneralOp, LINEAR_DIMS, Tensor
+
+    rows, k, m = 64, 256, 40
+    blocks = Q.synth_q8_0(rows, k, 3).reshape(rows, -1, 34).copy()
+    blocks[5, 2, :2] = np.frombuffer(np.float16(20000.0).tobytes(), np.uint8)
+    blocks = blocks.reshape(rows, -1)
+    x = Q.synth_activation_f32(m, k, 4)
+    w = backend.upload_weight(Q.QuantizationType.Q8_0, blocks, rows, k)
+    got = backend.execute(DotGeneralOp(LINEAR_DIMS, (m, rows)), [Tensor.from_float_array(x), w])[0].data
+    w.close()
+    want = x.astype(np.float64) @ oracle.dequant(O.Q8_0, blocks, rows * k).reshape(rows, k).astype(np.float64).T
+    assert np.linalg.norm(got - want) <= 3.8e-6 * np.linalg.norm(want)

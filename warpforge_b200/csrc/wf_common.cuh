@@ -54,6 +54,7 @@ struct Weight {
     int64_t row0 = 0;        // first global row of this shard
     int64_t total_rows = 0;  // rows of the unsharded tensor
     uint8_t* d_tiles = nullptr;
+    bool beyond_fp16 = false;  // some block may hold values outside fp16's range
     int64_t tiles_held = 0;  // bytes allocated at d_tiles (a reused buffer may be larger than g.bytes())
     int programs = 0;        // live programs whose op lists point at d_tiles
     // how the several-token decode kernel cuts this weight, per activation dtype (bf16 / fp32) and column count:
@@ -65,12 +66,17 @@ struct Weight {
     }
 };
 
-// Scratch for the GEMV fix-up between CTAs, one per stream that launches GEMVs.
+// Scratch of the kernels, one per stream that launches them (calls on different streams may overlap).
 struct GemvScratch {
     uint2* d_slots = nullptr;  // [ctas][128] {value bits, tag}
     float* d_part = nullptr;   // several-token kernel: partial sums of k-sliced launches
     int* d_count = nullptr;    // several-token kernel: arrival counters per row-tile
     int ctas = 0;
+    // tensor-core GEMM
+    void* d_x16 = nullptr;                 // fp16 copy of the activations
+    int64_t x16_bytes = 0;
+    float* d_gemm_partial = nullptr;       // [sm_count][512][128] pieces of tiles cut by a share boundary
+    unsigned int* d_gemm_ready = nullptr;  // [sm_count][4] generation whose piece is complete, per 32-row quarter; then {generation, CTAs out}
 };
 
 struct Context {
@@ -80,7 +86,8 @@ struct Context {
     int cc_major = 0, cc_minor = 0;
     cudaStream_t stream = nullptr;  // the context's own compute stream
     int* d_status = nullptr;            // StatusBlock in device memory
-    volatile int* h_status = nullptr;   // its host words, pinned
+    volatile int* h_status = nullptr;   // its host words, pinned; one more, set by the repack kernels (launch_repack)
+    int* beyond_dev = nullptr;          // device address of that one
     int salt = 0;                            // instrumentation level, 2 = kernel timing stamps
     unsigned long long* d_timing = nullptr;  // [sm_count][8]
     std::mutex mu;  // guards against concurrent use (try_lock -> WF_ERR_BUSY)
@@ -107,10 +114,6 @@ struct Context {
     int64_t upload_chunk_bytes = 0;
     cudaStream_t upload_stream = nullptr;
     cudaEvent_t upload_done[UPLOAD_RING] = {}, upload_repacked[UPLOAD_RING] = {};  // chunk transferred / its tiles written
-    void* d_x16 = nullptr;  // fp16 copy of the activations for the tensor-core GEMM
-    int64_t x16_bytes = 0;
-    float* d_gemm_partial = nullptr;       // [sm_count][512][128] pieces of tiles cut by a share boundary
-    unsigned int* d_gemm_ready = nullptr;  // [sm_count][4] generation whose piece is complete, per 32-row quarter; then {generation, CTAs out}
     int64_t launches = 0;
     bool glue_exact = false;  // silu / softmax evaluate exp as the host does (double, one rounding) instead of expf
     int gemv_ctas_per_sm[3] = {0, 0, 0};
@@ -136,8 +139,9 @@ int weight_upload(Context* c, int qtype, const void* blocks, int64_t n_rows, int
                   int q4_0_order, int64_t* weight);
 
 // wf_repack.cu
+// *beyond (device address) is set to 1 when a block may hold values outside fp16's range
 cudaError_t launch_repack(int qtype, const uint8_t* d_raw, uint8_t* d_tiles, int64_t rows, int64_t k,
-                          int q4_0_order, cudaStream_t s);
+                          int q4_0_order, int* beyond, cudaStream_t s);
 cudaError_t launch_dequant_rows(const Weight& w, int64_t row0, int64_t nrows, float* d_out, cudaStream_t s);
 
 // wf_gemv.cu
@@ -158,6 +162,9 @@ int gemv_launch_noalloc(Context* c, const GemvCall& call, cudaStream_t s);
 // wf_gemm.cu
 bool gemm_supported(const Weight& w, int x_dtype, int64_t m, const void* d_x);
 int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s);
+// sizes the stream's scratch like the largest of the context's other streams (before a recording)
+int gemm_prepare_stream(Context* c, cudaStream_t s);
+void free_scratch(GemvScratch& sc);
 
 struct ScopedLock {
     Context* c;

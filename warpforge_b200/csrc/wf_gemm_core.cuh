@@ -1,0 +1,551 @@
+// Building blocks of the tensor-core GEMM kernels: tcgen05 / TMA / mbarrier wrappers, the conversion of the activations, the
+// epilogue's stores and the dequantization of weight tiles to fp16.
+#pragma once
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+#include <type_traits>
+
+#include "wf_common.cuh"
+
+namespace wf {
+
+constexpr int GEMM_BN = 128;             // weight rows per CTA and tile (UMMA M per CTA)
+constexpr int GEMM_BK = 128;             // k per unit of the work split: two stages of 64 k
+constexpr int GEMM_DEQUANT_WARPS = 8;    // a 16-row weight tile each (sixteen of eight rows: 3 - 14 % slower, 92 registers a thread)
+constexpr int GEMM_THREADS = (6 + GEMM_DEQUANT_WARPS) * 32;  // TMA, MMA, 4 epilogue, dequant warps
+constexpr int GEMM_WAIT_SPINS = 1 << 20;    // of an mbarrier wait, which suspends the thread for microseconds per try
+constexpr int GEMM_POLL_SPINS = 1 << 22;    // of a poll of global memory
+constexpr int GEMM_PIECE_TOKENS = 512;   // tokens a stream-K piece can hold
+
+struct GemmParams {
+    const uint8_t* tiles;
+    float* y;
+    const float* row_unscale;  // [m] power of two that undoes the scaling of token row m (convert_rows_kernel)
+    int* status;
+    int64_t ldy, col0;
+    int rows, kt_w;      // kt_w: weight k-tiles per row-tile stripe (tile_k of the format)
+    int rt_last;         // last row-tile in the weight buffer
+    int m;               // tokens
+    int bm;              // tokens per MMA (UMMA N: multiple of 16, <= 256)
+    int n_tiles, m_tiles, k_blocks;  // k_blocks = ceil(k / 128)
+    int stages;
+    int ranks;           // split kernel: CTAs of a cluster, which share a tile's K
+    uint32_t idesc;
+    // pair kernel, stream-K: the (tile, k-block) units form one sequence, pair b owns units [b*q + min(b,r), ...)
+    int unit_q, unit_r;
+    float* partial;        // [ctas][GEMM_PIECE_TOKENS][128] fp32: a CTA's piece of a tile that begins in an earlier pair
+    unsigned int* ready;   // [ctas][4] generation whose piece (per 32-row quarter) is complete in `partial`
+    unsigned int* gen;     // [0] generations completed so far, [1] CTAs that have left the current launch: the kernel
+                           // numbers its own launches, so a launch recorded in a CUDA graph is a new generation on every replay
+                           // (read after griddepcontrol.wait, when the previous launch's closing store is visible)
+};
+
+// ---------------------------------------------------------------- PTX wrappers
+__device__ __forceinline__ uint32_t g_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void g_mbar_init(void* bar, int count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(g_smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void g_mbar_arrive(void* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(g_smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void g_mbar_expect_tx(void* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(g_smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool g_mbar_wait(void* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        ".reg .u32 n;\n\t"
+        "mov.u32 n, 0;\n\t"
+        "WFG_WAIT_%=:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra WFG_DONE_%=;\n\t"
+        "add.u32 n, n, 1;\n\t"
+        "setp.lt.u32 q, n, %3;\n\t"
+        "@q bra WFG_WAIT_%=;\n\t"
+        "WFG_DONE_%=:\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(g_smem_u32(bar)), "r"(parity), "r"((uint32_t)GEMM_WAIT_SPINS)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// shared::cluster address of the same object in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+    return r;
+}
+// Default semantics (release at CTA scope): the operands handed over were put in place by the async-proxy fence and the
+// CTA's own barriers; `.release.cluster` costs a fence that waits for the thread's loads in flight, 0.9 us per stage.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, void* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            g_smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(g_smem_u32(bar))
+        : "memory");
+}
+__device__ __forceinline__ void tmem_alloc(void* smem_dst, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(g_smem_u32(smem_dst)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_commit(void* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(g_smem_u32(bar)) : "memory");
+}
+// One 64-k span of a tile: four MMAs of 16 k, 32 bytes (two descriptor units) apart in the swizzled rows.  Issued by the
+// thread whose `issue` is non-zero; the whole warp comes here with the same operands, which therefore sit in uniform
+// registers.  (Issued from a branch of one lane, every operand had to be moved there, and at about 200 cycles per MMA
+// the issuing thread, not the tensor core with its 128, set the pace.)  accumulate: 0 = the first MMA starts from zero.
+template <int GROUP> __device__ __forceinline__ void tc_mma_span(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t issue) {
+#define WF_MMA_SPAN(G)                                                                    \
+    asm volatile(                                                                         \
+        "{\n\t.reg .pred p, e, t;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"               \
+        "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"        \
+        "add.s64 a1, %1, 2;\n\tadd.s64 a2, %1, 4;\n\tadd.s64 a3, %1, 6;\n\t"               \
+        "add.s64 b1, %2, 2;\n\tadd.s64 b2, %2, 4;\n\tadd.s64 b3, %2, 6;\n\t"               \
+        "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], %1, %2, %3, p;\n\t"              \
+        "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], a1, b1, %3, t;\n\t"              \
+        "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], a2, b2, %3, t;\n\t"              \
+        "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], a3, b3, %3, t;\n\t}" ::"r"(d_tmem), \
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue)                   \
+        : "memory")
+    if (GROUP == 1) WF_MMA_SPAN("1");
+    else WF_MMA_SPAN("2");
+#undef WF_MMA_SPAN
+}
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e;
+}
+__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p) {
+    unsigned int v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release_u32(unsigned int* p, unsigned int v) {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+// K-major operand, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.
+__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);   // start address
+    d |= (uint64_t)1 << 16;                    // leading byte offset (unused with swizzle), 16 B
+    d |= (uint64_t)(1024 >> 4) << 32;          // stride byte offset: 8 rows x 128 B
+    d |= (uint64_t)1 << 46;                    // descriptor version (sm_100)
+    d |= (uint64_t)2 << 61;                    // SWIZZLE_128B
+    return d;
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
+          "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+          "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// The same of one accumulator, or the sum of two that lie bm columns apart.
+template <int ACCS> __device__ __forceinline__ void tmem_ld_accs(uint32_t taddr, int bm, uint32_t (&r)[32]) {
+    tmem_ld32(taddr, r);
+    if (ACCS == 2) {
+        uint32_t e[32];
+        tmem_ld32(taddr + (uint32_t)bm, e);
+#pragma unroll
+        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(e[j]));
+    }
+}
+
+// ---------------------------------------------------------------- the order of k inside a stage
+// A stage row is 64 k = eight 16-byte chunks; group q (eight k) of 32-k block j lies in chunk 2 q + j, in the weights' rows and
+// the activations' alike (the sum does not care).  A lane stores group q of both blocks of a row; a 16-byte shared-memory
+// store is served eight lanes at a time, two neighbouring rows x four groups of one block, which under the 128-byte
+// swizzle meet eight different chunks this way.  With the blocks one after the other they met four, a two-way conflict.
+__host__ __device__ inline int stage_chunk(int j, int q) { return 2 * q + j; }
+
+// ---------------------------------------------------------------- activations to fp16
+// x16[row] = fp16(x[row] * 2^s) with s chosen so that the row's largest magnitude lands in [2^14, 2^15); unscale[row] = 2^-s.
+//   bf16 (PLANES 1): exact whenever the scaled value is a normal fp16.
+// Rows are padded to whole stages of 64 k (zeros) and lie in the stages' order of k.
+//   fp32 (PLANES 3): v = hi + mid + lo, each the fp16 nearest to what is left: exact down to 2^-39 of the row's largest.
+// One CTA per row.  A kernel of its own: the GEMM's CTAs set themselves up and dequantize their first stages under it.
+// Measured and not kept: converting inside the GEMM, every CTA its share of the rows and a counter to wait for (64
+// tokens: 18 us a call instead of 16, the launch and set-up of the GEMM itself lie bare then); CTAs small enough to wait
+// beside the previous GEMM's, which triggers them early (the nested release takes 3 us longer than the overlap gains).
+constexpr int CONVERT_THREADS = 256;
+template <int PLANES>
+__global__ void __launch_bounds__(CONVERT_THREADS) convert_rows_kernel(const void* __restrict__ x, __half* __restrict__ x16, float* __restrict__ unscale,
+                                                                       int m, int k) {
+    __shared__ int s_max[CONVERT_THREADS / 32];
+    // Launched with programmatic stream serialization itself: its CTAs may be placed while the previous kernel of the
+    // stream drains, but nothing is read or written before that kernel has completed (it may have produced x, and a
+    // previous GEMM may still be reading the fp16 copy this kernel rewrites).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMM may set itself up while the rows are converted
+    constexpr int KEEP = PLANES == 1 ? 4 : 2;  // groups of eight elements a thread keeps between the scan and the conversion
+    const int groups = k >> 3, t = (int)threadIdx.x;  // k is a multiple of 32
+    const int padded = (groups + 7) & ~7;             // groups of a row of x16
+    const size_t plane = (size_t)m * padded;
+    struct G {
+        uint4 a, b;
+    };
+    const int row = (int)blockIdx.x;
+    const uint4* src = static_cast<const uint4*>(x) + (size_t)row * groups * (PLANES == 1 ? 1 : 2);
+    auto load = [&](int i) {
+        G g;
+        g.a = __ldg(src + (PLANES == 1 ? i : 2 * i));
+        g.b = PLANES == 1 ? g.a : __ldg(src + 2 * i + 1);
+        return g;
+    };
+    auto emax_of = [](const G& g) {  // largest biased exponent; Inf and NaN do not drive the scale
+        int e = 0;
+        auto one = [&](uint32_t v) { e = max(e, v == 0xFFu ? 0 : (int)v); };
+        const uint32_t w[8] = {g.a.x, g.a.y, g.a.z, g.a.w, g.b.x, g.b.y, g.b.z, g.b.w};
+#pragma unroll
+        for (int i = 0; i < (PLANES == 1 ? 4 : 8); i++) {
+            one((w[i] >> 23) & 0xFFu);
+            if (PLANES == 1) one((w[i] >> 7) & 0xFFu);
+        }
+        return e;
+    };
+    G keep[KEEP];
+    int emax = 0;
+#pragma unroll
+    for (int u = 0; u < KEEP; u++)
+        if (t + u * CONVERT_THREADS < groups) keep[u] = load(t + u * CONVERT_THREADS);
+#pragma unroll
+    for (int u = 0; u < KEEP; u++)
+        if (t + u * CONVERT_THREADS < groups) emax = max(emax, emax_of(keep[u]));
+    for (int i = t + KEEP * CONVERT_THREADS; i < groups; i += CONVERT_THREADS) emax = max(emax, emax_of(load(i)));
+    emax = __reduce_max_sync(0xFFFFFFFFu, emax);
+    if ((t & 31) == 0) s_max[t >> 5] = emax;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < CONVERT_THREADS / 32; w++) emax = max(emax, s_max[w]);
+    const int shift = emax == 0 ? 0 : (127 + 14) - emax;  // multiply by 2^shift
+    const float scale = __uint_as_float((uint32_t)min(max(127 + shift, 1), 254) << 23);
+    uint4* out = reinterpret_cast<uint4*>(x16) + (size_t)row * padded;
+    auto convert = [&](int i, const G& g) {
+        float f[8];
+        const uint32_t w[8] = {g.a.x, g.a.y, g.a.z, g.a.w, g.b.x, g.b.y, g.b.z, g.b.w};
+        if (PLANES == 1) {
+#pragma unroll
+            for (int e = 0; e < 4; e++) f[2 * e] = __uint_as_float(w[e] << 16) * scale, f[2 * e + 1] = __uint_as_float(w[e] & 0xFFFF0000u) * scale;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; e++) f[e] = __uint_as_float(w[e]) * scale;
+        }
+#pragma unroll
+        for (int pl = 0; pl < PLANES; pl++) {
+            uint32_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const __half2 h = __floats2half2_rn(f[2 * e], f[2 * e + 1]);
+                o[e] = *reinterpret_cast<const uint32_t*>(&h);
+                if (pl + 1 < PLANES) {
+                    const float2 back = __half22float2(h);
+                    f[2 * e] -= back.x;
+                    f[2 * e + 1] -= back.y;
+                }
+            }
+            out[pl * plane + (i & ~7) + stage_chunk((i >> 2) & 1, i & 3)] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < KEEP; u++)
+        if (t + u * CONVERT_THREADS < groups) convert(t + u * CONVERT_THREADS, keep[u]);
+    for (int i = t + KEEP * CONVERT_THREADS; i < groups; i += CONVERT_THREADS) convert(i, load(i));
+    if (t < padded - groups)  // the block that K lacks of its last stage
+#pragma unroll
+        for (int pl = 0; pl < PLANES; pl++) out[pl * plane + (groups & ~7) + stage_chunk(1, t)] = make_uint4(0u, 0u, 0u, 0u);
+    if (t == 0) unscale[row] = __uint_as_float((uint32_t)min(max(127 - shift, 1), 254) << 23);
+}
+
+// ---------------------------------------------------------------- epilogue pieces (one lane = one weight row)
+// r[j] = accumulator of (token m0 + j, weight row n).  Rows of y are ldy floats apart; a warp writes 32
+// consecutive floats of one token row per store.  m0 is a multiple of 32, so the row scales load as float4.
+__device__ __forceinline__ void store_chunk(float* __restrict__ y, int64_t ldy, int64_t col0, const float* __restrict__ unscale,
+                                            const uint32_t (&r)[32], int m0, int m, int n, int rows) {
+    if (n >= rows || m0 >= m) return;
+    float* yp = y + (int64_t)m0 * ldy + col0 + n;
+    if (m0 + 32 <= m) {
+        float sc[32];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(unscale + m0) + i);
+            sc[4 * i] = v.x, sc[4 * i + 1] = v.y, sc[4 * i + 2] = v.z, sc[4 * i + 3] = v.w;
+        }
+#pragma unroll
+        for (int j = 0; j < 32; j++) yp[(int64_t)j * ldy] = __uint_as_float(r[j]) * sc[j];
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            if (m0 + j < m) yp[(int64_t)j * ldy] = __uint_as_float(r[j]) * __ldg(unscale + m0 + j);
+    }
+}
+// A stream-K piece holds four tokens of a weight row in 16 bytes, [tokens / 4][128 rows]: a warp moves 512 contiguous
+// bytes per access, eight accesses per 32 tokens (one float at a time the owner's tail read its pieces at a third of the
+// speed: 8 - 11 us after the last MMA for 256 KB).
+__device__ __forceinline__ void write_piece_chunk(float* __restrict__ piece, const uint32_t (&r)[32], int tok, int row) {
+    uint4* pp = reinterpret_cast<uint4*>(piece) + (size_t)(tok >> 2) * GEMM_BN + row;
+#pragma unroll
+    for (int j = 0; j < 8; j++) __stcg(pp + j * GEMM_BN, make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]));
+}
+__device__ __forceinline__ void load_piece_chunk(const float* __restrict__ piece, float4 (&v)[8], int tok, int row) {
+    const float4* pp = reinterpret_cast<const float4*>(piece) + (size_t)(tok >> 2) * GEMM_BN + row;
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = __ldcg(pp + j * GEMM_BN);
+}
+__device__ __forceinline__ void add_piece_chunk(uint32_t (&r)[32], const float4 (&v)[8]) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + v[j].x);
+        r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + v[j].y);
+        r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + v[j].z);
+        r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + v[j].w);
+    }
+}
+
+// ---------------------------------------------------------------- dequantization to fp16
+// A plane word holds the codes of 8 consecutive elements: rotated back by PLANE_ROT, nibble p of the
+// low half is element 2p and nibble p of the high half element 2p + 1.  As fp16 bit patterns
+//   (w & 0x000F000F) | 0x64006400  =  (1024 + e0, 1024 + e1)      codes in mantissa bits 3..0
+//   (w & 0x00F000F0) | 0x54005400  =  (  64 + e2,   64 + e3)      codes in mantissa bits 7..4
+// and the same two masks on the word rotated by a further 8 bits give elements 4..7.  Two rotates and
+// four logic ops per 8 codes; everything after that runs on the half / float pipes.
+struct Codes8 {
+    uint32_t k[2];  // 1024 + code: elements (0,1), (4,5)
+    uint32_t h[2];  // 64 + code:   elements (2,3), (6,7)
+};
+__device__ __forceinline__ Codes8 unpack8(uint32_t w) {
+    const uint32_t a = __funnelshift_r(w, w, PLANE_ROT), b = __funnelshift_r(w, w, PLANE_ROT + 8);
+    Codes8 c;
+    c.k[0] = (a & 0x000F000Fu) | 0x64006400u;
+    c.h[0] = (a & 0x00F000F0u) | 0x54005400u;
+    c.k[1] = (b & 0x000F000Fu) | 0x64006400u;
+    c.h[1] = (b & 0x00F000F0u) | 0x54005400u;
+    return c;
+}
+__device__ __forceinline__ __half2 as_half2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
+__device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
+
+// Q4_0: s * (code - 8) with s an fp16 value.  code - 8 is exact in fp16 and the product is rounded
+// once, exactly like the fp32 product rounded to fp16.
+__device__ __forceinline__ uint4 word_to_half8_q4_0(uint32_t w, __half2 s2) {
+    const Codes8 c = unpack8(w);
+    const __half2 m1032 = __float2half2_rn(-1032.f), m72 = __float2half2_rn(-72.f);
+    uint4 o;
+    o.x = as_u32(__hmul2(__hadd2(as_half2(c.k[0]), m1032), s2));
+    o.y = as_u32(__hmul2(__hadd2(as_half2(c.h[0]), m72), s2));
+    o.z = as_u32(__hmul2(__hadd2(as_half2(c.k[1]), m1032), s2));
+    o.w = as_u32(__hmul2(__hadd2(as_half2(c.h[1]), m72), s2));
+    return o;
+}
+// What rounding left, as a second fp16: fma(code - 8, s, -rounded) is exact, a multiple of s's last place.
+__device__ __forceinline__ void word_to_half8x2_q4_0(uint32_t w, __half2 s2, uint4& hi, uint4& lo) {
+    const Codes8 c = unpack8(w);
+    const __half2 m1032 = __float2half2_rn(-1032.f), m72 = __float2half2_rn(-72.f);
+    auto two = [&](uint32_t code, __half2 off, uint32_t& h, uint32_t& l) {
+        const __half2 q = __hadd2(as_half2(code), off), r = __hmul2(q, s2);
+        h = as_u32(r);
+        l = as_u32(__hfma2(q, s2, __hneg2(r)));
+    };
+    two(c.k[0], m1032, hi.x, lo.x);
+    two(c.h[0], m72, hi.y, lo.y);
+    two(c.k[1], m1032, hi.z, lo.z);
+    two(c.h[1], m72, hi.w, lo.w);
+}
+// Q8_0: s * (16 (hi - 8) + lo): the integer is exact in fp16 (|q| <= 128), one rounding in the product.
+__device__ __forceinline__ uint4 words_to_half8_q8(uint32_t wh, uint32_t wl, __half2 s2) {
+    const Codes8 h = unpack8(wh), l = unpack8(wl);
+    const __half2 m1032 = __float2half2_rn(-1032.f), m72 = __float2half2_rn(-72.f);
+    const __half2 m1024 = __float2half2_rn(-1024.f), m64 = __float2half2_rn(-64.f), sixteen = __float2half2_rn(16.f);
+    uint4 o;
+    o.x = as_u32(__hmul2(__hfma2(sixteen, __hadd2(as_half2(h.k[0]), m1032), __hadd2(as_half2(l.k[0]), m1024)), s2));
+    o.y = as_u32(__hmul2(__hfma2(sixteen, __hadd2(as_half2(h.h[0]), m72), __hadd2(as_half2(l.h[0]), m64)), s2));
+    o.z = as_u32(__hmul2(__hfma2(sixteen, __hadd2(as_half2(h.k[1]), m1032), __hadd2(as_half2(l.k[1]), m1024)), s2));
+    o.w = as_u32(__hmul2(__hfma2(sixteen, __hadd2(as_half2(h.h[1]), m72), __hadd2(as_half2(l.h[1]), m64)), s2));
+    return o;
+}
+__device__ __forceinline__ void words_to_half8x2_q8(uint32_t wh, uint32_t wl, __half2 s2, uint4& hi, uint4& lo) {
+    const Codes8 h = unpack8(wh), l = unpack8(wl);
+    const __half2 m1032 = __float2half2_rn(-1032.f), m72 = __float2half2_rn(-72.f);
+    const __half2 m1024 = __float2half2_rn(-1024.f), m64 = __float2half2_rn(-64.f), sixteen = __float2half2_rn(16.f);
+    auto two = [&](uint32_t ch, uint32_t cl, __half2 oh, __half2 ol, uint32_t& a, uint32_t& b) {
+        const __half2 q = __hfma2(sixteen, __hadd2(as_half2(ch), oh), __hadd2(as_half2(cl), ol)), r = __hmul2(q, s2);
+        a = as_u32(r);
+        b = as_u32(__hfma2(q, s2, __hneg2(r)));
+    };
+    two(h.k[0], l.k[0], m1032, m1024, hi.x, lo.x);
+    two(h.h[0], l.h[0], m72, m64, hi.y, lo.y);
+    two(h.k[1], l.k[1], m1032, m1024, hi.z, lo.z);
+    two(h.h[1], l.h[1], m72, m64, hi.w, lo.w);
+}
+// Q4_K: a * code + b in fp32 (a = d * sc and b = -dmin * m are exact in fp32), rounded once to fp16.
+__device__ __forceinline__ uint32_t pack_half2(float a, float b) {
+    __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&h);
+}
+__device__ __forceinline__ uint4 word_to_half8(uint32_t w, float a, float b) {
+    const Codes8 c = unpack8(w);
+    const float bk = fmaf(-1024.f, a, b), bh = fmaf(-64.f, a, b);  // the unpacked values carry 1024 / 64
+    const float2 f0 = __half22float2(as_half2(c.k[0])), f1 = __half22float2(as_half2(c.h[0]));
+    const float2 f2 = __half22float2(as_half2(c.k[1])), f3 = __half22float2(as_half2(c.h[1]));
+    uint4 o;
+    o.x = pack_half2(fmaf(a, f0.x, bk), fmaf(a, f0.y, bk));
+    o.y = pack_half2(fmaf(a, f1.x, bh), fmaf(a, f1.y, bh));
+    o.z = pack_half2(fmaf(a, f2.x, bk), fmaf(a, f2.y, bk));
+    o.w = pack_half2(fmaf(a, f3.x, bh), fmaf(a, f3.y, bh));
+    return o;
+}
+
+// The same as two fp16: 22 of the fp32 value's 24 bits (it is a multiple of 2^-24, as its fp16 factors are).
+__device__ __forceinline__ void word_to_half8x2(uint32_t w, float a, float b, uint4& hi, uint4& lo) {
+    const Codes8 c = unpack8(w);
+    auto two = [&](uint32_t code, float off, uint32_t& h, uint32_t& l) {  // code - off is exact
+        const float2 f = __half22float2(__hadd2(as_half2(code), __float2half2_rn(off)));
+        const float v0 = fmaf(a, f.x, b), v1 = fmaf(a, f.y, b);
+        const __half2 r = __floats2half2_rn(v0, v1);
+        const float2 back = __half22float2(r);
+        h = as_u32(r);
+        l = pack_half2(v0 - back.x, v1 - back.y);
+    };
+    two(c.k[0], -1024.f, hi.x, lo.x);
+    two(c.h[0], -64.f, hi.y, lo.y);
+    two(c.k[1], -1024.f, hi.z, lo.z);
+    two(c.h[1], -64.f, hi.w, lo.w);
+}
+
+// byte `i` of w times d, exactly: (2^23 + byte) * d - 2^23 * d
+__device__ __forceinline__ float byte_of(uint32_t w, uint32_t sel, float d, float neg_big_d) {
+    return fmaf(__uint_as_float(__byte_perm(w, 0x4B000000u, sel)), d, neg_big_d);
+}
+
+// What a lane holds of 8 + 8 rows x 128 k of a weight tile: for row half h (rows g = lane / 4 and g + 8) the words of
+// its element group (8 q .. 8 q + 7, q = lane & 3) in the four 32-k blocks, and those blocks' scales.  load() reads
+// them straight from global memory (16-byte pieces, the layout is fragment-ordered); pair<SUB>() converts blocks
+// 2 SUB and 2 SUB + 1 to fp16, one 16-byte chunk of the stage's row each, pair2<SUB>() to two fp16 per weight.
+template <int QT> struct DequantRegs;
+
+template <> struct DequantRegs<WF_QTYPE_Q4_0> {
+    uint4 c;
+    uint2 sc;  // fp16 scales of blocks (0, 1), (2, 3)
+    __device__ __forceinline__ void load(const uint8_t* tile, int, int lane, int h) {
+        c = __ldg(reinterpret_cast<const uint4*>(tile + h * 512 + lane * 16));
+        sc = __ldg(reinterpret_cast<const uint2*>(tile + Tile<WF_QTYPE_Q4_0>::SCALE_OFF + (lane >> 2) * 16 + h * 8));
+    }
+    template <int SUB> __device__ __forceinline__ void pair(uint4& o0, uint4& o1) const {
+        const uint32_t w0 = SUB ? c.z : c.x, w1 = SUB ? c.w : c.y, s = SUB ? sc.y : sc.x;
+        const __half2 sx = as_half2(__byte_perm(s, s, 0x1010u)), sy = as_half2(__byte_perm(s, s, 0x3232u));
+        o0 = word_to_half8_q4_0(w0, sx);
+        o1 = word_to_half8_q4_0(w1, sy);
+    }
+    template <int SUB> __device__ __forceinline__ void pair2(uint4& h0, uint4& h1, uint4& l0, uint4& l1) const {
+        const uint32_t w0 = SUB ? c.z : c.x, w1 = SUB ? c.w : c.y, s = SUB ? sc.y : sc.x;
+        const __half2 sx = as_half2(__byte_perm(s, s, 0x1010u)), sy = as_half2(__byte_perm(s, s, 0x3232u));
+        word_to_half8x2_q4_0(w0, sx, h0, l0);
+        word_to_half8x2_q4_0(w1, sy, h1, l1);
+    }
+};
+
+template <> struct DequantRegs<WF_QTYPE_Q4_1> {
+    uint4 c;
+    uint2 sc, mn;
+    __device__ __forceinline__ void load(const uint8_t* tile, int, int lane, int h) {
+        using T = Tile<WF_QTYPE_Q4_1>;
+        c = __ldg(reinterpret_cast<const uint4*>(tile + h * 512 + lane * 16));
+        sc = __ldg(reinterpret_cast<const uint2*>(tile + T::SCALE_OFF + (lane >> 2) * 16 + h * 8));
+        mn = __ldg(reinterpret_cast<const uint2*>(tile + T::MIN_OFF + (lane >> 2) * 16 + h * 8));
+    }
+    template <int SUB> __device__ __forceinline__ void pair(uint4& o0, uint4& o1) const {  // scale * code + min in fp32, rounded once
+        const uint32_t w0 = SUB ? c.z : c.x, w1 = SUB ? c.w : c.y;
+        const float2 s = __half22float2(as_half2(SUB ? sc.y : sc.x));
+        const float2 m = __half22float2(as_half2(SUB ? mn.y : mn.x));
+        o0 = word_to_half8(w0, s.x, m.x);
+        o1 = word_to_half8(w1, s.y, m.y);
+    }
+    template <int SUB> __device__ __forceinline__ void pair2(uint4& h0, uint4& h1, uint4& l0, uint4& l1) const {
+        const uint32_t w0 = SUB ? c.z : c.x, w1 = SUB ? c.w : c.y;
+        const float2 s = __half22float2(as_half2(SUB ? sc.y : sc.x));
+        const float2 m = __half22float2(as_half2(SUB ? mn.y : mn.x));
+        word_to_half8x2(w0, s.x, m.x, h0, l0);
+        word_to_half8x2(w1, s.y, m.y, h1, l1);
+    }
+};
+
+template <> struct DequantRegs<WF_QTYPE_Q8_0> {
+    uint4 ch, cl;
+    uint2 sc;
+    __device__ __forceinline__ void load(const uint8_t* tile, int, int lane, int h) {
+        ch = __ldg(reinterpret_cast<const uint4*>(tile + h * 512 + lane * 16));
+        cl = __ldg(reinterpret_cast<const uint4*>(tile + PLANE_BYTES + h * 512 + lane * 16));
+        sc = __ldg(reinterpret_cast<const uint2*>(tile + Tile<WF_QTYPE_Q8_0>::SCALE_OFF + (lane >> 2) * 16 + h * 8));
+    }
+    template <int SUB> __device__ __forceinline__ void pair(uint4& o0, uint4& o1) const {
+        const uint32_t h0 = SUB ? ch.z : ch.x, h1 = SUB ? ch.w : ch.y, l0 = SUB ? cl.z : cl.x, l1 = SUB ? cl.w : cl.y, s = SUB ? sc.y : sc.x;
+        const __half2 sx = as_half2(__byte_perm(s, s, 0x1010u)), sy = as_half2(__byte_perm(s, s, 0x3232u));
+        o0 = words_to_half8_q8(h0, l0, sx);
+        o1 = words_to_half8_q8(h1, l1, sy);
+    }
+    template <int SUB> __device__ __forceinline__ void pair2(uint4& r0, uint4& r1, uint4& e0, uint4& e1) const {
+        const uint32_t h0 = SUB ? ch.z : ch.x, h1 = SUB ? ch.w : ch.y, l0 = SUB ? cl.z : cl.x, l1 = SUB ? cl.w : cl.y, s = SUB ? sc.y : sc.x;
+        const __half2 sx = as_half2(__byte_perm(s, s, 0x1010u)), sy = as_half2(__byte_perm(s, s, 0x3232u));
+        words_to_half8x2_q8(h0, l0, sx, r0, e0);
+        words_to_half8x2_q8(h1, l1, sy, r1, e1);
+    }
+};
+
+template <> struct DequantRegs<WF_QTYPE_Q4_K> {  // one half (plane kb & 1) of a 256-k tile
+    uint4 c;
+    uint32_t dd, scw, mnw;  // (d, dmin); 8-bit scales / mins of the half's four sub-blocks
+    __device__ __forceinline__ void load(const uint8_t* tile, int plane, int lane, int h) {
+        using T = Tile<WF_QTYPE_Q4_K>;
+        const int g = lane >> 2;
+        c = __ldg(reinterpret_cast<const uint4*>(tile + plane * PLANE_BYTES + h * 512 + lane * 16));
+        dd = __ldg(reinterpret_cast<const uint32_t*>(tile + T::D_OFF + g * 8 + h * 4));
+        scw = __ldg(reinterpret_cast<const uint32_t*>(tile + T::SC_OFF + g * 16 + h * 8 + plane * 4));
+        mnw = __ldg(reinterpret_cast<const uint32_t*>(tile + T::MN_OFF + g * 16 + h * 8 + plane * 4));
+    }
+    template <int SUB> __device__ __forceinline__ void pair(uint4& o0, uint4& o1) const {  // (d * sc) * code - dmin * m
+        const float2 d = __half22float2(as_half2(dd));
+        const float nd = -8388608.f * d.x, nm = 8388608.f * d.y;
+        const uint32_t w0 = SUB ? c.z : c.x, w1 = SUB ? c.w : c.y;
+        const uint32_t first = 0x7540u + 2 * SUB, second = first + 1;
+        o0 = word_to_half8(w0, byte_of(scw, first, d.x, nd), byte_of(mnw, first, -d.y, nm));
+        o1 = word_to_half8(w1, byte_of(scw, second, d.x, nd), byte_of(mnw, second, -d.y, nm));
+    }
+    template <int SUB> __device__ __forceinline__ void pair2(uint4& h0, uint4& h1, uint4& l0, uint4& l1) const {
+        const float2 d = __half22float2(as_half2(dd));
+        const float nd = -8388608.f * d.x, nm = 8388608.f * d.y;
+        const uint32_t w0 = SUB ? c.z : c.x, w1 = SUB ? c.w : c.y;
+        const uint32_t first = 0x7540u + 2 * SUB, second = first + 1;
+        word_to_half8x2(w0, byte_of(scw, first, d.x, nd), byte_of(mnw, first, -d.y, nm), h0, l0);
+        word_to_half8x2(w1, byte_of(scw, second, d.x, nd), byte_of(mnw, second, -d.y, nm), h1, l1);
+    }
+};
+
+}  // namespace wf

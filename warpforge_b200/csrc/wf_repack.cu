@@ -15,11 +15,18 @@ __device__ __forceinline__ uint32_t pack8(const uint32_t (&nib)[8]) {
     return (w << PLANE_ROT) | (w >> (32 - PLANE_ROT));
 }
 
+// Raises *beyond when a block may hold values that fp16 cannot (bound = the largest magnitude its scales allow; an Inf or
+// NaN scale counts).  Almost never, so it costs a comparison per block.
+__device__ __forceinline__ void note_range(float bound, volatile int* beyond) {
+    if (!(bound < 65504.f)) *beyond = 1;
+}
+__device__ __forceinline__ float abs_half(uint16_t h) { return fabsf(__half2float(__ushort_as_half(h))); }
+
 __device__ __forceinline__ uint16_t ld_u16(const uint8_t* p) { return (uint16_t)(p[0] | (p[1] << 8)); }
 
 // One thread per (row, 32-k block, element group q).
 __global__ void repack_q4_0_kernel(const uint8_t* __restrict__ raw, uint8_t* __restrict__ tiles, int64_t rows,
-                                   int64_t nblk, int64_t kt, int ggml_order) {
+                                   int64_t nblk, int64_t kt, int ggml_order, volatile int* beyond) {
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= rows * nblk * 4) return;
     int q = idx & 3;
@@ -43,14 +50,16 @@ __global__ void repack_q4_0_kernel(const uint8_t* __restrict__ raw, uint8_t* __r
         }
     }
     *reinterpret_cast<uint32_t*>(tile + plane_word_off(ri, j, q)) = pack8(nib);
-    if (q == 0)
-        *reinterpret_cast<uint16_t*>(tile + Tile<WF_QTYPE_Q4_0>::SCALE_OFF + (ri & 7) * 16 + (ri >> 3) * 8 + j * 2) =
-            ld_u16(src);
+    if (q == 0) {
+        const uint16_t sc = ld_u16(src);
+        *reinterpret_cast<uint16_t*>(tile + Tile<WF_QTYPE_Q4_0>::SCALE_OFF + (ri & 7) * 16 + (ri >> 3) * 8 + j * 2) = sc;
+        note_range(8.f * abs_half(sc), beyond);
+    }
 }
 
 // Q4_1 (Dequantizer.java:304-358): fp16 scale, fp16 min, 16 code bytes in the same two nibble orders.
 __global__ void repack_q4_1_kernel(const uint8_t* __restrict__ raw, uint8_t* __restrict__ tiles, int64_t rows,
-                                   int64_t nblk, int64_t kt, int ggml_order) {
+                                   int64_t nblk, int64_t kt, int ggml_order, volatile int* beyond) {
     using T = Tile<WF_QTYPE_Q4_1>;
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= rows * nblk * 4) return;
@@ -79,11 +88,12 @@ __global__ void repack_q4_1_kernel(const uint8_t* __restrict__ raw, uint8_t* __r
         const int so = (ri & 7) * 16 + (ri >> 3) * 8 + j * 2;
         *reinterpret_cast<uint16_t*>(tile + T::SCALE_OFF + so) = ld_u16(src);
         *reinterpret_cast<uint16_t*>(tile + T::MIN_OFF + so) = ld_u16(src + 2);
+        note_range(15.f * abs_half(ld_u16(src)) + abs_half(ld_u16(src + 2)), beyond);
     }
 }
 
 __global__ void repack_q8_0_kernel(const uint8_t* __restrict__ raw, uint8_t* __restrict__ tiles, int64_t rows,
-                                   int64_t nblk, int64_t kt) {
+                                   int64_t nblk, int64_t kt, volatile int* beyond) {
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= rows * nblk * 4) return;
     int q = idx & 3;
@@ -101,16 +111,18 @@ __global__ void repack_q8_0_kernel(const uint8_t* __restrict__ raw, uint8_t* __r
     int off = plane_word_off(ri, j, q);
     *reinterpret_cast<uint32_t*>(tile + off) = pack8(hi);
     *reinterpret_cast<uint32_t*>(tile + PLANE_BYTES + off) = pack8(lo);
-    if (q == 0)
-        *reinterpret_cast<uint16_t*>(tile + Tile<WF_QTYPE_Q8_0>::SCALE_OFF + (ri & 7) * 16 + (ri >> 3) * 8 + j * 2) =
-            ld_u16(src);
+    if (q == 0) {
+        const uint16_t sc = ld_u16(src);
+        *reinterpret_cast<uint16_t*>(tile + Tile<WF_QTYPE_Q8_0>::SCALE_OFF + (ri & 7) * 16 + (ri >> 3) * 8 + j * 2) = sc;
+        note_range(128.f * abs_half(sc), beyond);
+    }
 }
 
 // Q5_0 (22 bytes: fp16 scale, 32 high bits, 16 nibble bytes; element i < 16 = low nibble of byte i, element
 // i + 16 = high nibble of byte i) into Q8_0 tiles: q = (nibble | bit << 4) - 16 is stored as the 8-bit integer
 // the Q8_0 kernels expect (nibbles of q ^ 0x80), with the block's own fp16 scale.
 __global__ void repack_q5_0_kernel(const uint8_t* __restrict__ raw, uint8_t* __restrict__ tiles, int64_t rows,
-                                   int64_t nblk, int64_t kt) {
+                                   int64_t nblk, int64_t kt, volatile int* beyond) {
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= rows * nblk * 4) return;
     int q = idx & 3;
@@ -133,9 +145,11 @@ __global__ void repack_q5_0_kernel(const uint8_t* __restrict__ raw, uint8_t* __r
     int off = plane_word_off(ri, j, q);
     *reinterpret_cast<uint32_t*>(tile + off) = pack8(hi);
     *reinterpret_cast<uint32_t*>(tile + PLANE_BYTES + off) = pack8(lo);
-    if (q == 0)
-        *reinterpret_cast<uint16_t*>(tile + Tile<WF_QTYPE_Q8_0>::SCALE_OFF + (ri & 7) * 16 + (ri >> 3) * 8 + j * 2) =
-            ld_u16(src);
+    if (q == 0) {
+        const uint16_t sc = ld_u16(src);
+        *reinterpret_cast<uint16_t*>(tile + Tile<WF_QTYPE_Q8_0>::SCALE_OFF + (ri & 7) * 16 + (ri >> 3) * 8 + j * 2) = sc;
+        note_range(16.f * abs_half(sc), beyond);
+    }
 }
 
 __device__ __forceinline__ void q4k_scale_min(const uint8_t* s, int j, uint32_t& sc, uint32_t& m) {
@@ -150,7 +164,7 @@ __device__ __forceinline__ void q4k_scale_min(const uint8_t* s, int j, uint32_t&
 
 // One thread per (row, super-block, sub-block jj, element group q).
 __global__ void repack_q4_k_kernel(const uint8_t* __restrict__ raw, uint8_t* __restrict__ tiles, int64_t rows,
-                                   int64_t nsb) {
+                                   int64_t nsb, volatile int* beyond) {
     using T = Tile<WF_QTYPE_Q4_K>;
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= rows * nsb * 32) return;
@@ -177,27 +191,28 @@ __global__ void repack_q4_k_kernel(const uint8_t* __restrict__ raw, uint8_t* __r
             uint16_t* dd = reinterpret_cast<uint16_t*>(tile + T::D_OFF + (ri & 7) * 8 + (ri >> 3) * 4);
             dd[0] = ld_u16(src);
             dd[1] = ld_u16(src + 2);
+            note_range(15.f * 63.f * abs_half(dd[0]) + 63.f * abs_half(dd[1]), beyond);
         }
     }
 }
 
 cudaError_t launch_repack(int qtype, const uint8_t* d_raw, uint8_t* d_tiles, int64_t rows, int64_t k,
-                          int q4_0_order, cudaStream_t s) {
+                          int q4_0_order, int* beyond, cudaStream_t s) {
     const int threads = 256;
     if (qtype == WF_QTYPE_Q4_K) {
         int64_t nsb = k / 256, n = rows * nsb * 32;
-        repack_q4_k_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, s>>>(d_raw, d_tiles, rows, nsb);
+        repack_q4_k_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, s>>>(d_raw, d_tiles, rows, nsb, beyond);
     } else {
         int64_t nblk = k / 32, n = rows * nblk * 4, kt = (k + 127) / 128;
         unsigned grid = (unsigned)((n + threads - 1) / threads);
         if (qtype == WF_QTYPE_Q4_0)
-            repack_q4_0_kernel<<<grid, threads, 0, s>>>(d_raw, d_tiles, rows, nblk, kt, q4_0_order == WF_Q4_0_ORDER_GGML);
+            repack_q4_0_kernel<<<grid, threads, 0, s>>>(d_raw, d_tiles, rows, nblk, kt, q4_0_order == WF_Q4_0_ORDER_GGML, beyond);
         else if (qtype == WF_QTYPE_Q4_1)
-            repack_q4_1_kernel<<<grid, threads, 0, s>>>(d_raw, d_tiles, rows, nblk, kt, q4_0_order == WF_Q4_0_ORDER_GGML);
+            repack_q4_1_kernel<<<grid, threads, 0, s>>>(d_raw, d_tiles, rows, nblk, kt, q4_0_order == WF_Q4_0_ORDER_GGML, beyond);
         else if (qtype == WF_QTYPE_Q5_0)
-            repack_q5_0_kernel<<<grid, threads, 0, s>>>(d_raw, d_tiles, rows, nblk, kt);
+            repack_q5_0_kernel<<<grid, threads, 0, s>>>(d_raw, d_tiles, rows, nblk, kt, beyond);
         else
-            repack_q8_0_kernel<<<grid, threads, 0, s>>>(d_raw, d_tiles, rows, nblk, kt);
+            repack_q8_0_kernel<<<grid, threads, 0, s>>>(d_raw, d_tiles, rows, nblk, kt, beyond);
     }
     return cudaGetLastError();
 }

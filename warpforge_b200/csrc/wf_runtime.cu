@@ -53,6 +53,16 @@ Weight* get_weight(Context* c, int64_t h) {
     return w;
 }
 
+void free_scratch(GemvScratch& sc) {
+    cudaFree(sc.d_slots);
+    cudaFree(sc.d_part);
+    cudaFree(sc.d_count);
+    cudaFree(sc.d_x16);
+    cudaFree(sc.d_gemm_partial);
+    cudaFree(sc.d_gemm_ready);
+    sc = GemvScratch{};
+}
+
 cudaStream_t resolve_stream(Context* c, int64_t stream) {
     return stream == 0 ? c->stream : reinterpret_cast<cudaStream_t>(stream);
 }
@@ -248,7 +258,7 @@ static cudaError_t upload_and_repack(Context* c, int qtype, const uint8_t* src, 
         if (e == cudaSuccess) e = cudaMemcpyAsync(d, h, (size_t)n, cudaMemcpyHostToDevice, c->upload_stream);
         if (e == cudaSuccess) e = cudaEventRecord(c->upload_done[i % UPLOAD_RING], c->upload_stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(s, c->upload_done[i % UPLOAD_RING], 0);
-        if (e == cudaSuccess) e = launch_repack(qtype, d, *d_tiles + r0 / TILE_ROWS * tile_row_bytes, n / row_bytes, k, q4_0_order, s);
+        if (e == cudaSuccess) e = launch_repack(qtype, d, *d_tiles + r0 / TILE_ROWS * tile_row_bytes, n / row_bytes, k, q4_0_order, c->beyond_dev, s);
         if (e == cudaSuccess) e = cudaEventRecord(c->upload_repacked[i % UPLOAD_RING], s);
     }
     stop.store(e != cudaSuccess);
@@ -311,7 +321,7 @@ int wf_init(int device, int64_t* ctx) {
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     StatusBlock block{0, 0, nullptr};
-    if (e == cudaSuccess) e = cudaHostAlloc((void**)&c->h_status, STATUS_BITS * sizeof(int), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostAlloc((void**)&c->h_status, (STATUS_BITS + 1) * sizeof(int), cudaHostAllocMapped);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&block.host, (void*)c->h_status, 0);
     if (e == cudaSuccess) e = cudaMalloc(&c->d_status, sizeof block);
     if (e == cudaSuccess) e = cudaMemcpy(c->d_status, &block, sizeof block, cudaMemcpyHostToDevice);
@@ -322,7 +332,8 @@ int wf_init(int device, int64_t* ctx) {
         delete c;
         return WF_ERR_CUDA_BASE + (int)e;
     }
-    for (int b = 0; b < STATUS_BITS; b++) c->h_status[b] = 0;
+    for (int b = 0; b <= STATUS_BITS; b++) c->h_status[b] = 0;
+    c->beyond_dev = block.host + STATUS_BITS;
     {
         std::lock_guard<std::mutex> lk(g_registry_mu);
         g_contexts.insert(c);
@@ -349,11 +360,7 @@ int wf_destroy(int64_t ctx) {
     release_spare_tiles(c);
     for (auto& kv : c->allocs) cudaFree(reinterpret_cast<void*>(kv.first));
     for (void* h : c->host_allocs) cudaFreeHost(h);
-    for (auto& kv : c->gemv_scratch) {
-        cudaFree(kv.second.d_slots);
-        cudaFree(kv.second.d_part);
-        cudaFree(kv.second.d_count);
-    }
+    for (auto& kv : c->gemv_scratch) free_scratch(kv.second);
     for (cudaGraphExec_t g : c->graphs) cudaGraphExecDestroy(g);
     for (cudaEvent_t ev : c->events) cudaEventDestroy(ev);
     for (cudaStream_t s : c->streams) cudaStreamDestroy(s);
@@ -366,9 +373,6 @@ int wf_destroy(int64_t ctx) {
         if (e) cudaEventDestroy(e);
     if (c->upload_stream) cudaStreamDestroy(c->upload_stream);
     if (c->d_stage) cudaFree(c->d_stage);
-    if (c->d_x16) cudaFree(c->d_x16);
-    if (c->d_gemm_partial) cudaFree(c->d_gemm_partial);
-    if (c->d_gemm_ready) cudaFree(c->d_gemm_ready);
     cudaFree(c->d_status);
     cudaFreeHost((void*)c->h_status);
     if (c->d_timing) cudaFree(c->d_timing);
@@ -409,9 +413,7 @@ int wf_stream_destroy(int64_t ctx, int64_t stream) {
     WF_CUDA(c, cudaStreamSynchronize(s));
     auto sc = c->gemv_scratch.find(s);
     if (sc != c->gemv_scratch.end()) {
-        cudaFree(sc->second.d_slots);
-        cudaFree(sc->second.d_part);
-        cudaFree(sc->second.d_count);
+        free_scratch(sc->second);
         c->gemv_scratch.erase(sc);
     }
     c->streams.erase(it);
@@ -557,6 +559,7 @@ int weight_upload(Context* c, int qtype, const void* blocks, int64_t n_rows, int
     w->g.rt_alloc = (w->g.rt + 7) / 8 * 8;
     w->row0 = row0;
     w->total_rows = n_rows;
+    c->h_status[STATUS_BITS] = 0;
     cudaError_t e = upload_and_repack(c, qtype, static_cast<const uint8_t*>(blocks) + row0 * row_bytes, rows, k, row_bytes, &w->d_tiles,
                                       &w->tiles_held, w->g.bytes(), w->g.kt * (int64_t)tile_bytes(w->g.qtype), q4_0_order, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -565,6 +568,7 @@ int weight_upload(Context* c, int qtype, const void* blocks, int64_t n_rows, int
         delete w;
         return cuda_status(c, e, "weight upload");
     }
+    w->beyond_fp16 = c->h_status[STATUS_BITS] != 0;
     c->launches++;
     c->weights.push_back(w);
     *weight = reinterpret_cast<int64_t>(w);
@@ -657,7 +661,9 @@ int wf_qlinear(int64_t ctx, int64_t weight, const void* x, int x_dtype, int x_on
     }
     GemvCall call{w, d_x, x_dtype, m, d_y, w->g.rows, 0};
     // many tokens: tensor-core GEMM; a few tokens: the HBM-bound GEMV
-    int rc = gemm_supported(*w, x_dtype, m, call.d_x) ? gemm_launch(c, call, s) : gemv_launch(c, call, s);
+    const bool gemm = gemm_supported(*w, x_dtype, m, call.d_x);
+    int rc = gemm ? gemm_launch(c, call, s) : gemv_launch(c, call, s);
+    if (gemm && rc == WF_ERR_RECORDING && x_dtype == WF_DTYPE_F32) rc = gemv_launch(c, call, s);  // takes fp32 tokens without more scratch
     if (rc != WF_OK) return rc;
     if (!y_on_device) {
         if (!y_direct) WF_CUDA(c, cudaMemcpyAsync(static_cast<uint8_t*>(c->h_stage) + yo, d_y, (size_t)yb, cudaMemcpyDeviceToHost, s));
@@ -690,6 +696,7 @@ int wf_graph_begin(int64_t ctx, int64_t stream) {
     WF_ENTER(ctx);
     cudaStream_t s = resolve_stream(c, stream);
     int rc = gemv_prepare_stream(c, s);  // no allocation may happen while recording
+    if (rc == WF_OK) rc = gemm_prepare_stream(c, s);
     if (rc != WF_OK) return rc;
     c->capture_launches = c->launches;
     WF_CUDA(c, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));

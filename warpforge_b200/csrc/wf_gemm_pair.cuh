@@ -151,13 +151,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
         // ------------------------------------------------ TMA producer: this CTA's tokens
         if (lane == 0) {
             asm volatile("griddepcontrol.wait;" ::: "memory");  // the fp16 activations
-            int it = 0;
+            StageCursor at;
             for (int u = u0; u < u1 && !*abort_flag;) {
                 const GemmSegment g = segment_at(p, u, u1);
                 const int mt = g.tile % p.m_tiles, nh = halves_of(mt);
-                for (int kb = 2 * g.kb0; kb < 2 * g.kb1; kb++, it++) {  // in stages
-                    const int s = it % stages;
-                    if (it >= stages && !g_mbar_wait(&s_empty[s], ((it / stages) - 1) & 1)) { fail(); break; }
+                for (int kb = 2 * g.kb0; kb < 2 * g.kb1; kb++, at.advance(stages)) {  // in stages
+                    const int s = at.s;
+                    if (!g_mbar_wait(&s_empty[s], at.phase ^ 1)) { fail(); break; }
                     uint8_t* b_stage = stage0 + (size_t)s * stage_bytes + PAIR_A_BYTES;
                     uint64_t* bar = leader ? &full[s] : &b_full[s];
                     g_mbar_expect_tx(bar, (uint32_t)nh * PAIR_B_HALF);
@@ -173,14 +173,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
             // ------------------------------------------------ MMA issuer of the pair (the whole warp walks the loop)
             const uint32_t issue = elect_one();
             const uint64_t a_desc0 = smem_desc_sw128(g_smem_u32(stage0)), b_desc0 = smem_desc_sw128(g_smem_u32(stage0) + PAIR_A_BYTES);
-            int s = 0, used[2] = {0, 0};
-            uint32_t phase = 0;
+            StageCursor at;
+            int used[2] = {0, 0};
             for (int u = u0; u < u1 && !*abort_flag;) {
                 const GemmSegment g = segment_at(p, u, u1);
                 const int nh = halves_of(g.tile % p.m_tiles);
                 bool ok = true;
                 for (int kb = 2 * g.kb0; kb < 2 * g.kb1 && ok; kb++) {
-                    if (!g_mbar_wait(&full[s], phase)) { fail(); ok = false; break; }
+                    const int s = at.s;
+                    if (!g_mbar_wait(&full[s], at.phase)) { fail(); ok = false; break; }
                     tc_fence_after();
                     const uint64_t off = (uint64_t)((uint32_t)s * stage_bytes >> 4);
                     for (int h = 0; h < nh; h++) {
@@ -197,10 +198,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
                     }
                     if (!ok) break;
                     if (issue) tc_commit_pair(&s_empty[s]);
-                    if (++s == stages) {
-                        s = 0;
-                        phase ^= 1;
-                    }
+                    at.advance(stages);
                 }
                 if (!ok) break;
                 if (issue && g.kb0 == 0 && g.kb1 < p.k_blocks) tc_commit_pair(tail_full);
@@ -209,10 +207,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
         } else if (lane == 0) {
             // ------------------------------------------------ rank 1: pass the word on that its TMA data has landed
             const int n = 2 * (u1 - u0);
-            for (int it = 0; it < n && !*abort_flag; it++) {
-                const int s = it % stages;
-                if (!g_mbar_wait(&b_full[s], (it / stages) & 1)) { fail(); break; }
-                mbar_arrive_cluster(map_to_rank(g_smem_u32(&full[s]), 0));
+            StageCursor at;
+            for (int it = 0; it < n && !*abort_flag; it++, at.advance(stages)) {
+                if (!g_mbar_wait(&b_full[at.s], at.phase)) { fail(); break; }
+                mbar_arrive_cluster(map_to_rank(g_smem_u32(&full[at.s]), 0));
             }
         }
     } else if (warp >= 4 && warp < 8) {
@@ -267,14 +265,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
 #pragma unroll
         for (int j = 0; j < 2; j++) a_off[j] = (uint32_t)((stage_chunk(j, dq4) ^ dg) << 4);
         // convert first, wait for the stage then, so that only the stores lie between "released" and "full"
-        int it = 0;
+        StageCursor at;
         auto finish_step = [&](const auto& regs, auto sub) {
-            const int s = it % stages;
+            const int s = at.s;
             uint4 out[2][2];
 #pragma unroll
             for (int hh = 0; hh < 2; hh++) regs[hh].template pair<decltype(sub)::value>(out[hh][0], out[hh][1]);
-            if (it == stages) asm volatile("griddepcontrol.wait;" ::: "memory");
-            if (it >= stages && !g_mbar_wait(&s_empty[s], ((it / stages) - 1) & 1)) {
+            if (!g_mbar_wait(&s_empty[s], at.phase ^ 1)) {
                 if (lane == 0) fail();
                 return false;
             }
@@ -286,7 +283,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> visible to the tensor core
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(full0 + (uint32_t)s * 8);
-            it++;
+            if (at.advance(stages)) asm volatile("griddepcontrol.wait;" ::: "memory");  // no bounded wait under earlier kernels
             return true;
         };
         constexpr int DEPTH = 3;  // register sets in turn, 128 k each

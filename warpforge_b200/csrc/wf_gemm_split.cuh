@@ -103,12 +103,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
         // ------------------------------------------------ TMA producer (activations)
         if (lane == 0) {
             asm volatile("griddepcontrol.wait;" ::: "memory");  // the fp16 activations
-            int it = 0;
+            StageCursor at;
             for (int tile = cluster; tile < tiles && !*abort_flag; tile += clusters) {
                 const int tok0 = (tile % p.m_tiles) * p.bm;
-                for (int st = 2 * kb0; st < 2 * kb1; st++, it++) {
-                    const int s = it % stages;
-                    if (it >= stages && !g_mbar_wait(&s_empty[s], ((it / stages) - 1) & 1)) { fail(); break; }
+                for (int st = 2 * kb0; st < 2 * kb1; st++, at.advance(stages)) {
+                    const int s = at.s;
+                    if (!g_mbar_wait(&s_empty[s], at.phase ^ 1)) { fail(); break; }
                     uint8_t* b_stage = stage0 + (size_t)s * stage_bytes + A_BYTES;
                     g_mbar_expect_tx(&b_full[s], PLANES * span_bytes);
 #pragma unroll
@@ -122,8 +122,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
         const uint32_t issue = elect_one();
         const uint64_t a_desc0 = smem_desc_sw128(g_smem_u32(stage0)), b_desc0 = smem_desc_sw128(g_smem_u32(stage0) + A_BYTES);
         const uint64_t span = span_bytes >> 4;
-        int s = 0, local = 0;
-        uint32_t phase = 0;
+        StageCursor at;
+        int local = 0;
         bool ok = true;
         for (int tile = cluster; tile < tiles && ok && !*abort_flag; tile += clusters) {
             for (int g0 = kb0; g0 < kb1 && ok; local++) {  // groups of units that share an accumulator
@@ -132,7 +132,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(buf * ACCS * p.bm), e_tmem = d_tmem + (uint32_t)p.bm;
                 for (int st = 2 * g0; st < 2 * g1; st++) {
-                    if (!g_mbar_wait(&b_full[s], phase) || !g_mbar_wait(&a_full[s], phase)) { fail(); ok = false; break; }
+                    const int s = at.s;
+                    if (!g_mbar_wait(&b_full[s], at.phase) || !g_mbar_wait(&a_full[s], at.phase)) { fail(); ok = false; break; }
                     tc_fence_after();
                     const uint64_t off = (uint64_t)((uint32_t)s * stage_bytes >> 4);
                     const uint64_t ad = a_desc0 + off, bd = b_desc0 + off;
@@ -146,10 +147,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
                         tc_mma_span<1>(e_tmem, ad, bd + 2 * span, p.idesc, 1u, issue);
                     }
                     if (issue) tc_commit(&s_empty[s]);  // frees the stage when these MMAs have read it
-                    if (++s == stages) {
-                        s = 0;
-                        phase ^= 1;
-                    }
+                    at.advance(stages);
                 }
                 if (ok && issue) tc_commit(&acc_full[buf]);
                 g0 = g1;
@@ -243,17 +241,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
         // One step: convert registers loaded earlier into fp16 rows (still in registers), wait for the stage, store them and
         // hand the stage over.  Converting before the wait keeps the arithmetic off the path between "the MMAs have
         // released the stage" and "the stage is full again".  (Both stages of a unit in one step: 7 - 14 % slower.)
-        int it = 0;
+        StageCursor at;
         auto finish_step = [&](const DequantRegs<QT> (&regs)[2], auto sub) {
-            const int s = it % stages;
+            const int s = at.s;
             uint4 out[2][2 * PIECES];
 #pragma unroll
             for (int hh = 0; hh < 2; hh++) {
                 if constexpr (PIECES == 1) regs[hh].template pair<decltype(sub)::value>(out[hh][0], out[hh][1]);
                 else regs[hh].template pair2<decltype(sub)::value>(out[hh][0], out[hh][1], out[hh][2], out[hh][3]);
             }
-            if (it == stages) asm volatile("griddepcontrol.wait;" ::: "memory");
-            if (it >= stages && !g_mbar_wait(&s_empty[s], ((it / stages) - 1) & 1)) {
+            if (!g_mbar_wait(&s_empty[s], at.phase ^ 1)) {
                 if (lane == 0) fail();
                 return false;
             }
@@ -266,7 +263,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> visible to the tensor core
             __syncwarp();
             if (lane == 0) g_mbar_arrive(&a_full[s]);
-            it++;
+            if (at.advance(stages)) asm volatile("griddepcontrol.wait;" ::: "memory");  // no bounded wait under earlier kernels
             return true;
         };
         // DEPTH register sets in turn (128 k each): the loads of the following DEPTH - 1 units are in flight while one is

@@ -106,17 +106,31 @@ static cudaError_t gemm_launch_one(Kernel kernel, const GemmParams& p, const CUt
     return cudaLaunchKernelEx(&cfg, kernel, p, map);
 }
 
-// CTAs per tile of the split kernel: the number of units the busiest CTA walks (rounds of tiles x its share of K), the
-// parts put together at the end (about three units' worth) and a little for every further round.
-static int split_ranks(const GemmDevice& d, int64_t tiles, int k_blocks, int* clusters) {
+// What a call costs in us by either kernel, fitted to measurements on one B200 (weights from HBM, calls back to back): 6 - 8 us
+// of conversion, launch and start; a cost per unit of 128 k on the busiest CTA or pair; the parts put together.
+//   us by the fit / measured: split, bf16, [4096 x 4096]: 33 tokens (4 ranks) 13 / 12.4, 100 tokens 15 / 15.6; [11008 x 4096],
+//   128 tokens (3 ranks) 30 / 28; [16000 x 1024], 400 tokens: 1 rank 31 / 30, 2 ranks 53 / 64.
+//   pair: [4096 x 4096] 256 tokens 24 / 23, 512 tokens 33 / 35; [11008 x 4096] 256 tokens 34 / 32, 300 tokens 49 / 46.
+static double split_cost(int64_t rounds, int units, int ranks, int bm, bool f32) {
+    const double b = bm / 128.0, unit = f32 ? 0.95 + 0.9 * b : 0.6 + 0.12 * b;
+    const double together = ranks == 1 ? 0.5 + 0.5 * b : (f32 ? 0.5 + 4.0 * b : 1.0 + 3.0 * b);
+    return 6.0 + (double)rounds * (units * unit + together);
+}
+static double pair_cost(int64_t units, int64_t m) {
+    const double half = m <= 256 ? 1.0 : 1.5;  // a token tile of one or two halves
+    return 8.0 + (double)units * half + (m <= 256 ? 8.0 : 13.0);
+}
+
+// CTAs per tile of the split kernel, the cheapest by split_cost.
+static int split_ranks(const GemmDevice& d, int64_t tiles, int k_blocks, int bm, bool f32, int* clusters, double* cost) {
     int best = 1;
-    double best_cost = 1e30;
+    *cost = 1e30;
     for (int n = 1; n <= SPLIT_MAX_RANKS && n <= k_blocks; n++) {
         if (d.clusters[n] < 1) continue;
         const int64_t rounds = (tiles + d.clusters[n] - 1) / d.clusters[n];
-        const double cost = (double)rounds * ((k_blocks + n - 1) / n) + (n > 1 ? 3.0 : 1.5) + 0.5 * (double)(rounds - 1);
-        if (cost < best_cost - 1e-9) {
-            best_cost = cost;
+        const double t = split_cost(rounds, (k_blocks + n - 1) / n, n, bm, f32);
+        if (t < *cost) {
+            *cost = t;
             best = n;
         }
     }
@@ -183,44 +197,42 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     p.m = (int)call.m;
     p.k_blocks = (int)((w.g.k + GEMM_BK - 1) / GEMM_BK);
 
-    // Pairs of CTAs on 256 x 512 tiles for more tokens than one tile of the other kernel takes, clusters on 128 x 128 tiles
-    // up to there, where there are few of the large tiles (a dozen: below it stream-K leaves pairs idle), and for fp32 tokens.
-    // us, pair / split: [11008 x 4096] 128 tokens 30 / 33, 250 tokens 33 / 54; [4096 x 4096] 250 24 / 27, 512 34 / 34.5,
-    // 2048 75 / 122; [1024 x 8192] 2048 (16 tiles) 58 / 77; [600 x 1024] 1500 (9 tiles) 24 / 20; [128 x 8192] 2048 49 / 27.
-    const int64_t pair_tiles = ((w.g.rows + 2 * GEMM_BN - 1) / (2 * GEMM_BN)) * ((call.m + PAIR_TOKENS - 1) / PAIR_TOKENS);
-    const bool pair = !f32 && call.m > SPLIT_MAX_TOKENS && dev->pairs > 0 && pair_tiles >= 12;
-    int grid, cluster;
+    int grid, cluster, clusters = 0;
     size_t stage_bytes, exchange = 0;
+    // Clusters on tiles of 128 rows x up to 128 tokens.  Token tiles are of one size, in steps of 32 where there are several (the
+    // epilogue works on 32 tokens at a time and must not reach into a neighbour); fp32: 96, so that two stages and the
+    // exchange buffer fit.
+    const int most = f32 ? 96 : SPLIT_MAX_TOKENS;
+    const int64_t token_tiles = (call.m + most - 1) / most, grain = token_tiles > 1 ? 32 : 16;
+    p.bm = (int)(((call.m + token_tiles - 1) / token_tiles + grain - 1) / grain * grain);
+    p.n_tiles = (int)((w.g.rows + GEMM_BN - 1) / GEMM_BN);
+    p.m_tiles = (int)((call.m + p.bm - 1) / p.bm);
+    // the last 128-row block may reach past the padded row-tiles: the weight buffer must cover it
+    if ((int64_t)p.n_tiles * (GEMM_BN / 16) > w.g.rt_alloc)
+        return set_error(c, WF_ERR_SHAPE, "weight buffer does not cover the last 128-row block");
+    double cost = 0;
+    p.ranks = split_ranks(*dev, (int64_t)p.n_tiles * p.m_tiles, p.k_blocks, p.bm, f32, &clusters, &cost);
+    // Pairs of CTAs on tiles of 256 rows x 512 tokens, stream-K shares.  A tile of U units shared by n pairs costs about U / n
+    // units plus n - 1 pieces added by its owner, a piece costing about two units: no share is shorter than sqrt(2 U)
+    // units, which bounds n for weights with few tiles.
+    const int pair_n = (int)((w.g.rows + 2 * GEMM_BN - 1) / (2 * GEMM_BN)), pair_m = (int)((call.m + PAIR_TOKENS - 1) / PAIR_TOKENS);
+    const int64_t units = (int64_t)pair_n * pair_m * p.k_blocks;
+    int min_units = 1;
+    while ((int64_t)min_units * min_units < 2 * p.k_blocks) min_units++;
+    const int workers = (int)std::min<int64_t>(dev->pairs, std::max<int64_t>(1, units / min_units));
+    const bool pair = !f32 && call.m > 64 && workers > 0 && pair_cost((units + workers - 1) / workers, call.m) < cost && !f32;
+    if (std::max(units, (int64_t)p.n_tiles * p.m_tiles * p.k_blocks) >= (1LL << 30)) return set_error(c, WF_ERR_TOO_LARGE, "GEMM has too many tile steps");
     if (pair) {
         p.bm = 256;
-        p.n_tiles = (int)((w.g.rows + 2 * GEMM_BN - 1) / (2 * GEMM_BN));
-        p.m_tiles = (int)((call.m + PAIR_TOKENS - 1) / PAIR_TOKENS);
-        // Stream-K shares.  A tile of U units shared by n pairs costs about U / n units plus n - 1 pieces added by its owner, a
-        // piece costing about two units: no share is shorter than sqrt(2 U) units, which bounds n for weights with few tiles.
-        const int64_t units = (int64_t)p.n_tiles * p.m_tiles * p.k_blocks;
-        if (units >= (1LL << 31)) return set_error(c, WF_ERR_TOO_LARGE, "GEMM has too many tile steps");
-        int min_units = 1;
-        while ((int64_t)min_units * min_units < 2 * p.k_blocks) min_units++;
-        const int workers = (int)std::min<int64_t>(dev->pairs, std::max<int64_t>(1, units / min_units));
+        p.n_tiles = pair_n;
+        p.m_tiles = pair_m;
         p.unit_q = (int)(units / workers);
         p.unit_r = (int)(units % workers);
         cluster = 2;
         grid = 2 * workers;
         stage_bytes = PAIR_A_BYTES + 2 * PAIR_B_HALF;
     } else {
-        // token tiles of one size, in steps of 32 where there are several (the epilogue works on 32 tokens at a time and must
-        // not reach into a neighbour); fp32: 96, so that two stages and the exchange buffer fit
-        const int most = f32 ? 96 : SPLIT_MAX_TOKENS;
-        const int64_t token_tiles = (call.m + most - 1) / most, grain = token_tiles > 1 ? 32 : 16;
-        p.bm = (int)(((call.m + token_tiles - 1) / token_tiles + grain - 1) / grain * grain);
-        p.n_tiles = (int)((w.g.rows + GEMM_BN - 1) / GEMM_BN);
-        p.m_tiles = (int)((call.m + p.bm - 1) / p.bm);
-        // the last 128-row block may reach past the padded row-tiles: the weight buffer must cover it
-        if ((int64_t)p.n_tiles * (GEMM_BN / 16) > w.g.rt_alloc)
-            return set_error(c, WF_ERR_SHAPE, "weight buffer does not cover the last 128-row block");
-        if ((int64_t)p.n_tiles * p.m_tiles * p.k_blocks >= (1LL << 30)) return set_error(c, WF_ERR_TOO_LARGE, "GEMM has too many tile steps");
-        int clusters = 0;
-        cluster = p.ranks = split_ranks(*dev, (int64_t)p.n_tiles * p.m_tiles, p.k_blocks, &clusters);
+        cluster = p.ranks;
         grid = clusters * cluster;
         stage_bytes = (size_t)split_stage_bytes(pieces, planes, p.bm);
         exchange = (size_t)split_exchange_bytes(p.bm, cluster);

@@ -44,7 +44,9 @@ __device__ __forceinline__ void st_async_16(uint32_t cluster_addr, uint32_t a, u
                  : "memory");
 }
 
-// smem: [0, 1024) barriers + tmem slot | stages x (A | B), 1024-byte aligned | exchange buffer
+__device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
+// smem: [0, 1024) barriers, tmem slot, token scales | stages x (A | B), 1024-byte aligned | exchange buffer
 template <int QT, int PIECES, int PLANES>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap) {
     constexpr int ACCS = PIECES;
@@ -66,6 +68,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
     const int stages = p.stages, S = p.ranks;
     uint8_t* stage0 = smem + 1024;
     float4* ex = reinterpret_cast<float4*>(stage0 + (size_t)stages * stage_bytes);
+    float* scale = reinterpret_cast<float*>(smem + 512);  // [128] row_unscale of the tile's tokens
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int rank = (int)blockIdx.x % S, cluster = (int)blockIdx.x / S, clusters = (int)gridDim.x / S;
     const int tiles = p.n_tiles * p.m_tiles;
@@ -170,9 +173,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
             const int nt = tile / p.m_tiles, tok0 = (tile % p.m_tiles) * p.bm;
             const int n = nt * GEMM_BN + row;
             if (S > 1) {
-                if (threadIdx.x == 128 && mine > 0) g_mbar_expect_tx(ex_full, (uint32_t)(S * mine * GEMM_BN * 16));
+                const int t = (int)threadIdx.x - 128;
+                const float mine_scale = t < p.bm && tok0 + t < p.m ? __ldg(p.row_unscale + tok0 + t) : 0.f;
+                if (round > 0) epilogue_sync();  // every warp is through with the previous tile's scales
+                scale[t] = mine_scale;
+                if (t == 0 && mine > 0) g_mbar_expect_tx(ex_full, (uint32_t)(S * mine * GEMM_BN * 16));
                 if (round > 0 && !g_mbar_wait(ex_empty, (round - 1) & 1)) { if (lane == 0) fail(); break; }
+                epilogue_sync();
             }
+            uint32_t to = 0, in = 0;  // rank and place there of the next group of four tokens
+            uint32_t to_addr = map_to_rank(ex_addr, 0), to_bar = map_to_rank(bar_addr, 0);
             for (int g0 = kb0; g0 < kb1; local++) {
                 const int g1 = min(kb1, g0 + min(FLUSH, kb1 - g0)), buf = local & 1;
                 const bool last = g1 == kb1;
@@ -196,9 +206,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
                         for (int j = 0; j < 8; j++) {
                             const int gr = (c >> 2) + j;
                             if (gr < groups) {
-                                const uint32_t to = (uint32_t)(gr / per);
-                                st_async_16(map_to_rank(ex_addr + (uint32_t)(gr - (int)to * per) * (GEMM_BN * 16), to), r[4 * j], r[4 * j + 1], r[4 * j + 2],
-                                            r[4 * j + 3], map_to_rank(bar_addr, to));
+                                st_async_16(to_addr + in * (GEMM_BN * 16), r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3], to_bar);
+                                if (++in == (uint32_t)per && gr + 1 < groups) {
+                                    in = 0;
+                                    to++;
+                                    to_addr = map_to_rank(ex_addr, to);
+                                    to_bar = map_to_rank(bar_addr, to);
+                                }
                             }
                         }
                     }
@@ -211,19 +225,22 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
             if (!ok) break;
             if (S > 1) {  // this rank's tokens: the ranks' parts in rank order
                 if (mine > 0 && !g_mbar_wait(ex_full, round & 1)) { if (lane == 0) fail(); break; }
-                for (int gi = 0; gi < mine; gi++) {
+                const int left = min(mine * 4, p.m - tok0 - rank * per * 4);  // tokens of this rank that exist
+                float* yp = p.y + (int64_t)(tok0 + rank * per * 4) * p.ldy + p.col0 + n;
+                const float* sc = scale + rank * per * 4;
+#pragma unroll 2
+                for (int gi = 0; gi * 4 < left; gi++) {
                     float4 v = ex[(size_t)gi * GEMM_BN + row];
                     for (int src = 1; src < S; src++) {
                         const float4 w = ex[(size_t)(src * per + gi) * GEMM_BN + row];
                         v.x += w.x, v.y += w.y, v.z += w.z, v.w += w.w;
                     }
-                    const int tok = tok0 + (rank * per + gi) * 4;
+                    const float4 u = *reinterpret_cast<const float4*>(sc + gi * 4);
+                    const float o[4] = {v.x * u.x, v.y * u.y, v.z * u.z, v.w * u.w};
                     if (n < p.rows) {
-                        float* yp = p.y + (int64_t)tok * p.ldy + p.col0 + n;
-                        const float o[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                         for (int e = 0; e < 4; e++)
-                            if (tok + e < p.m) yp[(int64_t)e * p.ldy] = o[e] * __ldg(p.row_unscale + tok + e);
+                            if (gi * 4 + e < left) yp[(int64_t)(gi * 4 + e) * p.ldy] = o[e];
                     }
                 }
                 __syncwarp();

@@ -80,7 +80,11 @@ template <int QT> static cudaError_t gemm_prepare(int device, GemmDevice** out) 
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_split_kernel<QT, 2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
     if (e == cudaSuccess) e = max_clusters(gemm_pair_kernel<QT>, 2, &d.pairs);
-    for (int n = 1; n <= SPLIT_MAX_RANKS && e == cudaSuccess; n++) e = max_clusters(gemm_split_kernel<QT, 1, 1>, n, &d.clusters[n]);
+    for (int n = 1; n <= SPLIT_MAX_RANKS && e == cudaSuccess; n++) {
+        e = max_clusters(gemm_split_kernel<QT, 1, 1>, n, &d.clusters[n]);
+        // one fewer than the device says: a cluster that does not find its place in the first wave costs a whole round
+        if (n >= 3 && d.clusters[n] > 16) d.clusters[n]--;
+    }
     d.ready = e == cudaSuccess;
     return e;
 }
@@ -110,25 +114,25 @@ static cudaError_t gemm_launch_one(Kernel kernel, const GemmParams& p, const CUt
 // of conversion, launch and start; a cost per unit of 128 k on the busiest CTA or pair; the parts put together.
 //   us by the fit / measured: split, bf16, [4096 x 4096]: 33 tokens (4 ranks) 13 / 12.4, 100 tokens 15 / 15.6; [11008 x 4096],
 //   128 tokens (3 ranks) 30 / 28; [16000 x 1024], 400 tokens: 1 rank 31 / 30, 2 ranks 53 / 64.
-//   pair: [4096 x 4096] 256 tokens 24 / 23, 512 tokens 33 / 35; [11008 x 4096] 256 tokens 34 / 32, 300 tokens 49 / 46.
-static double split_cost(int64_t rounds, int units, int ranks, int bm, bool f32) {
-    const double b = bm / 128.0, unit = f32 ? 0.95 + 0.9 * b : 0.6 + 0.12 * b;
+//   pair: [4096 x 4096] 256 tokens 25 / 23, 512 tokens 38 / 35; [11008 x 4096] 256 tokens 31 / 32; [600 x 6976] 2000 tokens 47 / 47.5.
+static double split_cost(int qt, int64_t rounds, int units, int ranks, int bm, bool f32) {
+    const double b = bm / 128.0, unit = f32 ? 0.95 + 0.9 * b : (qt == WF_QTYPE_Q4_0 ? 0.6 : qt == WF_QTYPE_Q8_0 ? 0.8 : 0.7) + 0.12 * b;
     const double together = ranks == 1 ? 0.5 + 0.5 * b : (f32 ? 0.5 + 4.0 * b : 1.0 + 3.0 * b);
     return 6.0 + (double)rounds * (units * unit + together);
 }
-static double pair_cost(int64_t units, int64_t m) {
-    const double half = m <= 256 ? 1.0 : 1.5;  // a token tile of one or two halves
-    return 8.0 + (double)units * half + (m <= 256 ? 8.0 : 13.0);
+// share: units of the busiest pair; a tile of U units is put together from the pieces of U / share pairs
+static double pair_cost(int64_t share, int k_blocks, int halves) {
+    return 8.0 + (double)share * (halves == 2 ? 1.5 : 1.0) + (double)((k_blocks + share - 1) / share) * (halves == 2 ? 4.5 : 2.2);
 }
 
 // CTAs per tile of the split kernel, the cheapest by split_cost.
-static int split_ranks(const GemmDevice& d, int64_t tiles, int k_blocks, int bm, bool f32, int* clusters, double* cost) {
+static int split_ranks(const GemmDevice& d, int qt, int64_t tiles, int k_blocks, int bm, bool f32, int* clusters, double* cost) {
     int best = 1;
     *cost = 1e30;
     for (int n = 1; n <= SPLIT_MAX_RANKS && n <= k_blocks; n++) {
         if (d.clusters[n] < 1) continue;
         const int64_t rounds = (tiles + d.clusters[n] - 1) / d.clusters[n];
-        const double t = split_cost(rounds, (k_blocks + n - 1) / n, n, bm, f32);
+        const double t = split_cost(qt, rounds, (k_blocks + n - 1) / n, n, bm, f32);
         if (t < *cost) {
             *cost = t;
             best = n;
@@ -211,26 +215,37 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     if ((int64_t)p.n_tiles * (GEMM_BN / 16) > w.g.rt_alloc)
         return set_error(c, WF_ERR_SHAPE, "weight buffer does not cover the last 128-row block");
     double cost = 0;
-    p.ranks = split_ranks(*dev, (int64_t)p.n_tiles * p.m_tiles, p.k_blocks, p.bm, f32, &clusters, &cost);
-    // Pairs of CTAs on tiles of 256 rows x 512 tokens, stream-K shares.  A tile of U units shared by n pairs costs about U / n
+    p.ranks = split_ranks(*dev, qt, (int64_t)p.n_tiles * p.m_tiles, p.k_blocks, p.bm, f32, &clusters, &cost);
+    // Pairs of CTAs on tiles of 256 rows x 512 or 256 tokens, stream-K shares.  A tile of U units shared by n pairs costs about U / n
     // units plus n - 1 pieces added by its owner, a piece costing about two units: no share is shorter than sqrt(2 U)
     // units, which bounds n for weights with few tiles.
-    const int pair_n = (int)((w.g.rows + 2 * GEMM_BN - 1) / (2 * GEMM_BN)), pair_m = (int)((call.m + PAIR_TOKENS - 1) / PAIR_TOKENS);
-    const int64_t units = (int64_t)pair_n * pair_m * p.k_blocks;
+    const int pair_n = (int)((w.g.rows + 2 * GEMM_BN - 1) / (2 * GEMM_BN));
     int min_units = 1;
     while ((int64_t)min_units * min_units < 2 * p.k_blocks) min_units++;
-    const int workers = (int)std::min<int64_t>(dev->pairs, std::max<int64_t>(1, units / min_units));
-    const bool pair = !f32 && call.m > 64 && workers > 0 && pair_cost((units + workers - 1) / workers, call.m) < cost && !f32;
+    int64_t units = 0;
+    int workers = 0;
+    bool pair = false;
+    for (int halves = 1; halves <= 2 && !f32 && call.m > 64 && dev->pairs > 0; halves++) {
+        const int64_t u = (int64_t)pair_n * ((call.m + halves * 256 - 1) / (halves * 256)) * p.k_blocks;
+        const int n = (int)std::min<int64_t>(dev->pairs, std::max<int64_t>(1, u / min_units));
+        const double t = pair_cost((u + n - 1) / n, p.k_blocks, halves);
+        if (t >= cost) continue;
+        cost = t;
+        pair = true;
+        p.halves = halves;
+        units = u;
+        workers = n;
+    }
     if (std::max(units, (int64_t)p.n_tiles * p.m_tiles * p.k_blocks) >= (1LL << 30)) return set_error(c, WF_ERR_TOO_LARGE, "GEMM has too many tile steps");
     if (pair) {
         p.bm = 256;
         p.n_tiles = pair_n;
-        p.m_tiles = pair_m;
+        p.m_tiles = (int)((call.m + p.halves * 256 - 1) / (p.halves * 256));
         p.unit_q = (int)(units / workers);
         p.unit_r = (int)(units % workers);
         cluster = 2;
         grid = 2 * workers;
-        stage_bytes = PAIR_A_BYTES + 2 * PAIR_B_HALF;
+        stage_bytes = (size_t)pair_stage_bytes(p.halves);
     } else {
         cluster = p.ranks;
         grid = clusters * cluster;

@@ -30,6 +30,7 @@ struct GemmParams {
     int bm;              // tokens per MMA (UMMA N: multiple of 16, <= 256)
     int n_tiles, m_tiles, k_blocks;  // k_blocks = ceil(k / 128)
     int stages;
+    int halves;          // pair kernel: 256-token halves of a token tile, 1 or 2
     int ranks;           // split kernel: CTAs of a cluster, which share a tile's K
     uint32_t idesc;
     // pair kernel, stream-K: the (tile, k-block) units form one sequence, pair b owns units [b*q + min(b,r), ...)

@@ -1,6 +1,6 @@
 // Prefill GEMM for more than 256 tokens: y[m, rows] = x[m, K] . W[rows, K]^T on pairs of CTAs (tcgen05 cta_group::2).
 //
-// A pair computes 256 weight rows x 512 tokens: one tcgen05.mma of M = 256, N = 256 spans both SMs, each SM holding its
+// A pair computes 256 weight rows x 512 tokens (or 256, where there are few tiles): one tcgen05.mma of M = 256, N = 256 spans both SMs, each SM holding its
 // own 128 rows of A (dequantized weights, fp16), HALF of the tokens of B and its own 128 accumulator rows in TMEM.
 // What bounds the kernel is shared memory and power: per 64 k and 512 tokens (1024 MMA cycles) an SM moves 16 KB of A
 // in by generic stores, 32 KB of B in by TMA, and 32 + 32 KB out to the tensor core -- 109 bytes per cycle of the 128 it
@@ -33,7 +33,7 @@ constexpr int PAIR_BK = 64;                              // k per stage; a unit 
 constexpr int PAIR_A_BYTES = GEMM_BN * PAIR_BK * 2;      // 16 KB: this CTA's weight rows
 constexpr int PAIR_B_HALF = 128 * PAIR_BK * 2;           // 16 KB: this CTA's 128 of a half's 256 tokens
 constexpr int PAIR_MAX_STAGES = 8;
-constexpr int PAIR_TOKENS = 512;                         // tokens of a tile: two halves of 256, an accumulator each
+inline __host__ __device__ int pair_stage_bytes(int halves) { return PAIR_A_BYTES + halves * PAIR_B_HALF; }
 
 // A pair's share of the unit sequence, cut into segments: a segment is a run of k-blocks of one tile.
 struct GemmSegment {
@@ -106,7 +106,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
     uint64_t* tail_full = acc_empty + 2;                          // the accumulators of the tile shared with the following pairs
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail_full + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    constexpr uint32_t stage_bytes = PAIR_A_BYTES + 2 * PAIR_B_HALF;
+    const bool wide = p.halves == 2;
+    const int tile_tokens = p.halves * 256;
+    const uint32_t stage_bytes = (uint32_t)pair_stage_bytes(p.halves);
     uint8_t* stage0 = smem + 1024;
 
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -144,8 +146,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
         *abort_flag = 1;
     };
     // 256-token halves of token tile mt that hold tokens
-    auto halves_of = [&](int mt) { return p.m - mt * PAIR_TOKENS > 256 ? 2 : 1; };
-    // Half h of a tile accumulates in TMEM columns 256 h ..; used[h] counts the tiles that have used it so far.
+    auto halves_of = [&](int mt) { return wide && p.m - mt * 512 > 256 ? 2 : 1; };
+    // Accumulators are TMEM columns 0 .. 255 and 256 .. 511: one per half of a tile, or by turns for tiles of one half (`local`
+    // counts the segments).  used[acc] counts the uses so far.
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer: this CTA's tokens
@@ -162,7 +165,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
                     uint64_t* bar = leader ? &full[s] : &b_full[s];
                     g_mbar_expect_tx(bar, (uint32_t)nh * PAIR_B_HALF);
                     for (int h = 0; h < nh; h++)
-                        tma_load_2d(b_stage + h * PAIR_B_HALF, &xmap, kb * PAIR_BK, mt * PAIR_TOKENS + h * 256 + (int)rank * 128, bar);
+                        tma_load_2d(b_stage + h * PAIR_B_HALF, &xmap, kb * PAIR_BK, mt * tile_tokens + h * 256 + (int)rank * 128, bar);
                 }
                 u += g.kb1 - g.kb0;
             }
@@ -174,8 +177,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
             const uint32_t issue = elect_one();
             const uint64_t a_desc0 = smem_desc_sw128(g_smem_u32(stage0)), b_desc0 = smem_desc_sw128(g_smem_u32(stage0) + PAIR_A_BYTES);
             StageCursor at;
-            int used[2] = {0, 0};
-            for (int u = u0; u < u1 && !*abort_flag;) {
+            int local = 0, used[2] = {0, 0};
+            for (int u = u0; u < u1 && !*abort_flag; local++) {
                 const GemmSegment g = segment_at(p, u, u1);
                 const int nh = halves_of(g.tile % p.m_tiles);
                 bool ok = true;
@@ -185,15 +188,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
                     tc_fence_after();
                     const uint64_t off = (uint64_t)((uint32_t)s * stage_bytes >> 4);
                     for (int h = 0; h < nh; h++) {
-                        if (kb == 2 * g.kb0 && used[h] >= 1) {  // the epilogues must have drained this accumulator's previous tile
-                            if (!g_mbar_wait(&acc_empty[h], (used[h] - 1) & 1)) { fail(); ok = false; break; }
+                        const int acc = wide ? h : (local & 1);
+                        if (kb == 2 * g.kb0 && used[acc] >= 1) {  // the epilogues must have drained this accumulator's previous tile
+                            if (!g_mbar_wait(&acc_empty[acc], (used[acc] - 1) & 1)) { fail(); ok = false; break; }
                             tc_fence_after();
                         }
-                        tc_mma_span<2>(tmem_base + (uint32_t)(h * 256), a_desc0 + off, b_desc0 + off + (uint64_t)(h * (PAIR_B_HALF >> 4)), p.idesc,
+                        tc_mma_span<2>(tmem_base + (uint32_t)(acc * 256), a_desc0 + off, b_desc0 + off + (uint64_t)(h * (PAIR_B_HALF >> 4)), p.idesc,
                                        (uint32_t)(kb - 2 * g.kb0), issue);
                         if (kb == 2 * g.kb1 - 1) {
-                            if (issue) tc_commit_pair(&acc_full[h]);
-                            used[h]++;
+                            if (issue) tc_commit_pair(&acc_full[acc]);
+                            used[acc]++;
                         }
                     }
                     if (!ok) break;
@@ -218,13 +222,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
         // Every segment except the tile this pair owns the beginning of and shares with the following pairs.
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
-        int used[2] = {0, 0};
+        int local = 0, used[2] = {0, 0};
         bool dead = false;
         asm volatile("griddepcontrol.wait;" ::: "memory");  // the row scales; gen
         unsigned int launch_gen = ld_acquire_u32(p.gen) + 1u;  // this launch's generation: see GemmParams
         if (launch_gen == 0u) launch_gen = 1u;                 // 0 is what untouched flags hold
         float* mine = p.partial + (size_t)blockIdx.x * GEMM_PIECE_TOKENS * GEMM_BN;
-        for (int u = u0; u < u1 && !*abort_flag && !dead;) {
+        for (int u = u0; u < u1 && !*abort_flag && !dead; local++) {
             const GemmSegment g = segment_at(p, u, u1);
             const int nt = g.tile / p.m_tiles, mt = g.tile % p.m_tiles;
             const int n = nt * (2 * GEMM_BN) + (int)rank * GEMM_BN + row;
@@ -232,19 +236,20 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
             if (starts && !ends) break;
             const int parts = halves_of(mt);
             for (int h = 0; h < parts; h++) {
-                if (!g_mbar_wait(&acc_full[h], used[h] & 1)) { if (lane == 0) fail(); dead = true; break; }
+                const int acc = wide ? h : (local & 1);
+                if (!g_mbar_wait(&acc_full[acc], used[acc] & 1)) { if (lane == 0) fail(); dead = true; break; }
                 tc_fence_after();
-                used[h]++;
-                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * 256);
+                used[acc]++;
+                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * 256);
                 for (int c = 0; c < 256; c += 32) {
                     uint32_t r[32];
                     tmem_ld32(taddr + (uint32_t)c, r);
                     if (!starts) write_piece_chunk(mine, r, h * 256 + c, row);
-                    else store_chunk(p.y, p.ldy, p.col0, p.row_unscale, r, mt * PAIR_TOKENS + h * 256 + c, p.m, n, p.rows);
+                    else store_chunk(p.y, p.ldy, p.col0, p.row_unscale, r, mt * tile_tokens + h * 256 + c, p.m, n, p.rows);
                 }
                 tc_fence_before();  // the accumulator has been read: the MMA issuer may overwrite it
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(map_to_rank(g_smem_u32(&acc_empty[h]), 0));
+                if (lane == 0) mbar_arrive_cluster(map_to_rank(g_smem_u32(&acc_empty[acc]), 0));
             }
             if (dead) break;
             if (!starts) {  // publish this warp's 32 rows of the piece
@@ -317,6 +322,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
             const int row = quarter * 32 + lane;
             const int nt = tile / p.m_tiles, mt = tile % p.m_tiles;
             const int n = nt * (2 * GEMM_BN) + (int)rank * GEMM_BN + row;
+            int local = 0;  // number of this segment
+            for (int u = u0; u < u1; local++) {
+                const GemmSegment g = segment_at(p, u, u1);
+                if (g.tile == tile) break;
+                u += g.kb1 - g.kb0;
+            }
+            const uint32_t col0 = wide ? 0u : (uint32_t)((local & 1) * 256);
             int last_pair = pair;
             bool ok = !*abort_flag;
             const int tile_end = (tile + 1) * p.k_blocks;
@@ -341,14 +353,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
             if (ok && slice < chunks) fetch(pair + 1, slice);  // the next pair always holds a piece
             for (int ci = slice; ci < chunks && ok; ci += 3) {
                 uint32_t r[32];
-                tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ci * 32), r);
+                tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + col0 + (uint32_t)(ci * 32), r);
                 add_piece_chunk(r, v);
                 for (int cc = pair + 2; cc <= last_pair; cc++) {  // pieces in pair order
                     fetch(cc, ci);
                     add_piece_chunk(r, v);
                 }
                 if (ci + 3 < chunks) fetch(pair + 1, ci + 3);  // under the stores of this one
-                store_chunk(p.y, p.ldy, p.col0, p.row_unscale, r, mt * PAIR_TOKENS + ci * 32, p.m, n, p.rows);
+                store_chunk(p.y, p.ldy, p.col0, p.row_unscale, r, mt * tile_tokens + ci * 32, p.m, n, p.rows);
             }
         }
     }

@@ -1,0 +1,40 @@
+"""The ways a several-token product takes from its warps' sums to y: one slice (straight to y, or through shared memory for
+fp32 tokens), a cluster of slices in one and in several batches of row-tiles, and partial sums in memory where eight slices
+do not fit; the last slice and the last batch shorter than the others, fewer tiles than warps.
+
+Weights are the codes themselves (unit scales) and activations small multiples of a power of two, so every product and every
+partial sum is a multiple of 2^-9 below 2^15: exact in fp32 however the additions are ordered.  fp32 tokens need their second
+bf16 part."""
+import numpy as np
+import pytest
+
+from warpforge_b200 import quant as Q
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,k,m,f32", [
+    (16, 32, 2, False), (50, 96, 9, False), (4700, 2048, 8, False),     # one slice
+    (260, 2080, 16, False), (7000, 2560, 31, False), (3100, 11008, 17, False),  # clusters; several batches
+    (30, 65536, 32, False), (700, 27008, 31, False),                    # memory
+    (9000, 1024, 2, True), (3001, 4128, 10, True), (100, 3200, 5, True),
+])
+def test_exact(rows, k, m, f32):
+    from warpforge_b200.backend import DotGeneralOp, LINEAR_DIMS, NvidiaBackend, Tensor
+
+    rng = np.random.default_rng(rows + k + m)
+    codes = rng.integers(0, 16, (rows, k), dtype=np.uint8)
+    blocks = np.zeros((rows, k // 32, 18), np.uint8)
+    blocks[:, :, 0:2] = np.frombuffer(np.float16(1.0).tobytes(), np.uint8)
+    c = codes.reshape(rows, k // 32, 32)
+    blocks[:, :, 2:] = c[:, :, 0::2] | (c[:, :, 1::2] << 4)
+    # |y| <= 8 K max|x| stays below 2^15
+    x = (rng.integers(-511, 512, (m, k)) / 512.0 if f32 else rng.integers(-8, 9, (m, k)) / 128.0).astype(np.float32)
+    backend = NvidiaBackend(0)
+    w = backend.upload_weight(Q.QuantizationType.Q4_0, blocks.reshape(rows, -1), rows, k)
+    t = Tensor.from_float_array(x) if f32 else Tensor.from_bf16_bits(Q.float_to_bf16_bits(x).reshape(m, k))
+    got = [backend.execute(DotGeneralOp(LINEAR_DIMS, (m, rows)), [t, w])[0].data for _ in range(2)]
+    want = x.astype(np.float64) @ (codes.astype(np.float64) - 8.0).T
+    w.close()
+    backend.close()
+    assert np.array_equal(got[0], want) and np.array_equal(got[1], want)

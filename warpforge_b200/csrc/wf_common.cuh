@@ -24,6 +24,18 @@ constexpr int STATUS_GEMM_PIPE_TIMEOUT = 2;
 constexpr int STATUS_PEER_WAIT_TIMEOUT = 4;
 constexpr int STATUS_BAD_INDEX = 8;  // an embedding index outside the table
 
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+    return r;
+}
+// 16 bytes into the shared memory of a CTA of the cluster; the bytes count on the barrier there when they have arrived
+__device__ __forceinline__ void st_async_16(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t cluster_bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(cluster_addr), "r"(a), "r"(b),
+                 "r"(c), "r"(d), "r"(cluster_bar)
+                 : "memory");
+}
+
 // The status block: `bits` collects what kernels report (and is what running kernels look at); `host` is the device
 // address of one int per bit in pinned host memory, set with it, so that the host learns the outcome of a stream it
 // has waited for from its own memory.  Copying the bits back instead cost every synchronising call about 10 us.

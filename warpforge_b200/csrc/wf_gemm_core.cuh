@@ -84,11 +84,6 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 // shared::cluster address of the same object in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-    return r;
-}
 // Default semantics (release at CTA scope): the operands handed over were put in place by the async-proxy fence and the
 // CTA's own barriers; `.release.cluster` costs a fence that waits for the thread's loads in flight, 0.9 us per stage.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {

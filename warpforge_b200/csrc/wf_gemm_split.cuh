@@ -37,13 +37,6 @@ inline __host__ __device__ int split_stage_bytes(int pieces, int planes, int bm)
 inline __host__ __device__ int split_groups(int bm, int ranks) { return (bm / 4 + ranks - 1) / ranks; }
 inline __host__ __device__ int split_exchange_bytes(int bm, int ranks) { return ranks == 1 ? 0 : ranks * split_groups(bm, ranks) * GEMM_BN * 16; }
 
-// 16 bytes into the shared memory of a CTA of the cluster; the bytes count on the barrier there when they have arrived
-__device__ __forceinline__ void st_async_16(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t cluster_bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(cluster_addr), "r"(a), "r"(b),
-                 "r"(c), "r"(d), "r"(cluster_bar)
-                 : "memory");
-}
-
 __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // smem: [0, 1024) barriers, tmem slot, token scales | stages x (A | B), 1024-byte aligned | exchange buffer

@@ -81,22 +81,66 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvPara
 // ---------------------------------------------------------------- host side
 constexpr size_t GEMV_SMEM_LIMIT = 227 * 1024;
 
-// The cut of a weight for `cols` activation columns, worked out once per weight (the search walks a few thousand
+// Without a device to ask: a GPC's SMs are seldom a multiple of a cluster, so about a tenth of the SMs stay out of
+// clusters of three and more.
+static void gemvn_clusters_estimate(int sm_count, int* clusters) {
+    for (int n = 1; n <= GEMVN_MAX_CLUSTER; n++) clusters[n] = n <= 2 ? sm_count / n : sm_count * 9 / (10 * n);
+}
+
+// How many clusters of each size the current device holds at a time (every instance of the kernel takes a whole SM), asked once.
+static const int* gemvn_clusters(int sm_count) {
+    struct Capacity {
+        bool ready = false;
+        int clusters[GEMVN_MAX_CLUSTER + 1] = {};
+    };
+    static Capacity devs[64];
+    static std::mutex mu;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    Capacity& d = devs[dev & 63];
+    if (d.ready) return d.clusters;
+    gemvn_clusters_estimate(sm_count, d.clusters);
+    const auto kernel = gemvn_kernel<WF_QTYPE_Q4_0, 1, WAY_CLUSTER>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_LIMIT) == cudaSuccess) {
+        for (int n = 2; n <= GEMVN_MAX_CLUSTER; n++) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)n);
+            cfg.blockDim = dim3(GEMV_CONSUMERS);
+            cfg.dynamicSmemBytes = GEMVN_SMEM;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)n;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int count = 0;
+            // one fewer of the larger ones: a cluster that does not find its place in the first wave costs a whole round
+            if (cudaOccupancyMaxActiveClusters(&count, kernel, &cfg) == cudaSuccess) d.clusters[n] = n >= 3 && count > 16 ? count - 1 : count;
+        }
+        d.ready = true;
+    }
+    cudaGetLastError();  // a failed question leaves the estimate
+    return d.clusters;
+}
+
+// The cut of a weight for `cols` activation columns, worked out once per weight (the search walks dozens of
 // candidates: too slow for every call of a microsecond-scale kernel).
 static GemvNPlan cached_plan(int sm_count, const Weight& w, int cols, bool x_f32) {
     short* e = const_cast<Weight&>(w).split_cache[x_f32 ? 1 : 0][cols];
     if (e[0] < 0) {
-        const GemvNPlan p = gemvn_plan(sm_count, w.g.qtype, w.g.rt, w.g.kt, cols, x_f32);
+        const GemvNPlan p = gemvn_plan(gemvn_clusters(sm_count), w.g.qtype, w.g.rt, w.g.kt, cols, x_f32);
         e[1] = (short)p.kc;
-        e[2] = (short)p.team;
-        e[3] = (short)p.uses_part;
+        e[2] = (short)p.batch;
+        e[3] = (short)p.ctas;
         e[0] = (short)p.slices;
     }
     GemvNPlan p;
     p.slices = e[0];
     p.kc = e[1];
-    p.team = e[2];
-    p.uses_part = e[3] != 0;
+    p.batch = e[2];
+    p.ctas = e[3];
+    p.part = p.slices > GEMVN_MAX_CLUSTER;
     return p;
 }
 
@@ -147,13 +191,13 @@ static cudaError_t launch_qt_one_token(int qt, const GemvParams& p, int grid, si
                                  : launch_one_token<WF_QTYPE_Q4_K>(p, grid, smem, s);
 }
 
-template <int QT, int NG>
+template <int QT, int NG, int WAY>
 static cudaError_t launch_several(const GemvNParams& p, int grid, size_t smem, cudaStream_t s) {
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && !attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemvn_kernel<QT, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_LIMIT);
+        cudaError_t e = cudaFuncSetAttribute(gemvn_kernel<QT, NG, WAY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_LIMIT);
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
@@ -162,19 +206,28 @@ static cudaError_t launch_several(const GemvNParams& p, int grid, size_t smem, c
     cfg.blockDim = dim3(GEMV_CONSUMERS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)p.slices;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemvn_kernel<QT, NG>, p);
+    cfg.numAttrs = p.cluster ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, gemvn_kernel<QT, NG, WAY>, p);
+}
+template <int QT, int NG>
+static cudaError_t launch_way(const GemvNParams& p, int grid, size_t smem, cudaStream_t s) {
+    if (!p.x_f32 && p.slices == 1) return launch_several<QT, NG, WAY_DIRECT>(p, grid, smem, s);
+    if (!p.x_f32 && p.cluster) return launch_several<QT, NG, WAY_CLUSTER>(p, grid, smem, s);
+    return launch_several<QT, NG, WAY_ANY>(p, grid, smem, s);
 }
 template <int NG>
 static cudaError_t launch_qt_several(int qt, const GemvNParams& p, int grid, size_t smem, cudaStream_t s) {
-    return qt == WF_QTYPE_Q4_0   ? launch_several<WF_QTYPE_Q4_0, NG>(p, grid, smem, s)
-           : qt == WF_QTYPE_Q4_1 ? launch_several<WF_QTYPE_Q4_1, NG>(p, grid, smem, s)
-           : qt == WF_QTYPE_Q8_0 ? launch_several<WF_QTYPE_Q8_0, NG>(p, grid, smem, s)
-                                 : launch_several<WF_QTYPE_Q4_K, NG>(p, grid, smem, s);
+    return qt == WF_QTYPE_Q4_0   ? launch_way<WF_QTYPE_Q4_0, NG>(p, grid, smem, s)
+           : qt == WF_QTYPE_Q4_1 ? launch_way<WF_QTYPE_Q4_1, NG>(p, grid, smem, s)
+           : qt == WF_QTYPE_Q8_0 ? launch_way<WF_QTYPE_Q8_0, NG>(p, grid, smem, s)
+                                 : launch_way<WF_QTYPE_Q4_K, NG>(p, grid, smem, s);
 }
 
 // Allocates (once per stream) what the kernels of that stream exchange partial results through: the one-token
@@ -270,13 +323,15 @@ static int launch_passes(Context* c, const GemvCall& call, cudaStream_t s, const
         if (plan.slices < 1) return set_error(c, WF_ERR_TOO_LARGE, "no split of K=%lld fits %d activation columns", (long long)w.g.k, p.cols);
         p.slices = plan.slices;
         p.kc = plan.kc;
-        p.team = plan.team;
+        p.batch = plan.batch;
+        p.cluster = plan.slices > 1 && !plan.part;
         const int ng = p.cols <= 8 ? 1 : p.cols <= 16 ? 2 : 4;
-        const size_t smem = gemvn_smem(qt, p.kc, p.cols, ng, p.team, &p.sx, &p.piece_off);
-        if (clear && plan.uses_part) WF_CUDA(c, cudaMemsetAsync(buf.count, 0, (size_t)w.g.rt * sizeof(int), s));
-        const cudaError_t e = ng == 1   ? launch_qt_several<1>(qt, p, c->sm_count, smem, s)
-                              : ng == 2 ? launch_qt_several<2>(qt, p, c->sm_count, smem, s)
-                                        : launch_qt_several<4>(qt, p, c->sm_count, smem, s);
+        const int grid = plan.part ? c->sm_count : plan.ctas * plan.slices;
+        const size_t smem = gemvn_smem(qt, p.kc, p.cols, f32, p.slices, p.batch, &p.sx, &p.piece_off, &p.ex_off);
+        if (clear && plan.part) WF_CUDA(c, cudaMemsetAsync(buf.count, 0, (size_t)w.g.rt * sizeof(int), s));
+        const cudaError_t e = ng == 1   ? launch_qt_several<1>(qt, p, grid, smem, s)
+                              : ng == 2 ? launch_qt_several<2>(qt, p, grid, smem, s)
+                                        : launch_qt_several<4>(qt, p, grid, smem, s);
         if (e != cudaSuccess) return cuda_status(c, e, what);
         c->launches++;
     }
@@ -355,12 +410,15 @@ extern "C" int wf_plan_several_tokens(int qtype, int64_t rows, int64_t k, int co
     if (qt != WF_QTYPE_Q4_0 && qt != WF_QTYPE_Q4_1 && qt != WF_QTYPE_Q8_0 && qt != WF_QTYPE_Q4_K) return WF_ERR_UNSUPPORTED_TYPE;
     if (rows < 1 || k < 1 || cols < 1 || cols > GEMVN_MAX_COLS || sm_count < 1 || !slices || !k_tiles_per_slice || !team) return WF_ERR_INVALID_ARGUMENT;
     const int64_t rt = (rows + 15) / 16, kt = (k + tile_k(qt) - 1) / tile_k(qt);
-    const GemvNPlan p = gemvn_plan(sm_count, qt, rt, kt, cols, x_is_f32 != 0);
+    int clusters[GEMVN_MAX_CLUSTER + 1];
+    gemvn_clusters_estimate(sm_count, clusters);
+    const GemvNPlan p = gemvn_plan(clusters, qt, rt, kt, cols, x_is_f32 != 0);
     *slices = p.slices;
     *k_tiles_per_slice = p.kc;
-    *team = p.team;
-    if (uses_partial_sums) *uses_partial_sums = p.uses_part ? 1 : 0;
-    const int ng = cols <= 8 ? 1 : cols <= 16 ? 2 : 4;
-    if (smem_bytes) *smem_bytes = p.slices > 0 ? (int64_t)gemvn_smem(qt, p.kc, cols, ng, p.team, nullptr, nullptr) : 0;
+    // the warps of a CTA cut its tiles evenly: about this many share a row-tile
+    const int share = p.slices > 0 ? GEMV_WARPS / (int)std::min<int64_t>((rt + p.ctas - 1) / p.ctas, GEMV_WARPS) : 1;
+    *team = share >= 16 ? 16 : share >= 8 ? 8 : share;
+    if (uses_partial_sums) *uses_partial_sums = p.slices > 1 || x_is_f32 ? 1 : 0;
+    if (smem_bytes) *smem_bytes = p.slices > 0 ? (int64_t)gemvn_smem(qt, p.kc, cols, x_is_f32 != 0, p.slices, p.batch, nullptr, nullptr, nullptr) : 0;
     return WF_OK;
 }

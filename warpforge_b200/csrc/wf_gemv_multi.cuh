@@ -6,21 +6,27 @@
 // integer work per weight byte does not grow with the number of tokens.  fp32 activations enter as three exact
 // bf16 columns per token (x = hi + mid + lo), as in the one-pass ring kernel this replaces.
 //
-// Work split.  A unit is one row-tile (16 rows) times one k-slice (kc consecutive k-tiles, contiguous in memory).
-// A team of W warps of one CTA owns whole units: its members cut a unit's k-tiles among themselves, keep their
-// sums in registers from their first to their last tile, and hand them to the team's first member through
-// shared memory (one named barrier per unit).  The number of k-slices S and the team size W are chosen on the
-// host so that (i) a slice of the activations (all columns, kc tiles of k) fits in shared memory whatever K is,
-// and (ii) every warp of the grid has about the same number of tiles however few rows the weight has (a
-// 1024-row shard has 64 row-tiles for 2368 warps).  The CTAs are dealt to the slices round-robin (CTA c works
-// on slice c mod S); the CTAs of a slice split its row-tiles evenly, and so do the teams of a CTA.  A CTA stages
-// only its own slice of x.
+// Work split.  K is cut into S slices of kc k-tiles so that a slice of the activations (all columns) fits in shared memory
+// and, where a weight has few rows, so that every SM gets some of it.  A unit is one row-tile (16 rows) times one slice.
+// A CTA owns consecutive units of one slice; its 16 warps cut the run of their tiles into 16 equal runs, wherever that
+// falls: a warp keeps its sums in registers while it stays inside a unit and leaves them in shared memory (a "piece") when
+// it leaves the unit or its run ends.  After a barrier the warps add each unit's pieces in warp order.  Units are taken in
+// batches as large as the pieces' shared memory allows: mostly one; the first tiles of the next batch are requested before
+// a batch is added up.
 //
-// With S > 1 (or fp32 activations, whose three columns per token are combined at the end) a unit's sums go to a
-// partial-sum buffer [slice][column][row]; the warp then counts itself on the row-tile's arrival counter, and
-// the warp that finds all other slices already counted adds the S partial sums in slice order and stores y
-// (it also puts the counter back to zero).  The order of the additions is fixed, so the result does not depend
-// on which warp comes last; nobody waits for anybody.  With S = 1 and bf16 activations y is stored directly.
+// Slices.  With S = 1 the sums are y.  With S = 2 .. 8 the CTAs of the S slices form a cluster that shares its row-tiles
+// out: each CTA sends the sums of a unit to the CTA that owns the row-tile (st.async into its shared memory, counted by an
+// mbarrier there), which adds the slices in order and stores y.  Only a K too long for eight slices (32 columns beyond
+// 25600, 16 beyond 51200) goes through memory: partial sums [row-tile][slice], an arrival counter per row-tile, and the
+// warp that finds all other slices already counted adds them, in slice order, and puts the counter back to zero.  Nowhere
+// does the result depend on who comes last, and nobody waits for a CTA outside its cluster.
+//
+// What bounds it: at few columns the weight bytes; at 9 and more the instructions (per 32-k block and eight columns a
+// 16-byte and an 8-byte shared load, two MMAs, four FMAs); on small shards the chain launch - activations - tiles - sums.
+// Teams of warps per row-tile and partial
+// sums in memory for every S > 1 took, 16 columns, Q4_K: 1024 x 8192 10.1 us, 3584 x 8192 15.8, 1024 x 28672 19.3; the even
+// cut and the clusters take 5.8, 11.9 and 13.0.  4096 x 4096 Q4_0, one slice: 5.5 -> 4.6 at 4 columns, 9.2 -> 6.7 at 16,
+// 17.0 -> 9.9 at 32.
 //
 // Replaces, for up to 32 tokens, the fp32 batch_matmul_f32 launch of
 // warpforge-backend-nvidia/src/main/java/io/surfworks/warpforge/backend/nvidia/ops/DotGeneralKernel.java:263-281.
@@ -29,11 +35,11 @@
 
 namespace wf {
 
-// weight of a staged activation byte against a streamed weight byte in the planner's estimate (measured: 1 - 3 give
-// the same cuts for up to 8 columns, 2 the best ones for 16; 6 and more cut K too finely)
-constexpr int GEMVN_STAGE_COST = 2;
 constexpr int GEMVN_MAX_COLS = 32;
 constexpr int GEMVN_MAX_SLICES = 64;
+constexpr int GEMVN_MAX_CLUSTER = 8;  // slices that meet in a cluster (the largest portable size)
+constexpr int GEMVN_MAX_BATCH = 64;   // units a CTA adds up at a time
+constexpr size_t GEMVN_SMEM = 200 * 1024;
 constexpr size_t GEMVN_PART_BYTES = 8u << 20;  // partial sums a launch may use (the static array of the no-alloc entry is this large)
 constexpr int GEMVN_MAX_ROW_TILES = 1 << 16;   // arrival counters
 
@@ -41,78 +47,86 @@ struct GemvNParams {
     const uint8_t* tiles;
     const void* x;
     float* y;
-    float* part;  // [slices][cols][rt * 16], used unless slices == 1 with bf16 activations
+    float* part;  // [rt][slices][column pairs][8] float4, used beyond GEMVN_MAX_CLUSTER slices
     int* count;   // [rt] arrivals per row-tile, zero between launches
     int* status;
     int64_t ldy, col0, ldx;
     int rows, k, kt, rt;
-    int m, x_f32, cols;  // cols = activation columns = m (bf16) or 3 m (fp32)
-    int slices, kc;      // k-slices; k-tiles per slice (the last slice may have fewer)
-    int team;            // warps that share a unit (they cut its k-tiles among themselves)
-    int sx;              // bytes per staged activation row
-    int piece_off;       // byte offset of the team hand-over buffers in shared memory
+    int m, x_f32, cols;     // cols = activation columns = m (bf16) or 3 m (fp32)
+    int slices, kc, batch;  // k-slices; k-tiles per slice (the last slice may have fewer); units added up at a time
+    int cluster;            // the slices of a row-tile are the CTAs of a cluster
+    int sx;                 // bytes per staged activation row
+    int piece_off, ex_off;  // byte offsets in shared memory: pieces; sums on their way to y
     unsigned long long* timing;
 };
 
 template <int QT, int NG> struct GemvNGeom {
     // tiles a warp holds in registers while it multiplies: what 128 registers per thread leave room for
-    static constexpr int DEPTH = (QT == WF_QTYPE_Q4_0) ? (NG == 4 ? 3 : 4) : (QT == WF_QTYPE_Q4_1) ? 3 : 2;
+        static constexpr int DEPTH = (QT == WF_QTYPE_Q4_0) ? (NG == 4 ? 3 : 4) : (QT == WF_QTYPE_Q4_1) ? 3 : (QT == WF_QTYPE_Q8_0 && NG == 1) ? 3 : 2;
 };
 
-// Shared memory: start values [kc * TK / 32][NG][4] float2 | staged x [cols][sx] | team hand-over [2][16][32] NG float4.
-inline size_t gemvn_smem(int qt, int kc, int cols, int ng, int team, int* sx_out, int* piece_off_out) {
-    const int kslice = kc * tile_k(qt);
+// Shared memory: control 128 | start values [kc * TK / 32][NG][4] float2 | staged x [cols][sx] | pieces [batch + 15][NG][32]
+// float4 | sums of the CTA's own row-tiles [slices][ceil(batch / slices)][NG][32] float4 (a cluster's exchange, or fp32
+// tokens, whose three columns meet there).
+inline size_t gemvn_smem(int qt, int kc, int cols, bool x_f32, int slices, int batch, int* sx_out, int* piece_off_out, int* ex_off_out) {
+    const int kslice = kc * tile_k(qt), ng = cols <= 8 ? 1 : cols <= 16 ? 2 : 4;
     const int sx = kslice * 2 + 64;  // +64: consecutive rows start 16 banks apart
     if (sx_out) *sx_out = sx;
     size_t b = 128 + (size_t)(kslice / 32) * ng * 32 + (size_t)cols * sx;
     b = (b + 127) & ~(size_t)127;
     if (piece_off_out) *piece_off_out = (int)b;
-    if (team > 1) b += (size_t)2 * GEMV_WARPS * 32 * ng * 16;
+    b += (size_t)(batch + GEMV_WARPS - 1) * ng * 512;
+    if (ex_off_out) *ex_off_out = (int)b;
+    if (slices <= GEMVN_MAX_CLUSTER && (slices > 1 || x_f32)) b += (size_t)slices * ((batch + slices - 1) / slices) * ng * 512;
     return b;
 }
 
 struct GemvNPlan {
-    int slices = 0, kc = 0, team = 1;  // slices == 0: no plan fits
-    bool uses_part = false;
+    int slices = 0, kc = 0, batch = 0;  // slices == 0: no plan fits
+    int ctas = 0;                       // CTAs (per slice, where the slices form clusters)
+    bool part = false;                  // partial sums go through memory
 };
-// The cheapest (S, W) by the estimate "what the busiest warp moves", in sixteenths of a tile: per slice,
-// ceil(row-tiles / teams of the slice) units; per unit the member's share of the kc tiles, the hand-over inside
-// the team (W > 1) and the partial sums written (cols x 64 bytes, S > 1); for the warp that completes a row-tile
-// the S partial sums read back and two tiles' worth of round trips; for every warp its sixteenth of the CTA's
-// activation staging (cols x kc tiles of k, bf16; all CTAs of a slice read the same lines of the L2).
-inline GemvNPlan gemvn_plan(int sm_count, int qt, int64_t rt, int64_t kt, int cols, bool x_f32) {
+// clusters[S]: how many clusters of S CTAs the device holds at a time (S = 1: SMs).  The cheapest cut by an estimate in
+// nanoseconds: the busiest warp's tiles, the staging of the slice, and per batch the way of its sums to y.  The constants
+// are a fit to 78 measured weights from 128 x 8192 to 28014 x 2496 with 2 .. 32 columns, each at every S up to 8: its choices
+// are 1.5 % slower than the best S on average, 19 % at worst.  Memory is the way where eight slices do not fit (against a
+// cluster of the same S it measured 1 - 4 us more on small weights and within 8 % either way on tall ones).
+inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt, int cols, bool x_f32) {
     GemvNPlan best;
-    const int ng = cols <= 8 ? 1 : cols <= 16 ? 2 : 4;
-    int64_t best_cost = -1;
+    const int ng = cols <= 8 ? 1 : cols <= 16 ? 2 : 4, tk = tile_k(qt), sms = clusters[1];
+    const double per_group = 15.9 + (qt == WF_QTYPE_Q4_1 ? 3.3 : qt == WF_QTYPE_Q8_0 ? 16.3 : qt == WF_QTYPE_Q4_K ? 5.0 : 0.0);
+    const double tile_ns = (tk / 128) * (17.3 + per_group * ng);  // one SM's time per tile
+    double best_ns = 0;
     int last_kc = 0;
-    static const int team_sizes[] = {1, 2, 3, 4, 5, 8, 16};
-    for (int s = 1; s <= GEMVN_MAX_SLICES && s <= kt && s <= sm_count; s++) {
+    for (int s = 1; s <= GEMVN_MAX_SLICES && s <= kt && s <= sms; s++) {
         const int kc = (int)((kt + s - 1) / s), slices = (int)((kt + kc - 1) / kc);
         if (kc == last_kc) continue;
         last_kc = kc;
-        const bool part = slices > 1 || x_f32;
-        if (part && (size_t)slices * cols * rt * 16 * 4 > GEMVN_PART_BYTES) continue;
-        const int64_t tb = tile_bytes(qt), part16 = part ? ((int64_t)cols * 64 * 16 + tb - 1) / tb : 0;
-        for (int w : team_sizes) {
-            if (gemvn_smem(qt, kc, cols, ng, w, nullptr, nullptr) > 200 * 1024) continue;
-            const int teams = GEMV_WARPS / w;
-            int64_t cost = 0;
-            for (int sl = 0; sl < slices; sl++) {
-                const int64_t ctas = (sm_count - sl + slices - 1) / slices;
-                const int64_t kcs = std::min<int64_t>(kc, kt - (int64_t)sl * kc);
-                const int64_t units_cta = (rt + ctas - 1) / ctas, units_team = (units_cta + teams - 1) / teams;
-                cost = std::max(cost, units_team * (((kcs + w - 1) / w) * 16 + (w > 1 ? 4 + w : 0) + part16));
-            }
-            if (part) cost += slices * part16 + 32;
-            // every CTA stages cols x kc tiles of k of the activations (from L2, by all its warps together)
-            cost += ((int64_t)cols * kc * tile_k(qt) * GEMVN_STAGE_COST + tb - 1) / tb;
-            if (best_cost < 0 || cost < best_cost) {
-                best_cost = cost;
-                best.slices = slices;
-                best.kc = kc;
-                best.team = w;
-                best.uses_part = part;
-            }
+        const bool part = slices > GEMVN_MAX_CLUSTER;
+        // (what wf_plan_several_tokens promises of every cut; a cluster's sums do not need the buffer)
+        if (slices > 1 && (size_t)slices * ((cols + 1) & ~1) * rt * 16 * 4 > GEMVN_PART_BYTES) continue;
+        const int64_t room = part ? sms / slices : clusters[slices];  // CTAs a slice gets, at least
+        if (room < 1) continue;
+        const int64_t units = (rt + std::min(room, rt) - 1) / std::min(room, rt);  // of the busiest CTA
+        int batch = (int)std::min<int64_t>(units, GEMVN_MAX_BATCH);
+        while (batch >= 1 && gemvn_smem(qt, kc, cols, x_f32, slices, batch, nullptr, nullptr, nullptr) > GEMVN_SMEM) batch--;
+        if (batch < 1) continue;
+        double ns = (double)cols * kc * tk * 2 / (x_f32 ? 27.2 : 87.3);
+        for (int64_t left = units; left > 0; left -= batch) {
+            const int nb = (int)std::min<int64_t>(batch, left), own = (nb + slices - 1) / slices;
+            ns += ((nb * kc + GEMV_WARPS - 1) / GEMV_WARPS) * GEMV_WARPS * tile_ns;
+            ns += 847.0 + (x_f32 ? 270.0 : 223.0) * ((nb * ng + GEMV_WARPS - 1) / GEMV_WARPS);
+            if (part) ns += 1313.0 + 119.4 * nb * ng + 145.2 * slices;
+            else if (slices > 1) ns += 616.0 + slices * (6.1 + 32.1 * ((own * ng + GEMV_WARPS - 1) / GEMV_WARPS));
+            if (x_f32 && !part) ns += 31.1 * slices * ((own * (cols / 3) * 16 + GEMV_CONSUMERS - 1) / GEMV_CONSUMERS);
+        }
+        if (best.slices == 0 || ns < best_ns) {
+            best_ns = ns;
+            best.slices = slices;
+            best.kc = kc;
+            best.batch = batch;
+            best.ctas = (int)std::min(room, rt);
+            best.part = part;
         }
     }
     return best;
@@ -129,11 +143,12 @@ inline GemvNPlan gemvn_plan(int sm_count, int qt, int64_t rt, int64_t kt, int co
 static __device__ void stage_x_slice_bulk(const GemvNParams& p, uint8_t* xs, float* cinit, int k_lo, int kslice, int ng, float beta,
                                           int nthreads, uint32_t bar, uint32_t abort32) {
     const int valid = max(0, min(kslice, p.k - k_lo));  // elements of the slice that exist
-    if (threadIdx.x == 0) {
-        mbar_expect_tx(bar, (uint32_t)(p.m * valid * 2));
-        for (int t = 0; t < p.m; t++)
-            if (valid > 0)
-                bulk_load(smem_u32(xs + (size_t)t * p.sx), static_cast<const uint16_t*>(p.x) + (size_t)t * p.ldx + k_lo, (uint32_t)valid * 2, bar);
+    if (threadIdx.x < 32) {  // one token per lane
+        if (threadIdx.x == 0) mbar_expect_tx(bar, (uint32_t)(p.m * valid * 2));
+        __syncwarp();
+        const int t = threadIdx.x;
+        if (t < p.m && valid > 0)
+            bulk_load(smem_u32(xs + (size_t)t * p.sx), static_cast<const uint16_t*>(p.x) + (size_t)t * p.ldx + k_lo, (uint32_t)valid * 2, bar);
     }
     if (valid < kslice) {  // K ends inside the slice: zeros behind it (k is a multiple of 32, so whole 16-byte pieces)
         const int pieces = (kslice - valid) >> 3;
@@ -144,14 +159,17 @@ static __device__ void stage_x_slice_bulk(const GemvNParams& p, uint8_t* xs, flo
         __syncthreads();
     }
     mbar_wait_or_abort(bar, 0, abort32);
+    // Neighbouring threads take neighbouring tokens of one block: their rows start 16 banks apart, so every second one
+    // meets the banks of the first, and each such pair starts at another of the block's four 16-byte runs (taken
+    // through an exclusive or, which leaves the pairs of the final additions what they are).
     const int nblk = kslice >> 5;
     for (int i = threadIdx.x; i < p.m * nblk; i += nthreads) {
-        const int t = i / nblk, b = i - t * nblk;
+        const int b = i / p.m, t = i - b * p.m, rot = (threadIdx.x >> 1) & 3;
         const uint4* src = reinterpret_cast<const uint4*>(xs + (size_t)t * p.sx + (size_t)b * 64);
         float part[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const uint4 v = src[j];
+            const uint4 v = src[j ^ rot];
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
             float sum = 0.f;
 #pragma unroll
@@ -193,46 +211,66 @@ static __device__ void stage_x_slice(const GemvNParams& p, uint8_t* xs, float* c
             for (int s = 0; s < parts; s++) blk[p.x_f32 ? 3 * t + s : t] = beta * sum[s];
         }
     };
-    for (int raw = threadIdx.x; raw < padded; raw += nthreads) {  // warp-uniform trip counts
-        const int idx = item(raw);
-        const bool live = idx < total;
-        const int t = live ? idx / groups : 0, c8 = live ? idx - t * groups : 0;
-        const int kk = k_lo + c8 * 8;
-        const bool in_k = live && kk < p.k;
-        float sum[3] = {0.f, 0.f, 0.f};
-        float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (in_k) {
-            const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(p.x) + (size_t)t * p.ldx + kk);
-            const float4 a = __ldcg(src), b = __ldcg(src + 1);
-            f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-        }
-        uint32_t hi[4], mid[4], lo[4];
+    // four items' loads in flight: one after the other, each paid a trip to the L2
+    constexpr int AHEAD = 4;
+    for (int raw0 = threadIdx.x; raw0 < padded; raw0 += AHEAD * nthreads) {  // warp-uniform trip counts
+        float4 va[AHEAD], vb[AHEAD];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float x0 = f[2 * i], x1 = f[2 * i + 1];
-            const float h0 = __uint_as_float(__float_as_uint(x0) & 0xFFFF0000u);
-            const float h1 = __uint_as_float(__float_as_uint(x1) & 0xFFFF0000u);
-            const float r0 = x0 - h0, r1 = x1 - h1;
-            const float m0 = __uint_as_float(__float_as_uint(r0) & 0xFFFF0000u);
-            const float m1 = __uint_as_float(__float_as_uint(r1) & 0xFFFF0000u);
-            const float l0 = r0 - m0, l1 = r1 - m1;  // at most 8 significant bits left: exact in bf16
-            hi[i] = pack_bf16_trunc(h0, h1);
-            mid[i] = pack_bf16_trunc(m0, m1);
-            lo[i] = pack_bf16_trunc(l0, l1);
-            sum[0] += h0 + h1;
-            sum[1] += m0 + m1;
-            sum[2] += l0 + l1;
+        for (int j = 0; j < AHEAD; j++) {
+            const int raw = raw0 + j * nthreads, idx = raw < padded ? item(raw) : total;
+            const int t = idx < total ? idx / groups : 0, c8 = idx - t * groups, kk = k_lo + c8 * 8;
+            va[j] = vb[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (idx < total && kk < p.k) {
+                const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(p.x) + (size_t)t * p.ldx + kk);
+                va[j] = __ldcg(src);
+                vb[j] = __ldcg(src + 1);
+            }
         }
-        if (live) {
-            *reinterpret_cast<uint4*>(xs + (size_t)(3 * t) * p.sx + c8 * 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(xs + (size_t)(3 * t + 1) * p.sx + c8 * 16) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
-            *reinterpret_cast<uint4*>(xs + (size_t)(3 * t + 2) * p.sx + c8 * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) {
+            const int raw = raw0 + j * nthreads;
+            if (raw >= padded) break;
+            const int idx = item(raw);
+            const bool live = idx < total;
+            const int t = live ? idx / groups : 0, c8 = live ? idx - t * groups : 0;
+            float sum[3] = {0.f, 0.f, 0.f};
+            const float f[8] = {va[j].x, va[j].y, va[j].z, va[j].w, vb[j].x, vb[j].y, vb[j].z, vb[j].w};
+            uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float x0 = f[2 * i], x1 = f[2 * i + 1];
+                const float h0 = __uint_as_float(__float_as_uint(x0) & 0xFFFF0000u);
+                const float h1 = __uint_as_float(__float_as_uint(x1) & 0xFFFF0000u);
+                const float r0 = x0 - h0, r1 = x1 - h1;
+                const float m0 = __uint_as_float(__float_as_uint(r0) & 0xFFFF0000u);
+                const float m1 = __uint_as_float(__float_as_uint(r1) & 0xFFFF0000u);
+                const float l0 = r0 - m0, l1 = r1 - m1;  // at most 8 significant bits left: exact in bf16
+                hi[i] = pack_bf16_trunc(h0, h1);
+                mid[i] = pack_bf16_trunc(m0, m1);
+                lo[i] = pack_bf16_trunc(l0, l1);
+                sum[0] += h0 + h1;
+                sum[1] += m0 + m1;
+                sum[2] += l0 + l1;
+            }
+            if (live) {
+                *reinterpret_cast<uint4*>(xs + (size_t)(3 * t) * p.sx + c8 * 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(xs + (size_t)(3 * t + 1) * p.sx + c8 * 16) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+                *reinterpret_cast<uint4*>(xs + (size_t)(3 * t + 2) * p.sx + c8 * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            }
+            block_sums(sum, live, t, c8);
         }
-        block_sums(sum, live, t, c8);
     }
 }
 
-template <int QT, int NG>
+// What lies between a unit's sums and y.  Its own kernel for each of the two ways that most calls take: the code after the
+// last tile runs once and is fetched from the L2, so the branches it would jump over cost a small call 0.4 us.
+enum GemvNWay {
+    WAY_DIRECT,   // one slice, bf16 tokens: straight to y
+    WAY_CLUSTER,  // the slices of bf16 tokens meet in a cluster
+    WAY_ANY       // fp32 tokens, or partial sums in memory
+};
+
+template <int QT, int NG, int WAY>
 __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNParams p) {
     using T = Tile<QT>;
     using R = TileRegs<QT>;
@@ -242,20 +280,11 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNPar
 
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    const int S = p.slices, slice = (int)blockIdx.x % S, idx = (int)blockIdx.x / S;
-    const int ctas = ((int)gridDim.x - slice + S - 1) / S;  // CTAs working on this slice
+    const int S = WAY == WAY_DIRECT ? 1 : p.slices, slice = (int)blockIdx.x % S, idx = (int)blockIdx.x / S;  // slice = rank in the cluster
+    const int ctas = ((int)gridDim.x - slice + S - 1) / S;                                                    // CTAs working on this slice
     const int k0t = slice * p.kc, kcs = min(p.kc, p.kt - k0t);
-    // teams of W warps; a team owns whole units, its members cut a unit's k-tiles among themselves
-    const int W = p.team, teams = GEMV_WARPS / W;
-    const int team = warp / W, member = warp - team * W;
-    const bool idle = team >= teams;
-    // this CTA's row-tiles of the slice, this team's share of them
-    const int u0 = (int)((int64_t)idx * p.rt / ctas), u1 = (int)((int64_t)(idx + 1) * p.rt / ctas);
-    const int nu = u1 - u0, tq = nu / teams, tr = nu - tq * teams;
-    const int ua = idle ? 0 : u0 + team * tq + min(team, tr), ub = idle ? 0 : ua + tq + (team < tr ? 1 : 0);
-    // this member's k-tiles inside every unit
-    const int ma = member * kcs / W, mb = (member + 1) * kcs / W, ml = mb - ma;
-    const int nt = (ub - ua) * ml;  // tiles of this warp
+    const int u0 = (int)((unsigned)(idx * p.rt) / (unsigned)ctas), nu = (int)((unsigned)((idx + 1) * p.rt) / (unsigned)ctas) - u0;  // its units
+    const bool cluster = WAY == WAY_CLUSTER || (WAY == WAY_ANY && p.cluster), f32 = WAY == WAY_ANY && p.x_f32;
 
     auto stamp = [&](int i) {
         if (p.timing != nullptr && threadIdx.x == 0) {
@@ -268,175 +297,240 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNPar
     // tiles are requested before the wait for the previous grid.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     stamp(3);
+    // A batch: its units and tiles, this warp's run of them [lo, lo + nt), the unit and k-tile the run starts in.
+    int nb = 0, total = 0, nt = 0, unit = 0, kk = 0;
     R slots[DEPTH];
-    const uint8_t* lptr = p.tiles + ((size_t)ua * p.kt + k0t + ma) * T::BYTES;
-    int lkk = 0, lrem = nt;
+    const uint8_t* lptr = p.tiles;
+    int lkk = 0, lrem = 0;
     auto load_next = [&](R& slot) {
         if (lrem > 0) {
             slot.load_global_n(lptr, lane);
             lrem--;
             lptr += T::BYTES;
-            if (++lkk == ml) {  // next unit: the same k-tiles of the next row-tile
+            if (++lkk == kcs) {  // next unit: the same k-tiles of the next row-tile
                 lkk = 0;
-                lptr += (size_t)(p.kt - ml) * T::BYTES;
+                lptr += (size_t)(p.kt - kcs) * T::BYTES;
             }
         }
     };
-    static_for<DEPTH>([&](auto J) { load_next(slots[decltype(J)::value]); });
-    // control words: mbarrier of the activation copies at 0, abort word at 8
+    auto open_batch = [&](int b0) {
+        nb = min(p.batch, nu - b0);
+        total = nb * kcs;
+        // 16 equal runs; one tile for each of the first warps where there are fewer
+        const bool each = total < GEMV_WARPS;
+        const int lo = each ? min(warp, total) : (int)((unsigned)(warp * total) / GEMV_WARPS);
+        nt = (each ? min(warp + 1, total) : (int)((unsigned)((warp + 1) * total) / GEMV_WARPS)) - lo;
+        unit = (int)((unsigned)lo / (unsigned)kcs);
+        kk = lkk = lo - unit * kcs;
+        lrem = nt;
+        lptr = p.tiles + ((size_t)(u0 + b0 + unit) * p.kt + k0t + kk) * T::BYTES;
+        static_for<DEPTH>([&](auto J) { load_next(slots[decltype(J)::value]); });
+    };
+    open_batch(0);
+    // control words: mbarrier of the activation copies at 0, abort word at 8, mbarrier of the cluster's sums at 16, the units
+    // that this CTA completed: their number at 24, they at 32 .. 95
+    const uint32_t abort32 = smem_u32(smem + 8), sums_bar = smem_u32(smem + 16);
     if (threadIdx.x == 0) {
         *reinterpret_cast<volatile int*>(smem + 8) = 0;
         mbar_init(smem_u32(smem), 1);
+        mbar_init(sums_bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    // the others may send sums here from now on; waited for before the first ones are sent
+    if (cluster) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
 
     float* cinit = reinterpret_cast<float*>(smem + 128);  // [kslice / 32][NG][4] float2
     const int kslice = kcs * T::K;
     uint8_t* xs = reinterpret_cast<uint8_t*>(cinit + (size_t)(p.kc * T::K / 32) * NG * 8);
-    // team hand-over: [2][warp][lane] NG float4, after the staged activations
-    float4* pieces = reinterpret_cast<float4*>(smem + p.piece_off);
+    float4* const pieces = reinterpret_cast<float4*>(smem + p.piece_off);  // [unit of the batch + warp][NG][32]
+    float4* const sums = reinterpret_cast<float4*>(smem + p.ex_off);       // [slice][own unit][NG][32]
 
     asm volatile("griddepcontrol.wait;" ::: "memory");
     stamp(0);
-    if (p.x_f32) stage_x_slice(p, xs, cinit, k0t * T::K, kslice, NG, R::BETA, GEMV_CONSUMERS);
-    else stage_x_slice_bulk(p, xs, cinit, k0t * T::K, kslice, NG, R::BETA, GEMV_CONSUMERS, smem_u32(smem), smem_u32(smem + 8));
+    if (f32) stage_x_slice(p, xs, cinit, k0t * T::K, kslice, NG, R::BETA, GEMV_CONSUMERS);
+    else stage_x_slice_bulk(p, xs, cinit, k0t * T::K, kslice, NG, R::BETA, GEMV_CONSUMERS, smem_u32(smem), abort32);
     __syncthreads();
     stamp(1);
-    if (*reinterpret_cast<volatile int*>(smem + 8)) {  // the copies did not land in time: y would be garbage
+    if (*reinterpret_cast<volatile int*>(smem + 8)) {  // the copies did not land in time: y will be garbage, the status says so
         if (threadIdx.x == 0) report_status(p.status, STATUS_GEMV_FIXUP_TIMEOUT);
         drain_after_abort();
-        return;
     }
-    if (idle) return;
 
     // dead columns read the last live row: their results are computed and never stored
     uint32_t xg[NG];
 #pragma unroll
-    for (int gi = 0; gi < NG; gi++) xg[gi] = smem_u32(xs) + (uint32_t)min(8 * gi + g, p.cols - 1) * p.sx + q * 16 + (uint32_t)ma * XSTEP;
-    const uint32_t c32 = smem_u32(cinit) + q * 8 + (uint32_t)ma * CSTEP;
-    const bool direct = S == 1 && !p.x_f32;
-    const int64_t prow = (int64_t)p.rt * 16;
+    for (int gi = 0; gi < NG; gi++) xg[gi] = smem_u32(xs) + (uint32_t)min(8 * gi + g, p.cols - 1) * p.sx + q * 16;
+    const uint32_t c32 = smem_u32(cinit) + q * 8;
+    const int pairs = (p.cols + 1) >> 1;  // live column pairs: a lane's float4 is one of them in two rows
 
-    float acc[NG][4];
-#pragma unroll
-    for (int gi = 0; gi < NG; gi++) acc[gi][0] = acc[gi][1] = acc[gi][2] = acc[gi][3] = 0.f;
-
-    // member 0 of the team, holding the unit's complete sums: store them (or count the slice in and add the slices)
-    auto store_unit = [&](int u) {
-        const int r0 = u * 16 + g, r1 = r0 + 8;
-        if (direct) {
-#pragma unroll
-            for (int gi = 0; gi < NG; gi++)
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int col = 8 * gi + 2 * q + e;
-                    if (col < p.cols) {
-                        if (r0 < p.rows) p.y[(int64_t)col * p.ldy + p.col0 + r0] = acc[gi][e];
-                        if (r1 < p.rows) p.y[(int64_t)col * p.ldy + p.col0 + r1] = acc[gi][2 + e];
-                    }
-                }
-            return;
+    // a unit's sums of eight columns, as the lanes hold them, to y (bf16 tokens)
+    auto store_y = [&](int u, int gi, const float4& v) {
+        const int r0 = u * 16 + g, r1 = r0 + 8, col = 8 * gi + 2 * q;
+        float* const y = p.y + (int64_t)col * p.ldy + p.col0 + r0;
+        if (col < p.cols) {
+            if (r0 < p.rows) y[0] = v.x;
+            if (r1 < p.rows) y[8] = v.z;
         }
-        float* mine = p.part + (int64_t)slice * p.cols * prow;
-#pragma unroll
-        for (int gi = 0; gi < NG; gi++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int col = 8 * gi + 2 * q + e;
-                if (col < p.cols) {
-                    __stcg(mine + (int64_t)col * prow + r0, acc[gi][e]);
-                    __stcg(mine + (int64_t)col * prow + r1, acc[gi][2 + e]);
-                }
-            }
-        // count this slice in; the warp that completes the row-tile adds the slices in order
-        __syncwarp();
-        int old = 0;
-        if (lane == 0) {
-            __threadfence();
-            old = atomicAdd(p.count + u, 1);
-        }
-        old = __shfl_sync(0xFFFFFFFFu, old, 0);
-        if (old != S - 1) return;
-        if (lane == 0) p.count[u] = 0;  // nobody else touches it again in this launch
-        __threadfence();
-        // four (token, row) sums per lane at a time, so that the loads of a slice do not wait for one another
-        const int items = p.m * 16;
-        const int64_t sstride = (int64_t)p.cols * prow;
-        for (int i0 = lane; i0 < items; i0 += 128) {
-            float v[4] = {0.f, 0.f, 0.f, 0.f};
-            const float* src[4];
-#pragma unroll
-            for (int w = 0; w < 4; w++) {
-                const int i = min(i0 + 32 * w, items - 1), tok = i >> 4;
-                src[w] = p.part + (int64_t)(p.x_f32 ? 3 * tok : tok) * prow + u * 16 + (i & 15);
-            }
-            for (int s = 0; s < S; s++) {
-#pragma unroll
-                for (int w = 0; w < 4; w++) {
-                    const float* ps = src[w] + (int64_t)s * sstride;
-                    // fp32 activations: columns 3t, 3t+1, 3t+2 are the hi / mid / lo parts of token t
-                    v[w] += p.x_f32 ? (__ldcg(ps + 2 * prow) + __ldcg(ps + prow)) + __ldcg(ps) : __ldcg(ps);
-                }
-            }
-#pragma unroll
-            for (int w = 0; w < 4; w++) {
-                const int i = i0 + 32 * w, row = u * 16 + (i & 15);
-                if (i < items && row < p.rows) p.y[(int64_t)(i >> 4) * p.ldy + p.col0 + row] = v[w];
-            }
+        if (col + 1 < p.cols) {
+            if (r0 < p.rows) y[p.ldy] = v.y;
+            if (r1 < p.rows) y[p.ldy + 8] = v.w;
         }
     };
+    // place of (column, row) among a unit's float4s, in floats
+    auto place = [](int col, int row) { return ((col >> 3) * 32 + (row & 7) * 4 + ((col & 7) >> 1)) * 4 + (row >> 3) * 2 + (col & 1); };
 
-    // end of a unit: the members hand their sums to member 0 through shared memory (two buffers, alternating by
-    // unit, one named barrier per team and unit), member 0 adds them in member order
-    int parity = 0;
-    auto finish_unit = [&](int u) {
-        if (W > 1) {
-            float4* buf = pieces + ((size_t)parity * GEMV_WARPS + warp) * 32 * NG + lane;
-            if (member != 0) {
-#pragma unroll
-                for (int gi = 0; gi < NG; gi++) buf[gi * 32] = make_float4(acc[gi][0], acc[gi][1], acc[gi][2], acc[gi][3]);
-            }
-            asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(W * 32) : "memory");
-            if (member == 0) {
-                for (int j = 1; j < W; j++) {
-#pragma unroll
-                    for (int gi = 0; gi < NG; gi++) {
-                        const float4 v = buf[(size_t)j * 32 * NG + gi * 32];
-                        acc[gi][0] += v.x;
-                        acc[gi][1] += v.y;
-                        acc[gi][2] += v.z;
-                        acc[gi][3] += v.w;
-                    }
-                }
-            }
-            parity ^= 1;
-        }
-        if (member == 0) store_unit(u);
+    for (int b0 = 0, round = 0; b0 < nu; b0 += p.batch, round++) {
+        float acc[NG][4];
 #pragma unroll
         for (int gi = 0; gi < NG; gi++) acc[gi][0] = acc[gi][1] = acc[gi][2] = acc[gi][3] = 0.f;
-    };
+        for (int g0 = 0; g0 < nt; g0 += DEPTH) {
+            static_for<DEPTH>([&](auto J) {
+                constexpr int j = decltype(J)::value;
+                if (g0 + j < nt) {
+                    slots[j].template compute_n<NG>(acc, xg, (uint32_t)kk * XSTEP, c32 + (uint32_t)kk * CSTEP);
+                    load_next(slots[j]);
+                    if (++kk == kcs || g0 + j + 1 == nt) {  // the piece's place is its own: unit + warp grows along the run
+                        float4* const to = pieces + (size_t)(unit + warp) * NG * 32 + lane;
+#pragma unroll
+                        for (int gi = 0; gi < NG; gi++) {
+                            to[gi * 32] = make_float4(acc[gi][0], acc[gi][1], acc[gi][2], acc[gi][3]);
+                            acc[gi][0] = acc[gi][1] = acc[gi][2] = acc[gi][3] = 0.f;
+                        }
+                        unit++;
+                        kk = 0;
+                    }
+                }
+            });
+        }
+        const int bn = nb, btotal = total;
+        const bool more = b0 + p.batch < nu;
+        if (more) open_batch(b0 + p.batch);
+        if (b0 == 0) stamp(4);
+        // the warps whose runs, [w total / runs, (w + 1) total / runs), meet the tiles of unit i
+        int w0 = 0, w1 = 0;
+        const int runs = min(btotal, GEMV_WARPS);
+        auto holders = [&](int i) {
+            w0 = (int)((unsigned)((i * kcs + 1) * runs - 1) / (unsigned)btotal);
+            w1 = (int)((unsigned)((i + 1) * kcs * runs - 1) / (unsigned)btotal);
+        };
+        if (warp < bn * NG) holders(warp / NG);
+        __syncthreads();  // the batch's pieces are there
+        if (cluster) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        const int per_rank = (p.batch + S - 1) / S;                              // places for own units in `sums`
+        const int own = slice < bn ? (bn - slice + S - 1) / S : 0;               // units whose row-tiles this rank stores
+        if (cluster && own > 0 && threadIdx.x == 0) mbar_expect_tx(sums_bar, (uint32_t)(S * own * NG * 512));
 
-    if (ml == 0) {  // fewer k-tiles in the slice than members: this member only keeps the team's barriers company
-        for (int u = ua; u < ub; u++) finish_unit(u);
-        return;
-    }
-    int unit = ua, kk = 0;
-    for (int g0 = 0; g0 < nt; g0 += DEPTH) {
-        static_for<DEPTH>([&](auto J) {
-            constexpr int j = decltype(J)::value;
-            if (g0 + j < nt) {
-                slots[j].template compute_n<NG>(acc, xg, (uint32_t)kk * XSTEP, c32 + (uint32_t)kk * CSTEP);
-                load_next(slots[j]);
-                if (++kk == ml) {
-                    finish_unit(unit);
-                    unit++;
-                    kk = 0;
+        for (int it = warp; it < bn * NG; it += GEMV_WARPS) {
+            const int i = it / NG, gi = it % NG;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int w = w0; w <= w1; w += 4) {  // four pieces in flight
+                float4 a[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    a[j] = w + j <= w1 ? pieces[((size_t)(i + w + j) * NG + gi) * 32 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    v.x += a[j].x;
+                    v.y += a[j].y;
+                    v.z += a[j].z;
+                    v.w += a[j].w;
                 }
             }
-        });
+            if (cluster) {
+                const uint32_t to = smem_u32(sums + ((size_t)(slice * per_rank + i / S) * NG + gi) * 32 + lane);
+                st_async_16(map_to_rank(to, (uint32_t)(i % S)), __float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z),
+                            __float_as_uint(v.w), map_to_rank(sums_bar, (uint32_t)(i % S)));
+            } else if (S > 1) {
+                float4* const to = reinterpret_cast<float4*>(p.part) + (((size_t)(u0 + b0 + i) * S + slice) * pairs + 4 * gi + q) * 8 + g;
+                if (4 * gi + q < pairs) __stcg(to, v);
+            } else if (f32) {
+                sums[((size_t)i * NG + gi) * 32 + lane] = v;
+            } else {
+                store_y(u0 + b0 + i, gi, v);
+            }
+            if (it + GEMV_WARPS < bn * NG) holders((it + GEMV_WARPS) / NG);
+        }
+
+        if (WAY == WAY_DIRECT) {
+            // done
+        } else if (S == 1 || cluster) {
+            if (cluster) {
+                if (own > 0) mbar_wait_or_abort(sums_bar, round & 1, abort32);
+            } else if (f32) {
+                __syncthreads();
+            }
+            if (f32) {  // columns 3t, 3t + 1, 3t + 2 are the hi / mid / lo parts of token t
+                for (int e = threadIdx.x; e < own * p.m * 16; e += GEMV_CONSUMERS) {
+                    const int row = e & 15, j = (e >> 4) / p.m, t = (e >> 4) - j * p.m, r = (u0 + b0 + slice + j * S) * 16 + row;
+                    const int hi = place(3 * t, row), mid = place(3 * t + 1, row), lo = place(3 * t + 2, row);
+                    float v = 0.f;
+                    for (int s = 0; s < S; s++) {
+                        const float* const f = reinterpret_cast<const float*>(sums + (size_t)(s * per_rank + j) * NG * 32);
+                        v += (f[lo] + f[mid]) + f[hi];
+                    }
+                    if (r < p.rows) p.y[(int64_t)t * p.ldy + p.col0 + r] = v;
+                }
+            } else if (cluster) {
+                for (int it = warp; it < own * NG; it += GEMV_WARPS) {
+                    const int j = it / NG, gi = it % NG;
+                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int s = 0; s < S; s++) {
+                        const float4 a = sums[((size_t)(s * per_rank + j) * NG + gi) * 32 + lane];
+                        v.x += a.x;
+                        v.y += a.y;
+                        v.z += a.z;
+                        v.w += a.w;
+                    }
+                    store_y(u0 + b0 + slice + j * S, gi, v);
+                }
+            }
+        } else {
+            // count the units in, list those that this CTA completed, then add their slices
+            int* const listed = reinterpret_cast<int*>(smem + 24);
+            __syncthreads();
+            if (warp == 0) {
+                int n = 0;
+                for (int i = lane; i - lane < bn; i += 32) {
+                    int old = 0, *const count = p.count + u0 + b0 + i;
+                    if (i < bn) asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(old) : "l"(count) : "memory");
+                    const bool last = i < bn && old == S - 1;
+                    const unsigned all = __ballot_sync(0xFFFFFFFFu, last);
+                    if (last) {
+                        *count = 0;  // nobody else touches it again in this launch
+                        smem[32 + n + __popc(all & ((1u << lane) - 1))] = (uint8_t)i;
+                    }
+                    n += __popc(all);
+                }
+                if (lane == 0) *listed = n;
+            }
+            __syncthreads();
+            for (int e = threadIdx.x; e < *listed * p.m * 16; e += GEMV_CONSUMERS) {
+                const int j = e / (p.m * 16), row = e & 15, t = (e - j * p.m * 16) >> 4, u = u0 + b0 + smem[32 + j];
+                // [column pair][row & 7] float4 of {pair} x {row, row + 8}
+                auto at = [&](int col) { return ((col >> 1) * 8 + (row & 7)) * 4 + (row >> 3) * 2 + (col & 1); };
+                const float* const base = p.part + (size_t)u * S * pairs * 32;
+                float v = 0.f;
+#pragma unroll 4
+                for (int s = 0; s < S; s++) {
+                    const float* const f = base + (size_t)s * pairs * 32;
+                    v += f32 ? (__ldcg(f + at(3 * t + 2)) + __ldcg(f + at(3 * t + 1))) + __ldcg(f + at(3 * t)) : __ldcg(f + at(t));
+                }
+                if (u * 16 + row < p.rows) p.y[(int64_t)t * p.ldy + p.col0 + u * 16 + row] = v;
+            }
+        }
+        if (more) {  // this batch's pieces and sums are read
+            __syncthreads();
+            if (cluster) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        }
     }
-    stamp(4);
+    if (*reinterpret_cast<volatile int*>(smem + 8)) {  // a wait ran out: stay until the others' sums have landed
+        if (lane == 0) report_status(p.status, STATUS_GEMV_FIXUP_TIMEOUT);
+        if (cluster) {
+            asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        }
+    }
 }
 
 }  // namespace wf

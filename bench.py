@@ -5,8 +5,9 @@
 
 Workload (benchmark config 4): the 224 Q4_0 projections of a 7B-shape Llama decoder, batch 1,
 every weight a distinct buffer (3.64 GB per token, far larger than L2, so every step reads
-HBM cold).  One step = one token = all projections in layer order, run as ONE persistent
-kernel per GPU (`--mode graph`: one kernel per projection, recorded once as a CUDA graph).
+HBM cold).  One step = one token = all projections in layer order, run as one native program
+(one launch per group of projections that share their activations; with several ranks one
+persistent kernel per GPU; `--mode graph`: one kernel per projection, recorded once as a CUDA graph).
 With N > 1 ranks the weights are row-sharded and every rank ends with all rows of every
 projection: the persistent kernel stores its rows into the other ranks' buffers over NVLink
 from inside the GEMV epilogue (graph mode: a gather kernel after every projection).
@@ -443,8 +444,8 @@ def run_ours(args) -> None:
         stack.build_program(None)
         stack.mode = "program"
     elif mode == "program":
-        # one persistent kernel per token and rank; the row-shard gather is fused into the GEMV
-        # epilogue (peer stores), so no communicator is needed
+        # several ranks: one persistent kernel per token and rank; the row-shard gather is fused into
+        # the GEMV epilogue (peer stores), so no communicator is needed
         stack = ProjectionStack(ctx, spec, tokens=1, rank=rank, world=world, layers=args.layers or None)
         handles = None
         if world > 1:
@@ -524,7 +525,7 @@ def run_ours(args) -> None:
         ms_step = ms / args.steps
         tok_s = 1e3 / ms_step * (world if replicas else 1)
         alg_bytes = stack.algorithmic_bytes_per_step()          # this rank's shard
-        n_launch = 1 if mode in ("program", "replicas") else stack.layers * len(spec.projections)
+        n_launch = max(1, round(launches / args.steps))
         gbs = alg_bytes / (ms_step * 1e-3) / 1e9
         h2d = sum(v.nbytes for v in stack.x_host.values())
         line = {
@@ -535,14 +536,15 @@ def run_ours(args) -> None:
                        "parallelism": (f"{world} independent replicas, one token stream each" if replicas
                                        else f"row-sharded tp{world}" if world > 1 else "single GPU"),
                        "execution": ("one persistent kernel per token, gather fused into the GEMV epilogue (peer stores)"
-                                     if mode == "program" else "one persistent kernel per token and replica" if replicas else "CUDA graph of one GEMV kernel per projection"
+                                     if mode == "program" and world > 1 else "one launch per group of projections that share their activations"
+                                     if mode in ("program", "replicas") else "CUDA graph of one GEMV kernel per projection"
                                      + (" + its gather (one kernel of peer stores; NCCL with WF_GATHER=nccl)" if world > 1 else "")),
                        "l2": "inputs larger than L2: 3.64 GB of distinct weights per step", "bytes_per_token": spec.bytes_per_token()},
             "e2e": {"value": 1e3 / (e2e_ms / args.steps) * (world if replicas else 1), "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": int(y_out.nbytes)},
             "gpu_launches": int(launches),
             "parity": parity,
             "clocks": clocks,
-            "roofline": {"bound": "hbm", "kernel": ("gemv1_program_kernel" if mode in ("program", "replicas") else "gemv1_kernel") + "<Q4_0> (one token)", "achieved": gbs, "peak": hbm_peak, "unit": "GB/s",
+            "roofline": {"bound": "hbm", "kernel": ("gemv1_program_kernel" if mode == "program" and world > 1 else "gemv1_group_kernel" if mode in ("program", "replicas") else "gemv1_kernel") + "<Q4_0> (one token)", "achieved": gbs, "peak": hbm_peak, "unit": "GB/s",
                          "frac": gbs / hbm_peak, "frac_of_8TBs_nominal": gbs / 8000.0, "peak_source": peak_src,
                          "bytes_per_launch": alg_bytes / n_launch, "us_per_launch": ms_step * 1e3 / n_launch,
                          "traffic": NCU_TRAFFIC_BYTES_PER_LAYER * stack.layers / (1 if replicas else world) / n_launch,
@@ -586,7 +588,7 @@ def main() -> None:
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--mode", default="auto", choices=["auto", "graph", "program", "replicas"],
-                    help="program: one persistent kernel per token (default); graph: one kernel per projection in a CUDA graph; "
+                    help="program: the step as one native program (default): a launch per group of projections, with several ranks one persistent kernel; graph: one kernel per projection in a CUDA graph; "
                          "replicas: N > 1 ranks each decode their own stream on the whole model (weak scaling, no exchange)")
     ap.add_argument("--layers", type=int, default=0,
                     help="profiling aid: run only this many of the 32 layers (the line is then marked partial and is not a bench value)")

@@ -261,8 +261,10 @@ int wf_allgather(int64_t ctx, int64_t comm, int64_t send_dev, int64_t recv_dev, 
 /* ---- decode programs ----------------------------------------------------------------
  * A decode step is a fixed list of quantized projections.  The reference would run it as
  * one Backend.execute per op from GraphExecutor's loop (warpforge-core/.../graph/GraphExecutor.java:75-104),
- * each with its own launch and synchronisation; a program runs the whole list as ONE
- * persistent kernel per GPU, streaming the weights of consecutive ops back to back.
+ * each with its own launch and synchronisation; a program issues the whole list in one call, without any host
+ * synchronisation: on one rank as one launch per group of ops that share their activations, each overlapping the
+ * tail of the one before it (programmatic stream serialization); with several ranks as ONE persistent kernel per
+ * GPU, streaming the weights of consecutive ops back to back.
  *   weights[n_ops]           weight handles, all of one quantization type
  *   x_dev[n_ops]             bf16 activations [m, k] each op reads (device pointers)
  *   y_dev[n_ops]             this rank's fp32 output buffer [m, n_total] of each op; after the run it

@@ -38,3 +38,54 @@ def test_exact(rows, k, m, f32):
     w.close()
     backend.close()
     assert np.array_equal(got[0], want) and np.array_equal(got[1], want)
+
+
+@pytest.mark.parametrize("m", [1, 2, 7])
+@pytest.mark.parametrize("ks,shared", [
+    ((1024,) * 6, (0, 1, 1, 1, 1, 1)),      # six weights on one input: two launches
+    ((2080, 2080, 96, 3232), (0, 1, 0, 0)),  # groups of two, one and one
+    ((8192, 8192), (0, 1)),                  # several slices at seven tokens
+    ((1024, 512), (0, 1)),                   # the second reads the first half of what the first staged: the persistent kernel
+])
+def test_program_of_one_rank(m, ks, shared):
+    """A program's projections, joined where they read the same activations; exact as above."""
+    import ctypes
+
+    from warpforge_b200 import _native as N
+    from warpforge_b200.backend import CudaContext, QuantizedWeight
+
+    rng = np.random.default_rng(len(ks) + m)
+    ctx = CudaContext(0)
+    arr = lambda v, t: (t * len(v))(*v)
+    ws, xs, ys, want = [], [], [], []
+    for i, (k, same) in enumerate(zip(ks, shared)):
+        rows = (16, 5000, 33, 700, 1, 2368)[i]
+        codes = rng.integers(0, 16, (rows, k), dtype=np.uint8)
+        blocks = np.zeros((rows, k // 32, 18), np.uint8)
+        blocks[:, :, 0:2] = np.frombuffer(np.float16(1.0).tobytes(), np.uint8)
+        c = codes.reshape(rows, k // 32, 32)
+        blocks[:, :, 2:] = c[:, :, 0::2] | (c[:, :, 1::2] << 4)
+        ws.append(QuantizedWeight(ctx, Q.QuantizationType.Q4_0, blocks.reshape(rows, -1), rows, k))
+        if not same:
+            x = (rng.integers(-8, 9, (m, k)) / 128.0).astype(np.float32)
+            bits = Q.float_to_bf16_bits(x).reshape(m, k)
+            d = ctx.allocate(bits.nbytes)
+            ctx.copy_to_device(d, bits)
+        xs.append(d)
+        ys.append(ctx.allocate(m * rows * 4))
+        want.append(x[:, :k].astype(np.float64) @ (codes.astype(np.float64) - 8.0).T)
+    flags = [0 if same else N.WF_OP_NEW_X | (N.WF_OP_DEPENDS if i else 0) for i, same in enumerate(shared)]
+    prog = ctypes.c_int64()
+    try:
+        ctx._ck("create", ctx._lib.wf_program_create(ctx.handle, len(ws), arr([w.handle for w in ws], ctypes.c_int64), arr(xs, ctypes.c_int64),
+                                                     arr(ys, ctypes.c_int64), arr(flags, ctypes.c_int), m, 1, 0, None, ctypes.byref(prog)))
+        for _ in range(2):
+            ctx._ck("run", ctx._lib.wf_program_run(ctx.handle, prog.value, 0))
+        ctx.synchronize()
+        for y, w in zip(ys, want):
+            got = np.empty(w.shape, np.float32)
+            ctx.copy_to_host(got, y)
+            assert np.array_equal(got, w)
+        ctx._ck("destroy", ctx._lib.wf_program_destroy(ctx.handle, prog.value))
+    finally:
+        ctx.close()

@@ -78,6 +78,102 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvPara
     stamp(5);
 }
 
+// The same for a program: several weights, the fp32 operations before the projection in its staging, a residual in its store.
+// Its own kernel, because what a plain call does not need it would fetch cold and jump over: 2 % of a 4 - 8 us call.
+template <int QT>
+__global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Gemv1GroupParams p) {
+    using T = Tile<QT>;
+    using R = TileRegs<QT>;
+    extern __shared__ __align__(128) uint8_t smem[];
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem);
+    WsPiece* pieces = reinterpret_cast<WsPiece*>(smem + WS_CTRL_BYTES);
+    uint8_t* recs = smem + WS_CTRL_BYTES + WS_PIECE_BYTES;
+    const int kp = p.kt * T::K;
+    uint8_t* xd = recs + (size_t)(kp >> 5) * 32;
+
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);
+    const int lane = threadIdx.x & 31;
+    const int bx = blockIdx.x;
+    int t0, t1;
+    ws_cta_share(bx, (int)gridDim.x, p.chunk_q, p.chunk_r, p.aligned, p.kt, t0, t1);
+    // start, waited, staged, done
+    auto stamp = [&](int i) {
+        if (p.timing != nullptr && threadIdx.x == 0) {
+            unsigned long long tm;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(tm));
+            if (p.timing_at + i < 64) p.timing[(size_t)bx * 64 + p.timing_at + i] = tm;
+        }
+    };
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    stamp(0);
+    auto share_of = [&](int o) {  // this CTA's part of weight o
+        const int begin = o > 0 ? p.op[o - 1].rt_end * p.kt : 0, end = p.op[o].rt_end * p.kt;
+        const int a = max(t0, begin), b = min(t1, end);
+        return WsShare{p.op[o].tiles, a < b ? a - begin : 0, a < b ? b - begin : 0, p.kt, 0, {0, 0}};
+    };
+    constexpr int DEPTH = WsGeom<QT, true>::DEPTH;
+    R slots[DEPTH];
+    WsCursor cur;
+    ws_prime<QT, DEPTH>(slots, cur, share_of, p.n_ops, warp, lane);
+    if (threadIdx.x == 0) {
+        *abort_flag = 0;
+        mbar_init(smem_u32(smem + 16), 1);
+        ws_bars_init(smem);
+    }
+    ws_clear_digits(xd, kp, GEMV_CONSUMERS);
+    __syncthreads();
+    const WsBars bar = ws_bars(smem);
+
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    stamp(1);
+    const int kind = p.x_kind;
+    if (kind == XK_BF16) {
+        stage_x_q8<R::BETA_INT, XK_BF16>(p.x, p.k, xd, recs, kp, GEMV_CONSUMERS);
+    } else if (kind == XK_F32) {
+        stage_x_q8<R::BETA_INT, XK_F32>(p.x, p.k, xd, recs, kp, GEMV_CONSUMERS);
+    } else if (kind == XK_SWIGLU_F32) {
+        stage_x_q8<R::BETA_INT, XK_SWIGLU_F32>(p.x, p.k, xd, recs, kp, GEMV_CONSUMERS, p.aux);
+    } else if (p.x_bytes > 0) {  // two passes over x: from shared memory
+        uint8_t* const xs = xd + (size_t)kp * 8;
+        const float* const gamma = p.aux != nullptr ? reinterpret_cast<const float*>(xs + p.x_bytes) : nullptr;
+        const uint32_t bar_x = smem_u32(smem + 16);
+        if (threadIdx.x == 0) {
+            mbar_expect_tx(bar_x, (uint32_t)(p.x_bytes * (gamma ? 2 : 1)));
+            bulk_load(smem_u32(xs), p.x, (uint32_t)p.x_bytes, bar_x);
+            if (gamma) bulk_load(smem_u32(gamma), p.aux, (uint32_t)p.x_bytes, bar_x);
+        }
+        mbar_wait_or_abort(bar_x, 0, smem_u32(const_cast<int*>(abort_flag)));
+        const float inv = cta_rms_inv<true>(reinterpret_cast<const float*>(xs), p.k, p.eps, reinterpret_cast<float*>(smem + 192), GEMV_CONSUMERS);
+        stage_x_q8<R::BETA_INT, XK_RMSNORM_F32, true>(xs, p.k, xd, recs, kp, GEMV_CONSUMERS, gamma, inv);
+    } else {
+        const float inv = cta_rms_inv(static_cast<const float*>(p.x), p.k, p.eps, reinterpret_cast<float*>(smem + 192), GEMV_CONSUMERS);
+        stage_x_q8<R::BETA_INT, XK_RMSNORM_F32>(p.x, p.k, xd, recs, kp, GEMV_CONSUMERS, p.aux, inv);
+    }
+    __syncthreads();
+    stamp(2);
+    uint32_t seq = 0;
+    for (int o = 0; o < p.n_ops; o++) {
+        const WsShare share = share_of(o);
+        if (share.t0 == share.t1) continue;  // the same for the whole CTA
+        float* const y = p.op[o].y;
+        const float* const residual = p.op[o].residual;
+        const int rows = p.op[o].rows;
+        auto emit_row = [&](int n, float v) {
+            if (n < rows) {
+                if (residual != nullptr) v += __ldcg(residual + n);
+                y[n] = v;
+            }
+        };
+        ws_consume<QT, DEPTH>(share, p.chunk_q, p.chunk_r, warp, lane, slots, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
+                       smem_u32(recs) + (uint32_t)(kp >> 5) * 16, p.scratch, p.status, smem_u32(const_cast<int*>(abort_flag)), share_of,
+                       p.n_ops, emit_row);
+    }
+    stamp(3);
+    if (*abort_flag) {  // a wait ran out somewhere in this CTA
+        if (lane == 0) report_status(p.status, STATUS_GEMV_FIXUP_TIMEOUT);
+    }
+}
+
 // ---------------------------------------------------------------- host side
 constexpr size_t GEMV_SMEM_LIMIT = 227 * 1024;
 
@@ -101,7 +197,7 @@ static const int* gemvn_clusters(int sm_count) {
     Capacity& d = devs[dev & 63];
     if (d.ready) return d.clusters;
     gemvn_clusters_estimate(sm_count, d.clusters);
-    const auto kernel = gemvn_kernel<WF_QTYPE_Q4_0, 1, WAY_CLUSTER>;
+    const auto kernel = gemvn_kernel<WF_QTYPE_Q4_0, 1, WAY_CLUSTER, false>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_LIMIT) == cudaSuccess) {
         for (int n = 2; n <= GEMVN_MAX_CLUSTER; n++) {
             cudaLaunchConfig_t cfg = {};
@@ -161,13 +257,12 @@ int gemv_max_tokens_per_pass(const Weight& w, int x_dtype) {
     return n;
 }
 
-template <int QT>
-static cudaError_t launch_one_token(const GemvParams& p, int grid, size_t smem, cudaStream_t s) {
-    static bool attr_set[64] = {};
+template <class Params>
+static cudaError_t launch_one_token(void (*kernel)(const Params), bool (&attr_set)[64], const Params& p, int grid, size_t smem, cudaStream_t s) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && !attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemv1_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_LIMIT);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_LIMIT);
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
@@ -181,23 +276,30 @@ static cudaError_t launch_one_token(const GemvParams& p, int grid, size_t smem, 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemv1_kernel<QT>, p);
+    return cudaLaunchKernelEx(&cfg, kernel, p);
 }
-
-static cudaError_t launch_qt_one_token(int qt, const GemvParams& p, int grid, size_t smem, cudaStream_t s) {
+template <int QT> static cudaError_t launch_one_token(const GemvParams& p, int grid, size_t smem, cudaStream_t s) {
+    static bool attr_set[64] = {};
+    return launch_one_token(gemv1_kernel<QT>, attr_set, p, grid, smem, s);
+}
+template <int QT> static cudaError_t launch_one_token(const Gemv1GroupParams& p, int grid, size_t smem, cudaStream_t s) {
+    static bool attr_set[64] = {};
+    return launch_one_token(gemv1_group_kernel<QT>, attr_set, p, grid, smem, s);
+}
+template <class Params> static cudaError_t launch_qt_one_token(int qt, const Params& p, int grid, size_t smem, cudaStream_t s) {
     return qt == WF_QTYPE_Q4_0   ? launch_one_token<WF_QTYPE_Q4_0>(p, grid, smem, s)
            : qt == WF_QTYPE_Q4_1 ? launch_one_token<WF_QTYPE_Q4_1>(p, grid, smem, s)
            : qt == WF_QTYPE_Q8_0 ? launch_one_token<WF_QTYPE_Q8_0>(p, grid, smem, s)
                                  : launch_one_token<WF_QTYPE_Q4_K>(p, grid, smem, s);
 }
 
-template <int QT, int NG, int WAY>
-static cudaError_t launch_several(const GemvNParams& p, int grid, size_t smem, cudaStream_t s) {
+template <int QT, int NG, int WAY, bool GROUP>
+static cudaError_t launch_several(const GemvNParams<GROUP ? GEMV_GROUP : 1>& p, int grid, size_t smem, cudaStream_t s) {
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && !attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemvn_kernel<QT, NG, WAY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_LIMIT);
+        cudaError_t e = cudaFuncSetAttribute(gemvn_kernel<QT, NG, WAY, GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_LIMIT);
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
@@ -214,20 +316,22 @@ static cudaError_t launch_several(const GemvNParams& p, int grid, size_t smem, c
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p.cluster ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, gemvn_kernel<QT, NG, WAY>, p);
+    return cudaLaunchKernelEx(&cfg, gemvn_kernel<QT, NG, WAY, GROUP>, p);
 }
-template <int QT, int NG>
-static cudaError_t launch_way(const GemvNParams& p, int grid, size_t smem, cudaStream_t s) {
-    if (!p.x_f32 && p.slices == 1) return launch_several<QT, NG, WAY_DIRECT>(p, grid, smem, s);
-    if (!p.x_f32 && p.cluster) return launch_several<QT, NG, WAY_CLUSTER>(p, grid, smem, s);
-    return launch_several<QT, NG, WAY_ANY>(p, grid, smem, s);
+template <int QT, int NG, bool GROUP>
+static cudaError_t launch_way(const GemvNParams<GROUP ? GEMV_GROUP : 1>& p, int grid, size_t smem, cudaStream_t s) {
+    if (!p.x_f32 && p.slices == 1) return launch_several<QT, NG, WAY_DIRECT, GROUP>(p, grid, smem, s);
+    if constexpr (!GROUP) {
+        if (p.x_f32 || !p.cluster) return launch_several<QT, NG, WAY_ANY, GROUP>(p, grid, smem, s);
+    }
+    return launch_several<QT, NG, WAY_CLUSTER, GROUP>(p, grid, smem, s);
 }
-template <int NG>
-static cudaError_t launch_qt_several(int qt, const GemvNParams& p, int grid, size_t smem, cudaStream_t s) {
-    return qt == WF_QTYPE_Q4_0   ? launch_way<WF_QTYPE_Q4_0, NG>(p, grid, smem, s)
-           : qt == WF_QTYPE_Q4_1 ? launch_way<WF_QTYPE_Q4_1, NG>(p, grid, smem, s)
-           : qt == WF_QTYPE_Q8_0 ? launch_way<WF_QTYPE_Q8_0, NG>(p, grid, smem, s)
-                                 : launch_way<WF_QTYPE_Q4_K, NG>(p, grid, smem, s);
+template <int NG, bool GROUP>
+static cudaError_t launch_qt_several(int qt, const GemvNParams<GROUP ? GEMV_GROUP : 1>& p, int grid, size_t smem, cudaStream_t s) {
+    return qt == WF_QTYPE_Q4_0   ? launch_way<WF_QTYPE_Q4_0, NG, GROUP>(p, grid, smem, s)
+           : qt == WF_QTYPE_Q4_1 ? launch_way<WF_QTYPE_Q4_1, NG, GROUP>(p, grid, smem, s)
+           : qt == WF_QTYPE_Q8_0 ? launch_way<WF_QTYPE_Q8_0, NG, GROUP>(p, grid, smem, s)
+                                 : launch_way<WF_QTYPE_Q4_K, NG, GROUP>(p, grid, smem, s);
 }
 
 // Allocates (once per stream) what the kernels of that stream exchange partial results through: the one-token
@@ -301,18 +405,16 @@ static int launch_passes(Context* c, const GemvCall& call, cudaStream_t s, const
     if (per_pass < 1) return set_error(c, WF_ERR_TOO_LARGE, "weight [%lld x %lld] is beyond the decode kernels", (long long)w.g.rows, (long long)w.g.k);
     if (w.g.rt > GEMVN_MAX_ROW_TILES) return set_error(c, WF_ERR_TOO_LARGE, "%lld rows: more than %d row-tiles", (long long)w.g.rows, GEMVN_MAX_ROW_TILES);
     for (int64_t m0 = 0; m0 < call.m; m0 += per_pass) {
-        GemvNParams p{};
-        p.tiles = w.d_tiles;
+        GemvNParams<1> p{};
+        p.w[0] = GemvNWeight{w.d_tiles, call.d_y + m0 * call.ldy + call.col0, call.ldy, (int)w.g.rows, (int)w.g.rt};
+        p.n_w = 1;
         p.x = static_cast<const uint8_t*>(call.d_x) + (size_t)m0 * w.g.k * esz;
-        p.y = call.d_y + m0 * call.ldy;
         p.part = buf.part;
         p.count = buf.count;
         p.status = c->d_status;
         p.timing = timing;
-        p.ldy = call.ldy;
-        p.col0 = call.col0;
+        p.timing_at = -1;
         p.ldx = w.g.k;
-        p.rows = (int)w.g.rows;
         p.k = (int)w.g.k;
         p.kt = (int)w.g.kt;
         p.rt = (int)w.g.rt;
@@ -329,9 +431,9 @@ static int launch_passes(Context* c, const GemvCall& call, cudaStream_t s, const
         const int grid = plan.part ? c->sm_count : plan.ctas * plan.slices;
         const size_t smem = gemvn_smem(qt, p.kc, p.cols, f32, p.slices, p.batch, &p.sx, &p.piece_off, &p.ex_off);
         if (clear && plan.part) WF_CUDA(c, cudaMemsetAsync(buf.count, 0, (size_t)w.g.rt * sizeof(int), s));
-        const cudaError_t e = ng == 1   ? launch_qt_several<1>(qt, p, grid, smem, s)
-                              : ng == 2 ? launch_qt_several<2>(qt, p, grid, smem, s)
-                                        : launch_qt_several<4>(qt, p, grid, smem, s);
+        const cudaError_t e = ng == 1   ? launch_qt_several<1, false>(qt, p, grid, smem, s)
+                              : ng == 2 ? launch_qt_several<2, false>(qt, p, grid, smem, s)
+                                        : launch_qt_several<4, false>(qt, p, grid, smem, s);
         if (e != cudaSuccess) return cuda_status(c, e, what);
         c->launches++;
     }
@@ -353,6 +455,94 @@ int gemv_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     if (rc != WF_OK) return rc;
     const GemvScratch& sc = c->gemv_scratch[s];
     return launch_passes(c, call, s, GemvBuffers{sc.d_slots, sc.d_part, sc.d_count}, false, c->salt >= 2 ? c->d_timing : nullptr, "gemv launch");
+}
+
+// ---------------------------------------------------------------- a program's launches
+bool gemv_prepare_group(Context* c, const GemvGroup& g, GemvPrepared* out) {
+    if (g.n < 1 || g.n > GEMV_GROUP || g.m < 1 || g.m > 8) return false;
+    const Weight& first = *g.w[0];
+    const int qt = first.g.qtype, kt = (int)first.g.kt, kp = kt * tile_k(qt);
+    int64_t rt = 0;
+    for (int i = 0; i < g.n; i++) {
+        if (g.w[i]->g.qtype != qt || g.w[i]->g.k != first.g.k) return false;
+        rt += g.w[i]->g.rt;
+    }
+    if (rt * kt >= (1LL << 31) || rt > GEMVN_MAX_ROW_TILES) return false;
+    out->qt = qt;
+    out->m = g.m;
+    if (g.m == 1) {
+        if (!ws_fits(kp, 0)) return false;
+        Gemv1GroupParams& p = out->one;
+        p = {};
+        int64_t end = 0;
+        for (int i = 0; i < g.n; i++) {
+            end += g.w[i]->g.rt;
+            p.op[i] = Gemv1Op{g.w[i]->d_tiles, g.y[i], g.residual[i], (int)g.w[i]->g.rows, (int)end};
+        }
+        p.n_ops = g.n;
+        p.x = g.x;
+        p.aux = g.aux;
+        p.eps = g.eps;
+        p.x_kind = g.x_kind;
+        p.k = (int)first.g.k;
+        p.kt = kt;
+        if (g.n == 1) {
+            const WsSplit sp = ws_split(c->sm_count, rt, kt);
+            out->grid = sp.ctas;
+            p.aligned = sp.aligned;
+            p.chunk_q = sp.chunk_q;
+            p.chunk_r = sp.chunk_r;
+        } else {  // whole row-tiles of the list: nothing is finished between CTAs
+            out->grid = (int)std::min<int64_t>(c->sm_count, rt);
+            p.aligned = 1;
+            p.chunk_q = (int)(rt / out->grid);
+            p.chunk_r = (int)(rt % out->grid);
+        }
+        p.scratch = g.scratch;
+        p.status = c->d_status;
+        p.timing = g.timing;
+        p.timing_at = g.timing_at;
+        out->smem = ws_smem(kp, 0);
+        if (g.x_kind == XK_RMSNORM_F32) {  // x and gamma as they are in memory behind the digits, where there is room
+            const size_t rows = (size_t)p.k * 4 * (g.aux ? 2 : 1);
+            if (out->smem + rows <= GEMV_SMEM_LIMIT) {
+                p.x_bytes = p.k * 4;
+                out->smem += rows;
+            }
+        }
+        return true;
+    }
+    if (g.x_kind != XK_BF16) return false;
+    const GemvNPlan plan = gemvn_plan(gemvn_clusters(c->sm_count), qt, rt, kt, g.m, false);
+    if (plan.slices < 1 || plan.part) return false;
+    GemvNParams<GEMV_GROUP>& p = out->several;
+    p = {};
+    int64_t end = 0;
+    for (int i = 0; i < g.n; i++) {
+        end += g.w[i]->g.rt;
+        p.w[i] = GemvNWeight{g.w[i]->d_tiles, g.y[i], g.ldy[i], (int)g.w[i]->g.rows, (int)end};
+    }
+    p.n_w = g.n;
+    p.x = g.x;
+    p.status = c->d_status;
+    p.timing = g.timing;
+    p.timing_at = g.timing_at;
+    p.ldx = first.g.k;
+    p.k = (int)first.g.k;
+    p.kt = kt;
+    p.rt = (int)rt;
+    p.m = p.cols = g.m;
+    p.slices = plan.slices;
+    p.kc = plan.kc;
+    p.batch = plan.batch;
+    p.cluster = plan.slices > 1;
+    out->grid = plan.ctas * plan.slices;
+    out->smem = gemvn_smem(qt, p.kc, p.cols, false, p.slices, p.batch, &p.sx, &p.piece_off, &p.ex_off);
+    return true;
+}
+cudaError_t gemv_launch_group(const GemvPrepared& g, cudaStream_t s) {
+    return g.m == 1 ? launch_qt_one_token(g.qt, g.one, g.grid, g.smem, s)
+                    : launch_qt_several<1, true>(g.qt, g.several, g.grid, g.smem, s);
 }
 
 // ---------------------------------------------------------------- allocation-free variant

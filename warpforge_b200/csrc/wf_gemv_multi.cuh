@@ -43,22 +43,53 @@ constexpr size_t GEMVN_SMEM = 200 * 1024;
 constexpr size_t GEMVN_PART_BYTES = 8u << 20;  // partial sums a launch may use (the static array of the no-alloc entry is this large)
 constexpr int GEMVN_MAX_ROW_TILES = 1 << 16;   // arrival counters
 
-struct GemvNParams {
+struct GemvNWeight {
     const uint8_t* tiles;
+    float* y;  // its first row of the first token
+    int64_t ldy;
+    int rows, rt_end;  // rt_end: row-tiles of the launch's weights up to and with this one
+};
+template <int GROUP> struct GemvNParams {
+    GemvNWeight w[GROUP];  // one weight, or several of the same K that read the same activations, as one list of row-tiles
+    int n_w;
     const void* x;
-    float* y;
     float* part;  // [rt][slices][column pairs][8] float4, used beyond GEMVN_MAX_CLUSTER slices
     int* count;   // [rt] arrivals per row-tile, zero between launches
     int* status;
-    int64_t ldy, col0, ldx;
-    int rows, k, kt, rt;
+    int64_t ldx;
+    int k, kt, rt;
     int m, x_f32, cols;     // cols = activation columns = m (bf16) or 3 m (fp32)
     int slices, kc, batch;  // k-slices; k-tiles per slice (the last slice may have fewer); units added up at a time
     int cluster;            // the slices of a row-tile are the CTAs of a cluster
     int sx;                 // bytes per staged activation row
     int piece_off, ex_off;  // byte offsets in shared memory: pieces; sums on their way to y
-    unsigned long long* timing;
+    unsigned long long* timing;  // optional globaltimer stamps: [ctas][8], or a program's [ctas][64]
+    int timing_at;               // -1, or this launch's first stamp in a program's row
 };
+
+// A program's launch: weights of one type and K that read the same activations.
+struct GemvGroup {
+    int n = 0, m = 1;
+    const Weight* w[GEMV_GROUP] = {};
+    float* y[GEMV_GROUP] = {};
+    int64_t ldy[GEMV_GROUP] = {};
+    const float* residual[GEMV_GROUP] = {};
+    const void* x = nullptr;
+    int x_kind = 0;
+    const float* aux = nullptr;
+    float eps = 0.f;
+    uint2* scratch = nullptr;
+    unsigned long long* timing = nullptr;
+    int timing_at = -1;
+};
+struct GemvPrepared {
+    int qt = 0, m = 1, grid = 0;
+    size_t smem = 0;
+    Gemv1GroupParams one;
+    GemvNParams<GEMV_GROUP> several;
+};
+bool gemv_prepare_group(Context* c, const GemvGroup& g, GemvPrepared* out);  // false: beyond the kernels
+cudaError_t gemv_launch_group(const GemvPrepared& g, cudaStream_t s);
 
 template <int QT, int NG> struct GemvNGeom {
     // tiles a warp holds in registers while it multiplies: what 128 registers per thread leave room for
@@ -140,7 +171,7 @@ inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt,
 // memory (no registers, no per-thread load latency; `bar` is an initialised mbarrier with one arrival pending),
 // and the block sums are taken from shared memory afterwards, one (column, block) per thread, in the association
 // ((s0 + s1) + (s2 + s3)) of four eight-element runs.
-static __device__ void stage_x_slice_bulk(const GemvNParams& p, uint8_t* xs, float* cinit, int k_lo, int kslice, int ng, float beta,
+template <class Params> static __device__ void stage_x_slice_bulk(const Params& p, uint8_t* xs, float* cinit, int k_lo, int kslice, int ng, float beta,
                                           int nthreads, uint32_t bar, uint32_t abort32) {
     const int valid = max(0, min(kslice, p.k - k_lo));  // elements of the slice that exist
     if (threadIdx.x < 32) {  // one token per lane
@@ -185,7 +216,7 @@ static __device__ void stage_x_slice_bulk(const GemvNParams& p, uint8_t* xs, flo
 }
 
 // fp32 activations (three bf16 columns per token), through registers.
-static __device__ void stage_x_slice(const GemvNParams& p, uint8_t* xs, float* cinit, int k_lo, int kslice, int ng, float beta,
+template <class Params> static __device__ void stage_x_slice(const Params& p, uint8_t* xs, float* cinit, int k_lo, int kslice, int ng, float beta,
                                      int nthreads) {
     const int groups = kslice >> 3;  // 8 elements per thread step; a multiple of 4
     const int total = p.m * groups;
@@ -270,8 +301,8 @@ enum GemvNWay {
     WAY_ANY       // fp32 tokens, or partial sums in memory
 };
 
-template <int QT, int NG, int WAY>
-__global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNParams p) {
+template <int QT, int NG, int WAY, bool GROUP>
+__global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNParams<GROUP ? GEMV_GROUP : 1> p) {
     using T = Tile<QT>;
     using R = TileRegs<QT>;
     constexpr int DEPTH = GemvNGeom<QT, NG>::DEPTH;
@@ -290,7 +321,12 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNPar
         if (p.timing != nullptr && threadIdx.x == 0) {
             unsigned long long tm;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(tm));
-            p.timing[(size_t)blockIdx.x * 8 + i] = tm;
+            if (!GROUP || p.timing_at < 0) {
+                p.timing[(size_t)blockIdx.x * 8 + i] = tm;
+            } else {  // a program's op: start, waited, staged, done
+                const int at = p.timing_at + (i == 3 ? 0 : i == 4 ? 3 : i + 1);
+                if (at < 64) p.timing[(size_t)blockIdx.x * 64 + at] = tm;
+            }
         }
     };
     // Programmatic stream serialization, as in the one-token kernel: the weights depend on nothing, so the first
@@ -300,8 +336,9 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNPar
     // A batch: its units and tiles, this warp's run of them [lo, lo + nt), the unit and k-tile the run starts in.
     int nb = 0, total = 0, nt = 0, unit = 0, kk = 0;
     R slots[DEPTH];
-    const uint8_t* lptr = p.tiles;
+    const uint8_t* lptr = nullptr;
     int lkk = 0, lrem = 0;
+    int lw = 0, lleft = 0;  // GROUP: the weight being requested from and its row-tiles from here on
     auto load_next = [&](R& slot) {
         if (lrem > 0) {
             slot.load_global_n(lptr, lane);
@@ -310,6 +347,11 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNPar
             if (++lkk == kcs) {  // next unit: the same k-tiles of the next row-tile
                 lkk = 0;
                 lptr += (size_t)(p.kt - kcs) * T::BYTES;
+                if (GROUP && --lleft == 0 && lw + 1 < p.n_w) {
+                    lw++;
+                    lleft = p.w[lw].rt_end - p.w[lw - 1].rt_end;
+                    lptr = p.w[lw].tiles + (size_t)k0t * T::BYTES;
+                }
             }
         }
     };
@@ -323,7 +365,13 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNPar
         unit = (int)((unsigned)lo / (unsigned)kcs);
         kk = lkk = lo - unit * kcs;
         lrem = nt;
-        lptr = p.tiles + ((size_t)(u0 + b0 + unit) * p.kt + k0t + kk) * T::BYTES;
+        int u = u0 + b0 + unit;
+        if (GROUP) {
+            for (lw = 0; lw + 1 < p.n_w && u >= p.w[lw].rt_end; lw++) {}
+            lleft = p.w[lw].rt_end - u;
+            u -= lw > 0 ? p.w[lw - 1].rt_end : 0;
+        }
+        lptr = p.w[GROUP ? lw : 0].tiles + ((size_t)u * p.kt + k0t + kk) * T::BYTES;
         static_for<DEPTH>([&](auto J) { load_next(slots[decltype(J)::value]); });
     };
     open_batch(0);
@@ -366,15 +414,21 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNPar
 
     // a unit's sums of eight columns, as the lanes hold them, to y (bf16 tokens)
     auto store_y = [&](int u, int gi, const float4& v) {
+        int at = 0;
+        if (GROUP) {
+            while (at + 1 < p.n_w && u >= p.w[at].rt_end) at++;
+            u -= at > 0 ? p.w[at - 1].rt_end : 0;
+        }
+        const GemvNWeight& w = p.w[at];
         const int r0 = u * 16 + g, r1 = r0 + 8, col = 8 * gi + 2 * q;
-        float* const y = p.y + (int64_t)col * p.ldy + p.col0 + r0;
+        float* const y = w.y + (int64_t)col * w.ldy + r0;
         if (col < p.cols) {
-            if (r0 < p.rows) y[0] = v.x;
-            if (r1 < p.rows) y[8] = v.z;
+            if (r0 < w.rows) y[0] = v.x;
+            if (r1 < w.rows) y[8] = v.z;
         }
         if (col + 1 < p.cols) {
-            if (r0 < p.rows) y[p.ldy] = v.y;
-            if (r1 < p.rows) y[p.ldy + 8] = v.w;
+            if (r0 < w.rows) y[w.ldy] = v.y;
+            if (r1 < w.rows) y[w.ldy + 8] = v.w;
         }
     };
     // place of (column, row) among a unit's float4s, in floats
@@ -469,7 +523,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNPar
                         const float* const f = reinterpret_cast<const float*>(sums + (size_t)(s * per_rank + j) * NG * 32);
                         v += (f[lo] + f[mid]) + f[hi];
                     }
-                    if (r < p.rows) p.y[(int64_t)t * p.ldy + p.col0 + r] = v;
+                    if (r < p.w[0].rows) p.w[0].y[(int64_t)t * p.w[0].ldy + r] = v;
                 }
             } else if (cluster) {
                 for (int it = warp; it < own * NG; it += GEMV_WARPS) {
@@ -516,7 +570,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNPar
                     const float* const f = base + (size_t)s * pairs * 32;
                     v += f32 ? (__ldcg(f + at(3 * t + 2)) + __ldcg(f + at(3 * t + 1))) + __ldcg(f + at(3 * t)) : __ldcg(f + at(t));
                 }
-                if (u * 16 + row < p.rows) p.y[(int64_t)t * p.ldy + p.col0 + u * 16 + row] = v;
+                if (u * 16 + row < p.w[0].rows) p.w[0].y[(int64_t)t * p.w[0].ldy + u * 16 + row] = v;
             }
         }
         if (more) {  // this batch's pieces and sums are read

@@ -40,8 +40,9 @@ struct WsPiece {  // the sums of one cut row-tile as far as one warp's run cover
 };
 constexpr int WS_PIECE_BYTES = WS_SLOTS * GEMV_WARPS * 2 * (int)sizeof(WsPiece);
 
-// Tiles a warp holds in registers.  The per-projection kernel has room for six 1.1 KB tiles; the program kernel, which
-// keeps more state alive around the tile loop, spills from five on (506 against 791 tok/s at six), so it holds four.
+// Tiles a warp holds in registers.  The per-projection kernel has room for six 1.1 KB tiles.  The kernels of a program hold
+// four: the persistent one spills from five on (506 against 791 tok/s at six), and in a group's launch the requests ahead
+// of the activations hold those up (a 32-layer step: 1172 us at six, 1163 at five, 1144 at four, 1160 at three).
 #ifndef WS_DEPTH_SINGLE
 #define WS_DEPTH_SINGLE 6
 #endif
@@ -102,6 +103,30 @@ struct WsShare {  // a CTA's share of one weight (32 bytes: the entry of the sha
     int kt;
     int flags;
     int pad[2];
+};
+
+// What one launch of a program multiplies: up to GEMV_GROUP weights of the same K that read the same activations, cut as one
+// list of row-tiles.
+constexpr int GEMV_GROUP = 4;
+struct Gemv1Op {
+    const uint8_t* tiles;
+    float* y;               // its first row
+    const float* residual;  // y[n] = (x . W[n]) + residual[n] (null: plain store); may be y itself
+    int rows, rt_end;       // rt_end: row-tiles of the list up to and with this weight
+};
+struct Gemv1GroupParams {
+    Gemv1Op op[GEMV_GROUP];
+    int n_ops;
+    const void* x;
+    const float* aux;  // XK_RMSNORM_F32: gamma or null; XK_SWIGLU_F32: the up projection's output
+    float eps;
+    int x_kind, k, kt;
+    int x_bytes;                    // XK_RMSNORM_F32: of a row of x (and gamma) to keep in shared memory; 0: no room
+    int chunk_q, chunk_r, aligned;  // how the list is cut over the CTAs (ws_cta_share)
+    uint2* scratch;                 // [ctas][128] exchange slots
+    int* status;
+    unsigned long long* timing;     // optional globaltimer stamps [ctas][64]: the program's first ops
+    int timing_at;                  // this launch's first stamp
 };
 
 // This warp's run [a, b) of the share [t0, t1).

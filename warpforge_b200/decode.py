@@ -85,7 +85,7 @@ class ProjectionStack:
         self.ctx, self.spec, self.m, self.comm = context, spec, tokens, comm
         self.rank = comm.rank if comm else rank
         self.world = comm.world if comm else world
-        self.mode = "graph"  # "graph": one kernel (+ NCCL all-gather) per projection; "program": one persistent kernel
+        self.mode = "graph"  # "graph": one kernel (+ NCCL all-gather) per projection; "program": one native call
         self.layers = layers if layers is not None else spec.layers
         self.weights: List[List[QuantizedWeight]] = []
         self.blocks = {}
@@ -132,7 +132,7 @@ class ProjectionStack:
                                                   self.m, self.y_dev[name], stream)
                     ctx._ck("wf_qlinear_allgather", rc)
 
-    # ---- the step as one persistent kernel ("program")
+    # ---- the step as one native call ("program"): a few launches on one rank, one persistent kernel on several
     OP_NEW_X, OP_DEPENDS = 1, 2
 
     def op_flags(self) -> List[int]:
@@ -266,7 +266,7 @@ class FusedDecoderStack:
         gate, up  = W{gate,up} . rms_norm(h_mid, gamma2)
         h_next    = h_mid + Wdown . (silu(gate) * up)
 
-    All activations are fp32 device buffers that the projections read and write directly; one kernel launch per
+    All activations are fp32 device buffers that the projections read and write directly; one native call per
     token.  Single rank.  `dims` = (d_model, ffn); weights are seeded synthetic blocks of `qtype`."""
 
     NAMES = ("wq", "wk", "wv", "wo", "wgate", "wup", "wdown")

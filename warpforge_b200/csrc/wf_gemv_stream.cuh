@@ -40,14 +40,12 @@ struct WsPiece {  // the sums of one cut row-tile as far as one warp's run cover
 };
 constexpr int WS_PIECE_BYTES = WS_SLOTS * GEMV_WARPS * 2 * (int)sizeof(WsPiece);
 
-// Tiles a warp holds in registers.  The per-projection kernel has room for six 1.1 KB tiles.  The kernels of a program hold
-// four: the persistent one spills from five on (506 against 791 tok/s at six), and in a group's launch the requests ahead
-// of the activations hold those up (a 32-layer step: 1172 us at six, 1163 at five, 1144 at four, 1160 at three).
-#ifndef WS_DEPTH_SINGLE
-#define WS_DEPTH_SINGLE 6
-#endif
+// Tiles a warp holds in registers.  The per-projection kernel has room for six Q4_0 tiles; with Q4_1's minima four are
+// quicker (7000 x 3008: 5.2 us at six, 4.8 at four).  The kernels of a program hold four: the persistent one spills from
+// five on (506 against 791 tok/s at six), and in a group's launch the requests ahead of the activations hold those up (a
+// 32-layer step: 1172 us at six, 1163 at five, 1144 at four, 1160 at three).
 template <int QT, bool PROGRAM> struct WsGeom {
-    static constexpr int DEPTH = Tile<QT>::BYTES <= 1280 ? (PROGRAM ? 4 : WS_DEPTH_SINGLE) : 2;
+    static constexpr int DEPTH = Tile<QT>::BYTES > 1280 ? 2 : QT == WF_QTYPE_Q4_0 && !PROGRAM ? 6 : 4;
 };
 
 // Shared memory of the one-token kernels:
@@ -287,12 +285,13 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, int chunk_q, int c
             int ncnt;
             ws_next_group<QT, DEPTH>(cur, share_of, n_ops, warp, nbase, ncnt);
             const WsLanePtrs<QT> lp(nbase, lane);
-            if (g0 + DEPTH <= len && kk + DEPTH <= kt && ncnt == DEPTH) {
-                // a whole group inside one row-tile, a whole group to request: straight-line code, immediate offsets
+            if (g0 + DEPTH <= len && kk + DEPTH <= kt) {
+                // a whole group inside one row-tile: straight-line code, immediate offsets; the requests are predicated, so
+                // that a run's last group takes this way too (a third of the groups of a decode step: 1140 -> 1094 us)
                 static_for<DEPTH>([&](auto J) {
                     constexpr int j = decltype(J)::value;
                     slots[j].template compute_q8<j>(acc, qa, dg);
-                    slots[j].template load_global<j * T::BYTES>(lp.pc, lp.ps);
+                    if (j < ncnt) slots[j].template load_global<j * T::BYTES>(lp.pc, lp.ps);
                 });
                 kk += DEPTH;
                 qa.x += DEPTH * XSTEP;

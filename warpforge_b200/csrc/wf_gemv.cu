@@ -257,6 +257,7 @@ int gemv_max_tokens_per_pass(const Weight& w, int x_dtype) {
     return n;
 }
 
+// grid 0: only make the kernel ready (its first use loads it, which can take milliseconds).
 template <class Params>
 static cudaError_t launch_one_token(void (*kernel)(const Params), bool (&attr_set)[64], const Params& p, int grid, size_t smem, cudaStream_t s) {
     int dev = 0;
@@ -266,6 +267,7 @@ static cudaError_t launch_one_token(void (*kernel)(const Params), bool (&attr_se
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
+    if (grid == 0) return cudaSuccess;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(GEMV_CONSUMERS);
@@ -303,6 +305,7 @@ static cudaError_t launch_several(const GemvNParams<GROUP ? GEMV_GROUP : 1>& p, 
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
+    if (grid == 0) return cudaSuccess;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(GEMV_CONSUMERS);
@@ -458,6 +461,7 @@ int gemv_launch(Context* c, const GemvCall& call, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------- a program's launches
+static cudaError_t launch_group(const GemvPrepared& g, int grid, cudaStream_t s);
 bool gemv_prepare_group(Context* c, const GemvGroup& g, GemvPrepared* out) {
     if (g.n < 1 || g.n > GEMV_GROUP || g.m < 1 || g.m > 8) return false;
     const Weight& first = *g.w[0];
@@ -510,7 +514,7 @@ bool gemv_prepare_group(Context* c, const GemvGroup& g, GemvPrepared* out) {
                 out->smem += rows;
             }
         }
-        return true;
+        return launch_group(*out, 0, nullptr) == cudaSuccess;
     }
     if (g.x_kind != XK_BF16) return false;
     const GemvNPlan plan = gemvn_plan(gemvn_clusters(c->sm_count), qt, rt, kt, g.m, false);
@@ -538,12 +542,12 @@ bool gemv_prepare_group(Context* c, const GemvGroup& g, GemvPrepared* out) {
     p.cluster = plan.slices > 1;
     out->grid = plan.ctas * plan.slices;
     out->smem = gemvn_smem(qt, p.kc, p.cols, false, p.slices, p.batch, &p.sx, &p.piece_off, &p.ex_off);
-    return true;
+    return launch_group(*out, 0, nullptr) == cudaSuccess;
 }
-cudaError_t gemv_launch_group(const GemvPrepared& g, cudaStream_t s) {
-    return g.m == 1 ? launch_qt_one_token(g.qt, g.one, g.grid, g.smem, s)
-                    : launch_qt_several<1, true>(g.qt, g.several, g.grid, g.smem, s);
+static cudaError_t launch_group(const GemvPrepared& g, int grid, cudaStream_t s) {
+    return g.m == 1 ? launch_qt_one_token(g.qt, g.one, grid, g.smem, s) : launch_qt_several<1, true>(g.qt, g.several, grid, g.smem, s);
 }
+cudaError_t gemv_launch_group(const GemvPrepared& g, cudaStream_t s) { return launch_group(g, g.grid, s); }
 
 // ---------------------------------------------------------------- allocation-free variant
 // What the kernels exchange partial results through lives, for wf_qlinear_noalloc, in these statically sized

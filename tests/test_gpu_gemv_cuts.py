@@ -89,3 +89,43 @@ def test_program_of_one_rank(m, ks, shared):
         ctx._ck("destroy", ctx._lib.wf_program_destroy(ctx.handle, prog.value))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("d,ffn", [(512, 736), (96, 32), (256, 5024)])
+def test_swiglu_between_launches(d, ffn):
+    """silu(gate) * up made by the launch of a gate and an up projection, in that order, or (up first) by the staging of the
+    projection that reads it: the same float operations on gate and up rows whose sums are cut between warps at other places
+    (as between the program and the per-projection kernels: 1e-5 of the output scale)."""
+    import ctypes
+
+    from warpforge_b200 import _native as N
+    from warpforge_b200.backend import CudaContext, QuantizedWeight
+
+    ctx = CudaContext(0)
+    arr = lambda v, t: (t * len(v))(*v)
+    qt = Q.QuantizationType.Q8_0
+    try:
+        gate, up = (QuantizedWeight(ctx, qt, Q.synth_weight(qt, ffn, d, s), ffn, d) for s in (1, 2))
+        down = QuantizedWeight(ctx, qt, Q.synth_weight(qt, d, ffn, 3), d, ffn)
+        x = Q.synth_activation_f32(1, d, 4)
+        dx, yg, yu, yd = ctx.allocate(x.nbytes), ctx.allocate(ffn * 4), ctx.allocate(ffn * 4), ctx.allocate(d * 4)
+        ctx.copy_to_device(dx, x)
+        outs = []
+        for first, second in (((gate, yg), (up, yu)), ((up, yu), (gate, yg))):
+            prog = ctypes.c_int64()
+            ctx._ck("create", ctx._lib.wf_program_create_fused(
+                ctx.handle, 3, arr([first[0].handle, second[0].handle, down.handle], ctypes.c_int64), arr([dx, dx, yg], ctypes.c_int64),
+                arr([first[1], second[1], yd], ctypes.c_int64), arr([N.WF_OP_NEW_X, 0, N.WF_OP_NEW_X | N.WF_OP_DEPENDS], ctypes.c_int),
+                arr([1, 1, 3], ctypes.c_int), arr([0, 0, yu], ctypes.c_int64), None, None, 1, 1, 0, None, ctypes.byref(prog)))
+            for _ in range(2):
+                ctx._ck("run", ctx._lib.wf_program_run(ctx.handle, prog.value, 0))
+            ctx.synchronize()
+            outs.append([np.empty(n, np.float32) for n in (ffn, ffn, d)])
+            for a, p in zip(outs[-1], (yg, yu, yd)):
+                ctx.copy_to_host(a, p)
+            ctx._ck("destroy", ctx._lib.wf_program_destroy(ctx.handle, prog.value))
+        assert np.isfinite(outs[0][2]).all() and np.any(outs[0][2])
+        for a, b in zip(*outs):
+            assert np.max(np.abs(a - b)) <= 1e-5 * np.max(np.abs(b))
+    finally:
+        ctx.close()

@@ -463,16 +463,32 @@ struct Program {
     uint2* d_scratch = nullptr;
     int2* d_shares = nullptr;
     unsigned long long* d_timing = nullptr;
+    float* d_act = nullptr;       // silu(gate) * up on its way from the launch that makes it to the one that reads it
     std::vector<GemvPrepared> launches;  // one rank: the projections' own kernels, one launch per group; empty: the persistent kernel
     ProgParams params{};
     size_t smem = 0;
     int grid = 0;
 };
 
+static bool rows_overlap(const float* a, int64_t na, const float* b, int64_t nb) { return a < b + nb && b < a + na; }
+
+// Whether op o's input silu(gate) * up can be made by the launch of ops i, i + 1 = its gate and up projections: they are alone
+// on their input, and nothing in between writes what they stored.
+static bool makes_act(const std::vector<ProgOp>& ops, int i, int o) {
+    const ProgOp &gate = ops[i], &up = ops[i + 1], &down = ops[o];
+    if (down.x_kind != XK_SWIGLU_F32 || !(down.flags & OP_NEW_X) || down.x != gate.y || down.x_aux != up.y) return false;
+    if (gate.rows != down.k || up.rows != down.k || rows_overlap(gate.y, gate.rows, up.y, up.rows)) return false;
+    for (int k = i + 2; k < o; k++)
+        if (rows_overlap(ops[k].y, ops[k].rows, gate.y, gate.rows) || rows_overlap(ops[k].y, ops[k].rows, up.y, up.rows)) return false;
+    return true;
+}
+
 // One rank's program as launches of the per-projection kernels (false: something in it needs the persistent kernel).
 // Projections that reuse the staged activations of the one before them join its launch.
 static bool program_launches(Context* c, const std::vector<ProgOp>& ops, Program* pr) {
     const int n_ops = (int)ops.size();
+    int made_for = -1, act_rows = 0;
+    for (const ProgOp& op : ops) act_rows = std::max(act_rows, op.k);
     pr->launches.clear();
     for (int i = 0, head = 0; i < n_ops;) {
         if (ops[i].flags & OP_NEW_X) head = i;
@@ -492,6 +508,19 @@ static bool program_launches(Context* c, const std::vector<ProgOp>& ops, Program
         g.x_kind = ops[head].x_kind;
         g.aux = ops[head].x_aux;
         g.eps = ops[head].eps;
+        if (i == head && made_for == i) {  // the launch before left this op's input in d_act
+            g.x = pr->d_act;
+            g.x_kind = XK_F32;
+            g.aux = nullptr;
+        }
+        if (g.n == 2 && j < n_ops && makes_act(ops, i, j)) {
+            if (!pr->d_act && cudaMalloc(&pr->d_act, (size_t)act_rows * sizeof(float)) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+            g.act = pr->d_act;
+            made_for = j;
+        }
         g.scratch = pr->d_scratch;
         g.timing = pr->d_timing;
         g.timing_at = 1 + 4 * i;
@@ -738,6 +767,7 @@ int wf_program_create_fused(int64_t ctx, int n_ops, const int64_t* weights, cons
         cudaFree(pr->d_scratch);
         cudaFree(pr->d_shares);
         cudaFree(pr->d_timing);
+        cudaFree(pr->d_act);
         delete pr;
         return cuda_status(c, e, "program allocation");
     }
@@ -850,6 +880,7 @@ int wf_program_destroy(int64_t ctx, int64_t program) {
     cudaFree(pr->d_sync);
     cudaFree(pr->d_scratch);
     cudaFree(pr->d_shares);
+    cudaFree(pr->d_act);
     if (pr->d_timing) cudaFree(pr->d_timing);
     for (Weight* w : pr->held) w->programs--;
     pr->magic = 0;

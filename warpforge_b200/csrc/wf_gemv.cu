@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Ge
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     stamp(0);
     auto share_of = [&](int o) {  // this CTA's part of weight o
-        const int begin = o > 0 ? p.op[o - 1].rt_end * p.kt : 0, end = p.op[o].rt_end * p.kt;
+        const int begin = p.op[o].rt_begin * p.kt, end = p.op[o].rt_end * p.kt;
         const int a = max(t0, begin), b = min(t1, end);
         return WsShare{p.op[o].tiles, a < b ? a - begin : 0, a < b ? b - begin : 0, p.kt, 0, {0, 0}};
     };
@@ -167,6 +167,16 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Ge
         ws_consume<QT, DEPTH>(share, p.chunk_q, p.chunk_r, warp, lane, slots, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
                        smem_u32(recs) + (uint32_t)(kp >> 5) * 16, p.scratch, p.status, smem_u32(const_cast<int*>(abort_flag)), share_of,
                        p.n_ops, emit_row);
+    }
+    // silu(gate) * up by the CTA that has stored both: in the staging of the projection that reads it every CTA would read all
+    // of gate and up and take all sigmoids (11008 rows: 6.0 us of staging instead of 2.3)
+    if (p.act != nullptr) {
+        __syncthreads();
+        const int row1 = min(t1 / p.kt * 16, p.op[0].rows);
+        for (int n = t0 / p.kt * 16 + threadIdx.x; n < row1; n += GEMV_CONSUMERS) {
+            const float f = p.op[0].y[n], sig = 1.0f / (1.0f + expf(-f));
+            p.act[n] = (f * sig) * p.op[1].y[n];
+        }
     }
     stamp(3);
     if (*abort_flag) {  // a wait ran out somewhere in this CTA
@@ -480,8 +490,9 @@ bool gemv_prepare_group(Context* c, const GemvGroup& g, GemvPrepared* out) {
         p = {};
         int64_t end = 0;
         for (int i = 0; i < g.n; i++) {
-            end += g.w[i]->g.rt;
-            p.op[i] = Gemv1Op{g.w[i]->d_tiles, g.y[i], g.residual[i], (int)g.w[i]->g.rows, (int)end};
+            const int64_t begin = g.act != nullptr ? 0 : end;
+            end = begin + g.w[i]->g.rt;
+            p.op[i] = Gemv1Op{g.w[i]->d_tiles, g.y[i], g.residual[i], (int)g.w[i]->g.rows, (int)begin, (int)end};
         }
         p.n_ops = g.n;
         p.x = g.x;
@@ -496,6 +507,13 @@ bool gemv_prepare_group(Context* c, const GemvGroup& g, GemvPrepared* out) {
             p.aligned = sp.aligned;
             p.chunk_q = sp.chunk_q;
             p.chunk_r = sp.chunk_r;
+        } else if (g.act != nullptr) {
+            const int64_t one = first.g.rt;
+            out->grid = (int)std::min<int64_t>(c->sm_count, one);
+            p.aligned = 1;
+            p.chunk_q = (int)(one / out->grid);
+            p.chunk_r = (int)(one % out->grid);
+            p.act = g.act;
         } else {  // whole row-tiles of the list: nothing is finished between CTAs
             out->grid = (int)std::min<int64_t>(c->sm_count, rt);
             p.aligned = 1;

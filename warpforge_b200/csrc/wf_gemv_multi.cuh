@@ -78,6 +78,7 @@ struct GemvGroup {
     int x_kind = 0;
     const float* aux = nullptr;
     float eps = 0.f;
+    float* act = nullptr;  // two weights, a gate and an up projection: silu(gate) * up goes here as well
     uint2* scratch = nullptr;
     unsigned long long* timing = nullptr;
     int timing_at = -1;

@@ -110,7 +110,7 @@ struct Gemv1Op {
     const uint8_t* tiles;
     float* y;               // its first row
     const float* residual;  // y[n] = (x . W[n]) + residual[n] (null: plain store); may be y itself
-    int rows, rt_end;       // rt_end: row-tiles of the list up to and with this weight
+    int rows, rt_begin, rt_end;  // its row-tiles in the launch's list
 };
 struct Gemv1GroupParams {
     Gemv1Op op[GEMV_GROUP];
@@ -121,6 +121,9 @@ struct Gemv1GroupParams {
     int x_kind, k, kt;
     int x_bytes;                    // XK_RMSNORM_F32: of a row of x (and gamma) to keep in shared memory; 0: no room
     int chunk_q, chunk_r, aligned;  // how the list is cut over the CTAs (ws_cta_share)
+    float* act;                     // null, or: op[0] is a gate, op[1] the up projection of the same rows, both have the list's
+                                    // first row-tiles, so that a CTA has the same rows of both, and act[n] = silu(gate[n]) * up[n]
+                                    // is stored too
     uint2* scratch;                 // [ctas][128] exchange slots
     int* status;
     unsigned long long* timing;     // optional globaltimer stamps [ctas][64]: the program's first ops

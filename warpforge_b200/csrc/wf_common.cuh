@@ -112,7 +112,11 @@ struct Context {
     std::unordered_map<int64_t, int64_t> allocs;  // device ptr -> bytes
     std::vector<void*> host_allocs;
     std::vector<Weight*> weights;
-    std::multimap<int64_t, uint8_t*> spare_tiles;  // tile buffers of freed weights by size, at most SPARE_TILES_BYTES in all
+    struct SpareTiles {
+        int64_t bytes;
+        uint8_t* tiles;
+    };
+    std::vector<SpareTiles> spare_tiles;  // tile buffers of freed weights, oldest first, at most SPARE_TILES_BYTES in all
     int64_t spare_tiles_bytes = 0;
     std::unordered_map<cudaStream_t, GemvScratch> gemv_scratch;
     // pinned staging for host-pointer calls

@@ -224,3 +224,14 @@ def test_error_paths(backend):
     assert lib.wf_embedding(ctx.handle, d, d, d, 1, 0, 4, 0) == N.WF_ERR_SHAPE
     assert lib.wf_silu(12345, d, d, 4, 0) == N.WF_ERR_INVALID_HANDLE
     ctx.free(d)
+
+
+@pytest.mark.parametrize("n", [513, 1000, 2048, 2049])
+@pytest.mark.parametrize("rows", [1, 296, 297])
+def test_few_rows(backend, oracle, rows, n):
+    """Both sides of the lines between row groups: up to 296 rows of up to 2048 columns are held by twice the threads."""
+    rng = np.random.default_rng(rows * 43 + n)
+    x = (rng.standard_normal((rows, n)) * 2.5 + 0.5).astype(np.float32)
+    _check_rows(oracle, _call(backend, "rms_norm", x), oracle.rms_norm(x))
+    _check_rows(oracle, _call(backend, "layer_norm", x), oracle.layer_norm(x))
+    _check_rows(oracle, _call(backend, "softmax", x), oracle.softmax(x))

@@ -26,6 +26,7 @@ namespace wf {
 // Bound by HBM as long as enough rows are in flight per SM to cover one row's chain of load, reductions and store, so
 // the group fits the row: 256 threads with room for 32 floats each left three quarters of their registers idle on a
 // row of 2048, and 64 floats per lane of a warp per row takes so many registers that softmax had 8 warps per SM.
+constexpr int FEW_ROWS = 296;  // two CTAs per SM
 constexpr int ROW_CTA = 256;  // threads of a CTA whose warps take a row each
 
 // Sum over the group's T threads, in double; every thread gets it.  `red` (T / 32 doubles, unused for a warp) is private
@@ -291,6 +292,9 @@ __global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) softmax_kernel(const fl
 template <class F> static void with_row_group(int64_t rows, int64_t n, F&& f) {
     const unsigned packed = (unsigned)((rows + ROW_CTA / 32 - 1) / (ROW_CTA / 32)), each = (unsigned)rows;
     using std::integral_constant;
+    // Rows that are all on the chip at once: what counts is one row's chain, so twice the threads hold half of it each (softmax of
+    // 256 rows of 2000: 4.6 -> 4.1 us a call).  Longer rows gain nothing from it and lose at 8192 (rms_norm of 64 rows 5.5 -> 6.2).
+    if (rows <= FEW_ROWS && n > 512 && n <= 2048) return f(integral_constant<int, 256>{}, integral_constant<int, 2>{}, each);
     if (n <= 512) f(integral_constant<int, 32>{}, integral_constant<int, 4>{}, packed);
     else if (n <= 1024) f(integral_constant<int, 64>{}, integral_constant<int, 4>{}, each);
     else if (n <= 2048) f(integral_constant<int, 128>{}, integral_constant<int, 4>{}, each);

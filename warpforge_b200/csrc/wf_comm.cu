@@ -17,6 +17,7 @@
 #include <algorithm>
 
 #include "wf_common.cuh"
+#include "wf_gather_route.h"
 #include "wf_gemv_core.cuh"
 
 namespace wf {
@@ -573,19 +574,7 @@ static void release_peer_landing(Comm* k) {
     k->peer_ok = false;
 }
 
-// True when this gather goes by peer stores: the mappings exist, the decode kernels produce the output (they
-// write a column block of a wider matrix in place) and both halves of the landing buffer hold it.
-static bool gather_by_peer_stores(const Comm* k, const Weight& w, int x_dtype, int64_t m, const void* x) {
-    if (!k->peer_ok || k->world < 2) return false;
-    if (gemm_supported(w, x_dtype, m, x)) return false;
-    const int64_t words = (int64_t)k->world * m * w.g.rows;
-    return words < (1ll << 31) && 2 * words * (int64_t)sizeof(uint2) <= GATHER_LAND_BYTES;
-}
-
-// True when a gather that is not small goes through the staging areas: every rank's block fits its own.
-static bool gather_by_peer_loads(const Comm* k, int64_t m, int64_t rows) {
-    return k->peer_ok && k->world > 1 && m * rows * 4 <= k->stage_bytes && (int64_t)k->world * m * rows < (1ll << 40);
-}
+static GatherRoom room_of(const Comm* k) { return GatherRoom{k->peer_ok, k->world, GATHER_LAND_BYTES, k->stage_bytes}; }
 
 }  // namespace wf
 
@@ -721,7 +710,8 @@ int wf_qlinear_allgather(int64_t ctx, int64_t comm, int64_t weight, const void* 
     cudaStream_t s = resolve_stream(c, stream);
     const int64_t rows = w->g.rows, n = w->total_rows;
     float* y = static_cast<float*>(y_full_dev);
-    if (gather_by_peer_stores(k, *w, x_dtype, m, x_dev)) {
+    const GatherRoute route = gather_route(room_of(k), x_dtype == WF_DTYPE_F32, m, rows);
+    if (route == GATHER_STORES) {
         // every rank computes its column block of y in place, then one kernel exchanges the blocks
         GemvCall call{w, x_dev, x_dtype, m, y, n, w->row0};
         int rc = gemv_launch(c, call, s);
@@ -736,14 +726,16 @@ int wf_qlinear_allgather(int64_t ctx, int64_t comm, int64_t weight, const void* 
         c->launches++;
         return WF_OK;
     }
-    if (gather_by_peer_loads(k, m, rows)) {
+    if (route == GATHER_LOADS) {
         GatherPeers peers;
         for (int r = 0; r < WF_MAX_GATHER_RANKS; r++) peers.land[r] = k->land[r];
-        gather_wait_done_kernel<<<1, 32, 0, s>>>(peers, k->d_epoch, c->d_status, k->world, k->rank, k->wait_ns);
-        WF_CUDA(c, cudaGetLastError());
         float* mine = reinterpret_cast<float*>(reinterpret_cast<char*>(k->land[k->rank]) + GATHER_LAND_BYTES + GATHER_FLAG_BYTES);
         GemvCall call{w, x_dev, x_dtype, m, mine, rows, 0};
-        int rc = gemm_supported(*w, x_dtype, m, call.d_x) ? gemm_launch(c, call, s) : gemv_launch(c, call, s);
+        int rc = qlinear_reserve(c, call, s);  // before anything is enqueued: a refused call leaves nothing behind
+        if (rc != WF_OK) return rc;
+        gather_wait_done_kernel<<<1, 32, 0, s>>>(peers, k->d_epoch, c->d_status, k->world, k->rank, k->wait_ns);
+        WF_CUDA(c, cudaGetLastError());
+        rc = qlinear_launch(c, call, s);
         if (rc != WF_OK) return rc;
         const int vec = (rows % 4 == 0) && (reinterpret_cast<uintptr_t>(y) % 16 == 0);
         const int64_t pieces = (int64_t)k->world * m * (vec ? rows / 4 : rows);
@@ -782,7 +774,7 @@ int wf_qlinear_allgather(int64_t ctx, int64_t comm, int64_t weight, const void* 
     }
     float* mine = k->d_tmp + (int64_t)k->world * m * rows;
     GemvCall call{w, x_dev, x_dtype, m, mine, rows, 0};
-    int rc = gemm_supported(*w, x_dtype, m, call.d_x) ? gemm_launch(c, call, s) : gemv_launch(c, call, s);
+    int rc = qlinear_launch(c, call, s);
     if (rc != WF_OK) return rc;
     int r = nccl().AllGather(mine, k->d_tmp, (size_t)(m * rows), NCCL_FLOAT32, k->comm, s);
     if (r != NCCL_SUCCESS) return nccl_status(c, r, "ncclAllGather");

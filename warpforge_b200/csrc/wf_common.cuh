@@ -171,6 +171,8 @@ struct GemvCall {
     int64_t col0;
 };
 int gemv_launch(Context* c, const GemvCall& call, cudaStream_t s);
+// what gemv_launch would refuse or allocate, without launching anything
+int gemv_reserve(Context* c, const GemvCall& call, cudaStream_t s);
 int gemv_max_tokens_per_pass(const Weight& w, int x_dtype);
 int gemv_prepare_stream(Context* c, cudaStream_t s);
 int gemv_launch_noalloc(Context* c, const GemvCall& call, cudaStream_t s);
@@ -178,6 +180,10 @@ int gemv_launch_noalloc(Context* c, const GemvCall& call, cudaStream_t s);
 // wf_gemm.cu
 bool gemm_supported(const Weight& w, int x_dtype, int64_t m, const void* d_x);
 int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s);
+// A projection by the kernel for its token count, wherever the result goes.  qlinear_reserve makes the scratch that
+// qlinear_launch will use, or refuses the call, before anything is enqueued.
+int qlinear_reserve(Context* c, const GemvCall& call, cudaStream_t s);
+int qlinear_launch(Context* c, const GemvCall& call, cudaStream_t s);
 // sizes the stream's scratch like the largest of the context's other streams (before a recording)
 int gemm_prepare_stream(Context* c, cudaStream_t s);
 void free_scratch(GemvScratch& sc);

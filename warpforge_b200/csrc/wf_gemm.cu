@@ -12,6 +12,7 @@
 // bf16 activations: weights are rounded once to fp16 (relative 2^-12) after the exact fp32 dequantization; products
 // and sums are fp32 in the tensor core.  Replaces the host transpose + batch_matmul_f32 of
 // warpforge-backend-nvidia/src/main/java/io/surfworks/warpforge/backend/nvidia/ops/DotGeneralKernel.java:169-298.
+#include "wf_gather_route.h"
 #include "wf_gemm_pair.cuh"
 #include "wf_gemm_split.cuh"
 
@@ -36,17 +37,13 @@ static EncodeTiledFn encode_tiled_fn() {
 
 constexpr size_t GEMM_SMEM_LIMIT = 227 * 1024;
 
-// Token counts from which on the tensor cores are used.  bf16: more than one launch of the memory-bound decode kernel takes.
-constexpr int GEMM_MIN_TOKENS_BF16 = 33, GEMM_MIN_TOKENS_F32 = 11;
-
 bool gemm_supported(const Weight& w, int x_dtype, int64_t m, const void* d_x) {
     // K a multiple of 8 elements and a 16-byte aligned activation pointer: rows are read in 16-byte pieces, the TMA row
     // stride must be a multiple of 16 bytes.  Whole 128-row blocks exist for any row count: the weight buffer is padded
     // to 8 row-tiles with zero scales.
     // fp32 activations keep fp32's range: a weight with values beyond fp16's stays on the decode kernel.
     if (x_dtype == WF_DTYPE_F32 && w.beyond_fp16) return false;
-    const int least = x_dtype == WF_DTYPE_BF16 ? GEMM_MIN_TOKENS_BF16 : GEMM_MIN_TOKENS_F32;
-    return m >= least && (w.g.k % 8) == 0 && (reinterpret_cast<uintptr_t>(d_x) & 15) == 0 && encode_tiled_fn() != nullptr;
+    return many_tokens(x_dtype == WF_DTYPE_F32, m) && (w.g.k % 8) == 0 && (reinterpret_cast<uintptr_t>(d_x) & 15) == 0 && encode_tiled_fn() != nullptr;
 }
 
 // What the kernels of one format need to know about a device, found out once: how many clusters of each size it holds
@@ -176,6 +173,31 @@ int gemm_prepare_stream(Context* c, cudaStream_t s) {
     return most > 0 ? gemm_scratch(c, s, c->gemv_scratch[s], most) : WF_OK;
 }
 
+// Bytes of a call's converted rows: the fp16 planes, and behind them (at *scales) the rows' scales.
+static int64_t gemm_x16_bytes(const GemvCall& call, int planes, int64_t* scales) {
+    const int64_t kx = (call.w->g.k + 63) & ~63LL;  // elements of a converted row
+    *scales = (planes * call.m * kx * 2 + 255) & ~255LL;
+    return *scales + ((call.m * 4 + 127) & ~127LL);
+}
+
+int qlinear_reserve(Context* c, const GemvCall& call, cudaStream_t s) {
+    if (gemm_supported(*call.w, call.x_dtype, call.m, call.d_x)) {
+        const bool f32 = call.x_dtype == WF_DTYPE_F32;
+        int64_t scales;
+        const int rc = gemm_scratch(c, s, c->gemv_scratch[s], gemm_x16_bytes(call, f32 ? 3 : 1, &scales));
+        if (rc != WF_ERR_RECORDING || !f32) return rc;
+    }
+    return gemv_reserve(c, call, s);
+}
+
+int qlinear_launch(Context* c, const GemvCall& call, cudaStream_t s) {
+    // many tokens: tensor-core GEMM; a few tokens: the HBM-bound GEMV
+    if (!gemm_supported(*call.w, call.x_dtype, call.m, call.d_x)) return gemv_launch(c, call, s);
+    const int rc = gemm_launch(c, call, s);
+    // the decode kernels take fp32 tokens without more scratch than a recorded stream has
+    return rc == WF_ERR_RECORDING && call.x_dtype == WF_DTYPE_F32 ? gemv_launch(c, call, s) : rc;
+}
+
 int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     const Weight& w = *call.w;
     const int qt = w.g.qtype;
@@ -257,8 +279,9 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     p.idesc = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(p.bm >> 3) << 17) | ((uint32_t)((pair ? 2 * GEMM_BN : GEMM_BN) >> 4) << 24);
 
     // the activations' fp16 planes and row scales
-    const int64_t kx = (w.g.k + 63) & ~63LL;  // elements of a converted row
-    const int64_t x16_plane = (planes * call.m * kx * 2 + 255) & ~255LL, x16_bytes = x16_plane + ((call.m * 4 + 127) & ~127LL);
+    const int64_t kx = (w.g.k + 63) & ~63LL;
+    int64_t x16_plane;
+    const int64_t x16_bytes = gemm_x16_bytes(call, planes, &x16_plane);
     GemvScratch& sc = c->gemv_scratch[s];
     {
         const int rc = gemm_scratch(c, s, sc, x16_bytes);

@@ -460,12 +460,15 @@ static int check_shape(Context* c, const Weight& w, int x_dtype) {
     return WF_OK;
 }
 
+int gemv_reserve(Context* c, const GemvCall& call, cudaStream_t s) {
+    const int rc = check_shape(c, *call.w, call.x_dtype);
+    return rc != WF_OK ? rc : gemv_prepare_stream(c, s);
+}
+
 int gemv_launch(Context* c, const GemvCall& call, cudaStream_t s) {
-    int rc = check_shape(c, *call.w, call.x_dtype);
+    const int rc = gemv_reserve(c, call, s);
     if (rc != WF_OK) return rc;
     if (call.w->g.rt * call.w->g.kt < 1) return WF_OK;
-    rc = gemv_prepare_stream(c, s);
-    if (rc != WF_OK) return rc;
     const GemvScratch& sc = c->gemv_scratch[s];
     return launch_passes(c, call, s, GemvBuffers{sc.d_slots, sc.d_part, sc.d_count}, false, c->salt >= 2 ? c->d_timing : nullptr, "gemv launch");
 }

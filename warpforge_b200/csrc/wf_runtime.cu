@@ -672,10 +672,7 @@ int wf_qlinear(int64_t ctx, int64_t weight, const void* x, int x_dtype, int x_on
         if (!y_on_device) d_y = reinterpret_cast<float*>(static_cast<uint8_t*>(y_direct ? c->h_stage_dev : c->d_stage) + yo);
     }
     GemvCall call{w, d_x, x_dtype, m, d_y, w->g.rows, 0};
-    // many tokens: tensor-core GEMM; a few tokens: the HBM-bound GEMV
-    const bool gemm = gemm_supported(*w, x_dtype, m, call.d_x);
-    int rc = gemm ? gemm_launch(c, call, s) : gemv_launch(c, call, s);
-    if (gemm && rc == WF_ERR_RECORDING && x_dtype == WF_DTYPE_F32) rc = gemv_launch(c, call, s);  // takes fp32 tokens without more scratch
+    const int rc = qlinear_launch(c, call, s);
     if (rc != WF_OK) return rc;
     if (!y_on_device) {
         if (!y_direct) WF_CUDA(c, cudaMemcpyAsync(static_cast<uint8_t*>(c->h_stage) + yo, d_y, (size_t)yb, cudaMemcpyDeviceToHost, s));

@@ -15,8 +15,9 @@
 //   warps 4-7   epilogue (TMEM lane quarter = warp % 4): accumulator -> the ranks' exchange buffers -> y
 //   warps 2,3,8-13  dequantization: quantized tiles from global memory -> fp16 rows in the swizzled A stage
 // A stage is 64 k.  The accumulator is double buffered in TMEM, so a tile is put together while the next one is computed.
-// Every wait is bounded; on expiry the CTA sets a status bit, stops issuing work and still frees its TMEM.  The epilogue's
-// warps meet on barriers of their own and leave only together, at one of them (epilogue_all).
+// Every wait is bounded; on expiry the CTA sets a status bit, stops issuing work and still frees its TMEM.  Warps leave their
+// loops on their own, so there is no barrier between some of them: they meet on mbarriers, whose waits are bounded, and
+// all together at the end.
 //
 // PIECES 1, PLANES 1: bf16 tokens, weights rounded once to fp16.
 // PIECES 2, PLANES 3: fp32 tokens.  Every weight is two fp16 (its value, and what rounding left), every token value three,
@@ -38,18 +39,7 @@ inline __host__ __device__ int split_stage_bytes(int pieces, int planes, int bm)
 inline __host__ __device__ int split_groups(int bm, int ranks) { return (bm / 4 + ranks - 1) / ranks; }
 inline __host__ __device__ int split_exchange_bytes(int bm, int ranks) { return ranks == 1 ? 0 : ranks * split_groups(bm, ranks) * GEMM_BN * 16; }
 
-// Barrier of the four epilogue warps; true for all of them when `ok` is true for all of their threads.  A warp that has given
-// up comes here like the others, so that they leave the tile loop together and none waits for one that has left.
-__device__ __forceinline__ bool epilogue_all(bool ok) {
-    uint32_t all;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                 : "=r"(all)
-                 : "r"((uint32_t)ok)
-                 : "memory");
-    return all != 0;
-}
-
-// smem: [0, 1024) barriers, tmem slot, token scales | stages x (A | B), 1024-byte aligned | exchange buffer
+// smem: [0, 1024) barriers, tmem slot | stages x (A | B), 1024-byte aligned | exchange buffer
 template <int QT, int PIECES, int PLANES>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap) {
     constexpr int ACCS = PIECES;
@@ -71,7 +61,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
     const int stages = p.stages, S = p.ranks;
     uint8_t* stage0 = smem + 1024;
     float4* ex = reinterpret_cast<float4*>(stage0 + (size_t)stages * stage_bytes);
-    float* scale = reinterpret_cast<float*>(smem + 512);  // [128] row_unscale of the tile's tokens
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int rank = (int)blockIdx.x % S, cluster = (int)blockIdx.x / S, clusters = (int)gridDim.x / S;
     const int tiles = p.n_tiles * p.m_tiles;
@@ -172,26 +161,23 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
         asm volatile("griddepcontrol.wait;" ::: "memory");  // the row scales; no bounded wait before
         float* sums = p.partial + (size_t)blockIdx.x * SPLIT_MAX_TOKENS * GEMM_BN;
         bool ok = true;
-        for (int tile = cluster; tile < tiles; tile += clusters, round++) {
+        for (int tile = cluster; tile < tiles && ok && !*abort_flag; tile += clusters, round++) {
             const int nt = tile / p.m_tiles, tok0 = (tile % p.m_tiles) * p.bm;
             const int n = nt * GEMM_BN + row;
+            const int first = tok0 + rank * per * 4;  // the first token of the tile that this rank finishes, of at most 64 (S > 1)
+            float scale[2];                           // their scales, two per lane: a warp shares nothing with the others
             if (S > 1) {
-                const int t = (int)threadIdx.x - 128;
-                const float mine_scale = t < p.bm && tok0 + t < p.m ? __ldg(p.row_unscale + tok0 + t) : 0.f;
-                if (round > 0 && !epilogue_all(ok && !*abort_flag)) break;  // every warp is through with the previous tile's scales
-                scale[t] = mine_scale;
-                if (t == 0 && mine > 0) g_mbar_expect_tx(ex_full, (uint32_t)(S * mine * GEMM_BN * 16));
-                if (round > 0 && !g_mbar_wait(ex_empty, (round - 1) & 1)) { if (lane == 0) fail(); ok = false; }
-                if (!epilogue_all(ok)) break;
-            } else if (__any_sync(0xFFFFFFFFu, !ok || *abort_flag)) {
-                break;
+#pragma unroll
+                for (int j = 0; j < 2; j++) scale[j] = 32 * j + lane < min(4 * mine, p.m - first) ? __ldg(p.row_unscale + first + 32 * j + lane) : 0.f;
+                if (threadIdx.x == 128 && mine > 0) g_mbar_expect_tx(ex_full, (uint32_t)(S * mine * GEMM_BN * 16));
+                if (round > 0 && !g_mbar_wait(ex_empty, (round - 1) & 1)) { if (lane == 0) fail(); break; }
             }
             uint32_t to = 0, in = 0;  // rank and place there of the next group of four tokens
             uint32_t to_addr = map_to_rank(ex_addr, 0), to_bar = map_to_rank(bar_addr, 0);
             for (int g0 = kb0; g0 < kb1; local++) {
                 const int g1 = min(kb1, g0 + min(FLUSH, kb1 - g0)), buf = local & 1;
                 const bool last = g1 == kb1;
-                if (!__all_sync(0xFFFFFFFFu, g_mbar_wait(&acc_full[buf], (local >> 1) & 1))) { if (lane == 0) fail(); ok = false; break; }
+                if (!g_mbar_wait(&acc_full[buf], (local >> 1) & 1)) { if (lane == 0) fail(); ok = false; break; }
                 tc_fence_after();
                 const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * ACCS * p.bm);
                 for (int c = 0; c < p.bm; c += 32) {  // 32 columns at a time (also past a BM that is not a multiple of 32)
@@ -227,12 +213,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
                 if (lane == 0) g_mbar_arrive(&acc_empty[buf]);
                 g0 = g1;
             }
-            if (!ok) continue;  // to the barrier at the next tile's start, where all four warps leave
+            if (!ok) break;
             if (S > 1) {  // this rank's tokens: the ranks' parts in rank order
-                if (mine > 0 && !__all_sync(0xFFFFFFFFu, g_mbar_wait(ex_full, round & 1))) { if (lane == 0) fail(); ok = false; continue; }
-                const int left = min(mine * 4, p.m - tok0 - rank * per * 4);  // tokens of this rank that exist
-                float* yp = p.y + (int64_t)(tok0 + rank * per * 4) * p.ldy + p.col0 + n;
-                const float* sc = scale + rank * per * 4;
+                if (mine > 0 && !g_mbar_wait(ex_full, round & 1)) { if (lane == 0) fail(); break; }
+                const int left = min(mine * 4, p.m - first);  // tokens of this rank that exist
+                float* yp = p.y + (int64_t)first * p.ldy + p.col0 + n;
 #pragma unroll 2
                 for (int gi = 0; gi * 4 < left; gi++) {
                     float4 v = ex[(size_t)gi * GEMM_BN + row];
@@ -240,8 +225,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
                         const float4 w = ex[(size_t)(src * per + gi) * GEMM_BN + row];
                         v.x += w.x, v.y += w.y, v.z += w.z, v.w += w.w;
                     }
-                    const float4 u = *reinterpret_cast<const float4*>(sc + gi * 4);
-                    const float o[4] = {v.x * u.x, v.y * u.y, v.z * u.z, v.w * u.w};
+                    float o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int e = 0; e < 4; e++) o[e] *= __shfl_sync(0xFFFFFFFFu, gi < 8 ? scale[0] : scale[1], (gi * 4 + e) & 31);
                     if (n < p.rows) {
 #pragma unroll
                         for (int e = 0; e < 4; e++)

@@ -52,6 +52,11 @@ __device__ __forceinline__ void report_status(int* status, int bit) {
     *reinterpret_cast<volatile int*>(b->host + (31 - __clz(bit))) = 1;
     __threadfence_system();
 }
+// After an abort: give this CTA's asynchronous copies still in flight (its own, and those that other CTAs of its cluster have
+// sent here) time to land before its shared memory is handed to another CTA (about a millisecond, bounded).
+__device__ __forceinline__ void drain_after_abort() {
+    for (int i = 0; i < 1000; i++) __nanosleep(1000);
+}
 #endif
 
 constexpr int UPLOAD_RING = 6;  // pinned chunks

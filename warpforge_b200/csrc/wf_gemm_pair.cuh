@@ -370,6 +370,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
     __syncwarp();
     tc_fence_before();
     __syncthreads();
+    if (warp == 1 && *abort_flag) drain_after_abort();  // operands and MMAs that nobody waited for, in either CTA
     cluster_sync();
     if (warp == 1) {
         tc_fence_after();

@@ -316,6 +316,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
     __syncthreads();
     if (S > 1) cluster_sync();
     if (warp == 1) {
+        if (*abort_flag) drain_after_abort();  // operands, MMAs and other ranks' parts that nobody waited for
         tc_fence_after();
         tmem_dealloc(tmem_base, 512);
     }

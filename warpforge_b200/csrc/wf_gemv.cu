@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Ge
     stamp(3);
     if (*abort_flag) {  // a wait ran out somewhere in this CTA
         if (lane == 0) report_status(p.status, STATUS_GEMV_FIXUP_TIMEOUT);
+        drain_after_abort();  // the activations' copies
     }
 }
 

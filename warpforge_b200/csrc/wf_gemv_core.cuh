@@ -171,11 +171,6 @@ __device__ __forceinline__ void mbar_wait_or_abort(uint32_t bar, uint32_t parity
         "r"(parity), "r"(abort32), "r"((uint32_t)GEMV_BAR_SPINS)
         : "memory");
 }
-// After an abort: give this CTA's bulk copies still in flight time to land before its shared memory
-// is handed to another CTA (about a millisecond, bounded).
-__device__ __forceinline__ void drain_after_abort() {
-    for (int i = 0; i < 1000; i++) __nanosleep(1000);
-}
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
                  "r"(bytes), "r"(bar)

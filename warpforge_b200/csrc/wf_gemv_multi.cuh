@@ -585,6 +585,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemvn_kernel(const GemvNPar
             asm volatile("barrier.cluster.arrive.release;" ::: "memory");
             asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
         }
+        drain_after_abort();
     }
 }
 

@@ -85,3 +85,31 @@ def test_fp32_tokens_keep_fp32s_range(backend, oracle):
     w.close()
     want = x.astype(np.float64) @ oracle.dequant(O.Q8_0, blocks, rows * k).reshape(rows, k).astype(np.float64).T
     assert np.linalg.norm(got - want) <= 3.8e-6 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("f32", [True, False])
+def test_rows_of_the_smallest_magnitudes(backend, oracle, f32):
+    """Rows whose largest magnitude lies on either side of 2^-112 (where the scale to fp16's range reaches its end), down to
+    subnormal floats, next to ordinary ones and a row of zeros.  Weights of magnitude 1e3 .. 1e4 keep y normal, so the bars
+    of the other tests hold row by row."""
+    from warpforge_b200.backend import DotGeneralOp, LINEAR_DIMS, Tensor
+
+    rows, k, m = 200, 544, 40
+    blocks = Q.synth_q8_0(rows, k, 3).reshape(rows, -1, 34).copy()
+    blocks[:, :, :2] = np.random.default_rng(1).uniform(100, 400, (rows, k // 32)).astype(np.float16)[..., None].view(np.uint8)
+    blocks = blocks.reshape(rows, -1)
+    x = Q.synth_activation_f32(m, k, 4)
+    small = {1: 2.0 ** -115, 2: 1e-35, 3: 2.0 ** -126, 4: 2.0 ** -132, 5: 0.0, 6: 2.0 ** -111, 7: 2.0 ** -100, 9: 1e30}
+    for r, scale in small.items():
+        x[r] = (x[r].astype(np.float64) * scale).astype(np.float32)
+    if not f32:
+        bits = Q.float_to_bf16_bits(x).reshape(m, k)
+        x = Q.bf16_bits_to_float(bits).reshape(m, k)
+    w = backend.upload_weight(Q.QuantizationType.Q8_0, blocks, rows, k)
+    t = Tensor.from_float_array(x) if f32 else Tensor.from_bf16_bits(bits)
+    got = backend.execute(DotGeneralOp(LINEAR_DIMS, (m, rows)), [t, w])[0].data
+    w.close()
+    want = x.astype(np.float64) @ oracle.dequant(O.Q8_0, blocks, rows * k).reshape(rows, k).astype(np.float64).T
+    assert np.any(x[4]) and np.max(np.abs(x[4])) < 2.0 ** -126 * 16 and not np.any(got[5])
+    for r in range(m):
+        assert np.linalg.norm(got[r] - want[r]) <= (3.8e-6 if f32 else 3e-4) * np.linalg.norm(want[r]), r

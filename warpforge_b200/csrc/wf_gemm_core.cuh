@@ -197,7 +197,8 @@ template <int ACCS> __device__ __forceinline__ void tmem_ld_accs(uint32_t taddr,
 __host__ __device__ inline int stage_chunk(int j, int q) { return 2 * q + j; }
 
 // ---------------------------------------------------------------- activations to fp16
-// x16[row] = fp16(x[row] * 2^s) with s chosen so that the row's largest magnitude lands in [2^14, 2^15); unscale[row] = 2^-s.
+// x16[row] = fp16(x[row] * 2^s) with s chosen so that the row's largest magnitude lands in [2^14, 2^15), or 126 where that
+// would take more (magnitudes below 2^-112, down to subnormal ones); unscale[row] = 2^-s.
 //   bf16 (PLANES 1): exact whenever the scaled value is a normal fp16.
 // Rows are padded to whole stages of 64 k (zeros) and lie in the stages' order of k.
 //   fp32 (PLANES 3): v = hi + mid + lo, each the fp16 nearest to what is left: exact down to 2^-39 of the row's largest.
@@ -255,8 +256,8 @@ __global__ void __launch_bounds__(CONVERT_THREADS) convert_rows_kernel(const voi
     __syncthreads();
 #pragma unroll
     for (int w = 0; w < CONVERT_THREADS / 32; w++) emax = max(emax, s_max[w]);
-    const int shift = emax == 0 ? 0 : (127 + 14) - emax;  // multiply by 2^shift
-    const float scale = __uint_as_float((uint32_t)min(max(127 + shift, 1), 254) << 23);
+    const int shift = min((127 + 14) - emax, 126);  // multiply by 2^shift; 2^126 is the largest power whose reciprocal is normal
+    const float scale = __uint_as_float((uint32_t)(127 + shift) << 23);
     uint4* out = reinterpret_cast<uint4*>(x16) + (size_t)row * padded;
     auto convert = [&](int i, const G& g) {
         float f[8];
@@ -291,7 +292,7 @@ __global__ void __launch_bounds__(CONVERT_THREADS) convert_rows_kernel(const voi
     if (t < padded - groups)  // the block that K lacks of its last stage
 #pragma unroll
         for (int pl = 0; pl < PLANES; pl++) out[pl * plane + (groups & ~7) + stage_chunk(1, t)] = make_uint4(0u, 0u, 0u, 0u);
-    if (t == 0) unscale[row] = __uint_as_float((uint32_t)min(max(127 - shift, 1), 254) << 23);
+    if (t == 0) unscale[row] = __uint_as_float((uint32_t)(127 - shift) << 23);
 }
 
 // ---------------------------------------------------------------- epilogue pieces (one lane = one weight row)

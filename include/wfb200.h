@@ -331,7 +331,10 @@ int wf_ipc_close(int64_t ctx, int64_t dptr);
  * recorded: wf_graph_begin sizes the decode kernels' scratch, and a recorded call that would have to
  * allocate or grow another buffer (the GEMM's activation copy and piece buffers, the gather buffer of
  * wf_qlinear_allgather) returns WF_ERR_RECORDING and records nothing -- issue the same call once
- * before wf_graph_begin. */
+ * before wf_graph_begin.
+ * A graph works in the scratch of the stream it was recorded on and keeps it: that stream may be destroyed, and a later
+ * call on it may need a larger buffer.  Launches of a graph, of other graphs recorded on the same stream and calls on that
+ * stream must therefore not run at the same time, whatever stream a graph is launched on. */
 int wf_graph_begin(int64_t ctx, int64_t stream);
 int wf_graph_end(int64_t ctx, int64_t stream, int64_t* graph);
 int wf_graph_launch(int64_t ctx, int64_t graph, int64_t stream);

@@ -3,7 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <unordered_map>
@@ -84,18 +84,27 @@ struct Weight {
     }
 };
 
-// Scratch of the kernels, one per stream that launches them (calls on different streams may overlap).
+// Scratch of the kernels, one per stream that launches them (calls on different streams may overlap).  A recorded graph keeps
+// a copy: its kernels hold these addresses however long it lives, whatever becomes of the stream it was recorded on and
+// though a later call there may need more and put a larger buffer in the place of one.
 struct GemvScratch {
-    uint2* d_slots = nullptr;  // [ctas][128] {value bits, tag}
-    float* d_part = nullptr;   // several-token kernel: partial sums of k-sliced launches
-    int* d_count = nullptr;    // several-token kernel: arrival counters per row-tile
+    std::shared_ptr<uint2> d_slots;  // [ctas][128] {value bits, tag}
+    std::shared_ptr<float> d_part;   // several-token kernel: partial sums of k-sliced launches
+    std::shared_ptr<int> d_count;    // several-token kernel: arrival counters per row-tile
     int ctas = 0;
     // tensor-core GEMM
-    void* d_x16 = nullptr;                 // fp16 copy of the activations
+    std::shared_ptr<uint8_t> d_x16;         // fp16 copy of the activations
     int64_t x16_bytes = 0;
-    float* d_gemm_partial = nullptr;       // [sm_count][512][128] pieces of tiles cut by a share boundary
-    unsigned int* d_gemm_ready = nullptr;  // [sm_count][4] generation whose piece is complete, per 32-row quarter; then {generation, CTAs out}
+    std::shared_ptr<float> d_gemm_partial;  // [sm_count][512][128] pieces of tiles cut by a share boundary
+    std::shared_ptr<unsigned int> d_gemm_ready;  // [sm_count][4] generation whose piece is complete, per 32-row quarter; then {generation, CTAs out}
 };
+// Device memory that is freed with the last reference to it.
+template <class T> inline cudaError_t make_shared_device(std::shared_ptr<T>& p, size_t bytes) {
+    void* q = nullptr;
+    const cudaError_t e = cudaMalloc(&q, bytes);
+    if (e == cudaSuccess) p.reset(static_cast<T*>(q), [](T* r) { cudaFree(r); });
+    return e;
+}
 
 struct Context {
     uint32_t magic = CTX_MAGIC;
@@ -115,6 +124,7 @@ struct Context {
     std::vector<cudaGraphExec_t> graphs;
     int64_t capture_launches = 0;  // product kernels recorded by the capture in progress
     std::unordered_map<cudaGraphExec_t, int64_t> graph_launches;
+    std::unordered_map<cudaGraphExec_t, GemvScratch> graph_scratch;  // of the stream it was recorded on
     std::unordered_map<int64_t, int64_t> allocs;  // device ptr -> bytes
     std::vector<void*> host_allocs;
     std::vector<Weight*> weights;
@@ -192,7 +202,6 @@ int qlinear_reserve(Context* c, const GemvCall& call, cudaStream_t s);
 int qlinear_launch(Context* c, const GemvCall& call, cudaStream_t s);
 // sizes the stream's scratch like the largest of the context's other streams (before a recording)
 int gemm_prepare_stream(Context* c, cudaStream_t s);
-void free_scratch(GemvScratch& sc);
 
 struct ScopedLock {
     Context* c;

@@ -144,24 +144,19 @@ static int gemm_scratch(Context* c, cudaStream_t s, GemvScratch& sc, int64_t x16
     if (x16_bytes > sc.x16_bytes) {
         const int rc = refuse_allocation_while_recording(c, s, "the fp16 activation scratch");
         if (rc != WF_OK) return rc;
-        if (sc.d_x16) cudaFree(sc.d_x16);
-        sc.d_x16 = nullptr;
+        sc.d_x16.reset();
         sc.x16_bytes = 0;
-        WF_CUDA(c, cudaMalloc(&sc.d_x16, (size_t)x16_bytes));
+        WF_CUDA(c, make_shared_device(sc.d_x16, (size_t)x16_bytes));
         sc.x16_bytes = x16_bytes;
     }
     if (!sc.d_gemm_ready) {
         const int rc = refuse_allocation_while_recording(c, s, "the GEMM's piece buffers");
         if (rc != WF_OK) return rc;
-        if (!sc.d_gemm_partial) WF_CUDA(c, cudaMalloc(&sc.d_gemm_partial, (size_t)c->sm_count * GEMM_PIECE_TOKENS * GEMM_BN * sizeof(float)));
+        if (!sc.d_gemm_partial) WF_CUDA(c, make_shared_device(sc.d_gemm_partial, (size_t)c->sm_count * GEMM_PIECE_TOKENS * GEMM_BN * sizeof(float)));
         const size_t bytes = ((size_t)c->sm_count * 4 + 2) * sizeof(unsigned int);
-        unsigned int* ready = nullptr;
-        WF_CUDA(c, cudaMalloc(&ready, bytes));
-        const cudaError_t e = cudaMemsetAsync(ready, 0, bytes, s);
-        if (e != cudaSuccess) {
-            cudaFree(ready);
-            return cuda_status(c, e, "cudaMemsetAsync");
-        }
+        std::shared_ptr<unsigned int> ready;
+        WF_CUDA(c, make_shared_device(ready, bytes));
+        WF_CUDA(c, cudaMemsetAsync(ready.get(), 0, bytes, s));
         sc.d_gemm_ready = ready;
     }
     return WF_OK;
@@ -287,11 +282,11 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
         const int rc = gemm_scratch(c, s, sc, x16_bytes);
         if (rc != WF_OK) return rc;
     }
-    p.partial = sc.d_gemm_partial;
-    p.ready = sc.d_gemm_ready;
-    p.gen = sc.d_gemm_ready + (size_t)c->sm_count * 4;
-    __half* x16 = static_cast<__half*>(sc.d_x16);
-    float* unscale = reinterpret_cast<float*>(static_cast<uint8_t*>(sc.d_x16) + x16_plane);
+    p.partial = sc.d_gemm_partial.get();
+    p.ready = sc.d_gemm_ready.get();
+    p.gen = p.ready + (size_t)c->sm_count * 4;
+    __half* x16 = reinterpret_cast<__half*>(sc.d_x16.get());
+    float* unscale = reinterpret_cast<float*>(sc.d_x16.get() + x16_plane);
     p.row_unscale = unscale;
 
     CUtensorMap map;

@@ -356,18 +356,12 @@ int gemv_prepare_stream(Context* c, cudaStream_t s) {
     if (sc.ctas >= c->sm_count) return WF_OK;
     const int rc = refuse_allocation_while_recording(c, s, "the decode kernels' scratch");
     if (rc != WF_OK) return rc;
-    if (sc.d_slots) cudaFree(sc.d_slots);
-    if (sc.d_part) cudaFree(sc.d_part);
-    if (sc.d_count) cudaFree(sc.d_count);
-    sc.d_slots = nullptr;
-    sc.d_part = nullptr;
-    sc.d_count = nullptr;
     sc.ctas = 0;
-    WF_CUDA(c, cudaMalloc(&sc.d_slots, (size_t)c->sm_count * 128 * sizeof(uint2)));
-    WF_CUDA(c, cudaMemset(sc.d_slots, 0, (size_t)c->sm_count * 128 * sizeof(uint2)));
-    WF_CUDA(c, cudaMalloc(&sc.d_part, GEMVN_PART_BYTES));
-    WF_CUDA(c, cudaMalloc(&sc.d_count, (size_t)GEMVN_MAX_ROW_TILES * sizeof(int)));
-    WF_CUDA(c, cudaMemset(sc.d_count, 0, (size_t)GEMVN_MAX_ROW_TILES * sizeof(int)));
+    WF_CUDA(c, make_shared_device(sc.d_slots, (size_t)c->sm_count * 128 * sizeof(uint2)));
+    WF_CUDA(c, cudaMemset(sc.d_slots.get(), 0, (size_t)c->sm_count * 128 * sizeof(uint2)));
+    WF_CUDA(c, make_shared_device(sc.d_part, GEMVN_PART_BYTES));
+    WF_CUDA(c, make_shared_device(sc.d_count, (size_t)GEMVN_MAX_ROW_TILES * sizeof(int)));
+    WF_CUDA(c, cudaMemset(sc.d_count.get(), 0, (size_t)GEMVN_MAX_ROW_TILES * sizeof(int)));
     sc.ctas = c->sm_count;
     return WF_OK;
 }
@@ -471,7 +465,7 @@ int gemv_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     if (rc != WF_OK) return rc;
     if (call.w->g.rt * call.w->g.kt < 1) return WF_OK;
     const GemvScratch& sc = c->gemv_scratch[s];
-    return launch_passes(c, call, s, GemvBuffers{sc.d_slots, sc.d_part, sc.d_count}, false, c->salt >= 2 ? c->d_timing : nullptr, "gemv launch");
+    return launch_passes(c, call, s, GemvBuffers{sc.d_slots.get(), sc.d_part.get(), sc.d_count.get()}, false, c->salt >= 2 ? c->d_timing : nullptr, "gemv launch");
 }
 
 // ---------------------------------------------------------------- a program's launches

@@ -53,16 +53,6 @@ Weight* get_weight(Context* c, int64_t h) {
     return w;
 }
 
-void free_scratch(GemvScratch& sc) {
-    cudaFree(sc.d_slots);
-    cudaFree(sc.d_part);
-    cudaFree(sc.d_count);
-    cudaFree(sc.d_x16);
-    cudaFree(sc.d_gemm_partial);
-    cudaFree(sc.d_gemm_ready);
-    sc = GemvScratch{};
-}
-
 cudaStream_t resolve_stream(Context* c, int64_t stream) {
     return stream == 0 ? c->stream : reinterpret_cast<cudaStream_t>(stream);
 }
@@ -372,8 +362,9 @@ int wf_destroy(int64_t ctx) {
     release_spare_tiles(c);
     for (auto& kv : c->allocs) cudaFree(reinterpret_cast<void*>(kv.first));
     for (void* h : c->host_allocs) cudaFreeHost(h);
-    for (auto& kv : c->gemv_scratch) free_scratch(kv.second);
     for (cudaGraphExec_t g : c->graphs) cudaGraphExecDestroy(g);
+    c->graph_scratch.clear();
+    c->gemv_scratch.clear();
     for (cudaEvent_t ev : c->events) cudaEventDestroy(ev);
     for (cudaStream_t s : c->streams) cudaStreamDestroy(s);
     if (c->h_stage) cudaFreeHost(c->h_stage);
@@ -423,11 +414,7 @@ int wf_stream_destroy(int64_t ctx, int64_t stream) {
     auto it = std::find(c->streams.begin(), c->streams.end(), s);
     if (stream == 0 || it == c->streams.end()) return WF_ERR_INVALID_HANDLE;
     WF_CUDA(c, cudaStreamSynchronize(s));
-    auto sc = c->gemv_scratch.find(s);
-    if (sc != c->gemv_scratch.end()) {
-        free_scratch(sc->second);
-        c->gemv_scratch.erase(sc);
-    }
+    c->gemv_scratch.erase(s);
     c->streams.erase(it);
     WF_CUDA(c, cudaStreamDestroy(s));
     return WF_OK;
@@ -717,13 +704,15 @@ int wf_graph_end(int64_t ctx, int64_t stream, int64_t* graph) {
     if (!graph) return WF_ERR_INVALID_ARGUMENT;
     *graph = 0;
     cudaGraph_t g = nullptr;
-    WF_CUDA(c, cudaStreamEndCapture(resolve_stream(c, stream), &g));
+    cudaStream_t s = resolve_stream(c, stream);
+    WF_CUDA(c, cudaStreamEndCapture(s, &g));
     cudaGraphExec_t exec = nullptr;
     cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return cuda_status(c, e, "cudaGraphInstantiate");
     c->graphs.push_back(exec);
     c->graph_launches[exec] = c->launches - c->capture_launches;
+    c->graph_scratch[exec] = c->gemv_scratch[s];
     c->launches = c->capture_launches;  // recorded, not yet run
     *graph = reinterpret_cast<int64_t>(exec);
     return WF_OK;
@@ -745,7 +734,9 @@ int wf_graph_destroy(int64_t ctx, int64_t graph) {
     if (it == c->graphs.end()) return WF_ERR_INVALID_HANDLE;
     c->graphs.erase(it);
     c->graph_launches.erase(exec);
-    WF_CUDA(c, cudaGraphExecDestroy(exec));
+    const cudaError_t e = cudaGraphExecDestroy(exec);
+    c->graph_scratch.erase(exec);  // (freeing device memory waits for a replay that is still running)
+    WF_CUDA(c, e);
     return WF_OK;
 }
 

@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_program_kernel(const 
 
     ProgRun run{P, reinterpret_cast<volatile int*>(smem) + 1, ld_acquire_gpu(&P.sync->epoch)};
     bool failed = false;
-    uint32_t seq = 0;
+    uint32_t seq = 0, sums32 = 0;  // sums32: the activation sums, which lie behind the records of the K that was staged
     int stamp_i = 0;
     auto stamp = [&]() {
         if (P.timing != nullptr && threadIdx.x == 0 && stamp_i < 64) {
@@ -424,6 +424,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_program_kernel(const 
                 default: stage_x_q8<R::BETA_INT, XK_BF16>(op.x, op.k, xd, recs, kt * T::K, GEMV_CONSUMERS); break;
             }
             run.consumers_sync();
+            sums32 = smem_u32(recs) + (uint32_t)((kt * T::K) >> 5) * 16;
             stamp();
         } else {
             stamp();
@@ -440,8 +441,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_program_kernel(const 
             }
         };
         ws_consume<QT, DEPTH>(sh, op.chunk_q, op.chunk_r, warp, lane, slots, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
-                       smem_u32(recs) + (uint32_t)((kt * T::K) >> 5) * 16, slots_g, P.status, smem_u32(const_cast<int*>(abort_flag)),
-                       share_of, P.n_ops, emit_row);
+                       sums32, slots_g, P.status, smem_u32(const_cast<int*>(abort_flag)), share_of, P.n_ops, emit_row);
         if (*abort_flag) failed = true;
         stamp();
     }

@@ -134,6 +134,7 @@ struct Context {
     };
     std::vector<SpareTiles> spare_tiles;  // tile buffers of freed weights, oldest first, at most SPARE_TILES_BYTES in all
     int64_t spare_tiles_bytes = 0;
+    bool foreign_streams = false;  // a stream that is not the context's own has been used: its work cannot be waited for by itself
     std::unordered_map<cudaStream_t, GemvScratch> gemv_scratch;
     // pinned staging for host-pointer calls
     void* h_stage = nullptr;

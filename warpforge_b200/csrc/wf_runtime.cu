@@ -54,7 +54,35 @@ Weight* get_weight(Context* c, int64_t h) {
 }
 
 cudaStream_t resolve_stream(Context* c, int64_t stream) {
-    return stream == 0 ? c->stream : reinterpret_cast<cudaStream_t>(stream);
+    if (stream == 0) return c->stream;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    if (!c->foreign_streams) c->foreign_streams = std::find(c->streams.begin(), c->streams.end(), s) == c->streams.end();
+    return s;
+}
+
+// While one lives, calls that CUDA refuses to a thread that is recording a stream (freeing memory, waiting for another
+// stream) are allowed: nothing that this library does under it belongs to the recording.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Waits for everything that the context has launched on its own streams.  *idle = false: some of it cannot be waited for (a
+// stream is being recorded, or one that is not the context's own has been used).
+static cudaError_t wait_for_own_streams(Context* c, bool* idle) {
+    *idle = !c->foreign_streams;
+    auto wait = [&](cudaStream_t s) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        cudaError_t e = cudaStreamIsCapturing(s, &st);
+        if (e == cudaSuccess && st == cudaStreamCaptureStatusNone) return cudaStreamSynchronize(s);
+        *idle = false;
+        return e;
+    };
+    cudaError_t e = wait(c->stream);
+    for (cudaStream_t s : c->streams)
+        if (e == cudaSuccess) e = wait(s);
+    return e;
 }
 
 int ensure_stage(Context* c, int64_t host_bytes, int64_t dev_bytes) {
@@ -103,7 +131,8 @@ static cudaError_t fetch_from_host(void* d_dst, const void* h_src_dev, int64_t b
 // Tile buffers of freed weights are kept for the next upload of about the same size: cudaMalloc and cudaFree of a
 // large buffer take 0.3 ms each, as much as 18 MB of blocks on the link, and far more when other processes of the
 // machine use the driver.  Bounded, emptied when an allocation of the context fails and when it is destroyed.
-// A buffer enters the pool after the device has been synchronised (wf_weight_free), so it is idle for every stream.
+// A buffer enters the pool when every stream it may have been read on has been waited for (wf_weight_free), so it is idle.
+// That wait is not cudaDeviceSynchronize, which fails while anything on the device is being recorded and ends the recording.
 // Where a buffer does not fit any more the oldest ones go: sizes of a model that is no longer loaded must not keep the
 // current one's out (Q4_0 [28672 x 4096], upload + one token + free, after a 430 MB model was closed: 2.3 - 5.9 ms when the
 // newcomer was freed instead, 1.5 - 1.7 ms).
@@ -583,9 +612,12 @@ int wf_weight_free(int64_t ctx, int64_t weight) {
     if (!w) return WF_ERR_INVALID_HANDLE;
     if (w->programs > 0)
         return set_error(c, WF_ERR_IN_USE, "weight is referenced by %d live program(s): destroy them first", w->programs);
+    RelaxedCapture relaxed;
+    bool idle = false;  // no kernel reads the tiles any more
+    WF_CUDA(c, wait_for_own_streams(c, &idle));
+    if (idle) give_back_tiles(c, w->d_tiles, w->tiles_held);
+    else WF_CUDA(c, cudaFree(w->d_tiles));  // waits for what is running
     c->weights.erase(std::find(c->weights.begin(), c->weights.end(), w));
-    WF_CUDA(c, cudaDeviceSynchronize());  // kernels of any stream may still read the tiles
-    give_back_tiles(c, w->d_tiles, w->tiles_held);
     w->magic = 0;
     delete w;
     return WF_OK;

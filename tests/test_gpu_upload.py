@@ -107,3 +107,21 @@ def test_freed_after_use_on_a_stream_of_another_library():
         v.close()
     finally:
         ctx.close()
+
+
+def test_kept_buffers_count_as_free_memory():
+    from warpforge_b200.backend import CudaContext, QuantizedWeight
+
+    ctx = CudaContext(0)
+    try:
+        def once():
+            QuantizedWeight(ctx, Q.QuantizationType.Q4_0, np.zeros(8192 * 4096 // 32 * 18, np.uint8), 8192, 4096).close()
+
+        once()  # the upload's own buffers
+        before = ctx.device_info()["free_mem"]
+        w = QuantizedWeight(ctx, Q.QuantizationType.Q4_0, np.zeros(8192 * 4096 // 32 * 18, np.uint8), 8192, 4096)
+        assert ctx.device_info()["free_mem"] <= before - w.device_bytes() // 2
+        w.close()
+        assert ctx.device_info()["free_mem"] >= before
+    finally:
+        ctx.close()

@@ -501,15 +501,15 @@ static void setup_peer_landing(Context* c, Comm* k) {
         const long long v = atoll(mb);
         if (v >= 0 && v <= 65536) stage = v << 20;
     }
-    ok = ok && cudaMalloc(&own, (size_t)(GATHER_LAND_BYTES + GATHER_FLAG_BYTES + stage)) == cudaSuccess;
+    ok = ok && device_alloc(c, &own, (size_t)(GATHER_LAND_BYTES + GATHER_FLAG_BYTES + stage)) == cudaSuccess;
     ok = ok && cudaMemset(own, 0, (size_t)(GATHER_LAND_BYTES + GATHER_FLAG_BYTES)) == cudaSuccess;
-    ok = ok && cudaMalloc(&k->d_epoch, 4 * sizeof(unsigned int)) == cudaSuccess;
+    ok = ok && device_alloc(c, &k->d_epoch, 4 * sizeof(unsigned int)) == cudaSuccess;
     ok = ok && cudaMemset(k->d_epoch, 0, 4 * sizeof(unsigned int)) == cudaSuccess;
     k->stage_bytes = stage;
     ok = ok && cudaIpcGetMemHandle(&h[k->rank], own) == cudaSuccess;
     cudaGetLastError();
     // the two exchanges run on every rank whatever happened above, so that no rank waits alone
-    if (cudaMalloc(&d_x, (size_t)k->world * 64 + (size_t)k->world * 4) != cudaSuccess) {
+    if (device_alloc(c, &d_x, (size_t)k->world * 64 + (size_t)k->world * 4) != cudaSuccess) {
         cudaGetLastError();
         if (own) cudaFree(own);
         if (k->d_epoch) cudaFree(k->d_epoch);
@@ -769,7 +769,7 @@ int wf_qlinear_allgather(int64_t ctx, int64_t comm, int64_t weight, const void* 
         if (k->d_tmp) cudaFree(k->d_tmp);
         k->d_tmp = nullptr;
         k->tmp_bytes = 0;
-        WF_CUDA(c, cudaMalloc(&k->d_tmp, (size_t)need));
+        WF_CUDA(c, device_alloc(c, &k->d_tmp, (size_t)need));
         k->tmp_bytes = need;
     }
     float* mine = k->d_tmp + (int64_t)k->world * m * rows;

@@ -98,10 +98,13 @@ struct GemvScratch {
     std::shared_ptr<float> d_gemm_partial;  // [sm_count][512][128] pieces of tiles cut by a share boundary
     std::shared_ptr<unsigned int> d_gemm_ready;  // [sm_count][4] generation whose piece is complete, per 32-row quarter; then {generation, CTAs out}
 };
+// cudaMalloc for everything that a context allocates: where memory is short, its kept tile buffers go first.
+cudaError_t device_alloc(Context* c, void** p, size_t bytes);
+template <class T> inline cudaError_t device_alloc(Context* c, T** p, size_t bytes) { return device_alloc(c, reinterpret_cast<void**>(p), bytes); }
 // Device memory that is freed with the last reference to it.
-template <class T> inline cudaError_t make_shared_device(std::shared_ptr<T>& p, size_t bytes) {
+template <class T> inline cudaError_t make_shared_device(Context* c, std::shared_ptr<T>& p, size_t bytes) {
     void* q = nullptr;
-    const cudaError_t e = cudaMalloc(&q, bytes);
+    const cudaError_t e = device_alloc(c, &q, bytes);
     if (e == cudaSuccess) p.reset(static_cast<T*>(q), [](T* r) { cudaFree(r); });
     return e;
 }

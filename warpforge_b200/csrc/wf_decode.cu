@@ -514,7 +514,7 @@ static bool program_launches(Context* c, const std::vector<ProgOp>& ops, Program
             g.aux = nullptr;
         }
         if (g.n == 2 && j < n_ops && makes_act(ops, i, j)) {
-            if (!pr->d_act && cudaMalloc(&pr->d_act, (size_t)act_rows * sizeof(float)) != cudaSuccess) {
+            if (!pr->d_act && device_alloc(c, &pr->d_act, (size_t)act_rows * sizeof(float)) != cudaSuccess) {
                 cudaGetLastError();
                 return false;
             }
@@ -748,15 +748,15 @@ int wf_program_create_fused(int64_t ctx, int n_ops, const int64_t* weights, cons
     pr->rank = rank;
     pr->grid = grid;
     pr->smem = fixed + (size_t)stages * stage;
-    cudaError_t e = cudaMalloc(&pr->d_scratch, (size_t)2 * grid * 128 * sizeof(uint2));
+    cudaError_t e = device_alloc(c, &pr->d_scratch, (size_t)2 * grid * 128 * sizeof(uint2));
     if (e == cudaSuccess) e = cudaMemset(pr->d_scratch, 0, (size_t)2 * grid * 128 * sizeof(uint2));
-    if (c->salt >= 2 && e == cudaSuccess && cudaMalloc(&pr->d_timing, (size_t)grid * 64 * 8) == cudaSuccess)
+    if (c->salt >= 2 && e == cudaSuccess && device_alloc(c, &pr->d_timing, (size_t)grid * 64 * 8) == cudaSuccess)
         cudaMemset(pr->d_timing, 0, (size_t)grid * 64 * 8);
     if (e == cudaSuccess && (world > 1 || !program_launches(c, ops, pr))) {
         pr->launches.clear();
-        e = cudaMalloc(&pr->d_ops, sizeof(ProgOp) * (size_t)n_ops);
-        if (e == cudaSuccess) e = cudaMalloc(&pr->d_sync, sizeof(ProgSync));
-        if (e == cudaSuccess && !shares.empty()) e = cudaMalloc(&pr->d_shares, shares.size() * sizeof(int2));
+        e = device_alloc(c, &pr->d_ops, sizeof(ProgOp) * (size_t)n_ops);
+        if (e == cudaSuccess) e = device_alloc(c, &pr->d_sync, sizeof(ProgSync));
+        if (e == cudaSuccess && !shares.empty()) e = device_alloc(c, &pr->d_shares, shares.size() * sizeof(int2));
         if (e == cudaSuccess && !shares.empty()) e = cudaMemcpy(pr->d_shares, shares.data(), shares.size() * sizeof(int2), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(pr->d_ops, ops.data(), sizeof(ProgOp) * (size_t)n_ops, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemset(pr->d_sync, 0, sizeof(ProgSync));

@@ -146,16 +146,16 @@ static int gemm_scratch(Context* c, cudaStream_t s, GemvScratch& sc, int64_t x16
         if (rc != WF_OK) return rc;
         sc.d_x16.reset();
         sc.x16_bytes = 0;
-        WF_CUDA(c, make_shared_device(sc.d_x16, (size_t)x16_bytes));
+        WF_CUDA(c, make_shared_device(c, sc.d_x16, (size_t)x16_bytes));
         sc.x16_bytes = x16_bytes;
     }
     if (!sc.d_gemm_ready) {
         const int rc = refuse_allocation_while_recording(c, s, "the GEMM's piece buffers");
         if (rc != WF_OK) return rc;
-        if (!sc.d_gemm_partial) WF_CUDA(c, make_shared_device(sc.d_gemm_partial, (size_t)c->sm_count * GEMM_PIECE_TOKENS * GEMM_BN * sizeof(float)));
+        if (!sc.d_gemm_partial) WF_CUDA(c, make_shared_device(c, sc.d_gemm_partial, (size_t)c->sm_count * GEMM_PIECE_TOKENS * GEMM_BN * sizeof(float)));
         const size_t bytes = ((size_t)c->sm_count * 4 + 2) * sizeof(unsigned int);
         std::shared_ptr<unsigned int> ready;
-        WF_CUDA(c, make_shared_device(ready, bytes));
+        WF_CUDA(c, make_shared_device(c, ready, bytes));
         WF_CUDA(c, cudaMemsetAsync(ready.get(), 0, bytes, s));
         sc.d_gemm_ready = ready;
     }

@@ -357,10 +357,10 @@ int gemv_prepare_stream(Context* c, cudaStream_t s) {
     const int rc = refuse_allocation_while_recording(c, s, "the decode kernels' scratch");
     if (rc != WF_OK) return rc;
     sc.ctas = 0;
-    WF_CUDA(c, make_shared_device(sc.d_slots, (size_t)c->sm_count * 128 * sizeof(uint2)));
+    WF_CUDA(c, make_shared_device(c, sc.d_slots, (size_t)c->sm_count * 128 * sizeof(uint2)));
     WF_CUDA(c, cudaMemset(sc.d_slots.get(), 0, (size_t)c->sm_count * 128 * sizeof(uint2)));
-    WF_CUDA(c, make_shared_device(sc.d_part, GEMVN_PART_BYTES));
-    WF_CUDA(c, make_shared_device(sc.d_count, (size_t)GEMVN_MAX_ROW_TILES * sizeof(int)));
+    WF_CUDA(c, make_shared_device(c, sc.d_part, GEMVN_PART_BYTES));
+    WF_CUDA(c, make_shared_device(c, sc.d_count, (size_t)GEMVN_MAX_ROW_TILES * sizeof(int)));
     WF_CUDA(c, cudaMemset(sc.d_count.get(), 0, (size_t)GEMVN_MAX_ROW_TILES * sizeof(int)));
     sc.ctas = c->sm_count;
     return WF_OK;

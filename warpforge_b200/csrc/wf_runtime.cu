@@ -98,7 +98,7 @@ int ensure_stage(Context* c, int64_t host_bytes, int64_t dev_bytes) {
         if (c->d_stage) cudaFree(c->d_stage);
         c->d_stage = nullptr;
         c->d_stage_bytes = 0;
-        WF_CUDA(c, cudaMalloc(&c->d_stage, (size_t)dev_bytes));
+        WF_CUDA(c, device_alloc(c, &c->d_stage, (size_t)dev_bytes));
         c->d_stage_bytes = dev_bytes;
     }
     return WF_OK;
@@ -151,19 +151,23 @@ cudaError_t take_tiles(Context* c, int64_t bytes, uint8_t** tiles, int64_t* held
         return cudaSuccess;
     }
     *held = bytes;
-    cudaError_t e = cudaMalloc(tiles, (size_t)bytes);
-    if (e == cudaErrorMemoryAllocation && !c->spare_tiles.empty()) {
-        cudaGetLastError();
-        release_spare_tiles(c);
-        e = cudaMalloc(tiles, (size_t)bytes);
-    }
-    return e;
+    return device_alloc(c, tiles, (size_t)bytes);
 }
 
 void release_spare_tiles(Context* c) {
     for (const auto& t : c->spare_tiles) cudaFree(t.tiles);
     c->spare_tiles.clear();
     c->spare_tiles_bytes = 0;
+}
+
+cudaError_t device_alloc(Context* c, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && !c->spare_tiles.empty()) {
+        cudaGetLastError();
+        release_spare_tiles(c);
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
 }
 
 static void give_back_tiles(Context* c, uint8_t* tiles, int64_t held) {
@@ -225,7 +229,7 @@ static cudaError_t upload_and_repack(Context* c, int qtype, const uint8_t* src, 
         c->h_upload = c->d_upload = nullptr;
         c->upload_chunk_bytes = 0;
         e = cudaMallocHost(&c->h_upload, (size_t)(UPLOAD_RING * chunk_bytes));
-        if (e == cudaSuccess) e = cudaMalloc(&c->d_upload, (size_t)(UPLOAD_RING * chunk_bytes));
+        if (e == cudaSuccess) e = device_alloc(c, &c->d_upload, (size_t)(UPLOAD_RING * chunk_bytes));
         if (e != cudaSuccess) return e;
         c->upload_chunk_bytes = chunk_bytes;
     }
@@ -423,7 +427,7 @@ int wf_device_info(int64_t ctx, int* sm_count, int* cc_major, int* cc_minor, int
     if (cc_major) *cc_major = c->cc_major;
     if (cc_minor) *cc_minor = c->cc_minor;
     if (total_mem) *total_mem = (int64_t)t;
-    if (free_mem) *free_mem = (int64_t)f;
+    if (free_mem) *free_mem = (int64_t)f + c->spare_tiles_bytes;  // kept tile buffers are given back when memory is short
     return WF_OK;
 }
 
@@ -489,13 +493,7 @@ int wf_malloc(int64_t ctx, int64_t bytes, int64_t* dptr) {
     WF_ENTER(ctx);
     if (!dptr || bytes < 0) return WF_ERR_INVALID_ARGUMENT;
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, (size_t)std::max<int64_t>(bytes, 1));
-    if (e == cudaErrorMemoryAllocation && !c->spare_tiles.empty()) {
-        cudaGetLastError();
-        release_spare_tiles(c);
-        e = cudaMalloc(&p, (size_t)std::max<int64_t>(bytes, 1));
-    }
-    if (e != cudaSuccess) return cuda_status(c, e, "cudaMalloc");
+    WF_CUDA(c, device_alloc(c, &p, (size_t)std::max<int64_t>(bytes, 1)));
     c->allocs[reinterpret_cast<int64_t>(p)] = bytes;
     *dptr = reinterpret_cast<int64_t>(p);
     return WF_OK;
@@ -647,7 +645,7 @@ int wf_dequant_rows(int64_t ctx, int64_t weight, int64_t row0, int64_t nrows, fl
     if (nrows == 0) return WF_OK;
     const int64_t bytes = nrows * w->g.k * (int64_t)sizeof(float);
     float* d_out = nullptr;
-    WF_CUDA(c, cudaMalloc(&d_out, (size_t)bytes));
+    WF_CUDA(c, device_alloc(c, &d_out, (size_t)bytes));
     cudaError_t e = launch_dequant_rows(*w, row0, nrows, d_out, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out_host, d_out, (size_t)bytes, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -849,7 +847,7 @@ int wf_set_salt(int64_t ctx, int salt) {
     WF_ENTER(ctx);
     if (salt < 0 || salt > 2) return WF_ERR_INVALID_ARGUMENT;
     if (salt >= 2 && !c->d_timing) {
-        WF_CUDA(c, cudaMalloc(&c->d_timing, (size_t)c->sm_count * 8 * sizeof(unsigned long long)));
+        WF_CUDA(c, device_alloc(c, &c->d_timing, (size_t)c->sm_count * 8 * sizeof(unsigned long long)));
         WF_CUDA(c, cudaMemset(c->d_timing, 0, (size_t)c->sm_count * 8 * sizeof(unsigned long long)));
     }
     c->salt = salt;

@@ -362,8 +362,10 @@ int wf_read_timing(int64_t ctx, int64_t* out, int64_t n);
 int wf_launch_count(int64_t ctx, int64_t* launches);
 /* How the several-token decode kernel would cut a [rows x k] weight of type qtype for `cols` activation columns
  * (1..32; an fp32 token counts three) on a device with sm_count SMs: k-slices, k-tiles per slice, about how many warps
- * share a row-tile, whether sums of several slices or columns are brought together, shared-memory bytes.  Needs no device (host arithmetic only); slices = 0 means
- * no cut fits and the call is run in several launches of fewer columns. */
+ * share a row-tile, whether sums of several slices or columns are brought together, shared-memory bytes.  Needs no device
+ * (host arithmetic only).  slices = 0: no cut whose sums come to 8 MB at most is the cheapest; the columns are then run as
+ * clusters whose sums meet in shared memory, or in several launches of fewer.  (A call of that many columns may take several
+ * launches in any case, where the estimate says that they are quicker.) */
 int wf_plan_several_tokens(int qtype, int64_t rows, int64_t k, int cols, int x_is_f32, int sm_count, int* slices,
                            int* k_tiles_per_slice, int* team, int* uses_partial_sums, int64_t* smem_bytes);
 

@@ -129,3 +129,14 @@ def test_swiglu_between_launches(d, ffn):
             assert np.max(np.abs(a - b)) <= 1e-5 * np.max(np.abs(b))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("rows,k,m,f32", [
+    (36000, 3072, 32, False),   # clusters whose sums come to more than the partial-sum buffer holds
+    (28014, 4992, 32, False),   # tall and many columns: two launches of sixteen
+    (28014, 4992, 31, False),   # sixteen and fifteen
+    (6704, 9728, 10, True),     # fp32 tokens: more than 200 KB of shared memory, one batch
+    (9001, 11008, 7, True),
+])
+def test_exact_tall(rows, k, m, f32):
+    test_exact(rows, k, m, f32)

@@ -77,13 +77,12 @@ struct Weight {
     bool beyond_fp16 = false;  // some block may hold values outside fp16's range
     int64_t tiles_held = 0;  // bytes allocated at d_tiles (a reused buffer may be larger than g.bytes())
     int programs = 0;        // live programs whose op lists point at d_tiles
-    // how the several-token decode kernel cuts this weight, per activation dtype (bf16 / fp32) and column count:
-    // {slices, k-tiles per slice, team size, uses partial sums}, slices = -1 until first asked for (0: no cut fits)
-    short split_cache[2][33][4];
-    Weight() {
-        for (auto& a : split_cache)
-            for (auto& b : a) b[0] = -1;
-    }
+    // how the several-token decode kernel cuts this weight, per activation dtype (bf16 / fp32) and column count
+    struct Split {
+        short slices = -1;  // -1: not asked for yet, 0: no cut fits
+        short kc = 0, batch = 0, ctas = 0;
+        float ns = 0.f;  // the estimate
+    } split_cache[2][33];
 };
 
 // Scratch of the kernels, one per stream that launches them (calls on different streams may overlap).  A recorded graph keeps

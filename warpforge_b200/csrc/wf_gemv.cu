@@ -234,29 +234,54 @@ static const int* gemvn_clusters(int sm_count) {
 // The cut of a weight for `cols` activation columns, worked out once per weight (the search walks dozens of
 // candidates: too slow for every call of a microsecond-scale kernel).
 static GemvNPlan cached_plan(int sm_count, const Weight& w, int cols, bool x_f32) {
-    short* e = const_cast<Weight&>(w).split_cache[x_f32 ? 1 : 0][cols];
-    if (e[0] < 0) {
+    Weight::Split& e = const_cast<Weight&>(w).split_cache[x_f32 ? 1 : 0][cols];
+    if (e.slices < 0) {
         const GemvNPlan p = gemvn_plan(gemvn_clusters(sm_count), w.g.qtype, w.g.rt, w.g.kt, cols, x_f32);
-        e[1] = (short)p.kc;
-        e[2] = (short)p.batch;
-        e[3] = (short)p.ctas;
-        e[0] = (short)p.slices;
+        e.kc = (short)p.kc;
+        e.batch = (short)p.batch;
+        e.ctas = (short)p.ctas;
+        e.ns = (float)p.ns;
+        e.slices = (short)p.slices;
     }
     GemvNPlan p;
-    p.slices = e[0];
-    p.kc = e[1];
-    p.batch = e[2];
-    p.ctas = e[3];
+    p.slices = e.slices;
+    p.kc = e.kc;
+    p.batch = e.batch;
+    p.ctas = e.ctas;
+    p.ns = e.ns;
     p.part = p.slices > GEMVN_MAX_CLUSTER;
     return p;
 }
 
-// Activation columns one launch of the several-token kernel can take for this weight: at most 32, fewer when the
-// partial sums of a k-sliced launch would not fit their buffer (very tall weights).
+// Activation columns one launch of the several-token kernel can take for this weight: at most 32, fewer when no slice of
+// them fits, or the partial sums of more than eight slices would not fit their buffer.
 static int gemvn_cols_per_pass(int sm_count, const Weight& w, bool x_f32) {
     for (int cols = GEMVN_MAX_COLS; cols >= (x_f32 ? 3 : 1); cols--)
         if (cached_plan(sm_count, w, cols, x_f32).slices > 0) return cols;
     return 0;
+}
+
+// Tokens per launch for a call of m tokens: as many as one launch can take, or 16 columns where the estimate says that
+// several launches, which read the weight again, are quicker than one whose activations leave little room for batches of
+// sums (a launch boundary costs about 2 us).  32 tokens: Q4_0 [28014 x 4992] 58.4 us in one launch, 50.3 in two; Q4_K
+// [28672 x 8192] 122 and 105; [4096 x 4096] 10.0 and 13.4.
+static int gemvn_tokens_per_pass(int sm_count, const Weight& w, bool x_f32, int64_t m) {
+    const int per_tok = x_f32 ? 3 : 1;
+    int best = 0;
+    double best_ns = 0;
+    for (int cols : {gemvn_cols_per_pass(sm_count, w, x_f32), 16}) {
+        const int64_t most = cols / per_tok;
+        if (most < 1 || (best > 0 && most >= best)) continue;
+        const int64_t passes = (m + most - 1) / most, tokens = (m + passes - 1) / passes;
+        const GemvNPlan p = cached_plan(sm_count, w, (int)tokens * per_tok, x_f32);
+        if (p.slices < 1) continue;
+        const double ns = (double)passes * (p.ns + 2000.0);
+        if (best == 0 || ns < best_ns) {
+            best_ns = ns;
+            best = (int)tokens;
+        }
+    }
+    return best;
 }
 
 // Largest number of tokens one launch can take (0: the weight does not fit any kernel).
@@ -409,7 +434,7 @@ static int launch_passes(Context* c, const GemvCall& call, cudaStream_t s, const
         return WF_OK;
     }
     const int per_tok = f32 ? 3 : 1;
-    const int per_pass = gemvn_cols_per_pass(c->sm_count, w, f32) / per_tok;
+    const int per_pass = gemvn_tokens_per_pass(c->sm_count, w, f32, call.m);
     if (per_pass < 1) return set_error(c, WF_ERR_TOO_LARGE, "weight [%lld x %lld] is beyond the decode kernels", (long long)w.g.rows, (long long)w.g.k);
     if (w.g.rt > GEMVN_MAX_ROW_TILES) return set_error(c, WF_ERR_TOO_LARGE, "%lld rows: more than %d row-tiles", (long long)w.g.rows, GEMVN_MAX_ROW_TILES);
     for (int64_t m0 = 0; m0 < call.m; m0 += per_pass) {
@@ -622,7 +647,9 @@ extern "C" int wf_plan_several_tokens(int qtype, int64_t rows, int64_t k, int co
     const int64_t rt = (rows + 15) / 16, kt = (k + tile_k(qt) - 1) / tile_k(qt);
     int clusters[GEMVN_MAX_CLUSTER + 1];
     gemvn_clusters_estimate(sm_count, clusters);
-    const GemvNPlan p = gemvn_plan(clusters, qt, rt, kt, cols, x_is_f32 != 0);
+    GemvNPlan p = gemvn_plan(clusters, qt, rt, kt, cols, x_is_f32 != 0);
+    // sums that meet in clusters need no buffer: a cut whose sums come to more than it holds is not described here
+    if (p.slices > 1 && gemvn_sum_bytes(p.slices, cols, rt) > GEMVN_PART_BYTES) p = GemvNPlan{};
     *slices = p.slices;
     *k_tiles_per_slice = p.kc;
     // the warps of a CTA cut its tiles evenly: about this many share a row-tile

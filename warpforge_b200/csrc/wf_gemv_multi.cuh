@@ -39,7 +39,10 @@ constexpr int GEMVN_MAX_COLS = 32;
 constexpr int GEMVN_MAX_SLICES = 64;
 constexpr int GEMVN_MAX_CLUSTER = 8;  // slices that meet in a cluster (the largest portable size)
 constexpr int GEMVN_MAX_BATCH = 64;   // units a CTA adds up at a time
-constexpr size_t GEMVN_SMEM = 200 * 1024;
+// Shared memory that a plan may fill.  bf16 tokens: what wf_plan_several_tokens has always kept to.  fp32 tokens, whose rows
+// are three columns, need more of it for their sums: with all there is, the units of a CTA are mostly one batch (ten tokens,
+// Q4_0 [6704 x 9728]: 34.7 -> 31.8 us).
+constexpr size_t GEMVN_SMEM = 200 * 1024, GEMVN_SMEM_F32 = 227 * 1024;
 constexpr size_t GEMVN_PART_BYTES = 8u << 20;  // partial sums a launch may use (the static array of the no-alloc entry is this large)
 constexpr int GEMVN_MAX_ROW_TILES = 1 << 16;   // arrival counters
 
@@ -113,16 +116,21 @@ inline size_t gemvn_smem(int qt, int kc, int cols, bool x_f32, int slices, int b
     return b;
 }
 
+inline size_t gemvn_sum_bytes(int slices, int cols, int64_t rt) { return (size_t)slices * ((cols + 1) & ~1) * rt * 16 * 4; }
+
 struct GemvNPlan {
     int slices = 0, kc = 0, batch = 0;  // slices == 0: no plan fits
     int ctas = 0;                       // CTAs (per slice, where the slices form clusters)
     bool part = false;                  // partial sums go through memory
+    double ns = 0;                      // the estimate
 };
 // clusters[S]: how many clusters of S CTAs the device holds at a time (S = 1: SMs).  The cheapest cut by an estimate in
 // nanoseconds: the busiest warp's tiles, the staging of the slice, and per batch the way of its sums to y.  The constants
-// are a fit to 78 measured weights from 128 x 8192 to 28014 x 2496 with 2 .. 32 columns, each at every S up to 8: its choices
-// are 1.5 % slower than the best S on average, 19 % at worst.  Memory is the way where eight slices do not fit (against a
-// cluster of the same S it measured 1 - 4 us more on small weights and within 8 % either way on tall ones).
+// are a fit to 78 measured weights from 128 x 8192 to 28014 x 2496 with 2 .. 32 columns, each at every S up to 8.  In calls of
+// more than 13 us clusters of 3, 5 and 7 take longer than that by 8 % and 4 %, and 20 % on devices whose GPCs hold an odd
+// number of 7s.  On 130 other weights, up to 32000 x 8192, the choices are 1.4 % slower than the best S on average and 14 % at
+// worst (2.4 % and 32 % without that correction).  Memory is the way where eight slices do not fit (against a cluster of the
+// same S it measured 1 - 4 us more on small weights, up to twice the time on tall ones).
 inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt, int cols, bool x_f32) {
     GemvNPlan best;
     const int ng = cols <= 8 ? 1 : cols <= 16 ? 2 : 4, tk = tile_k(qt), sms = clusters[1];
@@ -135,13 +143,12 @@ inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt,
         if (kc == last_kc) continue;
         last_kc = kc;
         const bool part = slices > GEMVN_MAX_CLUSTER;
-        // (what wf_plan_several_tokens promises of every cut; a cluster's sums do not need the buffer)
-        if (slices > 1 && (size_t)slices * ((cols + 1) & ~1) * rt * 16 * 4 > GEMVN_PART_BYTES) continue;
+        if (part && gemvn_sum_bytes(slices, cols, rt) > GEMVN_PART_BYTES) continue;
         const int64_t room = part ? sms / slices : clusters[slices];  // CTAs a slice gets, at least
         if (room < 1) continue;
         const int64_t units = (rt + std::min(room, rt) - 1) / std::min(room, rt);  // of the busiest CTA
         int batch = (int)std::min<int64_t>(units, GEMVN_MAX_BATCH);
-        while (batch >= 1 && gemvn_smem(qt, kc, cols, x_f32, slices, batch, nullptr, nullptr, nullptr) > GEMVN_SMEM) batch--;
+        while (batch >= 1 && gemvn_smem(qt, kc, cols, x_f32, slices, batch, nullptr, nullptr, nullptr) > (x_f32 ? GEMVN_SMEM_F32 : GEMVN_SMEM)) batch--;
         if (batch < 1) continue;
         double ns = (double)cols * kc * tk * 2 / (x_f32 ? 27.2 : 87.3);
         for (int64_t left = units; left > 0; left -= batch) {
@@ -152,6 +159,7 @@ inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt,
             else if (slices > 1) ns += 616.0 + slices * (6.1 + 32.1 * ((own * ng + GEMV_WARPS - 1) / GEMV_WARPS));
             if (x_f32 && !part) ns += 31.1 * slices * ((own * (cols / 3) * 16 + GEMV_CONSUMERS - 1) / GEMV_CONSUMERS);
         }
+        if (!part && ns > 13000.0) ns *= slices == 3 || slices == 7 ? 1.1 : slices == 5 ? 1.05 : 1.0;
         if (best.slices == 0 || ns < best_ns) {
             best_ns = ns;
             best.slices = slices;
@@ -159,6 +167,7 @@ inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt,
             best.batch = batch;
             best.ctas = (int)std::min(room, rt);
             best.part = part;
+            best.ns = ns;
         }
     }
     return best;

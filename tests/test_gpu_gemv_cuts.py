@@ -140,3 +140,13 @@ def test_swiglu_between_launches(d, ffn):
 ])
 def test_exact_tall(rows, k, m, f32):
     test_exact(rows, k, m, f32)
+
+
+@pytest.mark.parametrize("rows,k,m,f32", [
+    (16, 32, 17, False), (3001, 2016, 24, False),            # one slice
+    (260, 2080, 20, False), (7000, 3104, 23, False),         # clusters; several batches
+    (30, 65536, 24, False),                                  # memory
+    (100, 3200, 6, True), (3001, 4128, 8, True), (2000, 96, 7, True),
+])
+def test_exact_three_groups_of_columns(rows, k, m, f32):
+    test_exact(rows, k, m, f32)

@@ -460,12 +460,13 @@ static int launch_passes(Context* c, const GemvCall& call, cudaStream_t s, const
         p.kc = plan.kc;
         p.batch = plan.batch;
         p.cluster = plan.slices > 1 && !plan.part;
-        const int ng = p.cols <= 8 ? 1 : p.cols <= 16 ? 2 : 4;
+        const int ng = (p.cols + 7) / 8;
         const int grid = plan.part ? c->sm_count : plan.ctas * plan.slices;
         const size_t smem = gemvn_smem(qt, p.kc, p.cols, f32, p.slices, p.batch, &p.sx, &p.piece_off, &p.ex_off);
         if (clear && plan.part) WF_CUDA(c, cudaMemsetAsync(buf.count, 0, (size_t)w.g.rt * sizeof(int), s));
         const cudaError_t e = ng == 1   ? launch_qt_several<1, false>(qt, p, grid, smem, s)
                               : ng == 2 ? launch_qt_several<2, false>(qt, p, grid, smem, s)
+                              : ng == 3 ? launch_qt_several<3, false>(qt, p, grid, smem, s)
                                         : launch_qt_several<4, false>(qt, p, grid, smem, s);
         if (e != cudaSuccess) return cuda_status(c, e, what);
         c->launches++;

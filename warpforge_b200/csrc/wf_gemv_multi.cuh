@@ -2,7 +2,7 @@
 //
 // Every warp loads its tiles from global memory straight into registers (the tile layout is the MMA's fragment
 // order) and multiplies them on mma.m16n8k16 with exact bf16 operands and fp32 accumulation: the 4-bit codes of a
-// 32-k block become A fragments once (unpack8) and meet NG = 1, 2 or 4 groups of eight activation columns, so the
+// 32-k block become A fragments once (unpack8) and meet NG = 1 .. 4 groups of eight activation columns, so the
 // integer work per weight byte does not grow with the number of tokens.  fp32 activations enter as three exact
 // bf16 columns per token (x = hi + mid + lo), as in the one-pass ring kernel this replaces.
 //
@@ -97,14 +97,14 @@ cudaError_t gemv_launch_group(const GemvPrepared& g, cudaStream_t s);
 
 template <int QT, int NG> struct GemvNGeom {
     // tiles a warp holds in registers while it multiplies: what 128 registers per thread leave room for
-        static constexpr int DEPTH = (QT == WF_QTYPE_Q4_0) ? (NG == 4 ? 3 : 4) : (QT == WF_QTYPE_Q4_1) ? 3 : (QT == WF_QTYPE_Q8_0 && NG == 1) ? 3 : 2;
+    static constexpr int DEPTH = (QT == WF_QTYPE_Q4_0) ? (NG >= 3 ? 3 : 4) : (QT == WF_QTYPE_Q4_1) ? 3 : (QT == WF_QTYPE_Q8_0 && NG == 1) ? 3 : 2;
 };
 
 // Shared memory: control 128 | start values [kc * TK / 32][NG][4] float2 | staged x [cols][sx] | pieces [batch + 15][NG][32]
 // float4 | sums of the CTA's own row-tiles [slices][ceil(batch / slices)][NG][32] float4 (a cluster's exchange, or fp32
 // tokens, whose three columns meet there).
 inline size_t gemvn_smem(int qt, int kc, int cols, bool x_f32, int slices, int batch, int* sx_out, int* piece_off_out, int* ex_off_out) {
-    const int kslice = kc * tile_k(qt), ng = cols <= 8 ? 1 : cols <= 16 ? 2 : 4;
+    const int kslice = kc * tile_k(qt), ng = (cols + 7) / 8;
     const int sx = kslice * 2 + 64;  // +64: consecutive rows start 16 banks apart
     if (sx_out) *sx_out = sx;
     size_t b = 128 + (size_t)(kslice / 32) * ng * 32 + (size_t)cols * sx;
@@ -133,7 +133,7 @@ struct GemvNPlan {
 // same S it measured 1 - 4 us more on small weights, up to twice the time on tall ones).
 inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt, int cols, bool x_f32) {
     GemvNPlan best;
-    const int ng = cols <= 8 ? 1 : cols <= 16 ? 2 : 4, tk = tile_k(qt), sms = clusters[1];
+    const int ng = (cols + 7) / 8, tk = tile_k(qt), sms = clusters[1];
     const double per_group = 15.9 + (qt == WF_QTYPE_Q4_1 ? 3.3 : qt == WF_QTYPE_Q8_0 ? 16.3 : qt == WF_QTYPE_Q4_K ? 5.0 : 0.0);
     const double tile_ns = (tk / 128) * (17.3 + per_group * ng);  // one SM's time per tile
     double best_ns = 0;

@@ -43,11 +43,12 @@ WORKLOAD = ("benchmark config 4: 7B-shape Llama decode, 224 Q4_0 projections (32
             "{4x[4096x4096], 2x[11008x4096], [4096x11008]}), batch 1, bf16 activations, fp32 out")
 
 
-# DRAM traffic of the decode kernel, from the ncu capture summarised in profiles/gemv1_program_q4_0_decode_7b.md
-# (dram__bytes_read.sum + dram__bytes_write.sum of one launch over two layers of this workload);
-# traffic grows in proportion to the layers run and splits evenly over row shards.  To be re-captured whenever the
-# kernel changes.
-NCU_TRAFFIC_BYTES_PER_LAYER = (227.78e6 + 4.19e6) / 2
+# DRAM traffic of the decode kernels per layer of this workload (dram__bytes_read.sum + dram__bytes_write.sum), from the
+# ncu captures summarised in the named files; it grows in proportion to the layers run and splits evenly over row shards.
+# To be re-captured whenever a kernel changes.  A kernel without a capture has no figure.
+NCU_TRAFFIC_PER_LAYER = {
+    "gemv1_program_kernel": ((227.78e6 + 4.19e6) / 2, "profiles/gemv1_program_q4_0_decode_7b.md"),
+}
 
 
 def tensor_peaks():
@@ -528,6 +529,10 @@ def run_ours(args) -> None:
         n_launch = max(1, round(launches / args.steps))
         gbs = alg_bytes / (ms_step * 1e-3) / 1e9
         h2d = sum(v.nbytes for v in stack.x_host.values())
+        kernel = ("gemv1_program_kernel" if mode == "program" and world > 1 else
+                  "gemv1_group_kernel" if mode in ("program", "replicas") else "gemv1_kernel")
+        per_layer, captured = NCU_TRAFFIC_PER_LAYER.get(kernel, (None, None))
+        traffic = per_layer * stack.layers / (1 if replicas else world) / n_launch if per_layer else None
         line = {
             "metric": METRIC, "value": tok_s, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": max(args.warmup, 3),
             "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak" if replicas else "strong", "vs_baseline": None,
@@ -544,11 +549,11 @@ def run_ours(args) -> None:
             "gpu_launches": int(launches),
             "parity": parity,
             "clocks": clocks,
-            "roofline": {"bound": "hbm", "kernel": ("gemv1_program_kernel" if mode == "program" and world > 1 else "gemv1_group_kernel" if mode in ("program", "replicas") else "gemv1_kernel") + "<Q4_0> (one token)", "achieved": gbs, "peak": hbm_peak, "unit": "GB/s",
+            "roofline": {"bound": "hbm", "kernel": kernel + "<Q4_0> (one token)", "achieved": gbs, "peak": hbm_peak, "unit": "GB/s",
                          "frac": gbs / hbm_peak, "frac_of_8TBs_nominal": gbs / 8000.0, "peak_source": peak_src,
                          "bytes_per_launch": alg_bytes / n_launch, "us_per_launch": ms_step * 1e3 / n_launch,
-                         "traffic": NCU_TRAFFIC_BYTES_PER_LAYER * stack.layers / (1 if replicas else world) / n_launch,
-                         "traffic_source": "ncu dram bytes of a 2-layer capture (profiles/gemv1_program_q4_0_decode_7b.md), scaled by layers (and 1 / ranks)"},
+                         "traffic": traffic,
+                         "traffic_source": f"ncu dram bytes of a 2-layer capture ({captured}), scaled by layers (and 1 / ranks)" if captured else "not captured"},
         }
         if stack.layers != spec.layers:
             line["partial"] = f"{stack.layers} of {spec.layers} layers: a profiling run, not a bench value"

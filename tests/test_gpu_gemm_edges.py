@@ -1,5 +1,5 @@
-"""The tensor-core kernels at the edges of their tiles: CTA pairs (256 rows x 512 tokens, from 129 tokens and a dozen tiles
-on) and K-splitting clusters (128 rows x 128 tokens; ranks with no tokens of their own to finish, several tiles per
+"""The tensor-core kernels at the edges of their tiles: CTA pairs (256 rows x 512 or 256 tokens; the cost function takes them
+from 65 tokens on where there are tiles enough) and K-splitting clusters (128 rows x 128 tokens; ranks with no tokens of their own to finish, several tiles per
 cluster), K that ends inside a stage of 64, and fp32 tokens.
 
 bf16 tokens: the bars of test_gpu_gemm.py.  fp32 tokens: products are exact to 2^-22 and an accumulator takes at most 32

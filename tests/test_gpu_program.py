@@ -1,9 +1,9 @@
-"""The decode step as one persistent kernel (wf_program_*): its outputs must agree with those of
-the same projections run one kernel at a time and with the CPU oracle.  The program and the
-per-projection kernels cut a row's k-range into different pieces (the program cuts projections that
-share their activations as one list of row-tiles; the per-projection kernels cut K into slices): the
-same exact block sums, a different order of the final fp32 additions -- equal to 1e-5 of the output
-scale, and the same bits from run to run.  A two-rank variant (row-sharded, gather fused into the epilogue over peer
+"""The decode step as one call (wf_program_*: on one rank grouped launches, on several one persistent kernel, which
+test_gpu_persistent_program.py covers on one rank): its outputs must agree with those of the same projections run one
+kernel at a time and with the CPU oracle.  The program and the per-projection kernels cut a row's k-range into different
+pieces (the program cuts projections that share their activations as one list of row-tiles; the per-projection kernels
+cut K into slices): the same exact block sums, a different order of the final fp32 additions -- equal to 1e-5 of the
+output scale, and the same bits from run to run.  A two-rank variant (row-sharded, gather fused into the epilogue over peer
 memory) runs when two GPUs are visible."""
 import os
 import subprocess
@@ -58,8 +58,8 @@ def test_program_equals_per_op_kernels(oracle, tokens):
 @pytest.mark.parametrize("qname", ["Q4_0", "Q4_1", "Q8_0", "Q4_K", "Q5_0"])
 @pytest.mark.parametrize("tokens", [1, 5])
 def test_program_every_quantization_type(oracle, qname, tokens):
-    """A small two-layer stack per type: the program's outputs equal the per-projection kernels' (bit for bit with
-    several tokens) and the oracle within the matmul tolerance (1 token: the integer one-token kernel, 5: the
+    """A small two-layer stack per type: the program's outputs equal the per-projection kernels' to 1e-5 of the output
+    scale and the oracle within the matmul tolerance (1 token: the integer one-token kernel, 5: the
     eight-column one)."""
     from warpforge_b200.backend import CudaContext
     from warpforge_b200.decode import ProjectionStack, StackSpec

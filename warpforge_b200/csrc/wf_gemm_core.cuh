@@ -83,8 +83,7 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
-// shared::cluster address of the same object in CTA `rank` of the cluster
-// Default semantics (release at CTA scope): the operands handed over were put in place by the async-proxy fence and the
+// Arrives on a barrier of another CTA of the cluster (its address there: map_to_rank).  Default semantics (release at CTA scope): the operands handed over were put in place by the async-proxy fence and the
 // CTA's own barriers; `.release.cluster` costs a fence that waits for the thread's loads in flight, 0.9 us per stage.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
@@ -201,7 +200,8 @@ __host__ __device__ inline int stage_chunk(int j, int q) { return 2 * q + j; }
 // would take more (magnitudes below 2^-112, down to subnormal ones); unscale[row] = 2^-s.
 //   bf16 (PLANES 1): exact whenever the scaled value is a normal fp16.
 // Rows are padded to whole stages of 64 k (zeros) and lie in the stages' order of k.
-//   fp32 (PLANES 3): v = hi + mid + lo, each the fp16 nearest to what is left: exact down to 2^-39 of the row's largest.
+//   fp32 (PLANES 3): v = hi + mid + lo, each the fp16 nearest to what is left: exact down to 2^-39 of the row's largest
+//   (below that, what fp32 rounding leaves of a sum that the largest takes part in).
 // One CTA per row.  A kernel of its own: the GEMM's CTAs set themselves up and dequantize their first stages under it.
 // Measured and not kept: converting inside the GEMM, every CTA its share of the rows and a counter to wait for (64
 // tokens: 18 us a call instead of 16, the launch and set-up of the GEMM itself lie bare then); CTAs small enough to wait

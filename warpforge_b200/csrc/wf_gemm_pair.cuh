@@ -1,4 +1,5 @@
-// Prefill GEMM for more than 256 tokens: y[m, rows] = x[m, K] . W[rows, K]^T on pairs of CTAs (tcgen05 cta_group::2).
+// Prefill GEMM for many tokens and tiles (chosen by estimated cost from 65 tokens on, see gemm_launch): y[m, rows] =
+// x[m, K] . W[rows, K]^T on pairs of CTAs (tcgen05 cta_group::2).
 //
 // A pair computes 256 weight rows x 512 tokens (or 256, where there are few tiles): one tcgen05.mma of M = 256, N = 256 spans both SMs, each SM holding its
 // own 128 rows of A (dequantized weights, fp16), HALF of the tokens of B and its own 128 accumulator rows in TMEM.

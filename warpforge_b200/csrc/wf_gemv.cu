@@ -40,8 +40,9 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvPara
             p.timing[(size_t)blockIdx.x * 8 + i] = tm;
         }
     };
-    // Programmatic stream serialization: see gemv_kernel.  The weights depend on nothing, so every warp
-    // requests the first tiles of its run before waiting for the previous grid.
+    // Programmatic stream serialization: this grid may start while the previous one drains, and what follows
+    // griddepcontrol.wait sees all that it wrote.  The weights depend on nothing, so every warp requests the first tiles
+    // of its run before that.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const WsShare share{p.tiles, t0, t1, p.kt, 0, {0, 0}};
     auto share_of = [&](int) { return share; };

@@ -17,7 +17,7 @@
 // Slices.  With S = 1 the sums are y.  With S = 2 .. 8 the CTAs of the S slices form a cluster that shares its row-tiles
 // out: each CTA sends the sums of a unit to the CTA that owns the row-tile (st.async into its shared memory, counted by an
 // mbarrier there), which adds the slices in order and stores y.  Only a K too long for eight slices (32 columns beyond
-// 25600, 16 beyond 51200) goes through memory: partial sums [row-tile][slice], an arrival counter per row-tile, and the
+// 16384, 24 beyond 22528, 16 beyond 40960) goes through memory: partial sums [row-tile][slice], an arrival counter per row-tile, and the
 // warp that finds all other slices already counted adds them, in slice order, and puts the counter back to zero.  Nowhere
 // does the result depend on who comes last, and nobody waits for a CTA outside its cluster.
 //

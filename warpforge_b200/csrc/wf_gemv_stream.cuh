@@ -290,7 +290,8 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, int chunk_q, int c
             const WsLanePtrs<QT> lp(nbase, lane);
             if (g0 + DEPTH <= len && kk + DEPTH <= kt) {
                 // a whole group inside one row-tile: straight-line code, immediate offsets; the requests are predicated, so
-                // that a run's last group takes this way too (a third of the groups of a decode step: 1140 -> 1094 us)
+                // that a run's last whole group takes this way too, whatever is left to request (a 32-layer step: 1140 ->
+                // 1094 us); what remains behind it, fewer tiles than a group, takes the one below
                 static_for<DEPTH>([&](auto J) {
                     constexpr int j = decltype(J)::value;
                     slots[j].template compute_q8<j>(acc, qa, dg);

@@ -48,6 +48,7 @@ WORKLOAD = ("benchmark config 4: 7B-shape Llama decode, 224 Q4_0 projections (32
 # To be re-captured whenever a kernel changes.  A kernel without a capture has no figure.
 NCU_TRAFFIC_PER_LAYER = {
     "gemv1_program_kernel": ((227.78e6 + 4.19e6) / 2, "profiles/gemv1_program_q4_0_decode_7b.md"),
+    "gemv1_group_kernel": (28.387e6 + 9.511e6 + 50.800e6 + 25.451e6, "profiles/gemv1_group_q4_0_decode_7b.md"),
 }
 
 

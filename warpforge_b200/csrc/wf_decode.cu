@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_program_kernel(const 
                 if (P.world > 1) emit_to_peers(op.ll, P.world, P.rank, off, v, run.tag());
             }
         };
-        ws_consume<QT, DEPTH>(sh, op.chunk_q, op.chunk_r, warp, lane, slots, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
+        ws_consume<QT, DEPTH>(sh, ws_open(sh, warp), op.chunk_q, op.chunk_r, warp, lane, slots, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
                        sums32, slots_g, P.status, smem_u32(const_cast<int*>(abort_flag)), share_of, P.n_ops, emit_row);
         if (*abort_flag) failed = true;
         stamp();

@@ -15,9 +15,35 @@
 namespace wf {
 
 // ---------------------------------------------------------------- one token
+// Between the wait for the grid that writes x and the first tile lies a chain that nothing overlaps: request x, turn it into
+// digits, find the warp's run.  Four warps per scheduler hide little of it, so what does not depend on x is done before
+// the wait, and each input kind has its own kernel, whose staging is no call behind a switch: behind the wait it took 1000 cycles
+// until the first element was requested, and 900 - 1700 from the staged row to the first tile.  With that, half the
+// instructions per digit, digits without bank conflicts and the cut row-tiles added by both halves of a warp, a 32-layer step of
+// the 7B shape went from 1097 to 1007 us, [4096 x 11008] from 7.8 to 7.2 (Q4_0).
+// What the staging needs to know, in registers before the wait:
+struct StageArgs {
+    const void* x;
+    const float* aux;
+    int k, kp;
+};
+__device__ __forceinline__ StageArgs pinned(StageArgs a) {
+    asm volatile("" : "+l"(a.x), "+l"(a.aux), "+r"(a.k), "+r"(a.kp));
+    return a;
+}
+template <class Stage> __device__ __forceinline__ void stage_row(const StageArgs& a, uint8_t* xd, uint8_t* recs, float inv = 1.f) {
+    const int padded = ((a.kp >> 3) + 31) & ~31;
+#pragma unroll 1
+    for (int c0 = threadIdx.x; c0 < padded; c0 += GEMV_CONSUMERS * Stage::U) {  // warp-uniform trip counts
+        Stage s;
+        s.fetch(a.x, a.aux, a.k, c0, GEMV_CONSUMERS);
+        s.put(xd, recs, a.kp, c0, GEMV_CONSUMERS, a.aux != nullptr, inv);
+    }
+}
+
 // Integer MMAs on exact base-256 digits of the activations, every warp streaming its own run of tiles from
 // global memory into registers (wf_gemv_stream.cuh).  512 threads, all of them consumers.
-template <int QT>
+template <int QT, int KIND>
 __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvParams p) {
     using T = Tile<QT>;
     using R = TileRegs<QT>;
@@ -55,13 +81,15 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvPara
         ws_bars_init(smem);
     }
     ws_clear_digits(xd, kp, GEMV_CONSUMERS);
+    const WsRun run = ws_open(share, warp);
     __syncthreads();
     const WsBars bar = ws_bars(smem);
 
+    using Stage = StageQ8<R::BETA_INT, KIND>;
+    const StageArgs args = pinned(StageArgs{p.x, nullptr, p.k, kp});
     asm volatile("griddepcontrol.wait;" ::: "memory");
     stamp(0);
-    if (p.x_f32) stage_x_q8<R::BETA_INT, XK_F32>(p.x, p.k, xd, recs, kp, GEMV_CONSUMERS);
-    else stage_x_q8<R::BETA_INT, XK_BF16>(p.x, p.k, xd, recs, kp, GEMV_CONSUMERS);
+    stage_row<Stage>(args, xd, recs);
     __syncthreads();
     stamp(1);
     auto emit_row = [&](int n, float v) {
@@ -69,7 +97,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvPara
     };
     stamp(2);
     uint32_t seq = 0;
-    ws_consume<QT, DEPTH>(share, p.chunk_q, p.chunk_r, warp, lane, slots, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
+    ws_consume<QT, DEPTH>(share, run, p.chunk_q, p.chunk_r, warp, lane, slots, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
                    smem_u32(recs) + (uint32_t)(kp >> 5) * 16, p.scratch, p.status, smem_u32(const_cast<int*>(abort_flag)), share_of, 1,
                    emit_row);
     stamp(4);
@@ -81,7 +109,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvPara
 
 // The same for a program: several weights, the fp32 operations before the projection in its staging, a residual in its store.
 // Its own kernel, because what a plain call does not need it would fetch cold and jump over: 2 % of a 4 - 8 us call.
-template <int QT>
+template <int QT, int KIND>
 __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Gemv1GroupParams p) {
     using T = Tile<QT>;
     using R = TileRegs<QT>;
@@ -122,18 +150,19 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Ge
         ws_bars_init(smem);
     }
     ws_clear_digits(xd, kp, GEMV_CONSUMERS);
+    // the first weight this CTA has tiles of, and the warp's run of them
+    int o = 0;
+    WsShare share = share_of(0);
+    while (share.t0 == share.t1 && o + 1 < p.n_ops) share = share_of(++o);
+    WsRun run = ws_open(share, warp);
     __syncthreads();
     const WsBars bar = ws_bars(smem);
+    const StageArgs args = pinned(StageArgs{p.x, p.aux, p.k, kp});
 
     asm volatile("griddepcontrol.wait;" ::: "memory");
     stamp(1);
-    const int kind = p.x_kind;
-    if (kind == XK_BF16) {
-        stage_x_q8<R::BETA_INT, XK_BF16>(p.x, p.k, xd, recs, kp, GEMV_CONSUMERS);
-    } else if (kind == XK_F32) {
-        stage_x_q8<R::BETA_INT, XK_F32>(p.x, p.k, xd, recs, kp, GEMV_CONSUMERS);
-    } else if (kind == XK_SWIGLU_F32) {
-        stage_x_q8<R::BETA_INT, XK_SWIGLU_F32>(p.x, p.k, xd, recs, kp, GEMV_CONSUMERS, p.aux);
+    if constexpr (KIND != XK_RMSNORM_F32) {
+        stage_row<StageQ8<R::BETA_INT, KIND>>(args, xd, recs);
     } else if (p.x_bytes > 0) {  // two passes over x: from shared memory
         uint8_t* const xs = xd + (size_t)kp * 8;
         const float* const gamma = p.aux != nullptr ? reinterpret_cast<const float*>(xs + p.x_bytes) : nullptr;
@@ -153,9 +182,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Ge
     __syncthreads();
     stamp(2);
     uint32_t seq = 0;
-    for (int o = 0; o < p.n_ops; o++) {
-        const WsShare share = share_of(o);
-        if (share.t0 == share.t1) continue;  // the same for the whole CTA
+    while (true) {
         float* const y = p.op[o].y;
         const float* const residual = p.op[o].residual;
         const int rows = p.op[o].rows;
@@ -165,9 +192,15 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Ge
                 y[n] = v;
             }
         };
-        ws_consume<QT, DEPTH>(share, p.chunk_q, p.chunk_r, warp, lane, slots, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
+        ws_consume<QT, DEPTH>(share, run, p.chunk_q, p.chunk_r, warp, lane, slots, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
                        smem_u32(recs) + (uint32_t)(kp >> 5) * 16, p.scratch, p.status, smem_u32(const_cast<int*>(abort_flag)), share_of,
                        p.n_ops, emit_row);
+        do {  // the next one, the same for the whole CTA
+            if (++o >= p.n_ops) break;
+            share = share_of(o);
+        } while (share.t0 == share.t1);
+        if (o >= p.n_ops) break;
+        run = ws_open(share, warp);
     }
     // silu(gate) * up by the CTA that has stored both: in the staging of the projection that reads it every CTA would read all
     // of gate and up and take all sigmoids (11008 rows: 6.0 us of staging instead of 2.3)
@@ -317,13 +350,24 @@ static cudaError_t launch_one_token(void (*kernel)(const Params), bool (&attr_se
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, p);
 }
-template <int QT> static cudaError_t launch_one_token(const GemvParams& p, int grid, size_t smem, cudaStream_t s) {
+template <int QT, int KIND> static cudaError_t launch_one_token_of(const GemvParams& p, int grid, size_t smem, cudaStream_t s) {
     static bool attr_set[64] = {};
-    return launch_one_token(gemv1_kernel<QT>, attr_set, p, grid, smem, s);
+    return launch_one_token(gemv1_kernel<QT, KIND>, attr_set, p, grid, smem, s);
+}
+template <int QT, int KIND> static cudaError_t launch_one_token_of(const Gemv1GroupParams& p, int grid, size_t smem, cudaStream_t s) {
+    static bool attr_set[64] = {};
+    return launch_one_token(gemv1_group_kernel<QT, KIND>, attr_set, p, grid, smem, s);
+}
+template <int QT> static cudaError_t launch_one_token(const GemvParams& p, int grid, size_t smem, cudaStream_t s) {
+    return p.x_f32 ? launch_one_token_of<QT, XK_F32>(p, grid, smem, s) : launch_one_token_of<QT, XK_BF16>(p, grid, smem, s);
 }
 template <int QT> static cudaError_t launch_one_token(const Gemv1GroupParams& p, int grid, size_t smem, cudaStream_t s) {
-    static bool attr_set[64] = {};
-    return launch_one_token(gemv1_group_kernel<QT>, attr_set, p, grid, smem, s);
+    switch (p.x_kind) {
+        case XK_F32: return launch_one_token_of<QT, XK_F32>(p, grid, smem, s);
+        case XK_RMSNORM_F32: return launch_one_token_of<QT, XK_RMSNORM_F32>(p, grid, smem, s);
+        case XK_SWIGLU_F32: return launch_one_token_of<QT, XK_SWIGLU_F32>(p, grid, smem, s);
+        default: return launch_one_token_of<QT, XK_BF16>(p, grid, smem, s);
+    }
 }
 template <class Params> static cudaError_t launch_qt_one_token(int qt, const Params& p, int grid, size_t smem, cudaStream_t s) {
     return qt == WF_QTYPE_Q4_0   ? launch_one_token<WF_QTYPE_Q4_0>(p, grid, smem, s)

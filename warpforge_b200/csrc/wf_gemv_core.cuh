@@ -291,7 +291,8 @@ __device__ __forceinline__ float2 lds64f(uint32_t a) {
 // start value -64 * (sum of the block's digits), prepared with the digits.
 //
 // Staged form of one token, per 128 k (a "unit" = four blocks j = 0..3, block pairs A = (0, 2) and
-// B = (1, 3)): 1024 bytes of digits, lane L = 4 g + q reads 32 bytes at L * 32: for pair A and then for pair B
+// B = (1, 3)): 512 bytes of digits for pair A, of which lane L = 4 g + q reads 16 at L * 16, and 512 for pair B, of which it
+// reads 16 at (L ^ 4) * 16 (no bank conflicts here; the exclusive or keeps the staging's stores of the two pairs apart):
 // the words {lo, hi} of the first MMA (elements 0, 4, 1, 5 of the lane's block) and {lo, hi} of the second
 // (elements 2, 6, 3, 7), holding digit (g & 3) of elements 8q..8q+7 of block 2 (g >> 2) [pair A] / 2 (g >> 2) + 1
 // [pair B].  A lane is a live source for the low k-slots (its block is the pair's first) when g < 4 and for
@@ -343,7 +344,8 @@ __device__ __forceinline__ void pair_imma(int (&d)[4], uint32_t w00, uint32_t w1
 
 // Lane-specific shared addresses of the staged token for the tile at hand.
 struct Q8Addr {
-    uint32_t x;    // this lane's 32 digit bytes of the tile's first unit
+    uint32_t x;    // this lane's 16 digit bytes of pair A in the tile's first unit
+    uint32_t xb;   // of pair B
     uint32_t rec;  // this lane's record of the tile's first unit
     uint32_t sx;   // this lane's pair of activation sums
 };
@@ -352,12 +354,14 @@ struct Q8Addr {
 struct Q8Digits {
     uint4 a, b;
     uint32_t mul28 = 0x10000000u | (gridDim.y >> 16);  // 2^28 (a grid has fewer than 2^16 CTAs in y), opaque to the compiler
-    template <int OFF> __device__ __forceinline__ void load(uint32_t addr) {
-        a = lds128_at<OFF>(addr);
-        b = lds128_at<OFF + 16>(addr);
+    template <int OFF> __device__ __forceinline__ void load(const Q8Addr& at) {
+        a = lds128_at<OFF>(at.x);
+        b = lds128_at<OFF>(at.xb);
     }
 };
 constexpr int Q8_UNIT_BYTES = 1024;  // staged digits per 128 k: 32 lanes x 32 bytes
+__device__ __forceinline__ uint32_t q8_lane_a(int lane) { return (uint32_t)lane * 16; }
+__device__ __forceinline__ uint32_t q8_lane_b(int lane) { return 512u + (uint32_t)(lane ^ 4) * 16; }
 
 // 256 D_even + D_odd as a float (|D| < 2^20 for the 4-bit formats, so the integer is exact and the conversion rounds once)
 __device__ __forceinline__ float digits_to_float(int de, int dodd) { return (float)(de * 256 + dodd); }
@@ -408,7 +412,7 @@ template <> struct TileRegs<WF_QTYPE_Q4_0> {
     // J: the tile's position after the one the addresses point at (immediate offsets).
     template <int J> __device__ __forceinline__ void compute_q8(float (&acc)[4], const Q8Addr& a, Q8Digits& dg) const {
         constexpr int TK = Tile<WF_QTYPE_Q4_0>::K;
-        dg.template load<J * (TK / 128) * Q8_UNIT_BYTES>(a.x);
+        dg.template load<J * (TK / 128) * Q8_UNIT_BYTES>(a);
         const uint4 r = lds128_at<J * (TK >> 5) * 16>(a.rec);  // {W, f, W', f'}
         int da[4], db[4];
         pair_imma(da, c[0].x, c[1].x, c[0].z, c[1].z, dg.a.x, dg.a.y, dg.a.z, dg.a.w, dg.mul28);
@@ -511,7 +515,7 @@ template <> struct TileRegs<WF_QTYPE_Q4_1> {
     // activations), which only the lanes of the first digit pair carry (the others read zeros).
     template <int J> __device__ __forceinline__ void compute_q8(float (&acc)[4], const Q8Addr& a, Q8Digits& dg) const {
         constexpr int TK = Tile<WF_QTYPE_Q4_1>::K;
-        dg.template load<J * (TK / 128) * Q8_UNIT_BYTES>(a.x);
+        dg.template load<J * (TK / 128) * Q8_UNIT_BYTES>(a);
         const uint4 r = lds128_at<J * (TK >> 5) * 16>(a.rec);
         const uint2 sx = lds64(a.sx + J * (TK >> 5) * 8);
         int da[4], db[4];
@@ -613,7 +617,7 @@ template <> struct TileRegs<WF_QTYPE_Q8_0> {
     // One token: value = 16 (hi - 8) + lo; the two planes accumulate separately and combine as integers.
     template <int J> __device__ __forceinline__ void compute_q8(float (&acc)[4], const Q8Addr& a, Q8Digits& dg) const {
         constexpr int TK = Tile<WF_QTYPE_Q8_0>::K;
-        dg.template load<J * (TK / 128) * Q8_UNIT_BYTES>(a.x);
+        dg.template load<J * (TK / 128) * Q8_UNIT_BYTES>(a);
         const uint4 r = lds128_at<J * (TK >> 5) * 16>(a.rec);
         int la[4], lb[4], ha[4], hb[4];
         pair_imma(ha, c[0].x, c[1].x, c[0].z, c[1].z, dg.a.x, dg.a.y, dg.a.z, dg.a.w, dg.mul28);
@@ -743,8 +747,8 @@ template <> struct TileRegs<WF_QTYPE_Q4_K> {
         const float ngd = -BIG * g.x, ngm = BIG * g.y, nhd = -BIG * h.x, nhm = BIG * h.y;
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-            if (u == 0) dg.template load<(2 * J) * Q8_UNIT_BYTES>(a.x);
-            else dg.template load<(2 * J + 1) * Q8_UNIT_BYTES>(a.x);
+            if (u == 0) dg.template load<(2 * J) * Q8_UNIT_BYTES>(a);
+            else dg.template load<(2 * J + 1) * Q8_UNIT_BYTES>(a);
             const uint4 r = u == 0 ? lds128_at<(2 * J) * 64>(a.rec) : lds128_at<(2 * J + 1) * 64>(a.rec);
             const uint2 sx = lds64(a.sx + (2 * J + u) * 32);
             int da[4], db[4];
@@ -1165,29 +1169,34 @@ static __device__ __noinline__ float cta_rms_inv(const float* x, int k, float ep
     return 1.0f / rms;
 }
 
-template <int BETA_INT, int KIND, bool SHARED = false>
-static __device__ __noinline__ void stage_x_q8(const void* x, int k, uint8_t* xd, uint8_t* recs, int kp, int nthreads,
-                                               const float* aux = nullptr, float inv = 1.f) {
-    constexpr bool F32 = KIND != XK_BF16, AUX = KIND == XK_RMSNORM_F32 || KIND == XK_SWIGLU_F32;
-    const int groups = kp >> 3, padded = (groups + 31) & ~31, kgroups = k >> 3;
-    const uint4* src = static_cast<const uint4*>(x);
-    const uint4* asrc = reinterpret_cast<const uint4*>(aux);
-    const bool has_aux = AUX && aux != nullptr;
-    uint8_t* sums = recs + (size_t)(kp >> 5) * 16;  // the activation sums follow the records
-    constexpr int U = SHARED ? 1 : F32 ? 2 : 3;  // element groups in flight per thread
-    const uint32_t src32 = SHARED ? smem_u32(x) : 0, asrc32 = SHARED && has_aux ? smem_u32(aux) : 0;
-    for (int c0 = threadIdx.x; c0 < padded; c0 += nthreads * U) {  // warp-uniform trip counts
-        uint4 pre[U], pre2[U], ax[U], ax2[U];
+__device__ __forceinline__ float max_nan(float a, float b) {  // of the magnitudes; a NaN stays one
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(fabsf(a)), "f"(fabsf(b)));
+    return m;
+}
+// What a thread stages at a time: element groups c0, c0 + nthreads, ... of eight elements each.  fetch() only requests them, put()
+// turns them into digits, so that a kernel can have the addresses ready before it waits for the grid that writes x.
+template <int BETA_INT, int KIND, bool SHARED = false> struct StageQ8 {
+    static constexpr bool F32 = KIND != XK_BF16, AUX = KIND == XK_RMSNORM_F32 || KIND == XK_SWIGLU_F32;
+    static constexpr int U = SHARED ? 1 : F32 ? 2 : 3;  // element groups in flight per thread
+    uint4 pre[U], pre2[F32 ? U : 1], ax[AUX ? U : 1], ax2[AUX ? U : 1];
+
+    __device__ __forceinline__ void fetch(const void* x, const float* aux, int k, int c0, int nthreads) {
+        const int kgroups = k >> 3;
+        const uint4* const src = static_cast<const uint4*>(x);
+        const uint4* const asrc = reinterpret_cast<const uint4*>(aux);
+        const uint32_t src32 = SHARED ? smem_u32(x) : 0, asrc32 = SHARED && AUX && aux != nullptr ? smem_u32(aux) : 0;
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int c8 = c0 + u * nthreads;
-            pre[u] = pre2[u] = make_uint4(0u, 0u, 0u, 0u);
-            ax[u] = ax2[u] = make_uint4(0x3F800000u, 0x3F800000u, 0x3F800000u, 0x3F800000u);  // 1.0f
+            pre[u] = make_uint4(0u, 0u, 0u, 0u);
+            if (F32) pre2[u] = make_uint4(0u, 0u, 0u, 0u);
+            if (AUX) ax[u] = ax2[u] = make_uint4(0x3F800000u, 0x3F800000u, 0x3F800000u, 0x3F800000u);  // 1.0f
             if (c8 < kgroups) {
                 if (F32) {
                     pre[u] = SHARED ? lds128(src32 + c8 * 32) : __ldcg(src + 2 * c8);
                     pre2[u] = SHARED ? lds128(src32 + c8 * 32 + 16) : __ldcg(src + 2 * c8 + 1);
-                    if (has_aux) {
+                    if (AUX && aux != nullptr) {
                         ax[u] = SHARED ? lds128(asrc32 + c8 * 32) : __ldcg(asrc + 2 * c8);
                         ax2[u] = SHARED ? lds128(asrc32 + c8 * 32 + 16) : __ldcg(asrc + 2 * c8 + 1);
                     }
@@ -1196,12 +1205,16 @@ static __device__ __noinline__ void stage_x_q8(const void* x, int k, uint8_t* xd
                 }
             }
         }
+    }
+
+    __device__ __forceinline__ void put(uint8_t* xd, uint8_t* recs, int kp, int c0, int nthreads, bool has_aux, float inv) const {
+        const int groups = kp >> 3, padded = (groups + 31) & ~31;
+        uint8_t* const sums = recs + (size_t)(kp >> 5) * 16;  // the activation sums follow the records
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int c8 = c0 + u * nthreads;
             if ((c8 & ~31) >= padded) break;  // warp-uniform
             const uint4 v = pre[u];
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
             float f[8];
             if (F32) {
                 const uint4 v2 = pre2[u];
@@ -1223,29 +1236,46 @@ static __device__ __noinline__ void stage_x_q8(const void* x, int k, uint8_t* xd
                     }
                 }
             } else {
+                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     f[2 * i] = __uint_as_float(w[i] << 16);
                     f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
                 }
             }
-            float sum = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
-            float amax = fmaxf(fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3]))),
-                               fmaxf(fmaxf(fabsf(f[4]), fabsf(f[5])), fmaxf(fabsf(f[6]), fabsf(f[7]))));
-            amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-            amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
-            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
-            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
+            float amax = max_nan(max_nan(max_nan(f[0], f[1]), max_nan(f[2], f[3])), max_nan(max_nan(f[4], f[5]), max_nan(f[6], f[7])));
+            amax = max_nan(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+            amax = max_nan(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
+            float sum = 0.f;  // of the block
+            if (BETA_INT == 0) {
+                sum = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+                sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+                sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
+            }
             const int eeff = max((int)(__float_as_uint(amax) >> 23), 40);
-            const bool special = eeff == 0xFF || sum != sum;  // an Inf or a NaN in the block (a NaN makes the sum a NaN)
             const float scale = __uint_as_float((uint32_t)(283 - eeff) << 23);  // 2^(156 - e)
+            int X[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) X[i] = __float2int_rz(f[i] * scale);
+            // x = X * 2^(e - 156); the MMA multiplies 8 * code; the lanes of the first digit pair hold
+            // 256^3 D + 256^2 D' = 2^16 (256 D + D')
+            float f_hi = __uint_as_float((uint32_t)(eeff - 156 - 3 + 16 + 127) << 23);
+            float f_lo = __uint_as_float((uint32_t)(eeff - 156 - 3 + 127) << 23);
+            if (eeff == 0xFF) {  // an Inf or a NaN in the block: the same for its four threads
+                const unsigned quad = 0xFu << (threadIdx.x & 28);
+                float all = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+                all += __shfl_xor_sync(quad, all, 1);
+                all += __shfl_xor_sync(quad, all, 2);
+#pragma unroll
+                for (int i = 0; i < 8; i++) X[i] = (fabsf(f[i]) == __uint_as_float(0x7F800000u)) ? (f[i] < 0.f ? -1 : 1) : 0;
+                // a NaN sum: a NaN element, or Infs of both signs (which the CPU's sum of products turns into NaN as well)
+                const bool nan = all != all;
+                f_hi = nan ? __uint_as_float(0x7FC00000u) : 0.f;
+                f_lo = nan ? __uint_as_float(0x7FC00000u) : __uint_as_float(0x7F800000u);
+            }
             uint32_t z[8];  // per element the four signed digit bytes, least significant digit in byte 0
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                int X = __float2int_rz(f[i] * scale);
-                if (special) X = (fabsf(f[i]) == __uint_as_float(0x7F800000u)) ? (f[i] < 0.f ? -1 : 1) : 0;
-                z[i] = ((uint32_t)X + 0x00808080u) ^ 0x00808080u;
-            }
+            for (int i = 0; i < 8; i++) z[i] = ((uint32_t)X[i] + 0x00808080u) ^ 0x00808080u;
             // transpose to digit-major byte quadruples in the element order of the two MMAs: (0, 4, 1, 5) and (2, 6, 3, 7)
             uint32_t t1[4], t2[4];
             {
@@ -1260,47 +1290,54 @@ static __device__ __noinline__ void stage_x_q8(const void* x, int k, uint8_t* xd
                 t2[0] = __byte_perm(P, R, 0x5410); t2[1] = __byte_perm(P, R, 0x7632);
                 t2[2] = __byte_perm(Q, S, 0x5410); t2[3] = __byte_perm(Q, S, 0x7632);
             }
-            int dsum[4];
+            int d_hi = 0, d_lo = 0;  // 256 * (sum of digit 3) + (sum of digit 2) of the block, and of digits 1 and 0
+            if (BETA_INT != 0) {
+                int dsum[4];
 #pragma unroll
-            for (int t = 0; t < 4; t++) {
-                dsum[t] = BETA_INT == 0 ? 0 : __dp4a((int)t1[t], 0x01010101, __dp4a((int)t2[t], 0x01010101, 0));
-                if (BETA_INT != 0) {
-                    dsum[t] += __shfl_xor_sync(0xFFFFFFFFu, dsum[t], 1);
-                    dsum[t] += __shfl_xor_sync(0xFFFFFFFFu, dsum[t], 2);
-                }
+                for (int t = 0; t < 4; t++) dsum[t] = __dp4a((int)t1[t], 0x01010101, __dp4a((int)t2[t], 0x01010101, 0));
+                d_hi = 256 * dsum[3] + dsum[2];
+                d_lo = 256 * dsum[1] + dsum[0];
+                d_hi += __shfl_xor_sync(0xFFFFFFFFu, d_hi, 1);
+                d_lo += __shfl_xor_sync(0xFFFFFFFFu, d_lo, 1);
+                d_hi += __shfl_xor_sync(0xFFFFFFFFu, d_hi, 2);
+                d_lo += __shfl_xor_sync(0xFFFFFFFFu, d_lo, 2);
             }
             if (c8 < groups) {
                 const int b = c8 >> 2, q = c8 & 3, unit = b >> 2, j = b & 3, pair = j & 1, hcol = j >> 1;
-                // lane (g = 4 hcol + digit, q): 32 bytes {lo, hi} first MMA, {lo, hi} second MMA for pair A, then pair B;
-                // this block fills the lo words when it is its pair's first block (hcol 0), the hi words otherwise
-                uint8_t* base = xd + (size_t)unit * Q8_UNIT_BYTES + q * 32 + pair * 16 + hcol * 4;
-#pragma unroll
-                for (int t = 0; t < 4; t++) {  // digit t has weight 256^t; column digit index = 3 - t (most significant first)
-                    uint32_t* w = reinterpret_cast<uint32_t*>(base + (4 * hcol + (3 - t)) * 128);
-                    w[0] = t1[t];
-                    w[2] = t2[t];
-                }
+                // lane 4 (4 hcol + digit) + q: {lo, hi} first MMA, {lo, hi} second MMA; this block fills the lo words when it is
+                // its pair's first block (hcol 0), the hi words otherwise.  Column digit index = 3 - t (most significant first).
+                uint8_t* const base = xd + (size_t)unit * Q8_UNIT_BYTES + pair * 512 + hcol * 260 + q * 16;
+                uint32_t* const even = reinterpret_cast<uint32_t*>(base + pair * 64);  // column digits 0 and 2 of pair A, 1 and 3 of pair B
+                uint32_t* const odd = reinterpret_cast<uint32_t*>(base + 64 - pair * 64);
+                even[0] = t1[3]; even[2] = t2[3];
+                odd[0] = t1[2]; odd[2] = t2[2];
+                even[32] = t1[1]; even[34] = t2[1];
+                odd[32] = t1[0]; odd[34] = t2[0];
                 if (q == 0) {
-                    // x = X * 2^(e - 156); the MMA multiplies 8 * code; the lanes of the first digit pair hold
-                    // 256^3 D + 256^2 D' = 2^16 (256 D + D')
-                    float f_hi = __uint_as_float((uint32_t)(eeff - 156 - 3 + 16 + 127) << 23);
-                    float f_lo = __uint_as_float((uint32_t)(eeff - 156 - 3 + 127) << 23);
-                    if (special) {
-                        // a NaN sum: a NaN element, or Infs of both signs (which the CPU's sum of products turns into NaN as well)
-                        const bool nan = sum != sum;
-                        f_hi = nan ? __uint_as_float(0x7FC00000u) : 0.f;
-                        f_lo = nan ? __uint_as_float(0x7FC00000u) : __uint_as_float(0x7F800000u);
-                    }
                     // block j of the unit is block (j & 1) of lane position h = j >> 1; digit pair p: record at (2 h + p) * 16
-                    uint8_t* rec = recs + (size_t)unit * 64 + (size_t)(j >> 1) * 32 + (size_t)(j & 1) * 8;
-                    *reinterpret_cast<uint2*>(rec) = make_uint2((uint32_t)(BETA_INT * (256 * dsum[3] + dsum[2])), __float_as_uint(f_hi));
-                    *reinterpret_cast<uint2*>(rec + 16) = make_uint2((uint32_t)(BETA_INT * (256 * dsum[1] + dsum[0])), __float_as_uint(f_lo));
-                    float* sp = reinterpret_cast<float*>(sums + (size_t)unit * 32 + (size_t)(j >> 1) * 16 + (size_t)(j & 1) * 4);
-                    sp[0] = sum;
-                    sp[2] = 0.f;
+                    uint8_t* const rec = recs + (size_t)unit * 64 + (size_t)(j >> 1) * 32 + (size_t)(j & 1) * 8;
+                    *reinterpret_cast<uint2*>(rec) = make_uint2((uint32_t)(BETA_INT * d_hi), __float_as_uint(f_hi));
+                    *reinterpret_cast<uint2*>(rec + 16) = make_uint2((uint32_t)(BETA_INT * d_lo), __float_as_uint(f_lo));
+                    if (BETA_INT == 0) {
+                        float* const sp = reinterpret_cast<float*>(sums + (size_t)unit * 32 + (size_t)(j >> 1) * 16 + (size_t)(j & 1) * 4);
+                        sp[0] = sum;
+                        sp[2] = 0.f;
+                    }
                 }
             }
         }
+    }
+};
+
+template <int BETA_INT, int KIND, bool SHARED = false>
+static __device__ __noinline__ void stage_x_q8(const void* x, int k, uint8_t* xd, uint8_t* recs, int kp, int nthreads,
+                                               const float* aux = nullptr, float inv = 1.f) {
+    using S = StageQ8<BETA_INT, KIND, SHARED>;
+    const int padded = ((kp >> 3) + 31) & ~31;
+    for (int c0 = threadIdx.x; c0 < padded; c0 += nthreads * S::U) {  // warp-uniform trip counts
+        S s;
+        s.fetch(x, aux, k, c0, nthreads);
+        s.put(xd, recs, kp, c0, nthreads, aux != nullptr, inv);
     }
 }
 

@@ -204,13 +204,35 @@ __device__ __forceinline__ void ws_bars_init(uint8_t* smem) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
+// A warp's run of a share: its tiles and where it begins.
+struct WsRun {
+    int len, rt, kk;  // tiles; row-tile and k-tile of the first
+};
+__device__ __forceinline__ WsRun ws_open(const WsShare& sh, int warp) {
+    int a, b;
+    ws_run(sh.t0, sh.t1, warp, a, b);
+    WsRun r;
+    r.len = b - a;
+    r.rt = __float2int_rz(__fdividef((float)a, (float)sh.kt));  // a / kt without the integer division
+    r.kk = a - r.rt * sh.kt;
+    while (r.kk < 0) {  // the float quotient is off by one at most for tile counts below 2^24; loops cover the rest
+        r.rt--;
+        r.kk += sh.kt;
+    }
+    while (r.kk >= sh.kt) {
+        r.rt++;
+        r.kk -= sh.kt;
+    }
+    return r;
+}
+
 // One weight, one warp: walk the run, hand the cut pieces over, finish the row-tiles this warp is first to hold.
 //   slots: the register sets holding the first group of this run (requested earlier); cur: the request cursor;
 //   x32 / c32 / s32: shared addresses of the staged digits, the block records and the activation sums;
 //   emit_row(n, value): store output row n of this weight (called by one lane per row);
 //   share_of(o): the CTA's share of weight o of the program.
 template <int QT, int DEPTH, class EmitRow, class ShareFn>
-__device__ __forceinline__ void ws_consume(const WsShare& sh, int chunk_q, int chunk_r, int warp, int lane,
+__device__ __forceinline__ void ws_consume(const WsShare& sh, const WsRun& run, int chunk_q, int chunk_r, int warp, int lane,
                                            TileRegs<QT> (&slots)[DEPTH], WsCursor& cur, const WsBars& bar,
                                            WsPiece* pieces, uint32_t& seq, uint32_t x32, uint32_t c32, uint32_t s32,
                                            uint2* slots_g, int* status, uint32_t abort32, ShareFn& share_of, int n_ops,
@@ -219,9 +241,7 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, int chunk_q, int c
     constexpr uint32_t XSTEP = (T::K / 128) * Q8_UNIT_BYTES, RSTEP = (T::K >> 5) * 16, SSTEP = (T::K >> 5) * 8;  // staged bytes per tile
     const int g = lane >> 2, q = lane & 3, kt = sh.kt;
     const uint32_t lane_is_0 = lane == 0;
-    int a, b;
-    ws_run(sh.t0, sh.t1, warp, a, b);
-    const int len = b - a;
+    const int len = run.len;
 
     const int slot = (int)(seq % WS_SLOTS);
     const uint32_t gen = seq / WS_SLOTS;
@@ -233,19 +253,12 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, int chunk_q, int c
     int npieces = 0, rtag0 = 0, rtag1 = 0;
     bool first0 = false, first1 = false;
     if (len > 0) {
-        int rt = __float2int_rz(__fdividef((float)a, (float)kt)), kk = a - rt * kt;  // a / kt without the integer division
-        while (kk < 0) {  // the float quotient is off by one at most for tile counts below 2^24; loops cover the rest
-            rt--;
-            kk += kt;
-        }
-        while (kk >= kt) {
-            rt++;
-            kk -= kt;
-        }
+        int rt = run.rt, kk = run.kk;
         bool starts_here = kk == 0;  // the row-tile being walked began inside this run
-        const uint32_t x0 = x32 + lane * 32, rec0 = c32 + q * 16, sx0 = s32 + q * 8;
+        const uint32_t x0 = x32 + q8_lane_a(lane), b_from_a = q8_lane_b(lane) - q8_lane_a(lane), rec0 = c32 + q * 16, sx0 = s32 + q * 8;
         Q8Addr qa;
         qa.x = x0 + (uint32_t)kk * XSTEP;
+        qa.xb = qa.x + b_from_a;
         qa.rec = rec0 + (uint32_t)kk * RSTEP;
         qa.sx = sx0 + (uint32_t)kk * SSTEP;
         Q8Digits dg;
@@ -299,6 +312,7 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, int chunk_q, int c
                 });
                 kk += DEPTH;
                 qa.x += DEPTH * XSTEP;
+                qa.xb += DEPTH * XSTEP;
                 qa.rec += DEPTH * RSTEP;
                 qa.sx += DEPTH * SSTEP;
                 if (kk == kt) {
@@ -307,6 +321,7 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, int chunk_q, int c
                     rt++;
                     starts_here = true;
                     qa.x = x0;
+                    qa.xb = x0 + b_from_a;
                     qa.rec = rec0;
                     qa.sx = sx0;
                 }
@@ -321,10 +336,13 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, int chunk_q, int c
                             rt++;
                             starts_here = true;
                             qa.x = x0;
+                            qa.xb = x0 + b_from_a;
+                    qa.xb = x0 + b_from_a;
                             qa.rec = rec0;
                             qa.sx = sx0;
                         } else {
                             qa.x += XSTEP;
+                            qa.xb += XSTEP;
                             qa.rec += RSTEP;
                             qa.sx += SSTEP;
                         }
@@ -347,19 +365,22 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, int chunk_q, int c
             if (!(pi == 0 ? first0 : first1)) continue;  // an earlier warp holds this row-tile first
             const int r = pi == 0 ? rtag0 : rtag1;
             const int row_end = min((r + 1) * kt, sh.t1);
-            // the following warps whose runs begin inside the row-tile hold its next pieces, each as its first piece:
-            // all loads first (they do not depend on each other), then the additions in warp order
-            float pc[GEMV_WARPS];
-            const int li = lane & 15;
-#pragma unroll
-            for (int d = 1; d < GEMV_WARPS; d++) {
-                const int w2 = warp + d, a2 = sh.t0 + w2 * rq + min(w2, rr);
-                pc[d] = (w2 < GEMV_WARPS && a2 < row_end) ? all[w2 * 2].v[li] : 0.f;
-            }
+            // the following warps whose runs begin inside the row-tile hold its next pieces, each as its first piece: lanes
+            // 0 .. 15 find out how many they are, then either half of the warp adds every second one, in warp order
+            const int li = lane & 15, half = lane >> 4, a2 = sh.t0 + li * rq + min(li, rr);
+            const int more = __popc(__ballot_sync(0xFFFFFFFFu, lane > warp && half == 0 && a2 < row_end));
+            const float* const next = reinterpret_cast<const float*>(all + (warp + half) * 2) + li;
             float v[1];
-            v[0] = mine[pi].v[li];
+            v[0] = half == 0 ? mine[pi].v[li] : 0.f;
+            float pc[GEMV_WARPS / 2];
 #pragma unroll
-            for (int d = 1; d < GEMV_WARPS; d++) v[0] += pc[d];
+            for (int d = 0; d < GEMV_WARPS / 2; d++) {
+                const int i = 2 * d + half;  // its piece: of warp + i
+                pc[d] = i >= 1 && i <= more ? next[d * 64] : 0.f;
+            }
+#pragma unroll
+            for (int d = 0; d < GEMV_WARPS / 2; d++) v[0] += pc[d];
+            v[0] += __shfl_xor_sync(0xFFFFFFFFu, v[0], 16);
             const bool starts = r * kt >= sh.t0, ends = (r + 1) * kt <= sh.t1;
             if (!starts) {
                 publish_piece<16>(slots_g + (size_t)blockIdx.x * 128, v, lane, status);

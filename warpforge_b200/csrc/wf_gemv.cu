@@ -27,8 +27,9 @@ struct StageArgs {
     const float* aux;
     int k, kp;
 };
-__device__ __forceinline__ StageArgs pinned(StageArgs a) {
-    asm volatile("" : "+l"(a.x), "+l"(a.aux), "+r"(a.k), "+r"(a.kp));
+template <int KIND> __device__ __forceinline__ StageArgs pinned(StageArgs a) {
+    if (KIND != XK_RMSNORM_F32) asm volatile("" : "+l"(a.x), "+r"(a.k), "+r"(a.kp));
+    if (KIND == XK_SWIGLU_F32) asm volatile("" : "+l"(a.aux));
     return a;
 }
 template <class Stage> __device__ __forceinline__ void stage_row(const StageArgs& a, uint8_t* xd, uint8_t* recs, float inv = 1.f) {
@@ -75,7 +76,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvPara
     constexpr int DEPTH = WsGeom<QT, false>::DEPTH;
     R slots[DEPTH];
     WsCursor cur;
-    ws_prime<QT, DEPTH>(slots, cur, share_of, 1, warp, lane);
+    WsNext next = ws_prime<QT, DEPTH>(slots, cur, share_of, 1, warp, lane);
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         ws_bars_init(smem);
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvPara
     const WsBars bar = ws_bars(smem);
 
     using Stage = StageQ8<R::BETA_INT, KIND>;
-    const StageArgs args = pinned(StageArgs{p.x, nullptr, p.k, kp});
+    const StageArgs args = pinned<KIND>(StageArgs{p.x, nullptr, p.k, kp});
     asm volatile("griddepcontrol.wait;" ::: "memory");
     stamp(0);
     stage_row<Stage>(args, xd, recs);
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvPara
     };
     stamp(2);
     uint32_t seq = 0;
-    ws_consume<QT, DEPTH>(share, run, p.chunk_q, p.chunk_r, warp, lane, slots, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
+    ws_consume<QT, DEPTH>(share, run, p.chunk_q, p.chunk_r, warp, lane, slots, next, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
                    smem_u32(recs) + (uint32_t)(kp >> 5) * 16, p.scratch, p.status, smem_u32(const_cast<int*>(abort_flag)), share_of, 1,
                    emit_row);
     stamp(4);
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Ge
     constexpr int DEPTH = WsGeom<QT, true>::DEPTH;
     R slots[DEPTH];
     WsCursor cur;
-    ws_prime<QT, DEPTH>(slots, cur, share_of, p.n_ops, warp, lane);
+    WsNext next = ws_prime<QT, DEPTH>(slots, cur, share_of, p.n_ops, warp, lane);
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         mbar_init(smem_u32(smem + 16), 1);
@@ -155,9 +156,13 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Ge
     WsShare share = share_of(0);
     while (share.t0 == share.t1 && o + 1 < p.n_ops) share = share_of(++o);
     WsRun run = ws_open(share, warp);
+    float* y = p.op[o].y;
+    const float* residual = p.op[o].residual;
+    int rows = p.op[o].rows;
     __syncthreads();
     const WsBars bar = ws_bars(smem);
-    const StageArgs args = pinned(StageArgs{p.x, p.aux, p.k, kp});
+    const StageArgs args = pinned<KIND>(StageArgs{p.x, p.aux, p.k, kp});
+    asm volatile("" : "+l"(y), "+l"(residual), "+r"(rows));
 
     asm volatile("griddepcontrol.wait;" ::: "memory");
     stamp(1);
@@ -183,16 +188,13 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Ge
     stamp(2);
     uint32_t seq = 0;
     while (true) {
-        float* const y = p.op[o].y;
-        const float* const residual = p.op[o].residual;
-        const int rows = p.op[o].rows;
         auto emit_row = [&](int n, float v) {
             if (n < rows) {
                 if (residual != nullptr) v += __ldcg(residual + n);
                 y[n] = v;
             }
         };
-        ws_consume<QT, DEPTH>(share, run, p.chunk_q, p.chunk_r, warp, lane, slots, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
+        ws_consume<QT, DEPTH>(share, run, p.chunk_q, p.chunk_r, warp, lane, slots, next, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
                        smem_u32(recs) + (uint32_t)(kp >> 5) * 16, p.scratch, p.status, smem_u32(const_cast<int*>(abort_flag)), share_of,
                        p.n_ops, emit_row);
         do {  // the next one, the same for the whole CTA
@@ -201,6 +203,9 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Ge
         } while (share.t0 == share.t1);
         if (o >= p.n_ops) break;
         run = ws_open(share, warp);
+        y = p.op[o].y;
+        residual = p.op[o].residual;
+        rows = p.op[o].rows;
     }
     // silu(gate) * up by the CTA that has stored both: in the staging of the projection that reads it every CTA would read all
     // of gate and up and take all sigmoids (11008 rows: 6.0 us of staging instead of 2.3)

@@ -305,41 +305,34 @@ __device__ __forceinline__ float2 lds64f(uint32_t a) {
 
 constexpr uint32_t CODE8_MASK = 0x78787878u;
 
-// d += (8 * codes) x digits over one block pair: w00 / w10 = rows g / g+8 of the pair's first block,
+// d = (8 * codes) x digits over one block pair: w00 / w10 = rows g / g+8 of the pair's first block,
 // w01 / w11 = of its second block; bl = digit bytes for the low k-slots (first MMA, second MMA),
-// bh = for the high k-slots.
+// bh = for the high k-slots.  The first MMA starts from zero.
+// The rotation is a funnel shift: as a 64-bit product with 2^28 (four cycles of the multiplier, in whose way the MMA's issue gets:
+// eight cycles for an MMA, fourteen for the two) a 32-layer step of the 7B shape took 1007 instead of 983 us, four fused layers of Q4_K 161
+// instead of 153.
 __device__ __forceinline__ void pair_imma(int (&d)[4], uint32_t w00, uint32_t w10, uint32_t w01, uint32_t w11,
-                                          uint32_t bl1, uint32_t bh1, uint32_t bl2, uint32_t bh2, uint32_t mul28) {
-    // d = (not +=): the first MMA starts from zero.  bl / bh: digit bytes for the low / high k-slots, first and second MMA.
-    // The rotation by four bits for the second MMA goes through the multiplier (w * 2^28 as a 64-bit product:
-    // low word w << 28, high word w >> 4) and one three-input logic op ((lo | hi) & mask), which leaves two
-    // instead of three instructions per word on the half-rate integer pipe.  mul28 = 2^28, kept in a register the
-    // compiler cannot see through (a constant factor would be turned back into shifts).
+                                          uint32_t bl1, uint32_t bh1, uint32_t bl2, uint32_t bh2) {
     asm(
         "{\n\t"
-        ".reg .b32 a0, a1, a2, a3, l0, l1, l2, l3, h0, h1, h2, h3;\n\t"
-        ".reg .b64 p0, p1, p2, p3;\n\t"
+        ".reg .b32 a0, a1, a2, a3, r0, r1, r2, r3;\n\t"
         "and.b32 a0, %4, %12;\n\t"
         "and.b32 a1, %5, %12;\n\t"
         "and.b32 a2, %6, %12;\n\t"
         "and.b32 a3, %7, %12;\n\t"
-        "mul.wide.u32 p0, %4, %13;\n\t"
-        "mul.wide.u32 p1, %5, %13;\n\t"
-        "mul.wide.u32 p2, %6, %13;\n\t"
-        "mul.wide.u32 p3, %7, %13;\n\t"
-        "mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {a0,a1,a2,a3}, {%8,%9}, {%14,%14,%14,%14};\n\t"
-        "mov.b64 {l0, h0}, p0;\n\t"
-        "mov.b64 {l1, h1}, p1;\n\t"
-        "mov.b64 {l2, h2}, p2;\n\t"
-        "mov.b64 {l3, h3}, p3;\n\t"
-        "lop3.b32 a0, l0, h0, %12, 0xA8;\n\t"
-        "lop3.b32 a1, l1, h1, %12, 0xA8;\n\t"
-        "lop3.b32 a2, l2, h2, %12, 0xA8;\n\t"
-        "lop3.b32 a3, l3, h3, %12, 0xA8;\n\t"
+        "shf.r.wrap.b32 r0, %4, %4, 4;\n\t"
+        "shf.r.wrap.b32 r1, %5, %5, 4;\n\t"
+        "shf.r.wrap.b32 r2, %6, %6, 4;\n\t"
+        "shf.r.wrap.b32 r3, %7, %7, 4;\n\t"
+        "mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {a0,a1,a2,a3}, {%8,%9}, {%13,%13,%13,%13};\n\t"
+        "and.b32 a0, r0, %12;\n\t"
+        "and.b32 a1, r1, %12;\n\t"
+        "and.b32 a2, r2, %12;\n\t"
+        "and.b32 a3, r3, %12;\n\t"
         "mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {a0,a1,a2,a3}, {%10,%11}, {%0,%1,%2,%3};\n\t"
         "}\n"
         : "=&r"(d[0]), "=&r"(d[1]), "=&r"(d[2]), "=&r"(d[3])
-        : "r"(w00), "r"(w10), "r"(w01), "r"(w11), "r"(bl1), "r"(bh1), "r"(bl2), "r"(bh2), "r"(CODE8_MASK), "r"(mul28), "r"(0));
+        : "r"(w00), "r"(w10), "r"(w01), "r"(w11), "r"(bl1), "r"(bh1), "r"(bl2), "r"(bh2), "r"(CODE8_MASK), "r"(0));
 }
 
 // Lane-specific shared addresses of the staged token for the tile at hand.
@@ -353,7 +346,6 @@ struct Q8Addr {
 // and of pair B (b).  For a lane that feeds the low k-slots the hi words are zero in shared memory, and vice versa.
 struct Q8Digits {
     uint4 a, b;
-    uint32_t mul28 = 0x10000000u | (gridDim.y >> 16);  // 2^28 (a grid has fewer than 2^16 CTAs in y), opaque to the compiler
     template <int OFF> __device__ __forceinline__ void load(const Q8Addr& at) {
         a = lds128_at<OFF>(at.x);
         b = lds128_at<OFF>(at.xb);
@@ -415,8 +407,8 @@ template <> struct TileRegs<WF_QTYPE_Q4_0> {
         dg.template load<J * (TK / 128) * Q8_UNIT_BYTES>(a);
         const uint4 r = lds128_at<J * (TK >> 5) * 16>(a.rec);  // {W, f, W', f'}
         int da[4], db[4];
-        pair_imma(da, c[0].x, c[1].x, c[0].z, c[1].z, dg.a.x, dg.a.y, dg.a.z, dg.a.w, dg.mul28);
-        pair_imma(db, c[0].y, c[1].y, c[0].w, c[1].w, dg.b.x, dg.b.y, dg.b.z, dg.b.w, dg.mul28);
+        pair_imma(da, c[0].x, c[1].x, c[0].z, c[1].z, dg.a.x, dg.a.y, dg.a.z, dg.a.w);
+        pair_imma(db, c[0].y, c[1].y, c[0].w, c[1].w, dg.b.x, dg.b.y, dg.b.z, dg.b.w);
         const float2 sg = half2_bits_to_float2(sg2), sh = half2_bits_to_float2(sh2);
         const float ea = __uint_as_float(r.y), eb = __uint_as_float(r.w);
         const int wa = (int)r.x, wb = (int)r.z;
@@ -519,8 +511,8 @@ template <> struct TileRegs<WF_QTYPE_Q4_1> {
         const uint4 r = lds128_at<J * (TK >> 5) * 16>(a.rec);
         const uint2 sx = lds64(a.sx + J * (TK >> 5) * 8);
         int da[4], db[4];
-        pair_imma(da, c[0].x, c[1].x, c[0].z, c[1].z, dg.a.x, dg.a.y, dg.a.z, dg.a.w, dg.mul28);
-        pair_imma(db, c[0].y, c[1].y, c[0].w, c[1].w, dg.b.x, dg.b.y, dg.b.z, dg.b.w, dg.mul28);
+        pair_imma(da, c[0].x, c[1].x, c[0].z, c[1].z, dg.a.x, dg.a.y, dg.a.z, dg.a.w);
+        pair_imma(db, c[0].y, c[1].y, c[0].w, c[1].w, dg.b.x, dg.b.y, dg.b.z, dg.b.w);
         const float2 sg = half2_bits_to_float2(sg2), sh = half2_bits_to_float2(sh2);
         const float2 mg = half2_bits_to_float2(mg2), mh = half2_bits_to_float2(mh2);
         const float ea = __uint_as_float(r.y), eb = __uint_as_float(r.w);
@@ -620,10 +612,10 @@ template <> struct TileRegs<WF_QTYPE_Q8_0> {
         dg.template load<J * (TK / 128) * Q8_UNIT_BYTES>(a);
         const uint4 r = lds128_at<J * (TK >> 5) * 16>(a.rec);
         int la[4], lb[4], ha[4], hb[4];
-        pair_imma(ha, c[0].x, c[1].x, c[0].z, c[1].z, dg.a.x, dg.a.y, dg.a.z, dg.a.w, dg.mul28);
-        pair_imma(la, c[2].x, c[3].x, c[2].z, c[3].z, dg.a.x, dg.a.y, dg.a.z, dg.a.w, dg.mul28);
-        pair_imma(hb, c[0].y, c[1].y, c[0].w, c[1].w, dg.b.x, dg.b.y, dg.b.z, dg.b.w, dg.mul28);
-        pair_imma(lb, c[2].y, c[3].y, c[2].w, c[3].w, dg.b.x, dg.b.y, dg.b.z, dg.b.w, dg.mul28);
+        pair_imma(ha, c[0].x, c[1].x, c[0].z, c[1].z, dg.a.x, dg.a.y, dg.a.z, dg.a.w);
+        pair_imma(la, c[2].x, c[3].x, c[2].z, c[3].z, dg.a.x, dg.a.y, dg.a.z, dg.a.w);
+        pair_imma(hb, c[0].y, c[1].y, c[0].w, c[1].w, dg.b.x, dg.b.y, dg.b.z, dg.b.w);
+        pair_imma(lb, c[2].y, c[3].y, c[2].w, c[3].w, dg.b.x, dg.b.y, dg.b.z, dg.b.w);
         const float2 sg = half2_bits_to_float2(sg2), sh = half2_bits_to_float2(sh2);
         const float ea = __uint_as_float(r.y), eb = __uint_as_float(r.w);
         const int wa = (int)r.x, wb = (int)r.z;
@@ -752,8 +744,8 @@ template <> struct TileRegs<WF_QTYPE_Q4_K> {
             const uint4 r = u == 0 ? lds128_at<(2 * J) * 64>(a.rec) : lds128_at<(2 * J + 1) * 64>(a.rec);
             const uint2 sx = lds64(a.sx + (2 * J + u) * 32);
             int da[4], db[4];
-            pair_imma(da, c[2 * u].x, c[2 * u + 1].x, c[2 * u].z, c[2 * u + 1].z, dg.a.x, dg.a.y, dg.a.z, dg.a.w, dg.mul28);
-            pair_imma(db, c[2 * u].y, c[2 * u + 1].y, c[2 * u].w, c[2 * u + 1].w, dg.b.x, dg.b.y, dg.b.z, dg.b.w, dg.mul28);
+            pair_imma(da, c[2 * u].x, c[2 * u + 1].x, c[2 * u].z, c[2 * u + 1].z, dg.a.x, dg.a.y, dg.a.z, dg.a.w);
+            pair_imma(db, c[2 * u].y, c[2 * u + 1].y, c[2 * u].w, c[2 * u + 1].w, dg.b.x, dg.b.y, dg.b.z, dg.b.w);
             const uint32_t wsg = scg[u], wsh = sch[u], wmg = mng[u], wmh = mnh[u];
             const float ea = __uint_as_float(r.y), eb = __uint_as_float(r.w);
             const float xa = __uint_as_float(sx.x), xb = __uint_as_float(sx.y);

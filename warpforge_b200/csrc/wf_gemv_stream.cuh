@@ -144,24 +144,26 @@ struct WsCursor {
     int t = 0, end = 0;
     const uint8_t* tiles = nullptr;
 };
-// The next group to request: address of its first tile and its number of tiles (0 once the program is exhausted).
+// The group to request next: its first tile and its number of tiles (0 once the program is exhausted).
+struct WsNext {
+    const uint8_t* base;
+    int cnt;
+};
 template <int QT, int DEPTH, class ShareFn>
-__device__ __forceinline__ void ws_next_group(WsCursor& c, ShareFn& share_of, int n_ops, int warp, const uint8_t*& base, int& cnt) {
+__device__ __forceinline__ WsNext ws_next_group(WsCursor& c, ShareFn& share_of, int n_ops, int warp) {
     while (c.t >= c.end) {
         if (c.op + 1 >= n_ops) {
             c.op = n_ops;
-            base = nullptr;
-            cnt = 0;
-            return;
+            return WsNext{nullptr, 0};
         }
         c.op++;
         const WsShare sh = share_of(c.op);
         ws_run(sh.t0, sh.t1, warp, c.t, c.end);
         c.tiles = sh.tiles;
     }
-    cnt = min(DEPTH, c.end - c.t);
-    base = c.tiles + (size_t)c.t * Tile<QT>::BYTES;
-    c.t += cnt;
+    const WsNext n{c.tiles + (size_t)c.t * Tile<QT>::BYTES, min(DEPTH, c.end - c.t)};
+    c.t += n.cnt;
+    return n;
 }
 // The two lane pointers a tile is loaded through (see TileRegs::load_global).
 template <int QT> struct WsLanePtrs {
@@ -170,18 +172,16 @@ template <int QT> struct WsLanePtrs {
     __device__ __forceinline__ WsLanePtrs(const uint8_t* base, int lane)
         : pc(base + lane * 16), ps(base + TileRegs<QT>::lane_scale_offset(lane)) {}
 };
-// Request the first group of the stream (the weights depend on nothing, so this comes before any wait).
+// Request the first group of the stream (the weights depend on nothing, so this comes before any wait); the one after it.
 template <int QT, int DEPTH, class ShareFn>
-__device__ __forceinline__ void ws_prime(TileRegs<QT> (&slots)[DEPTH], WsCursor& c, ShareFn& share_of, int n_ops,
-                                         int warp, int lane) {
-    const uint8_t* base;
-    int cnt;
-    ws_next_group<QT, DEPTH>(c, share_of, n_ops, warp, base, cnt);
-    const WsLanePtrs<QT> lp(base, lane);
+__device__ __forceinline__ WsNext ws_prime(TileRegs<QT> (&slots)[DEPTH], WsCursor& c, ShareFn& share_of, int n_ops, int warp, int lane) {
+    const WsNext first = ws_next_group<QT, DEPTH>(c, share_of, n_ops, warp);
+    const WsLanePtrs<QT> lp(first.base, lane);
     static_for<DEPTH>([&](auto J) {
         constexpr int j = decltype(J)::value;
-        if (j < cnt) slots[j].template load_global<j * Tile<QT>::BYTES>(lp.pc, lp.ps);
+        if (j < first.cnt) slots[j].template load_global<j * Tile<QT>::BYTES>(lp.pc, lp.ps);
     });
+    return ws_next_group<QT, DEPTH>(c, share_of, n_ops, warp);
 }
 // Clear the digit words once per kernel: the staging only ever writes the word of the half a lane feeds.
 __device__ __forceinline__ void ws_clear_digits(uint8_t* xd, int kp, int nthreads) {
@@ -226,14 +226,24 @@ __device__ __forceinline__ WsRun ws_open(const WsShare& sh, int warp) {
     return r;
 }
 
+// A row-tile cut by the share's boundary: its first holder's CTA adds what the following CTAs publish.  Out of line, since most
+// shares are whole row-tiles and the code that follows would lie behind it.
+static __device__ __noinline__ float ws_exchange(uint2* slots_g, float sum, int lane, bool starts, int row_end, int chunk_q, int chunk_r, int* status) {
+    float v[1] = {sum};
+    if (!starts) publish_piece<16>(slots_g + (size_t)blockIdx.x * 128, v, lane, status);
+    else collect_pieces<16>(slots_g, v, lane, row_end, chunk_q, chunk_r, status);
+    return v[0];
+}
+
 // One weight, one warp: walk the run, hand the cut pieces over, finish the row-tiles this warp is first to hold.
-//   slots: the register sets holding the first group of this run (requested earlier); cur: the request cursor;
+//   slots: the register sets holding the first group of this run (requested earlier); next: the group to request next; cur: the
+//   request cursor behind it;
 //   x32 / c32 / s32: shared addresses of the staged digits, the block records and the activation sums;
 //   emit_row(n, value): store output row n of this weight (called by one lane per row);
 //   share_of(o): the CTA's share of weight o of the program.
 template <int QT, int DEPTH, class EmitRow, class ShareFn>
 __device__ __forceinline__ void ws_consume(const WsShare& sh, const WsRun& run, int chunk_q, int chunk_r, int warp, int lane,
-                                           TileRegs<QT> (&slots)[DEPTH], WsCursor& cur, const WsBars& bar,
+                                           TileRegs<QT> (&slots)[DEPTH], WsNext& next, WsCursor& cur, const WsBars& bar,
                                            WsPiece* pieces, uint32_t& seq, uint32_t x32, uint32_t c32, uint32_t s32,
                                            uint2* slots_g, int* status, uint32_t abort32, ShareFn& share_of, int n_ops,
                                            EmitRow&& emit_row) {
@@ -297,10 +307,7 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, const WsRun& run, 
         for (int g0 = 0; g0 < len; g0 += DEPTH) {
             // the group after this one in the warp's stream (maybe of a later weight): requested slot by slot as
             // the slots of this group are used up
-            const uint8_t* nbase;
-            int ncnt;
-            ws_next_group<QT, DEPTH>(cur, share_of, n_ops, warp, nbase, ncnt);
-            const WsLanePtrs<QT> lp(nbase, lane);
+            const WsLanePtrs<QT> lp(next.base, lane);
             if (g0 + DEPTH <= len && kk + DEPTH <= kt) {
                 // a whole group inside one row-tile: straight-line code, immediate offsets; the requests are predicated, so
                 // that a run's last whole group takes this way too, whatever is left to request (a 32-layer step: 1140 ->
@@ -308,7 +315,7 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, const WsRun& run, 
                 static_for<DEPTH>([&](auto J) {
                     constexpr int j = decltype(J)::value;
                     slots[j].template compute_q8<j>(acc, qa, dg);
-                    if (j < ncnt) slots[j].template load_global<j * T::BYTES>(lp.pc, lp.ps);
+                    if (j < next.cnt) slots[j].template load_global<j * T::BYTES>(lp.pc, lp.ps);
                 });
                 kk += DEPTH;
                 qa.x += DEPTH * XSTEP;
@@ -347,9 +354,10 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, const WsRun& run, 
                             qa.sx += SSTEP;
                         }
                     }
-                    if (j < ncnt) slots[j].template load_global<j * T::BYTES>(lp.pc, lp.ps);
+                    if (j < next.cnt) slots[j].template load_global<j * T::BYTES>(lp.pc, lp.ps);
                 });
             }
+            next = ws_next_group<QT, DEPTH>(cur, share_of, n_ops, warp);
         }
         if (kk != 0) flush(false);
     }
@@ -370,8 +378,7 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, const WsRun& run, 
             const int li = lane & 15, half = lane >> 4, a2 = sh.t0 + li * rq + min(li, rr);
             const int more = __popc(__ballot_sync(0xFFFFFFFFu, lane > warp && half == 0 && a2 < row_end));
             const float* const next = reinterpret_cast<const float*>(all + (warp + half) * 2) + li;
-            float v[1];
-            v[0] = half == 0 ? mine[pi].v[li] : 0.f;
+            float sum = half == 0 ? mine[pi].v[li] : 0.f;
             float pc[GEMV_WARPS / 2];
 #pragma unroll
             for (int d = 0; d < GEMV_WARPS / 2; d++) {
@@ -379,15 +386,11 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, const WsRun& run, 
                 pc[d] = i >= 1 && i <= more ? next[d * 64] : 0.f;
             }
 #pragma unroll
-            for (int d = 0; d < GEMV_WARPS / 2; d++) v[0] += pc[d];
-            v[0] += __shfl_xor_sync(0xFFFFFFFFu, v[0], 16);
+            for (int d = 0; d < GEMV_WARPS / 2; d++) sum += pc[d];
+            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 16);
             const bool starts = r * kt >= sh.t0, ends = (r + 1) * kt <= sh.t1;
-            if (!starts) {
-                publish_piece<16>(slots_g + (size_t)blockIdx.x * 128, v, lane, status);
-            } else {
-                if (!ends) collect_pieces<16>(slots_g, v, lane, (r + 1) * kt, chunk_q, chunk_r, status);
-                if (lane < 16) emit_row(r * 16 + lane, v[0]);
-            }
+            if (!starts || !ends) sum = ws_exchange(slots_g, sum, lane, starts, (r + 1) * kt, chunk_q, chunk_r, status);
+            if (starts && lane < 16) emit_row(r * 16 + lane, sum);
         }
     }
     __syncwarp();

@@ -209,6 +209,13 @@ template <int T, int V> struct Row {
     }
 };
 
+// Every kernel here is launched with programmatic stream serialization: it may be placed while the kernel before it drains, lets
+// the one behind it be placed in turn, and touches memory only when the one before it has completed.
+__device__ __forceinline__ void wait_for_previous() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // row of this thread's group, -1 for a group without one
 template <int T> __device__ __forceinline__ int64_t row_of_group(int64_t rows) {
     const int64_t r = T == 32 ? (int64_t)blockIdx.x * (ROW_CTA / 32) + (threadIdx.x >> 5) : (int64_t)blockIdx.x;
@@ -220,6 +227,7 @@ template <int T, int V>
 __global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
                                                                          float* __restrict__ y, int64_t rows, int n, float eps) {
     __shared__ double red[T / 32];
+    wait_for_previous();
     const int64_t r = row_of_group<T>(rows);
     if (r < 0) return;
     const Row<T, V> row(x + (size_t)r * n, n);
@@ -238,6 +246,7 @@ __global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) layer_norm_kernel(const
                                                                            const float* __restrict__ beta, float* __restrict__ y,
                                                                            int64_t rows, int n, float eps) {
     __shared__ double red[T / 32], red2[T / 32];
+    wait_for_previous();
     const int64_t r = row_of_group<T>(rows);
     if (r < 0) return;
     const Row<T, V> row(x + (size_t)r * n, n);
@@ -265,6 +274,7 @@ __global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) softmax_kernel(const fl
     __shared__ float redf[T / 32];
     __shared__ double tab[32];
     if (EXACT) load_exp_table(tab);
+    wait_for_previous();
     const int64_t r = row_of_group<T>(rows);
     if (r < 0) return;
     Row<T, V> row(x + (size_t)r * n, n);
@@ -343,6 +353,7 @@ __global__ void __launch_bounds__(256, (ElShape<OP, EXACT>::CTAS)) elementwise_k
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
     __shared__ double tab[32];
     if (OP != EL_ADD && OP != EL_GELU && EXACT) load_exp_table(tab);
+    wait_for_previous();
     if (vec) {
         const int64_t n4 = n / 4;
         for (int64_t i0 = tid; i0 < n4; i0 += EL_UNROLL * step) {
@@ -426,6 +437,7 @@ __global__ void __launch_bounds__(256) dot_f32_kernel(const float* __restrict__ 
 __global__ void __launch_bounds__(256) embedding_kernel(const int64_t* __restrict__ indices, const float* __restrict__ table,
                                                         float* __restrict__ y, int64_t count, int64_t vocab, int dim, int vec,
                                                         int* status) {
+    wait_for_previous();
     for (int64_t r = blockIdx.x; r < count; r += gridDim.x) {
         const int64_t idx = (int64_t)(int)indices[r];  // `(int) indexData.getAtIndex(JAVA_LONG, i)`
         const bool ok = idx >= 0 && idx < vocab;
@@ -455,11 +467,25 @@ __global__ void __launch_bounds__(256) embedding_kernel(const int64_t* __restric
 static bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 static bool aligned4(const void* p) { return reinterpret_cast<uintptr_t>(p) % 4 == 0; }
 
+template <class... Params, class... Args>
+static cudaError_t launch_glue(void (*kernel)(Params...), unsigned grid, unsigned threads, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 template <int OP, bool EXACT>
-static void launch_element(Context* c, const float* a, const float* b, float* y, int64_t n, int vec, cudaStream_t s) {
+static cudaError_t launch_element(Context* c, const float* a, const float* b, float* y, int64_t n, int vec, cudaStream_t s) {
     const int64_t want = (n / 4 + 255) / 256, most = (int64_t)c->sm_count * ElShape<OP, EXACT>::CTAS;
     const int grid = (int)std::max<int64_t>(1, std::min(want, most));
-    elementwise_kernel<OP, EXACT><<<grid, 256, 0, s>>>(a, b, y, n, vec);
+    return launch_glue(elementwise_kernel<OP, EXACT>, (unsigned)grid, 256, s, a, b, y, n, vec);
 }
 
 }  // namespace wf
@@ -474,8 +500,7 @@ using namespace wf;
     WF_CUDA(c, cudaSetDevice(c->device));                                  \
     cudaStream_t s = resolve_stream(c, stream)
 
-static int launched(Context* c, const char* what) {
-    const cudaError_t e = cudaGetLastError();
+static int launched(Context* c, const char* what, cudaError_t e) {
     if (e != cudaSuccess) return cuda_status(c, e, what);
     c->launches++;
     return WF_OK;
@@ -503,12 +528,13 @@ int wf_rms_norm(int64_t ctx, int64_t x_dev, int64_t gamma_dev, int64_t y_dev, in
     GLUE_ENTER(ctx);
     int rc = check_rows(c, "rms_norm", x_dev, y_dev, rows, n);
     if (rc != WF_OK || rows == 0) return rc;
+    cudaError_t e = cudaSuccess;
     with_row_group(rows, n, [&](auto t, auto v, unsigned grid) {
         constexpr int T = decltype(t)::value, V = decltype(v)::value;
-        rms_norm_kernel<T, V><<<grid, T == 32 ? ROW_CTA : T, 0, s>>>(reinterpret_cast<const float*>(x_dev), reinterpret_cast<const float*>(gamma_dev),
-                                                                    reinterpret_cast<float*>(y_dev), rows, (int)n, eps);
+        e = launch_glue(rms_norm_kernel<T, V>, grid, T == 32 ? ROW_CTA : T, s, reinterpret_cast<const float*>(x_dev), reinterpret_cast<const float*>(gamma_dev),
+                        reinterpret_cast<float*>(y_dev), rows, (int)n, eps);
     });
-    return launched(c, "rms_norm");
+    return launched(c, "rms_norm", e);
 }
 
 int wf_layer_norm(int64_t ctx, int64_t x_dev, int64_t gamma_dev, int64_t beta_dev, int64_t y_dev, int64_t rows, int64_t n, float eps,
@@ -516,27 +542,27 @@ int wf_layer_norm(int64_t ctx, int64_t x_dev, int64_t gamma_dev, int64_t beta_de
     GLUE_ENTER(ctx);
     int rc = check_rows(c, "layer_norm", x_dev, y_dev, rows, n);
     if (rc != WF_OK || rows == 0) return rc;
+    cudaError_t e = cudaSuccess;
     with_row_group(rows, n, [&](auto t, auto v, unsigned grid) {
         constexpr int T = decltype(t)::value, V = decltype(v)::value;
-        layer_norm_kernel<T, V><<<grid, T == 32 ? ROW_CTA : T, 0, s>>>(
-            reinterpret_cast<const float*>(x_dev), reinterpret_cast<const float*>(gamma_dev), reinterpret_cast<const float*>(beta_dev),
-            reinterpret_cast<float*>(y_dev), rows, (int)n, eps);
+        e = launch_glue(layer_norm_kernel<T, V>, grid, T == 32 ? ROW_CTA : T, s, reinterpret_cast<const float*>(x_dev), reinterpret_cast<const float*>(gamma_dev),
+                        reinterpret_cast<const float*>(beta_dev), reinterpret_cast<float*>(y_dev), rows, (int)n, eps);
     });
-    return launched(c, "layer_norm");
+    return launched(c, "layer_norm", e);
 }
 
 int wf_softmax(int64_t ctx, int64_t x_dev, int64_t y_dev, int64_t rows, int64_t n, int64_t stream) {
     GLUE_ENTER(ctx);
     int rc = check_rows(c, "softmax", x_dev, y_dev, rows, n);
     if (rc != WF_OK || rows == 0) return rc;
+    cudaError_t e = cudaSuccess;
     with_row_group(rows, n, [&](auto t, auto v, unsigned grid) {
         constexpr int T = decltype(t)::value, V = decltype(v)::value;
         const float* x = reinterpret_cast<const float*>(x_dev);
         float* y = reinterpret_cast<float*>(y_dev);
-        if (c->glue_exact) softmax_kernel<T, V, true><<<grid, T == 32 ? ROW_CTA : T, 0, s>>>(x, y, rows, (int)n);
-        else softmax_kernel<T, V, false><<<grid, T == 32 ? ROW_CTA : T, 0, s>>>(x, y, rows, (int)n);
+        e = launch_glue(c->glue_exact ? softmax_kernel<T, V, true> : softmax_kernel<T, V, false>, grid, T == 32 ? ROW_CTA : T, s, x, y, rows, (int)n);
     });
-    return launched(c, "softmax");
+    return launched(c, "softmax", e);
 }
 
 static int elementwise(int64_t ctx, int op, const char* what, int64_t a_dev, int64_t b_dev, int64_t y_dev, int64_t count, int64_t stream) {
@@ -550,13 +576,14 @@ static int elementwise(int64_t ctx, int op, const char* what, int64_t a_dev, int
     const int vec = aligned16(a) && aligned16(y) && (unary || aligned16(b));
     const float *fa = static_cast<const float*>(a), *fb = static_cast<const float*>(b);
     float* fy = reinterpret_cast<float*>(y_dev);
-    if (op == EL_GELU) launch_element<EL_GELU, false>(c, fa, fb, fy, count, vec, s);
-    else if (op == EL_SILU && c->glue_exact) launch_element<EL_SILU, true>(c, fa, fb, fy, count, vec, s);
-    else if (op == EL_SILU) launch_element<EL_SILU, false>(c, fa, fb, fy, count, vec, s);
-    else if (op == EL_SWIGLU && c->glue_exact) launch_element<EL_SWIGLU, true>(c, fa, fb, fy, count, vec, s);
-    else if (op == EL_SWIGLU) launch_element<EL_SWIGLU, false>(c, fa, fb, fy, count, vec, s);
-    else launch_element<EL_ADD, false>(c, fa, fb, fy, count, vec, s);
-    return launched(c, what);
+    cudaError_t e;
+    if (op == EL_GELU) e = launch_element<EL_GELU, false>(c, fa, fb, fy, count, vec, s);
+    else if (op == EL_SILU && c->glue_exact) e = launch_element<EL_SILU, true>(c, fa, fb, fy, count, vec, s);
+    else if (op == EL_SILU) e = launch_element<EL_SILU, false>(c, fa, fb, fy, count, vec, s);
+    else if (op == EL_SWIGLU && c->glue_exact) e = launch_element<EL_SWIGLU, true>(c, fa, fb, fy, count, vec, s);
+    else if (op == EL_SWIGLU) e = launch_element<EL_SWIGLU, false>(c, fa, fb, fy, count, vec, s);
+    else e = launch_element<EL_ADD, false>(c, fa, fb, fy, count, vec, s);
+    return launched(c, what, e);
 }
 
 int wf_silu(int64_t ctx, int64_t x_dev, int64_t y_dev, int64_t count, int64_t stream) {
@@ -572,7 +599,7 @@ int wf_dot_f32(int64_t ctx, int64_t a_dev, int64_t b_dev, int64_t c_dev, int64_t
     const dim3 grid((unsigned)((n + DOT_TILE - 1) / DOT_TILE), (unsigned)std::min<int64_t>((m + DOT_TILE - 1) / DOT_TILE, 65535));
     dot_f32_kernel<<<grid, dim3(16, 16), 0, s>>>(reinterpret_cast<const float*>(a_dev), reinterpret_cast<const float*>(b_dev),
                                                  reinterpret_cast<float*>(c_dev), (int)m, (int)n, (int)k);
-    return launched(c, "dot");
+    return launched(c, "dot", cudaGetLastError());
 }
 
 int wf_gelu(int64_t ctx, int64_t x_dev, int64_t y_dev, int64_t count, int64_t stream) {
@@ -595,9 +622,9 @@ int wf_embedding(int64_t ctx, int64_t indices_dev, int64_t table_dev, int64_t y_
     if (count == 0) return WF_OK;
     const int vec = dim % 4 == 0 && table_dev % 16 == 0 && y_dev % 16 == 0;
     const int grid = (int)std::min<int64_t>(count, (int64_t)c->sm_count * 8);
-    embedding_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const int64_t*>(indices_dev), reinterpret_cast<const float*>(table_dev),
-                                          reinterpret_cast<float*>(y_dev), count, vocab, (int)dim, vec, c->d_status);
-    return launched(c, "embedding");
+    return launched(c, "embedding",
+                    launch_glue(embedding_kernel, (unsigned)grid, 256, s, reinterpret_cast<const int64_t*>(indices_dev), reinterpret_cast<const float*>(table_dev),
+                                reinterpret_cast<float*>(y_dev), count, vocab, (int)dim, vec, c->d_status));
 }
 
 }  // extern "C"

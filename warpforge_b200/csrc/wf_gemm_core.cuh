@@ -208,15 +208,15 @@ __host__ __device__ inline int stage_chunk(int j, int q) { return 2 * q + j; }
 // beside the previous GEMM's, which triggers them early (the nested release takes 3 us longer than the overlap gains).
 constexpr int CONVERT_THREADS = 256;
 template <int PLANES>
-__global__ void __launch_bounds__(CONVERT_THREADS) convert_rows_kernel(const void* __restrict__ x, __half* __restrict__ x16, float* __restrict__ unscale,
+__global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 ? 8 : 1) convert_rows_kernel(const void* __restrict__ x, __half* __restrict__ x16, float* __restrict__ unscale,
                                                                        int m, int k) {
     __shared__ int s_max[CONVERT_THREADS / 32];
     // Launched with programmatic stream serialization itself: its CTAs may be placed while the previous kernel of the
     // stream drains, but nothing is read or written before that kernel has completed (it may have produced x, and a
     // previous GEMM may still be reading the fp16 copy this kernel rewrites).
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMM may set itself up while the rows are converted
-    constexpr int KEEP = PLANES == 1 ? 4 : 2;  // groups of eight elements a thread keeps between the scan and the conversion
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    constexpr int KEEP = 2;  // groups of eight elements a thread keeps between the scan and the conversion
     const int groups = k >> 3, t = (int)threadIdx.x;  // k is a multiple of 32
     const int padded = (groups + 7) & ~7;             // groups of a row of x16
     const size_t plane = (size_t)m * padded;
@@ -242,15 +242,30 @@ __global__ void __launch_bounds__(CONVERT_THREADS) convert_rows_kernel(const voi
         }
         return e;
     };
+    // bf16: the largest magnitude of each half of the words, which is enough unless there is an Inf or a NaN (0x7F80 and up)
+    auto mags_of = [](uint32_t m, const G& g) {
+        return __vmaxu2(__vmaxu2(m, __vmaxu2(g.a.x & 0x7FFF7FFFu, g.a.y & 0x7FFF7FFFu)), __vmaxu2(g.a.z & 0x7FFF7FFFu, g.a.w & 0x7FFF7FFFu));
+    };
     G keep[KEEP];
     int emax = 0;
+    uint32_t mags = 0;
 #pragma unroll
     for (int u = 0; u < KEEP; u++)
         if (t + u * CONVERT_THREADS < groups) keep[u] = load(t + u * CONVERT_THREADS);
+    if (PLANES == 1) {
 #pragma unroll
-    for (int u = 0; u < KEEP; u++)
-        if (t + u * CONVERT_THREADS < groups) emax = max(emax, emax_of(keep[u]));
-    for (int i = t + KEEP * CONVERT_THREADS; i < groups; i += CONVERT_THREADS) emax = max(emax, emax_of(load(i)));
+        for (int u = 0; u < KEEP; u++)
+            if (t + u * CONVERT_THREADS < groups) mags = mags_of(mags, keep[u]);
+        for (int i = t + KEEP * CONVERT_THREADS; i < groups; i += CONVERT_THREADS) mags = mags_of(mags, load(i));
+        emax = max((int)(mags & 0xFFFFu) >> 7, (int)(mags >> 23));
+    }
+    if (PLANES > 1 || emax == 0xFF) {
+        emax = 0;
+#pragma unroll
+        for (int u = 0; u < KEEP; u++)
+            if (t + u * CONVERT_THREADS < groups) emax = max(emax, emax_of(keep[u]));
+        for (int i = t + KEEP * CONVERT_THREADS; i < groups; i += CONVERT_THREADS) emax = max(emax, emax_of(load(i)));
+    }
     emax = __reduce_max_sync(0xFFFFFFFFu, emax);
     if ((t & 31) == 0) s_max[t >> 5] = emax;
     __syncthreads();

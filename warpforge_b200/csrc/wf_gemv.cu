@@ -609,7 +609,7 @@ bool gemv_prepare_group(Context* c, const GemvGroup& g, GemvPrepared* out) {
         return launch_group(*out, 0, nullptr) == cudaSuccess;
     }
     if (g.x_kind != XK_BF16) return false;
-    const GemvNPlan plan = gemvn_plan(gemvn_clusters(c->sm_count), qt, rt, kt, g.m, false);
+    const GemvNPlan plan = gemvn_plan(gemvn_clusters(c->sm_count), qt, rt, kt, g.m, false, 1500.0);
     if (plan.slices < 1 || plan.part) return false;
     GemvNParams<GEMV_GROUP>& p = out->several;
     p = {};

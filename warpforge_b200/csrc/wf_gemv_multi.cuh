@@ -131,7 +131,11 @@ struct GemvNPlan {
 // number of 7s.  On 130 other weights, up to 32000 x 8192, the choices are 1.4 % slower than the best S on average and 14 % at
 // worst (2.4 % and 32 % without that correction).  Memory is the way where eight slices do not fit (against a cluster of the
 // same S it measured 1 - 4 us more on small weights, up to twice the time on tall ones).
-inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt, int cols, bool x_f32) {
+// cluster_ns: what a launch of clusters costs its neighbours.  Its CTAs start 1 us after the end of the launch before it, plain ones
+// half a microsecond ahead of it, and the launch behind it starts late as well: a program takes clusters only where they gain
+// more than that (four tokens Q8_0, d 4096, three layers: 169 us with two slices for Wq, Wk, Wv and for Wgate, Wup, 166 with two
+// everywhere, 163 with none).
+inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt, int cols, bool x_f32, double cluster_ns = 0.0) {
     GemvNPlan best;
     const int ng = (cols + 7) / 8, tk = tile_k(qt), sms = clusters[1];
     const double per_group = 15.9 + (qt == WF_QTYPE_Q4_1 ? 3.3 : qt == WF_QTYPE_Q8_0 ? 16.3 : qt == WF_QTYPE_Q4_K ? 5.0 : 0.0);
@@ -159,6 +163,7 @@ inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt,
             else if (slices > 1) ns += 616.0 + slices * (6.1 + 32.1 * ((own * ng + GEMV_WARPS - 1) / GEMV_WARPS));
             if (x_f32 && !part) ns += 31.1 * slices * ((own * (cols / 3) * 16 + GEMV_CONSUMERS - 1) / GEMV_CONSUMERS);
         }
+        if (!part && slices > 1) ns += cluster_ns;
         if (!part && ns > 13000.0) ns *= slices == 3 || slices == 7 ? 1.1 : slices == 5 ? 1.05 : 1.0;
         if (best.slices == 0 || ns < best_ns) {
             best_ns = ns;

@@ -203,9 +203,10 @@ __host__ __device__ inline int stage_chunk(int j, int q) { return 2 * q + j; }
 //   fp32 (PLANES 3): v = hi + mid + lo, each the fp16 nearest to what is left: exact down to 2^-39 of the row's largest
 //   (below that, what fp32 rounding leaves of a sum that the largest takes part in).
 // One CTA per row.  A kernel of its own: the GEMM's CTAs set themselves up and dequantize their first stages under it.
+// bf16 rows: 32 registers a thread, so that a CTA fits beside one of the cluster GEMM's and can wait there, and exponents found as
+// the largest magnitude of packed pairs; with 40 registers and an exponent at a time 2048 rows of 4096 took 7.7 us.
 // Measured and not kept: converting inside the GEMM, every CTA its share of the rows and a counter to wait for (64
-// tokens: 18 us a call instead of 16, the launch and set-up of the GEMM itself lie bare then); CTAs small enough to wait
-// beside the previous GEMM's, which triggers them early (the nested release takes 3 us longer than the overlap gains).
+// tokens: 18 us a call instead of 16, the launch and set-up of the GEMM itself lie bare then).
 constexpr int CONVERT_THREADS = 256;
 template <int PLANES>
 __global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 ? 8 : 1) convert_rows_kernel(const void* __restrict__ x, __half* __restrict__ x16, float* __restrict__ unscale,

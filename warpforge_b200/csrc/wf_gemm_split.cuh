@@ -43,8 +43,8 @@ inline __host__ __device__ int split_exchange_bytes(int bm, int ranks) { return 
 template <int QT, int PIECES, int PLANES>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap) {
     // The next call's conversion, 32 registers a thread, fits beside a CTA of 128 and waits there; and the next GEMM takes the SM as
-    // soon as this one leaves it (77 tokens, [5003 x 2784]: 125.4 -> 119 us for eight calls; fp32 tokens, whose conversion does not
-    // fit beside: 92.8 -> 98).
+    // soon as this one leaves it (eight calls of [5003 x 2784], 77 tokens: 122 -> 108.5 us; fp32 tokens, whose conversion does not
+    // fit beside, would take 93 -> 98).
     if (PIECES == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr int ACCS = PIECES;
     constexpr int FLUSH = PIECES == 1 ? 1 << 30 : SPLIT_FLUSH;

@@ -349,26 +349,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_pair_kernel(const GemmPa
             if (!ok && lane == 0) fail();
             tc_fence_after();
             const int chunks = halves_of(mt) * 8;  // of 32 tokens, dealt to the three warps of a quarter
-            // The first two pieces of a chunk are on their way while the one before it is stored: fetched only when it was needed, the
-            // second one made its owners the launch's last, 53 us where the others took 46.6 (Q4_K [14336 x 4096], 512 tokens).
-            float4 v[8], v2[8];
-            const bool two = last_pair > pair + 1;
-            auto fetch_into = [&](float4 (&to)[8], int cc, int ci) { load_piece_chunk(p.partial + (size_t)(2 * cc + (int)rank) * GEMM_PIECE_TOKENS * GEMM_BN, to, ci * 32, row); };
-            auto fetch = [&](int ci) {
-                fetch_into(v, pair + 1, ci);  // the next pair always holds a piece
-                if (two) fetch_into(v2, pair + 2, ci);
-            };
-            if (ok && slice < chunks) fetch(slice);
+            float4 v[8];
+            auto fetch = [&](int cc, int ci) { load_piece_chunk(p.partial + (size_t)(2 * cc + (int)rank) * GEMM_PIECE_TOKENS * GEMM_BN, v, ci * 32, row); };
+            if (ok && slice < chunks) fetch(pair + 1, slice);  // the next pair always holds a piece
             for (int ci = slice; ci < chunks && ok; ci += 3) {
                 uint32_t r[32];
                 tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + col0 + (uint32_t)(ci * 32), r);
-                add_piece_chunk(r, v);  // pieces in pair order
-                if (two) add_piece_chunk(r, v2);
-                for (int cc = pair + 3; cc <= last_pair; cc++) {
-                    fetch_into(v, cc, ci);
+                add_piece_chunk(r, v);
+                for (int cc = pair + 2; cc <= last_pair; cc++) {  // pieces in pair order
+                    fetch(cc, ci);
                     add_piece_chunk(r, v);
                 }
-                if (ci + 3 < chunks) fetch(ci + 3);  // under the stores of this one
+                if (ci + 3 < chunks) fetch(pair + 1, ci + 3);  // under the stores of this one
                 store_chunk(p.y, p.ldy, p.col0, p.row_unscale, r, mt * tile_tokens + ci * 32, p.m, n, p.rows);
             }
         }

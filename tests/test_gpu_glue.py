@@ -235,3 +235,23 @@ def test_few_rows(backend, oracle, rows, n):
     _check_rows(oracle, _call(backend, "rms_norm", x), oracle.rms_norm(x))
     _check_rows(oracle, _call(backend, "layer_norm", x), oracle.layer_norm(x))
     _check_rows(oracle, _call(backend, "softmax", x), oracle.softmax(x))
+
+
+def test_a_refused_launch_is_reported_once(backend):
+    """A launch into a recording that has been spoilt fails; the next call, on another stream, does not inherit its error."""
+    torch = pytest.importorskip("torch")
+    ctx = backend.cuda_context
+    lib, h = ctx._lib, ctx.handle
+    x, y = torch.ones(64, 64, device="cuda"), torch.zeros(64, 64, device="cuda")
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    ctx.graph_begin(s.cuda_stream)
+    with pytest.raises(RuntimeError):
+        s.synchronize()  # not allowed while recording: the recording ends as invalid
+    assert lib.wf_add(h, x.data_ptr(), x.data_ptr(), y.data_ptr(), 4096, s.cuda_stream) != N.WF_OK
+    rc = lib.wf_dot_f32(h, x.data_ptr(), x.data_ptr(), y.data_ptr(), 64, 64, 64, 0)
+    with pytest.raises(Exception):
+        ctx.graph_end(s.cuda_stream)
+    assert rc == N.WF_OK
+    ctx.synchronize()
+    assert bool((y == 64).all())

@@ -36,6 +36,7 @@ int set_error(Context* c, int status, const char* fmt, ...) {
 }
 
 int cuda_status(Context* c, cudaError_t e, const char* what) {
+    cudaGetLastError();  // reported here, not once more by the next launch that asks for it
     return set_error(c, WF_ERR_CUDA_BASE + (int)e, "%s failed: %s (%d)", what, cudaGetErrorName(e), (int)e);
 }
 

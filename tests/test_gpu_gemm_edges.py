@@ -44,6 +44,7 @@ def _run(backend, oracle, name, rows, k, x, tensor):
     (130, 352, 33), (1000, 1120, 80), (700, 5152, 77), (2500, 672, 128),  # clusters; K ends inside a stage
     (3000, 544, 129), (3072, 1024, 257), (2900, 288, 513), (1600, 2080, 1100),  # pairs; 129 tokens: one half, 257: the next begins
     (300, 800, 300), (128, 4128, 600),  # few tiles: clusters on several token tiles
+    (2900, 4096, 300), (2900, 4128, 129), (2900, 8192, 130), (2900, 8224, 300),  # pairs; K at the ends of what the conversion's two forms hold
 ])
 def test_bf16_tokens(backend, oracle, name, rows, k, m):
     from warpforge_b200.backend import Tensor

@@ -308,7 +308,11 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        WF_CUDA(c, cudaLaunchKernelEx(&cfg, f32 ? convert_rows_kernel<3> : convert_rows_kernel<1>, call.d_x, x16, unscale, (int)call.m, (int)w.g.k));
+        const bool alone = pair && w.g.k > CONVERT_KEEP_BESIDE * CONVERT_THREADS * 8;
+        const auto convert = f32     ? convert_rows_kernel<3, 2>
+                             : alone ? convert_rows_kernel<1, CONVERT_KEEP_ALONE>
+                                     : convert_rows_kernel<1, CONVERT_KEEP_BESIDE>;
+        WF_CUDA(c, cudaLaunchKernelEx(&cfg, convert, call.d_x, x16, unscale, (int)call.m, (int)w.g.k));
     }
     c->launches++;
     const size_t smem = 1024 + (size_t)p.stages * stage_bytes + exchange;

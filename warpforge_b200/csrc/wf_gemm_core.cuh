@@ -203,13 +203,18 @@ __host__ __device__ inline int stage_chunk(int j, int q) { return 2 * q + j; }
 //   fp32 (PLANES 3): v = hi + mid + lo, each the fp16 nearest to what is left: exact down to 2^-39 of the row's largest
 //   (below that, what fp32 rounding leaves of a sum that the largest takes part in).
 // One CTA per row.  A kernel of its own: the GEMM's CTAs set themselves up and dequantize their first stages under it.
-// bf16 rows: 32 registers a thread, so that a CTA fits beside one of the cluster GEMM's and can wait there, and exponents found as
-// the largest magnitude of packed pairs; with 40 registers and an exponent at a time 2048 rows of 4096 took 7.7 us.
+// bf16 rows find their exponents as the largest magnitude of packed pairs.  Before the cluster GEMM the kernel takes 32 registers a
+// thread, so that a CTA fits beside one of the GEMM's and can wait there.  The pair GEMM triggers nothing early, so
+// before it rows of more than 4096 elements are held whole, in 48 registers ([4096 x 8192], Q4_0, 1024 tokens: 65.9 -> 64.5 us
+// a call, 512 tokens: 40.2 -> 39.3; rows that the smaller form holds gain nothing: [11008 x 4096], 2048 tokens, 143.9 against 145.1).
 // Measured and not kept: converting inside the GEMM, every CTA its share of the rows and a counter to wait for (64
 // tokens: 18 us a call instead of 16, the launch and set-up of the GEMM itself lie bare then).
 constexpr int CONVERT_THREADS = 256;
-template <int PLANES>
-__global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 ? 8 : 1) convert_rows_kernel(const void* __restrict__ x, __half* __restrict__ x16, float* __restrict__ unscale,
+// KEEP: groups of eight elements a thread keeps between the scan and the conversion; what is left of a longer row is read again.
+constexpr int CONVERT_KEEP_BESIDE = 2;  // rows of 4096: what 32 registers hold
+constexpr int CONVERT_KEEP_ALONE = 4;   // rows of 8192
+template <int PLANES, int KEEP>
+__global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 && KEEP == CONVERT_KEEP_BESIDE ? 8 : 5) convert_rows_kernel(const void* __restrict__ x, __half* __restrict__ x16, float* __restrict__ unscale,
                                                                        int m, int k) {
     __shared__ int s_max[CONVERT_THREADS / 32];
     // Launched with programmatic stream serialization itself: its CTAs may be placed while the previous kernel of the
@@ -217,7 +222,6 @@ __global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 ? 8 : 1) convert_
     // previous GEMM may still be reading the fp16 copy this kernel rewrites).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMM may set itself up while the rows are converted
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    constexpr int KEEP = 2;  // groups of eight elements a thread keeps between the scan and the conversion
     const int groups = k >> 3, t = (int)threadIdx.x;  // k is a multiple of 32
     const int padded = (groups + 7) & ~7;             // groups of a row of x16
     const size_t plane = (size_t)m * padded;

@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_program_kernel(const 
     constexpr int DEPTH = WsGeom<QT, true>::DEPTH;
     R slots[DEPTH];
     WsCursor cur;
-    WsNext next = ws_prime<QT, DEPTH>(slots, cur, share_of, P.n_ops, warp, lane);
+    WsNext next = ws_prime<QT, DEPTH, false>(slots, cur, share_of, P.n_ops, warp, lane);
 
     ProgRun run{P, reinterpret_cast<volatile int*>(smem) + 1, ld_acquire_gpu(&P.sync->epoch)};
     bool failed = false;
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_program_kernel(const 
                 if (P.world > 1) emit_to_peers(op.ll, P.world, P.rank, off, v, run.tag());
             }
         };
-        ws_consume<QT, DEPTH>(sh, ws_open(sh, warp), op.chunk_q, op.chunk_r, warp, lane, slots, next, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
+        ws_consume<QT, DEPTH, false>(sh, ws_open(sh, warp), op.chunk_q, op.chunk_r, warp, lane, slots, next, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
                        sums32, slots_g, P.status, smem_u32(const_cast<int*>(abort_flag)), share_of, P.n_ops, emit_row);
         if (*abort_flag) failed = true;
         stamp();

@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvPara
     constexpr int DEPTH = WsGeom<QT, false>::DEPTH;
     R slots[DEPTH];
     WsCursor cur;
-    WsNext next = ws_prime<QT, DEPTH>(slots, cur, share_of, 1, warp, lane);
+    WsNext next = ws_prime<QT, DEPTH, true>(slots, cur, share_of, 1, warp, lane);
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         ws_bars_init(smem);
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_kernel(const GemvPara
     };
     stamp(2);
     uint32_t seq = 0;
-    ws_consume<QT, DEPTH>(share, run, p.chunk_q, p.chunk_r, warp, lane, slots, next, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
+    ws_consume<QT, DEPTH, true>(share, run, p.chunk_q, p.chunk_r, warp, lane, slots, next, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
                    smem_u32(recs) + (uint32_t)(kp >> 5) * 16, p.scratch, p.status, smem_u32(const_cast<int*>(abort_flag)), share_of, 1,
                    emit_row);
     stamp(4);
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Ge
     constexpr int DEPTH = WsGeom<QT, true>::DEPTH;
     R slots[DEPTH];
     WsCursor cur;
-    WsNext next = ws_prime<QT, DEPTH>(slots, cur, share_of, p.n_ops, warp, lane);
+    WsNext next = ws_prime<QT, DEPTH, true>(slots, cur, share_of, p.n_ops, warp, lane);
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         mbar_init(smem_u32(smem + 16), 1);
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(GEMV_CONSUMERS, 1) gemv1_group_kernel(const Ge
                 y[n] = v;
             }
         };
-        ws_consume<QT, DEPTH>(share, run, p.chunk_q, p.chunk_r, warp, lane, slots, next, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
+        ws_consume<QT, DEPTH, true>(share, run, p.chunk_q, p.chunk_r, warp, lane, slots, next, cur, bar, pieces, seq, smem_u32(xd), smem_u32(recs),
                        smem_u32(recs) + (uint32_t)(kp >> 5) * 16, p.scratch, p.status, smem_u32(const_cast<int*>(abort_flag)), share_of,
                        p.n_ops, emit_row);
         do {  // the next one, the same for the whole CTA

@@ -17,7 +17,8 @@ namespace wf {
 // ---------------------------------------------------------------- one token
 // Between the wait for the grid that writes x and the first tile lies a chain that nothing overlaps: request x, turn it into
 // digits, find the warp's run.  Four warps per scheduler hide little of it, so what does not depend on x is done before
-// the wait, and each input kind has its own kernel, whose staging is no call behind a switch: behind the wait it took 1000 cycles
+// the wait, and each input kind has its own kernel, whose staging is no call behind a switch (rms_norm, which reads the row twice, still
+// calls its two passes): behind the wait it took 1000 cycles
 // until the first element was requested, and 900 - 1700 from the staged row to the first tile.  With that, half the
 // instructions per digit, digits without bank conflicts and the cut row-tiles added by both halves of a warp, a 32-layer step of
 // the 7B shape went from 1097 to 1007 us, [4096 x 11008] from 7.8 to 7.2 (Q4_0).

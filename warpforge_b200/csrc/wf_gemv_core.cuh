@@ -1260,7 +1260,8 @@ template <int BETA_INT, int KIND, bool SHARED = false> struct StageQ8 {
                 all += __shfl_xor_sync(quad, all, 2);
 #pragma unroll
                 for (int i = 0; i < 8; i++) X[i] = (fabsf(f[i]) == __uint_as_float(0x7F800000u)) ? (f[i] < 0.f ? -1 : 1) : 0;
-                // a NaN sum: a NaN element, or Infs of both signs (which the CPU's sum of products turns into NaN as well)
+                // a NaN sum: a NaN element, or Infs of both signs (NaN here whatever the weights' signs; the CPU's sum of products gives an
+                // Inf where those signs make the terms alike)
                 const bool nan = all != all;
                 f_hi = nan ? __uint_as_float(0x7FC00000u) : 0.f;
                 f_lo = nan ? __uint_as_float(0x7FC00000u) : __uint_as_float(0x7F800000u);
@@ -1299,7 +1300,7 @@ template <int BETA_INT, int KIND, bool SHARED = false> struct StageQ8 {
                 // lane 4 (4 hcol + digit) + q: {lo, hi} first MMA, {lo, hi} second MMA; this block fills the lo words when it is
                 // its pair's first block (hcol 0), the hi words otherwise.  Column digit index = 3 - t (most significant first).
                 uint8_t* const base = xd + (size_t)unit * Q8_UNIT_BYTES + pair * 512 + hcol * 260 + q * 16;
-                uint32_t* const even = reinterpret_cast<uint32_t*>(base + pair * 64);  // column digits 0 and 2 of pair A, 1 and 3 of pair B
+                uint32_t* const even = reinterpret_cast<uint32_t*>(base + pair * 64);  // column digits 0 and 2, at positions 0 and 2 for pair A, 1 and 3 for pair B
                 uint32_t* const odd = reinterpret_cast<uint32_t*>(base + 64 - pair * 64);
                 even[0] = t1[3]; even[2] = t2[3];
                 odd[0] = t1[2]; odd[2] = t2[2];

@@ -349,7 +349,6 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, const WsRun& run, 
                             starts_here = true;
                             qa.x = x0;
                             qa.xb = x0 + b_from_a;
-                    qa.xb = x0 + b_from_a;
                             qa.rec = rec0;
                             qa.sx = sx0;
                         } else {
@@ -382,13 +381,13 @@ __device__ __forceinline__ void ws_consume(const WsShare& sh, const WsRun& run, 
             // 0 .. 15 find out how many they are, then either half of the warp adds every second one, in warp order
             const int li = lane & 15, half = lane >> 4, a2 = sh.t0 + li * rq + min(li, rr);
             const int more = __popc(__ballot_sync(0xFFFFFFFFu, lane > warp && half == 0 && a2 < row_end));
-            const float* const next = reinterpret_cast<const float*>(all + (warp + half) * 2) + li;
+            const float* const held = reinterpret_cast<const float*>(all + (warp + half) * 2) + li;
             float sum = half == 0 ? mine[pi].v[li] : 0.f;
             float pc[GEMV_WARPS / 2];
 #pragma unroll
             for (int d = 0; d < GEMV_WARPS / 2; d++) {
                 const int i = 2 * d + half;  // its piece: of warp + i
-                pc[d] = i >= 1 && i <= more ? next[d * 64] : 0.f;
+                pc[d] = i >= 1 && i <= more ? held[d * 64] : 0.f;
             }
 #pragma unroll
             for (int d = 0; d < GEMV_WARPS / 2; d++) sum += pc[d];

@@ -368,6 +368,10 @@ int wf_launch_count(int64_t ctx, int64_t* launches);
  * launches in any case, where the estimate says that they are quicker.) */
 int wf_plan_several_tokens(int qtype, int64_t rows, int64_t k, int cols, int x_is_f32, int sm_count, int* slices,
                            int* k_tiles_per_slice, int* team, int* uses_partial_sums, int64_t* smem_bytes);
+/* The same for the n launches of a program of 2..8 bf16 tokens, in their order (rows[i]: of all projections that share launch i).  They
+ * bring the sums of their slices together in clusters of at most eight CTAs, and a change from clusters to one slice costs the launch
+ * behind.  slices = 0 throughout: a launch fits neither way, and the program runs as one persistent kernel. */
+int wf_plan_program(int qtype, int n, const int64_t* rows, const int64_t* k, int tokens, int sm_count, int* slices, int* k_tiles_per_slice);
 
 #ifdef __cplusplus
 }

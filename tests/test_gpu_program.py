@@ -90,6 +90,30 @@ def test_program_every_quantization_type(oracle, qname, tokens):
         ctx.close()
 
 
+@pytest.mark.parametrize("qname,rows,k,tokens", [("Q8_0", 1024, 9216, 4), ("Q4_K", 1024, 9216, 4), ("Q4_0", 256, 16896, 2)])
+def test_program_of_long_rows_stays_launches(oracle, qname, rows, k, tokens):
+    """The cheapest cut of such a weight among all would have its sums go through memory; the program's launches take the cheapest in
+    clusters and do not give way to the persistent kernel."""
+    from warpforge_b200.backend import CudaContext
+    from warpforge_b200.decode import ProjectionStack, StackSpec
+
+    qt = Q.QuantizationType[qname]
+    oq = {"Q4_0": O.Q4_0, "Q8_0": O.Q8_0, "Q4_K": O.Q4_K}[qname]
+    ctx = CudaContext(0)
+    try:
+        st = ProjectionStack(ctx, StackSpec("long rows", qt, 3, (("wo", rows, k),), 0), tokens=tokens)
+        st.build_program()
+        before = ctx.launch_count()
+        st.run_program()
+        ctx.synchronize()
+        assert ctx.launch_count() - before == 3, "one launch per projection"
+        want = oracle.qlinear(oq, st.blocks["wo"], rows, k, Q.bf16_bits_to_float(st.x_host[k]), nthreads=oracle.max_threads())
+        assert np.max(np.abs(st.read_output("wo") - want)) <= 1e-3 * np.max(np.abs(want))
+        st.close()
+    finally:
+        ctx.close()
+
+
 def test_program_rejects_bad_arguments():
     import ctypes
 

@@ -65,3 +65,46 @@ def test_fewer_sms_still_cut_sensibly():
     for sms in (1, 8, 132):
         slices, kc, team, _, smem = _plan(2, 11008, 4096, 8, sms=sms)
         assert 1 <= slices <= sms and smem <= 200 * 1024
+
+
+def _program_plan(qt, shapes, tokens, sms=148):
+    n = len(shapes)
+    rows, ks = ((ctypes.c_int64 * n)(*v) for v in zip(*shapes))
+    s, kc = (ctypes.c_int * n)(), (ctypes.c_int * n)()
+    assert N.load().wf_plan_program(qt, n, rows, ks, tokens, sms, s, kc) == N.WF_OK
+    return list(s), list(kc)
+
+
+@pytest.mark.parametrize("qt", sorted(QTYPES))
+def test_a_program_of_like_launches_is_cut_as_a_call_is(qt):
+    """Wherever a call runs in clusters or in one slice, a program's launches do, and never with sums through memory, which they do not
+    know.  Nothing changes from launch to launch, so with fewer row-tiles than SMs it is the call's own cut; beyond, clusters are
+    charged and may give way to one slice."""
+    tk, _ = QTYPES[qt]
+    rows = [16, 256, 512, 1024, 2560, 4096, 12288, 22016, 44032]
+    ks = [512, 1024, 4096, 8448, 9216, 11008, 12288, 16384, 16896, 21248, 22016, 25600, 26880]
+    for r, k, tokens in itertools.product(rows, ks, (2, 3, 4, 5, 8)):
+        slices, kc = _program_plan(qt, [(r, k)] * 3, tokens)
+        call = _plan(qt, r, k, tokens)
+        if 1 <= call[0] <= 8:
+            assert slices == [call[0]] * 3 or (r >= 148 * 16 and slices == [1] * 3), (qt, r, k, tokens)
+        kt = -(-k // tk)
+        for s, c in zip(slices, kc):
+            assert s == 0 or (s <= 8 and (s - 1) * c < kt <= s * c)
+
+
+@pytest.mark.parametrize("qt,rows,k,tokens", [(8, 1024, 9216, 4), (14, 1024, 9216, 4), (8, 1024, 9216, 5), (2, 256, 16896, 2), (2, 512, 25600, 2), (8, 1024, 22016, 2)])
+@pytest.mark.parametrize("others", [[], [(4096, 4096), (22016, 4096)]])
+def test_a_change_that_costs_is_no_reason_to_give_the_launches_up(qt, rows, k, tokens, others):
+    slices, _ = _program_plan(qt, [(rows, k)] + others, tokens)
+    assert all(1 <= s <= 8 for s in slices)
+
+
+def test_a_program_that_no_launch_fits_and_bad_arguments():
+    assert _program_plan(2, [(4096, 4096), (64, 1 << 20)], 8)[0] == [0, 0]
+    one, k = (ctypes.c_int64 * 1)(4096), (ctypes.c_int64 * 1)(4096)
+    s, kc = (ctypes.c_int * 1)(), (ctypes.c_int * 1)()
+    lib = N.load()
+    assert lib.wf_plan_program(2, 1, one, k, 9, 148, s, kc) == N.WF_ERR_INVALID_ARGUMENT
+    assert lib.wf_plan_program(2, 0, one, k, 4, 148, s, kc) == N.WF_ERR_INVALID_ARGUMENT
+    assert lib.wf_plan_program(12, 1, one, k, 4, 148, s, kc) == N.WF_ERR_UNSUPPORTED_TYPE

@@ -490,6 +490,7 @@ static bool program_launches(Context* c, const std::vector<ProgOp>& ops, Program
     int made_for = -1, act_rows = 0;
     for (const ProgOp& op : ops) act_rows = std::max(act_rows, op.k);
     pr->launches.clear();
+    std::vector<GemvGroup> groups;
     for (int i = 0, head = 0; i < n_ops;) {
         if (ops[i].flags & OP_NEW_X) head = i;
         int j = i + 1;
@@ -524,10 +525,14 @@ static bool program_launches(Context* c, const std::vector<ProgOp>& ops, Program
         g.scratch = pr->d_scratch;
         g.timing = pr->d_timing;
         g.timing_at = 1 + 4 * i;
+        groups.push_back(g);
+        i = j;
+    }
+    if (!gemv_plan_groups(c, groups)) return false;
+    for (const GemvGroup& g : groups) {
         GemvPrepared ready;
         if (!gemv_prepare_group(c, g, &ready)) return false;
         pr->launches.push_back(ready);
-        i = j;
     }
     return true;
 }

@@ -547,6 +547,24 @@ int gemv_launch(Context* c, const GemvCall& call, cudaStream_t s) {
 
 // ---------------------------------------------------------------- a program's launches
 static cudaError_t launch_group(const GemvPrepared& g, int grid, cudaStream_t s);
+static std::array<GemvNPlan, 2> program_ways(const int* clusters, int qt, int64_t rt, int64_t kt, int tokens) {
+    std::array<GemvNPlan, 2> ways = {gemvn_plan(clusters, qt, rt, kt, tokens, false, GEMVN_ONE_SLICE), gemvn_plan(clusters, qt, rt, kt, tokens, false, GEMVN_CLUSTERS)};
+    if (rt >= clusters[1]) ways[1].ns += GEMVN_CLUSTER_LATE_NS;
+    return ways;
+}
+bool gemv_plan_groups(Context* c, std::vector<GemvGroup>& groups) {
+    if (groups.empty() || groups[0].m < 2) return true;
+    std::vector<std::array<GemvNPlan, 2>> ways;
+    for (const GemvGroup& g : groups) {
+        int64_t rt = 0;
+        for (int i = 0; i < g.n; i++) rt += g.w[i]->g.rt;
+        ways.push_back(program_ways(gemvn_clusters(c->sm_count), g.w[0]->g.qtype, rt, g.w[0]->g.kt, g.m));
+    }
+    std::vector<GemvNPlan> plans;
+    if (!gemvn_plan_program(ways, &plans)) return false;
+    for (size_t i = 0; i < groups.size(); i++) groups[i].plan = plans[i];
+    return true;
+}
 bool gemv_prepare_group(Context* c, const GemvGroup& g, GemvPrepared* out) {
     if (g.n < 1 || g.n > GEMV_GROUP || g.m < 1 || g.m > 8) return false;
     const Weight& first = *g.w[0];
@@ -610,7 +628,7 @@ bool gemv_prepare_group(Context* c, const GemvGroup& g, GemvPrepared* out) {
         return launch_group(*out, 0, nullptr) == cudaSuccess;
     }
     if (g.x_kind != XK_BF16) return false;
-    const GemvNPlan plan = gemvn_plan(gemvn_clusters(c->sm_count), qt, rt, kt, g.m, false, 1500.0);
+    const GemvNPlan& plan = g.plan;
     if (plan.slices < 1 || plan.part) return false;
     GemvNParams<GEMV_GROUP>& p = out->several;
     p = {};
@@ -709,5 +727,27 @@ extern "C" int wf_plan_several_tokens(int qtype, int64_t rows, int64_t k, int co
     *team = share >= 16 ? 16 : share >= 8 ? 8 : share;
     if (uses_partial_sums) *uses_partial_sums = p.slices > 1 || x_is_f32 ? 1 : 0;
     if (smem_bytes) *smem_bytes = p.slices > 0 ? (int64_t)gemvn_smem(qt, p.kc, cols, x_is_f32 != 0, p.slices, p.batch, nullptr, nullptr, nullptr) : 0;
+    return WF_OK;
+}
+
+// The cuts of a program's launches without a device (clusters as gemvn_clusters_estimate has them).
+extern "C" int wf_plan_program(int qtype, int n, const int64_t* rows, const int64_t* k, int tokens, int sm_count, int* slices, int* k_tiles_per_slice) {
+    using namespace wf;
+    const int qt = device_qtype(qtype);
+    if (qt != WF_QTYPE_Q4_0 && qt != WF_QTYPE_Q4_1 && qt != WF_QTYPE_Q8_0 && qt != WF_QTYPE_Q4_K) return WF_ERR_UNSUPPORTED_TYPE;
+    if (n < 1 || n > (1 << 20) || !rows || !k || tokens < 2 || tokens > 8 || sm_count < 1 || !slices || !k_tiles_per_slice) return WF_ERR_INVALID_ARGUMENT;
+    int clusters[GEMVN_MAX_CLUSTER + 1];
+    gemvn_clusters_estimate(sm_count, clusters);
+    std::vector<std::array<GemvNPlan, 2>> ways;
+    for (int i = 0; i < n; i++) {
+        if (rows[i] < 1 || k[i] < 1) return WF_ERR_INVALID_ARGUMENT;
+        ways.push_back(program_ways(clusters, qt, (rows[i] + 15) / 16, (k[i] + tile_k(qt) - 1) / tile_k(qt), tokens));
+    }
+    std::vector<GemvNPlan> plans;
+    if (!gemvn_plan_program(ways, &plans)) plans.assign(n, GemvNPlan{});
+    for (int i = 0; i < n; i++) {
+        slices[i] = plans[i].slices;
+        k_tiles_per_slice[i] = plans[i].kc;
+    }
     return WF_OK;
 }

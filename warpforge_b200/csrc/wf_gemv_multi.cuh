@@ -31,6 +31,8 @@
 // Replaces, for up to 32 tokens, the fp32 batch_matmul_f32 launch of
 // warpforge-backend-nvidia/src/main/java/io/surfworks/warpforge/backend/nvidia/ops/DotGeneralKernel.java:263-281.
 #pragma once
+#include <array>
+
 #include "wf_gemv_stream.cuh"
 
 namespace wf {
@@ -70,6 +72,13 @@ template <int GROUP> struct GemvNParams {
     int timing_at;               // -1, or this launch's first stamp in a program's row
 };
 
+struct GemvNPlan {
+    int slices = 0, kc = 0, batch = 0;  // slices == 0: no plan fits
+    int ctas = 0;                       // CTAs (per slice, where the slices form clusters)
+    bool part = false;                  // partial sums go through memory
+    double ns = 0;                      // the estimate
+};
+
 // A program's launch: weights of one type and K that read the same activations.
 struct GemvGroup {
     int n = 0, m = 1;
@@ -85,6 +94,7 @@ struct GemvGroup {
     uint2* scratch = nullptr;
     unsigned long long* timing = nullptr;
     int timing_at = -1;
+    GemvNPlan plan;  // several tokens: gemv_plan_groups
 };
 struct GemvPrepared {
     int qt = 0, m = 1, grid = 0;
@@ -92,6 +102,7 @@ struct GemvPrepared {
     Gemv1GroupParams one;
     GemvNParams<GEMV_GROUP> several;
 };
+bool gemv_plan_groups(Context* c, std::vector<GemvGroup>& groups);  // a program's launches in their order; false: beyond the kernels
 bool gemv_prepare_group(Context* c, const GemvGroup& g, GemvPrepared* out);  // false: beyond the kernels
 cudaError_t gemv_launch_group(const GemvPrepared& g, cudaStream_t s);
 
@@ -118,12 +129,6 @@ inline size_t gemvn_smem(int qt, int kc, int cols, bool x_f32, int slices, int b
 
 inline size_t gemvn_sum_bytes(int slices, int cols, int64_t rt) { return (size_t)slices * ((cols + 1) & ~1) * rt * 16 * 4; }
 
-struct GemvNPlan {
-    int slices = 0, kc = 0, batch = 0;  // slices == 0: no plan fits
-    int ctas = 0;                       // CTAs (per slice, where the slices form clusters)
-    bool part = false;                  // partial sums go through memory
-    double ns = 0;                      // the estimate
-};
 // clusters[S]: how many clusters of S CTAs the device holds at a time (S = 1: SMs).  The cheapest cut by an estimate in
 // nanoseconds: the busiest warp's tiles, the staging of the slice, and per batch the way of its sums to y.  The constants
 // are a fit to 78 measured weights from 128 x 8192 to 28014 x 2496 with 2 .. 32 columns, each at every S up to 8.  In calls of
@@ -131,11 +136,9 @@ struct GemvNPlan {
 // number of 7s.  On 130 other weights, up to 32000 x 8192, the choices are 1.4 % slower than the best S on average and 14 % at
 // worst (2.4 % and 32 % without that correction).  Memory is the way where eight slices do not fit (against a cluster of the
 // same S it measured 1 - 4 us more on small weights, up to twice the time on tall ones).
-// cluster_ns: what a launch of clusters costs its neighbours.  Its CTAs start 1 us after the end of the launch before it, plain ones
-// half a microsecond ahead of it, and the launch behind it starts late as well: a program takes clusters only where they gain
-// more than that (four tokens Q8_0, d 4096, three layers: 169 us with two slices for Wq, Wk, Wv and for Wgate, Wup, 166 with two
-// everywhere, 163 with none).
-inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt, int cols, bool x_f32, double cluster_ns = 0.0) {
+// ways: which cuts are considered.
+constexpr int GEMVN_ONE_SLICE = 1, GEMVN_CLUSTERS = 2, GEMVN_MEMORY = 4, GEMVN_ANY = 7;
+inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt, int cols, bool x_f32, int ways = GEMVN_ANY) {
     GemvNPlan best;
     const int ng = (cols + 7) / 8, tk = tile_k(qt), sms = clusters[1];
     const double per_group = 15.9 + (qt == WF_QTYPE_Q4_1 ? 3.3 : qt == WF_QTYPE_Q8_0 ? 16.3 : qt == WF_QTYPE_Q4_K ? 5.0 : 0.0);
@@ -147,6 +150,7 @@ inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt,
         if (kc == last_kc) continue;
         last_kc = kc;
         const bool part = slices > GEMVN_MAX_CLUSTER;
+        if (!(ways & (slices == 1 ? GEMVN_ONE_SLICE : part ? GEMVN_MEMORY : GEMVN_CLUSTERS))) continue;
         if (part && gemvn_sum_bytes(slices, cols, rt) > GEMVN_PART_BYTES) continue;
         const int64_t room = part ? sms / slices : clusters[slices];  // CTAs a slice gets, at least
         if (room < 1) continue;
@@ -163,7 +167,6 @@ inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt,
             else if (slices > 1) ns += 616.0 + slices * (6.1 + 32.1 * ((own * ng + GEMV_WARPS - 1) / GEMV_WARPS));
             if (x_f32 && !part) ns += 31.1 * slices * ((own * (cols / 3) * 16 + GEMV_CONSUMERS - 1) / GEMV_CONSUMERS);
         }
-        if (!part && slices > 1) ns += cluster_ns;
         if (!part && ns > 13000.0) ns *= slices == 3 || slices == 7 ? 1.1 : slices == 5 ? 1.05 : 1.0;
         if (best.slices == 0 || ns < best_ns) {
             best_ns = ns;
@@ -176,6 +179,44 @@ inline GemvNPlan gemvn_plan(const int* clusters, int qt, int64_t rt, int64_t kt,
         }
     }
     return best;
+}
+
+// The cuts of a program's launches, which follow each other again and again: ways[i] = the cheapest cut of launch i into one slice and
+// into clusters (sums through memory are not for them; slices == 0: does not fit).  The estimates come from calls of one kind in a
+// row.  In a program a launch of one slice takes each SM half a microsecond before the launch in front of it ends, but behind
+// clusters, which need several SMs at once, it starts 1 us after that end, as clusters do themselves.  So a change from clusters to
+// one slice is charged, and clusters where one slice has work for every SM; what is least is the sum over the circle of
+// launches.  Measured: 204 programs (Q4_0, Q4_1, Q8_0, Q4_K; 2 - 8 tokens; decoder layers of d 1024 to 4096) at nine settings of
+// the two charges, and 14 programs of like launches.  Without them layers take 1.9 % more than with the best setting of each, up to
+// 21 % ([2816 x 7680] Q4_K); 1.5 us on every launch of clusters and nothing else: 0.2 %, up to 4 %, but programs of like launches
+// with few rows 9 %, up to 33 % ([1024 x 9216] Q4_K, four tokens).
+constexpr double GEMVN_CHANGE_NS = 700.0, GEMVN_CLUSTER_LATE_NS = 800.0;
+inline bool gemvn_plan_program(const std::vector<std::array<GemvNPlan, 2>>& ways, std::vector<GemvNPlan>* out) {
+    const size_t n = ways.size();
+    constexpr double NEVER = 1e30;
+    const auto cost = [&](size_t i, int w) { return ways[i][w].slices > 0 ? ways[i][w].ns : NEVER; };
+    const auto change = [](int from, int to) { return from == 1 && to == 0 ? GEMVN_CHANGE_NS : 0.0; };
+    double best = NEVER;
+    for (int first = 0; first < 2; first++) {  // the first launch's way, which the last one's successor has as well
+        std::vector<std::array<int, 2>> from(n);
+        double sum[2] = {first == 0 ? cost(0, 0) : NEVER, first == 1 ? cost(0, 1) : NEVER};
+        for (size_t i = 1; i < n; i++) {
+            double next[2];
+            for (int w = 0; w < 2; w++) {
+                from[i][w] = sum[1] + change(1, w) < sum[0] + change(0, w);
+                next[w] = sum[from[i][w]] + change(from[i][w], w) + cost(i, w);
+            }
+            sum[0] = next[0];
+            sum[1] = next[1];
+        }
+        int last = sum[1] + change(1, first) < sum[0] + change(0, first);
+        const double total = sum[last] + change(last, first);
+        if (total >= best) continue;
+        best = total;
+        out->assign(n, GemvNPlan{});
+        for (size_t i = n; i-- > 0; last = from[i][last]) (*out)[i] = ways[i][last];
+    }
+    return best < NEVER;
 }
 
 // Stage this CTA's k-slice [k_lo, k_lo + kslice) of every token: bf16 rows of kslice elements (zero beyond k) and,

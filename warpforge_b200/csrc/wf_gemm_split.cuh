@@ -42,10 +42,6 @@ inline __host__ __device__ int split_exchange_bytes(int bm, int ranks) { return 
 // smem: [0, 1024) barriers, tmem slot | stages x (A | B), 1024-byte aligned | exchange buffer
 template <int QT, int PIECES, int PLANES>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap) {
-    // The next call's conversion, 32 registers a thread, fits beside a CTA of 128 and waits there; and the next GEMM takes the SM as
-    // soon as this one leaves it (eight calls of [5003 x 2784], 77 tokens: 122 -> 108.5 us; fp32 tokens, whose conversion does not
-    // fit beside, would take 93 -> 98).
-    if (PIECES == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr int ACCS = PIECES;
     constexpr int FLUSH = PIECES == 1 ? 1 << 30 : SPLIT_FLUSH;
     constexpr int KBW = Tile<QT>::K / GEMM_BK;  // units per weight k-tile
@@ -101,10 +97,20 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
     if (warp == 0) {
         // ------------------------------------------------ TMA producer (activations)
         if (lane == 0) {
+            // The next call's conversion, 32 registers a thread, fits beside a CTA of 128 and waits there, and the next GEMM takes each
+            // SM as it becomes free (a call of [5003 x 2784], 77 tokens, Q4_0: 12.7 -> 11.6 us; 64 tokens of [4096 x 4096], where shared
+            // memory has no room for it beside, 12.7 -> 11.3 all the same).  Placed when the CTA begins its last tile: a conversion
+            // that waits beside longer delays clusters of several tiles ([11008 x 4096], 128 tokens, two tiles each: 27.6 us
+            // without, 28.9 placed at the start, 27.8 here).  fp32 tokens, whose conversion does not fit: 93 -> 98.
+            auto last_tile = [&](int tile) {
+                if (PIECES == 1 && tile + clusters >= tiles) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+            };
+            last_tile(cluster);
             asm volatile("griddepcontrol.wait;" ::: "memory");  // the fp16 activations
             StageCursor at;
             for (int tile = cluster; tile < tiles && !*abort_flag; tile += clusters) {
                 const int tok0 = (tile % p.m_tiles) * p.bm;
+                if (tile != cluster) last_tile(tile);
                 for (int st = 2 * kb0; st < 2 * kb1; st++, at.advance(stages)) {
                     const int s = at.s;
                     if (!g_mbar_wait(&s_empty[s], at.phase ^ 1)) { fail(); break; }

@@ -46,6 +46,21 @@ struct StatusBlock {
 };
 constexpr int STATUS_BITS = 4;
 #ifdef __CUDACC__
+// Behind griddepcontrol.wait, what earlier kernels of the stream may still have been writing when this one was placed is read by
+// plain loads through pointers that are not const __restrict__, or by these (of data that is read once): the non-coherent
+// path, __ldg and what the compiler makes of const __restrict__, wants data that nobody writes while the kernel lives, and may be
+// moved above the wait.  Volatile statements keep their order, plain loads do not pass a statement that clobbers memory.
+__device__ __forceinline__ float ld_once(const float* p) {
+    float v;
+    asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_once(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
 __device__ __forceinline__ void report_status(int* status, int bit) {
     StatusBlock* b = reinterpret_cast<StatusBlock*>(status);
     atomicOr(&b->bits, bit);

@@ -214,7 +214,7 @@ constexpr int CONVERT_THREADS = 256;
 constexpr int CONVERT_KEEP_BESIDE = 2;  // rows of 4096: what 32 registers hold
 constexpr int CONVERT_KEEP_ALONE = 4;   // rows of 8192
 template <int PLANES, int KEEP>
-__global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 && KEEP == CONVERT_KEEP_BESIDE ? 8 : 5) convert_rows_kernel(const void* __restrict__ x, __half* __restrict__ x16, float* __restrict__ unscale,
+__global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 && KEEP == CONVERT_KEEP_BESIDE ? 8 : 5) convert_rows_kernel(const void* x, __half* __restrict__ x16, float* __restrict__ unscale,
                                                                        int m, int k) {
     __shared__ int s_max[CONVERT_THREADS / 32];
     // Launched with programmatic stream serialization itself: its CTAs may be placed while the previous kernel of the
@@ -232,8 +232,8 @@ __global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 && KEEP == CONVER
     const uint4* src = static_cast<const uint4*>(x) + (size_t)row * groups * (PLANES == 1 ? 1 : 2);
     auto load = [&](int i) {
         G g;
-        g.a = __ldg(src + (PLANES == 1 ? i : 2 * i));
-        g.b = PLANES == 1 ? g.a : __ldg(src + 2 * i + 1);
+        g.a = src[PLANES == 1 ? i : 2 * i];
+        g.b = PLANES == 1 ? g.a : src[2 * i + 1];
         return g;
     };
     auto emax_of = [](const G& g) {  // largest biased exponent; Inf and NaN do not drive the scale
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 && KEEP == CONVER
 // ---------------------------------------------------------------- epilogue pieces (one lane = one weight row)
 // r[j] = accumulator of (token m0 + j, weight row n).  Rows of y are ldy floats apart; a warp writes 32
 // consecutive floats of one token row per store.  m0 is a multiple of 32, so the row scales load as float4.
-__device__ __forceinline__ void store_chunk(float* __restrict__ y, int64_t ldy, int64_t col0, const float* __restrict__ unscale,
+__device__ __forceinline__ void store_chunk(float* __restrict__ y, int64_t ldy, int64_t col0, const float* unscale,
                                             const uint32_t (&r)[32], int m0, int m, int n, int rows) {
     if (n >= rows || m0 >= m) return;
     float* yp = y + (int64_t)m0 * ldy + col0 + n;
@@ -326,7 +326,7 @@ __device__ __forceinline__ void store_chunk(float* __restrict__ y, int64_t ldy, 
         float sc[32];
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(unscale + m0) + i);
+            const float4 v = reinterpret_cast<const float4*>(unscale + m0)[i];
             sc[4 * i] = v.x, sc[4 * i + 1] = v.y, sc[4 * i + 2] = v.z, sc[4 * i + 3] = v.w;
         }
 #pragma unroll
@@ -334,7 +334,7 @@ __device__ __forceinline__ void store_chunk(float* __restrict__ y, int64_t ldy, 
     } else {
 #pragma unroll
         for (int j = 0; j < 32; j++)
-            if (m0 + j < m) yp[(int64_t)j * ldy] = __uint_as_float(r[j]) * __ldg(unscale + m0 + j);
+            if (m0 + j < m) yp[(int64_t)j * ldy] = __uint_as_float(r[j]) * unscale[m0 + j];
     }
 }
 // A stream-K piece holds four tokens of a weight row in 16 bytes, [tokens / 4][128 rows]: a warp moves 512 contiguous

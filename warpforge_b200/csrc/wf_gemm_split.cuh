@@ -180,9 +180,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_split_kernel(const GemmP
             const int first = tok0 + rank * per * 4, left = min(mine * 4, p.m - first);
             if (S > 1) {
 #pragma unroll
-                for (int j = 0; j < 2; j++) scale[32 * j + lane] = 32 * j + lane < left ? __ldg(p.row_unscale + first + 32 * j + lane) : 0.f;
+                for (int j = 0; j < 2; j++) scale[32 * j + lane] = 32 * j + lane < left ? p.row_unscale[first + 32 * j + lane] : 0.f;
                 if (threadIdx.x == 128 && mine > 0) g_mbar_expect_tx(ex_full, (uint32_t)(S * mine * GEMM_BN * 16));
                 if (round > 0 && !g_mbar_wait(ex_empty, (round - 1) & 1)) { if (lane == 0) fail(); break; }
+            } else if (8 * lane < p.bm && tok0 + 8 * lane < p.m) {  // brought into the L1 while the tile is multiplied
+                asm volatile("" ::"f"(p.row_unscale[tok0 + 8 * lane]));
             }
             uint32_t to = 0, in = 0;  // rank and place there of the next group of four tokens
             uint32_t to_addr = map_to_rank(ex_addr, 0), to_bar = map_to_rank(bar_addr, 0);

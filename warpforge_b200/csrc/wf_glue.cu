@@ -132,12 +132,12 @@ template <int T, int V> struct Row {
 #pragma unroll
             for (int j = 0; j < V; j++) {
                 const int i = at(j, 0);
-                const float4 v = i < n ? __ldcs(reinterpret_cast<const float4*>(x + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 v = i < n ? ld_once(reinterpret_cast<const float4*>(x + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 r[4 * j] = v.x, r[4 * j + 1] = v.y, r[4 * j + 2] = v.z, r[4 * j + 3] = v.w;
             }
         } else {
 #pragma unroll
-            for (int j = 0; j < 4 * V; j++) r[j] = j * T + t < n ? __ldcs(x + j * T + t) : 0.f;
+            for (int j = 0; j < 4 * V; j++) r[j] = j * T + t < n ? ld_once(x + j * T + t) : 0.f;
         }
     }
     // the sum of f(x[i]) over the row: fp32 over eight elements of a thread (32 where the row is walked in global
@@ -192,25 +192,43 @@ template <int T, int V> struct Row {
                 if (wide) {
                     const int i = at(j, 0);
                     if (i >= n) continue;
-                    const float4 p = a ? __ldg(reinterpret_cast<const float4*>(a + i)) : make_float4(1.f, 1.f, 1.f, 1.f);
-                    const float4 q = b ? __ldg(reinterpret_cast<const float4*>(b + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 p = a ? *reinterpret_cast<const float4*>(a + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+                    const float4 q = b ? *reinterpret_cast<const float4*>(b + i) : make_float4(0.f, 0.f, 0.f, 0.f);
                     __stcs(reinterpret_cast<float4*>(y + i), make_float4(g(r[4 * j], p.x, q.x), g(r[4 * j + 1], p.y, q.y), g(r[4 * j + 2], p.z, q.z), g(r[4 * j + 3], p.w, q.w)));
                 } else {
+                    float p[4], q[4];  // requested before the first of them is stored
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
                         const int i = at(j, e);
-                        if (i < n) __stcs(y + i, g(r[4 * j + e], a ? __ldg(a + i) : 1.f, b ? __ldg(b + i) : 0.f));
+                        p[e] = a && i < n ? a[i] : 1.f;
+                        q[e] = b && i < n ? b[i] : 0.f;
                     }
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+                        if (at(j, e) < n) __stcs(y + at(j, e), g(r[4 * j + e], p[e], q[e]));
                 }
             }
         } else {
-            for (int i = t; i < n; i += T) y[i] = g(x[i], a ? __ldg(a + i) : 1.f, b ? __ldg(b + i) : 0.f);
+            for (int i0 = t; i0 < n; i0 += 4 * T) {
+                float v[4], p[4], q[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int i = i0 + e * T;
+                    v[e] = i < n ? x[i] : 0.f;
+                    p[e] = a && i < n ? a[i] : 1.f;
+                    q[e] = b && i < n ? b[i] : 0.f;
+                }
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    if (i0 + e * T < n) y[i0 + e * T] = g(v[e], p[e], q[e]);
+            }
         }
     }
 };
 
 // Every kernel here is launched with programmatic stream serialization: it may be placed while the kernel before it drains, lets
-// the one behind it be placed in turn, and touches memory only when the one before it has completed.
+// the one behind it be placed in turn, and touches memory only when the one before it has completed.  What it reads may have been
+// written meanwhile: no __ldg and no const __restrict__ pointers.
 __device__ __forceinline__ void wait_for_previous() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -224,7 +242,7 @@ template <int T> __device__ __forceinline__ int64_t row_of_group(int64_t rows) {
 
 // CustomCallKernel.java:368-412: rms = (float) sqrt(sumSq / n + eps); y = x * (1 / rms) [* gamma]
 template <int T, int V>
-__global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
+__global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) rms_norm_kernel(const float* x, const float* gamma,
                                                                          float* __restrict__ y, int64_t rows, int n, float eps) {
     __shared__ double red[T / 32];
     wait_for_previous();
@@ -242,8 +260,8 @@ __global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) rms_norm_kernel(const f
 
 // CustomCallKernel.java:109-171: mean, then the variance of (x - mean), invStd = 1 / (float) sqrt(var + eps)
 template <int T, int V>
-__global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) layer_norm_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
-                                                                           const float* __restrict__ beta, float* __restrict__ y,
+__global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) layer_norm_kernel(const float* x, const float* gamma,
+                                                                           const float* beta, float* __restrict__ y,
                                                                            int64_t rows, int n, float eps) {
     __shared__ double red[T / 32], red2[T / 32];
     wait_for_previous();
@@ -269,7 +287,7 @@ __global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) layer_norm_kernel(const
 
 // CustomCallKernel.java:173-224, over the last dimension: (float) exp(x - max) / sum
 template <int T, int V, bool EXACT>
-__global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int64_t rows, int n) {
+__global__ void __launch_bounds__(T == 32 ? ROW_CTA : T) softmax_kernel(const float* x, float* __restrict__ y, int64_t rows, int n) {
     __shared__ double red[T / 32];
     __shared__ float redf[T / 32];
     __shared__ double tab[32];
@@ -346,7 +364,7 @@ template <int OP, bool EXACT> struct ElShape {
     static constexpr int UNROLL = UNARY || EXACT ? 2 : 4, CTAS = UNARY || EXACT ? 6 : OP == EL_SWIGLU ? 3 : 4;  // what the registers allow
 };
 template <int OP, bool EXACT>
-__global__ void __launch_bounds__(256, (ElShape<OP, EXACT>::CTAS)) elementwise_kernel(const float* __restrict__ a, const float* __restrict__ b,
+__global__ void __launch_bounds__(256, (ElShape<OP, EXACT>::CTAS)) elementwise_kernel(const float* a, const float* b,
                                                                                       float* __restrict__ y, int64_t n, int vec) {
     constexpr bool UNARY = ElShape<OP, EXACT>::UNARY;
     constexpr int EL_UNROLL = ElShape<OP, EXACT>::UNROLL;
@@ -362,8 +380,8 @@ __global__ void __launch_bounds__(256, (ElShape<OP, EXACT>::CTAS)) elementwise_k
             for (int j = 0; j < EL_UNROLL; j++) {
                 const int64_t i = i0 + j * step;
                 if (i < n4) {
-                    u[j] = __ldcs(reinterpret_cast<const float4*>(a) + i);
-                    if (!UNARY) v[j] = __ldcs(reinterpret_cast<const float4*>(b) + i);
+                    u[j] = ld_once(reinterpret_cast<const float4*>(a) + i);
+                    if (!UNARY) v[j] = ld_once(reinterpret_cast<const float4*>(b) + i);
                 }
             }
 #pragma unroll
@@ -373,9 +391,9 @@ __global__ void __launch_bounds__(256, (ElShape<OP, EXACT>::CTAS)) elementwise_k
                 if (i < n4) __stcs(reinterpret_cast<float4*>(y) + i, make_float4(el<OP, EXACT>(p.x, q.x, tab), el<OP, EXACT>(p.y, q.y, tab), el<OP, EXACT>(p.z, q.z, tab), el<OP, EXACT>(p.w, q.w, tab)));
             }
         }
-        for (int64_t i = n4 * 4 + tid; i < n; i += step) y[i] = el<OP, EXACT>(a[i], UNARY ? 0.f : b[i], tab);
+        for (int64_t i = n4 * 4 + tid; i < n; i += step) y[i] = el<OP, EXACT>(ld_once(a + i), UNARY ? 0.f : ld_once(b + i), tab);
     } else {
-        for (int64_t i = tid; i < n; i += step) y[i] = el<OP, EXACT>(a[i], UNARY ? 0.f : b[i], tab);
+        for (int64_t i = tid; i < n; i += step) y[i] = el<OP, EXACT>(ld_once(a + i), UNARY ? 0.f : ld_once(b + i), tab);
     }
 }
 
@@ -434,7 +452,7 @@ __global__ void __launch_bounds__(256) dot_f32_kernel(const float* __restrict__ 
 
 // CustomCallKernel.java:282-318: row `index` of the table per looked-up position.  The CPU throws on an
 // index outside the table; here such a row is filled with zeros and the status word says so.
-__global__ void __launch_bounds__(256) embedding_kernel(const int64_t* __restrict__ indices, const float* __restrict__ table,
+__global__ void __launch_bounds__(256) embedding_kernel(const int64_t* indices, const float* table,
                                                         float* __restrict__ y, int64_t count, int64_t vocab, int dim, int vec,
                                                         int* status) {
     wait_for_previous();
@@ -444,22 +462,27 @@ __global__ void __launch_bounds__(256) embedding_kernel(const int64_t* __restric
         if (!ok && threadIdx.x == 0) report_status(status, STATUS_BAD_INDEX);
         const float* src = table + (size_t)(ok ? idx : 0) * dim;
         float* dst = y + (size_t)r * dim;
+        if (!ok) {
+            for (int i = threadIdx.x; i < dim; i += blockDim.x) dst[i] = 0.f;
+            continue;
+        }
         if (vec) {
-            for (int i0 = threadIdx.x; i0 < dim / 4; i0 += 4 * blockDim.x) {  // four pieces of the row in flight per thread
+#pragma unroll 1
+            for (int i0 = threadIdx.x; i0 < dim / 4; i0 += 4 * 256) {  // four pieces of the row in flight per thread
                 float4 v[4];
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    const int i = i0 + j * blockDim.x;
-                    v[j] = ok && i < dim / 4 ? __ldg(reinterpret_cast<const float4*>(src) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const int i = i0 + j * 256;
+                    if (i < dim / 4) v[j] = reinterpret_cast<const float4*>(src)[i];
                 }
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    const int i = i0 + j * blockDim.x;
+                    const int i = i0 + j * 256;
                     if (i < dim / 4) reinterpret_cast<float4*>(dst)[i] = v[j];
                 }
             }
         } else {
-            for (int i = threadIdx.x; i < dim; i += blockDim.x) dst[i] = ok ? src[i] : 0.f;
+            for (int i = threadIdx.x; i < dim; i += blockDim.x) dst[i] = src[i];
         }
     }
 }

@@ -58,6 +58,29 @@ def test_bf16_tokens(backend, oracle, name, rows, k, m):
     assert np.linalg.norm(d) <= 3e-4 * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("name,f32", [("q4_0", False), ("q8_0", False), ("q4_k", False), ("q4_1", True), ("q8_0", True), ("q4_k", True)])
+@pytest.mark.parametrize("rows,k,tokens", [
+    (20600, 128, (40,)),  # more tiles than clusters of one unit each: the sets of dequantizing warps take tiles by turns
+    (300, 1184, (16, 33, 48, 65, 80, 95)),  # every length of the ring of weights in TMEM; a last tile of the weight that is partly empty
+    (2600, 2720, (64, 96, 113)),
+])
+def test_rings_of_weights_in_tmem(backend, oracle, name, f32, rows, k, tokens):
+    from warpforge_b200.backend import Tensor
+
+    if name == "q4_k":
+        k = max(256, k // 256 * 256)
+    for m in tokens:
+        if f32:
+            x = Q.synth_activation_f32(m, k, rows + m)
+            t = Tensor.from_float_array(x)
+        else:
+            bits = Q.synth_activation_bf16(m, k, rows + m)
+            x, t = Q.bf16_bits_to_float(bits), Tensor.from_bf16_bits(bits)
+        got, want = _run(backend, oracle, name, rows, k, x, t)
+        assert np.linalg.norm(got - want) <= (3.8e-6 if f32 else 3e-4) * np.linalg.norm(want)
+        assert np.max(np.abs(got - want)) <= (3.8e-5 if f32 else 1e-3) * np.max(np.abs(want))  # f32: ten times the 2-norm's bar
+
+
 @pytest.mark.parametrize("name", sorted(QT))
 @pytest.mark.parametrize("rows,k,m", [(100, 96, 11), (257, 2080, 24), (1000, 4000, 96), (640, 1024, 97), (2100, 544, 200)])
 def test_fp32_tokens(backend, oracle, name, rows, k, m):

@@ -53,10 +53,10 @@ struct GemmDevice {
     int pairs = 0;
     int clusters[SPLIT_MAX_RANKS + 1] = {};
 };
-template <class Kernel> static cudaError_t max_clusters(Kernel kernel, int size, int* out) {
+template <class Kernel> static cudaError_t max_clusters(Kernel kernel, int threads, int size, int* out) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)size);
-    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = GEMM_SMEM_LIMIT;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -76,9 +76,9 @@ template <int QT> static cudaError_t gemm_prepare(int device, GemmDevice** out) 
     cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel<QT, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_split_kernel<QT, 2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
-    if (e == cudaSuccess) e = max_clusters(gemm_pair_kernel<QT>, 2, &d.pairs);
+    if (e == cudaSuccess) e = max_clusters(gemm_pair_kernel<QT>, GEMM_THREADS, 2, &d.pairs);
     for (int n = 1; n <= SPLIT_MAX_RANKS && e == cudaSuccess; n++) {
-        e = max_clusters(gemm_split_kernel<QT, 1, 1>, n, &d.clusters[n]);
+        e = max_clusters(gemm_split_kernel<QT, 1, 1>, SPLIT_THREADS, n, &d.clusters[n]);
         // one fewer than the device says: a cluster that does not find its place in the first wave costs a whole round
         if (n >= 3 && d.clusters[n] > 16) d.clusters[n]--;
     }
@@ -87,13 +87,13 @@ template <int QT> static cudaError_t gemm_prepare(int device, GemmDevice** out) 
 }
 
 template <class Kernel>
-static cudaError_t gemm_launch_one(Kernel kernel, const GemmParams& p, const CUtensorMap& map, int grid, int cluster, size_t smem, cudaStream_t s) {
+static cudaError_t gemm_launch_one(Kernel kernel, const GemmParams& p, const CUtensorMap& map, int threads, int grid, int cluster, size_t smem, cudaStream_t s) {
     // Programmatic stream serialization: this kernel may start while the conversion of the activations (the previous launch
     // of the stream) is still running; what reads the conversion's output waits with griddepcontrol.wait, the rest
     // (barrier set-up, TMEM allocation, the first weight loads and conversions) runs under it.
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
@@ -197,7 +197,7 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     const Weight& w = *call.w;
     const int qt = w.g.qtype;
     const bool f32 = call.x_dtype == WF_DTYPE_F32;
-    const int planes = f32 ? 3 : 1, pieces = f32 ? 2 : 1;
+    const int planes = f32 ? 3 : 1;
     GemmDevice* dev = nullptr;
     {
         const cudaError_t e = qt == WF_QTYPE_Q4_0   ? gemm_prepare<WF_QTYPE_Q4_0>(c->device, &dev)
@@ -266,7 +266,11 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     } else {
         cluster = p.ranks;
         grid = clusters * cluster;
-        stage_bytes = (size_t)split_stage_bytes(pieces, planes, p.bm);
+        p.unit_q = p.k_blocks / p.ranks;
+        p.unit_r = p.k_blocks % p.ranks;
+        p.tile_q = p.n_tiles * p.m_tiles / clusters;
+        p.tile_r = p.n_tiles * p.m_tiles % clusters;
+        stage_bytes = (size_t)split_stage_bytes(planes, p.bm);
         exchange = (size_t)split_exchange_bytes(p.bm, cluster);
     }
     p.stages = (int)std::min<size_t>((GEMM_SMEM_LIMIT - 1024 - exchange) / stage_bytes, 8);
@@ -308,19 +312,20 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        const bool alone = pair && w.g.k > CONVERT_KEEP_BESIDE * CONVERT_THREADS * 8;
-        const auto convert = f32     ? convert_rows_kernel<3, 2>
-                             : alone ? convert_rows_kernel<1, CONVERT_KEEP_ALONE>
-                                     : convert_rows_kernel<1, CONVERT_KEEP_BESIDE>;
+        const bool alone = pair && w.g.k > CONVERT_KEEP_SHORT * CONVERT_THREADS * 8;
+        const auto convert = f32     ? convert_rows_kernel<3, 2, TMEM_ORDER>
+                             : !pair ? convert_rows_kernel<1, CONVERT_KEEP_SHORT, TMEM_ORDER>
+                             : alone ? convert_rows_kernel<1, CONVERT_KEEP_LONG, SMEM_ORDER>
+                                     : convert_rows_kernel<1, CONVERT_KEEP_SHORT, SMEM_ORDER>;
         WF_CUDA(c, cudaLaunchKernelEx(&cfg, convert, call.d_x, x16, unscale, (int)call.m, (int)w.g.k));
     }
     c->launches++;
     const size_t smem = 1024 + (size_t)p.stages * stage_bytes + exchange;
     auto launch = [&](auto tag) {
         constexpr int QT = decltype(tag)::value;
-        return pair  ? gemm_launch_one(gemm_pair_kernel<QT>, p, map, grid, cluster, smem, s)
-               : f32 ? gemm_launch_one(gemm_split_kernel<QT, 2, 3>, p, map, grid, cluster, smem, s)
-                     : gemm_launch_one(gemm_split_kernel<QT, 1, 1>, p, map, grid, cluster, smem, s);
+        return pair  ? gemm_launch_one(gemm_pair_kernel<QT>, p, map, GEMM_THREADS, grid, cluster, smem, s)
+               : f32 ? gemm_launch_one(gemm_split_kernel<QT, 2, 3>, p, map, SPLIT_THREADS, grid, cluster, smem, s)
+                     : gemm_launch_one(gemm_split_kernel<QT, 1, 1>, p, map, SPLIT_THREADS, grid, cluster, smem, s);
     };
     const cudaError_t e = qt == WF_QTYPE_Q4_0   ? launch(std::integral_constant<int, WF_QTYPE_Q4_0>{})
                           : qt == WF_QTYPE_Q4_1 ? launch(std::integral_constant<int, WF_QTYPE_Q4_1>{})

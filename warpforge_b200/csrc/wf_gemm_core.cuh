@@ -12,7 +12,7 @@ namespace wf {
 
 constexpr int GEMM_BN = 128;             // weight rows per CTA and tile (UMMA M per CTA)
 constexpr int GEMM_BK = 128;             // k per unit of the work split: two stages of 64 k
-constexpr int GEMM_DEQUANT_WARPS = 8;    // a 16-row weight tile each (sixteen of eight rows: 3 - 14 % slower, 92 registers a thread)
+constexpr int GEMM_DEQUANT_WARPS = 8;    // a set: a 16-row weight tile each (A in shared memory, sixteen of eight rows: 3 - 14 % slower)
 constexpr int GEMM_THREADS = (6 + GEMM_DEQUANT_WARPS) * 32;  // TMA, MMA, 4 epilogue, dequant warps
 constexpr int GEMM_WAIT_SPINS = 1 << 20;    // of an mbarrier wait, which suspends the thread for microseconds per try
 constexpr int GEMM_POLL_SPINS = 1 << 22;    // of a poll of global memory
@@ -34,7 +34,8 @@ struct GemmParams {
     int ranks;           // split kernel: CTAs of a cluster, which share a tile's K
     uint32_t idesc;
     // pair kernel, stream-K: the (tile, k-block) units form one sequence, pair b owns units [b*q + min(b,r), ...)
-    int unit_q, unit_r;
+    // split kernel: rank b owns those k-blocks of every tile, cluster c takes tile_q tiles, one more below tile_r
+    int unit_q, unit_r, tile_q, tile_r;
     float* partial;        // [ctas][GEMM_PIECE_TOKENS][128] fp32: a CTA's piece of a tile that begins in an earlier pair
     unsigned int* ready;   // [ctas][4] generation whose piece (per 32-row quarter) is complete in `partial`
     unsigned int* gen;     // [0] generations completed so far, [1] CTAs that have left the current launch: the kernel
@@ -78,6 +79,19 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
+}
+__device__ __forceinline__ uint32_t cluster_id() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_count() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%nclusterid.x;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
@@ -128,6 +142,33 @@ template <int GROUP> __device__ __forceinline__ void tc_mma_span(uint32_t d_tmem
     else WF_MMA_SPAN("2");
 #undef WF_MMA_SPAN
 }
+// The same with A in TMEM (cta_group::1): 16 k are eight columns there.  The tensor core then reads only B from shared memory, and keeps
+// its pace for any N from 32 on (cycles per MMA of 128 rows x 16 k, A in shared memory / in TMEM, measured: N = 16: 39 / 11, 48: 44 / 24,
+// 96: 56 / 48, 128: 64 / 64).
+__device__ __forceinline__ void tc_mma_span_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t issue) {
+    asm volatile(
+        "{\n\t.reg .pred p, e, t;\n\t.reg .b32 a1, a2, a3;\n\t.reg .b64 b1, b2, b3;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+        "add.s32 a1, %1, 8;\n\tadd.s32 a2, %1, 16;\n\tadd.s32 a3, %1, 24;\n\t"
+        "add.s64 b1, %2, 2;\n\tadd.s64 b2, %2, 4;\n\tadd.s64 b3, %2, 6;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, t;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, t;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue)
+        : "memory");
+}
+// 16 rows x 64 k of fp16 into 16 lanes x 32 columns of TMEM.  A lane holds rows g = lane / 4 (r0) and g + 8 (r1), of either 32-k block the
+// eight elements 8 q .. 8 q + 7 (q = lane % 4): of each 16-byte piece the first half goes into the columns of one MMA, the
+// second into those of the next (order of k: stage_piece).
+__device__ __forceinline__ void tmem_st_span(uint32_t taddr, const uint4& r0b0, const uint4& r0b1, const uint4& r1b0, const uint4& r1b1) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(r0b0.x), "r"(r0b0.y), "r"(r1b0.x), "r"(r1b0.y), "r"(r0b0.z), "r"(r0b0.w), "r"(r1b0.z), "r"(r1b0.w),
+        "r"(r0b1.x), "r"(r0b1.y), "r"(r1b1.x), "r"(r1b1.y), "r"(r0b1.z), "r"(r0b1.w), "r"(r1b1.z), "r"(r1b1.w)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t e;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
@@ -177,15 +218,24 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// The same of one accumulator, or the sum of two that lie bm columns apart.
-template <int ACCS> __device__ __forceinline__ void tmem_ld_accs(uint32_t taddr, int bm, uint32_t (&r)[32]) {
-    tmem_ld32(taddr, r);
-    if (ACCS == 2) {
-        uint32_t e[32];
-        tmem_ld32(taddr + (uint32_t)bm, e);
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// N columns of one accumulator (32), or of the sum of two that lie bm columns apart (16).
+__device__ __forceinline__ void tmem_ld_accs(uint32_t taddr, int, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
+__device__ __forceinline__ void tmem_ld_accs(uint32_t taddr, int bm, uint32_t (&r)[16]) {
+    uint32_t e[16];
+    tmem_ld16(taddr, r);
+    tmem_ld16(taddr + (uint32_t)bm, e);
 #pragma unroll
-        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(e[j]));
-    }
+    for (int j = 0; j < 16; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(e[j]));
 }
 
 // ---------------------------------------------------------------- the order of k inside a stage
@@ -194,100 +244,50 @@ template <int ACCS> __device__ __forceinline__ void tmem_ld_accs(uint32_t taddr,
 // store is served eight lanes at a time, two neighbouring rows x four groups of one block, which under the 128-byte
 // swizzle meet eight different chunks this way.  With the blocks one after the other they met four, a two-way conflict.
 __host__ __device__ inline int stage_chunk(int j, int q) { return 2 * q + j; }
+// Where the weights go to TMEM (tmem_st_span), elements 8 q + 4 h .. + 3 of block j are the q-th quarter of the 16 k of MMA 2 j + h: as
+// 8-byte pieces of a stage row, piece 4 (2 j + h) + q.
+__host__ __device__ inline int stage_piece(int j, int q, int h) { return 4 * (2 * j + h) + q; }
+enum RowOrder { SMEM_ORDER, TMEM_ORDER };
 
 // ---------------------------------------------------------------- activations to fp16
-// x16[row] = fp16(x[row] * 2^s) with s chosen so that the row's largest magnitude lands in [2^14, 2^15), or 126 where that
-// would take more (magnitudes below 2^-112, down to subnormal ones); unscale[row] = 2^-s.
+// x16 = fp16(x * 2^s) with s chosen so that the largest magnitude of the row lands in [2^14, 2^15), or 126
+// where that would take more (magnitudes below 2^-112, down to subnormal ones); 2^-s undoes it behind the MMAs.
 //   bf16 (PLANES 1): exact whenever the scaled value is a normal fp16.
-// Rows are padded to whole stages of 64 k (zeros) and lie in the stages' order of k.
-//   fp32 (PLANES 3): v = hi + mid + lo, each the fp16 nearest to what is left: exact down to 2^-39 of the row's largest
+//   fp32 (PLANES 3): v = hi + mid + lo, each the fp16 nearest to what is left: exact down to 2^-39 of the largest
 //   (below that, what fp32 rounding leaves of a sum that the largest takes part in).
-// One CTA per row.  A kernel of its own: the GEMM's CTAs set themselves up and dequantize their first stages under it.
-// bf16 rows find their exponents as the largest magnitude of packed pairs.  Before the cluster GEMM the kernel takes 32 registers a
-// thread, so that a CTA fits beside one of the GEMM's and can wait there.  The pair GEMM triggers nothing early, so
-// before it rows of more than 4096 elements are held whole, in 48 registers ([4096 x 8192], Q4_0, 1024 tokens: 65.9 -> 64.5 us
-// a call, 512 tokens: 40.2 -> 39.3; rows that the smaller form holds gain nothing: [11008 x 4096], 2048 tokens, 143.9 against 145.1).
-// Measured and not kept: converting inside the GEMM, every CTA its share of the rows and a counter to wait for (64
-// tokens: 18 us a call instead of 16, the launch and set-up of the GEMM itself lie bare then).
-constexpr int CONVERT_THREADS = 256;
-// KEEP: groups of eight elements a thread keeps between the scan and the conversion; what is left of a longer row is read again.
-constexpr int CONVERT_KEEP_BESIDE = 2;  // rows of 4096: what 32 registers hold
-constexpr int CONVERT_KEEP_ALONE = 4;   // rows of 8192
-template <int PLANES, int KEEP>
-__global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 && KEEP == CONVERT_KEEP_BESIDE ? 8 : 5) convert_rows_kernel(const void* x, __half* __restrict__ x16, float* __restrict__ unscale,
-                                                                       int m, int k) {
-    __shared__ int s_max[CONVERT_THREADS / 32];
-    // Launched with programmatic stream serialization itself: its CTAs may be placed while the previous kernel of the
-    // stream drains, but nothing is read or written before that kernel has completed (it may have produced x, and a
-    // previous GEMM may still be reading the fp16 copy this kernel rewrites).
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMM may set itself up while the rows are converted
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int groups = k >> 3, t = (int)threadIdx.x;  // k is a multiple of 32
-    const int padded = (groups + 7) & ~7;             // groups of a row of x16
-    const size_t plane = (size_t)m * padded;
-    struct G {
-        uint4 a, b;
-    };
-    const int row = (int)blockIdx.x;
-    const uint4* src = static_cast<const uint4*>(x) + (size_t)row * groups * (PLANES == 1 ? 1 : 2);
-    auto load = [&](int i) {
-        G g;
-        g.a = src[PLANES == 1 ? i : 2 * i];
-        g.b = PLANES == 1 ? g.a : src[2 * i + 1];
-        return g;
-    };
-    auto emax_of = [](const G& g) {  // largest biased exponent; Inf and NaN do not drive the scale
+// Rows are padded to whole stages of 64 k (zeros) and lie in the stages' order of k.
+template <int PLANES> struct RowGroup {  // eight elements of a row
+    uint4 a, b;                          // b: fp32 only
+    __device__ __forceinline__ void load(const void* row, int i) {
+        const uint4* src = static_cast<const uint4*>(row) + (size_t)i * (PLANES == 1 ? 1 : 2);
+        a = src[0];
+        if (PLANES > 1) b = src[1];
+    }
+    // The largest magnitude so far: for bf16 of either half of the words, which is enough unless there is an Inf or a NaN (0x7F80
+    // and up); for fp32 the bits of the largest exponent, Inf and NaN aside.
+    __device__ __forceinline__ uint32_t largest(uint32_t m) const {
+        if (PLANES == 1) return __vmaxu2(__vmaxu2(m, __vmaxu2(a.x & 0x7FFF7FFFu, a.y & 0x7FFF7FFFu)), __vmaxu2(a.z & 0x7FFF7FFFu, a.w & 0x7FFF7FFFu));
+        return max(m, (uint32_t)exponent() << 23);
+    }
+    __device__ __forceinline__ int exponent() const {  // largest biased exponent; Inf and NaN do not drive the scale
         int e = 0;
         auto one = [&](uint32_t v) { e = max(e, v == 0xFFu ? 0 : (int)v); };
-        const uint32_t w[8] = {g.a.x, g.a.y, g.a.z, g.a.w, g.b.x, g.b.y, g.b.z, g.b.w};
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
         for (int i = 0; i < (PLANES == 1 ? 4 : 8); i++) {
             one((w[i] >> 23) & 0xFFu);
             if (PLANES == 1) one((w[i] >> 7) & 0xFFu);
         }
         return e;
-    };
-    // bf16: the largest magnitude of each half of the words, which is enough unless there is an Inf or a NaN (0x7F80 and up)
-    auto mags_of = [](uint32_t m, const G& g) {
-        return __vmaxu2(__vmaxu2(m, __vmaxu2(g.a.x & 0x7FFF7FFFu, g.a.y & 0x7FFF7FFFu)), __vmaxu2(g.a.z & 0x7FFF7FFFu, g.a.w & 0x7FFF7FFFu));
-    };
-    G keep[KEEP];
-    int emax = 0;
-    uint32_t mags = 0;
-#pragma unroll
-    for (int u = 0; u < KEEP; u++)
-        if (t + u * CONVERT_THREADS < groups) keep[u] = load(t + u * CONVERT_THREADS);
-    if (PLANES == 1) {
-#pragma unroll
-        for (int u = 0; u < KEEP; u++)
-            if (t + u * CONVERT_THREADS < groups) mags = mags_of(mags, keep[u]);
-        for (int i = t + KEEP * CONVERT_THREADS; i < groups; i += CONVERT_THREADS) mags = mags_of(mags, load(i));
-        emax = max((int)(mags & 0xFFFFu) >> 7, (int)(mags >> 23));
     }
-    if (PLANES > 1 || emax == 0xFF) {
-        emax = 0;
-#pragma unroll
-        for (int u = 0; u < KEEP; u++)
-            if (t + u * CONVERT_THREADS < groups) emax = max(emax, emax_of(keep[u]));
-        for (int i = t + KEEP * CONVERT_THREADS; i < groups; i += CONVERT_THREADS) emax = max(emax, emax_of(load(i)));
-    }
-    emax = __reduce_max_sync(0xFFFFFFFFu, emax);
-    if ((t & 31) == 0) s_max[t >> 5] = emax;
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < CONVERT_THREADS / 32; w++) emax = max(emax, s_max[w]);
-    const int shift = min((127 + 14) - emax, 126);  // multiply by 2^shift; 2^126 is the largest power whose reciprocal is normal
-    const float scale = __uint_as_float((uint32_t)(127 + shift) << 23);
-    uint4* out = reinterpret_cast<uint4*>(x16) + (size_t)row * padded;
-    auto convert = [&](int i, const G& g) {
+    // store(plane, eight fp16)
+    template <class Store> __device__ __forceinline__ void convert(float scale, Store store) const {
         float f[8];
-        const uint32_t w[8] = {g.a.x, g.a.y, g.a.z, g.a.w, g.b.x, g.b.y, g.b.z, g.b.w};
-        if (PLANES == 1) {
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-            for (int e = 0; e < 4; e++) f[2 * e] = __uint_as_float(w[e] << 16) * scale, f[2 * e + 1] = __uint_as_float(w[e] & 0xFFFF0000u) * scale;
-        } else {
-#pragma unroll
-            for (int e = 0; e < 8; e++) f[e] = __uint_as_float(w[e]) * scale;
+        for (int e = 0; e < 4; e++) {
+            f[2 * e] = (PLANES == 1 ? __uint_as_float(w[e] << 16) : __uint_as_float(w[2 * e])) * scale;
+            f[2 * e + 1] = (PLANES == 1 ? __uint_as_float(w[e] & 0xFFFF0000u) : __uint_as_float(w[2 * e + 1])) * scale;
         }
 #pragma unroll
         for (int pl = 0; pl < PLANES; pl++) {
@@ -302,57 +302,135 @@ __global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 && KEEP == CONVER
                     f[2 * e + 1] -= back.y;
                 }
             }
-            out[pl * plane + (i & ~7) + stage_chunk((i >> 2) & 1, i & 3)] = make_uint4(o[0], o[1], o[2], o[3]);
+            store(pl, make_uint4(o[0], o[1], o[2], o[3]));
         }
+    }
+};
+// 2^s and 2^-s from the largest biased exponent; 2^126 is the largest power whose reciprocal is normal
+__device__ __forceinline__ float2 row_scale(int emax) {
+    const int shift = min((127 + 14) - emax, 126);
+    return make_float2(__uint_as_float((uint32_t)(127 + shift) << 23), __uint_as_float((uint32_t)(127 - shift) << 23));
+}
+
+// One CTA per row.  A kernel of its own: the GEMM's CTAs set themselves up and dequantize their first stages under it.  Measured and
+// not kept: converting inside the GEMM, every rank's warps their share of the rows, with tags to wait for: what a warp does for a
+// row and then for the tags is a chain of trips to the L2, 4 us longer until the first MMA (77 tokens of [5003 x 2784]: 12.7 ->
+// 14.4 us a call, 64 of [1000 x 1024]: 6.8 -> 9.8).
+// KEEP: groups a thread keeps between the scan and the conversion; what is left of a longer row is read again.  Before the cluster GEMM
+// and for rows of 4096 it takes 32 registers a thread.  The pair GEMM triggers nothing early, so before it rows of more than
+// 4096 elements are held whole, in 48 registers ([4096 x 8192], Q4_0, 1024 tokens: 65.9 -> 64.5 us a call, 512 tokens: 40.2 ->
+// 39.3; rows that the smaller form holds gain nothing: [11008 x 4096], 2048 tokens, 143.9 against 145.1).
+constexpr int CONVERT_THREADS = 256;
+constexpr int CONVERT_KEEP_SHORT = 2;  // rows of 4096 (bf16)
+constexpr int CONVERT_KEEP_LONG = 4;   // rows of 8192
+template <int PLANES, int KEEP, RowOrder ORDER>
+__global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 && KEEP == CONVERT_KEEP_SHORT ? 8 : 5) convert_rows_kernel(const void* x, __half* __restrict__ x16, float* __restrict__ unscale,
+                                                                       int m, int k) {
+    __shared__ int s_max[CONVERT_THREADS / 32];
+    // Launched with programmatic stream serialization itself: its CTAs may be placed while the previous kernel of the
+    // stream drains, but nothing is read or written before that kernel has completed (it may have produced x, and a
+    // previous GEMM may still be reading the fp16 copy this kernel rewrites).
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMM may set itself up while the rows are converted
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int groups = k >> 3, t = (int)threadIdx.x;  // k is a multiple of 32
+    const int padded = (groups + 7) & ~7;             // groups of a row of x16
+    const size_t plane = (size_t)m * padded;
+    const int row = (int)blockIdx.x;
+    const uint4* src = static_cast<const uint4*>(x) + (size_t)row * groups * (PLANES == 1 ? 1 : 2);
+    RowGroup<PLANES> keep[KEEP], g;
+    uint32_t mags = 0;
+#pragma unroll
+    for (int u = 0; u < KEEP; u++)
+        if (t + u * CONVERT_THREADS < groups) keep[u].load(src, t + u * CONVERT_THREADS);
+#pragma unroll
+    for (int u = 0; u < KEEP; u++)
+        if (t + u * CONVERT_THREADS < groups) mags = keep[u].largest(mags);
+    for (int i = t + KEEP * CONVERT_THREADS; i < groups; i += CONVERT_THREADS) {
+        g.load(src, i);
+        mags = g.largest(mags);
+    }
+    int emax = PLANES == 1 ? max((int)(mags & 0xFFFFu) >> 7, (int)(mags >> 23)) : (int)(mags >> 23);
+    if (PLANES == 1 && emax == 0xFF) {
+        emax = 0;
+#pragma unroll
+        for (int u = 0; u < KEEP; u++)
+            if (t + u * CONVERT_THREADS < groups) emax = max(emax, keep[u].exponent());
+        for (int i = t + KEEP * CONVERT_THREADS; i < groups; i += CONVERT_THREADS) {
+            g.load(src, i);
+            emax = max(emax, g.exponent());
+        }
+    }
+    emax = __reduce_max_sync(0xFFFFFFFFu, emax);
+    if ((t & 31) == 0) s_max[t >> 5] = emax;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < CONVERT_THREADS / 32; w++) emax = max(emax, s_max[w]);
+    const float2 scale = row_scale(emax);
+    uint4* out = reinterpret_cast<uint4*>(x16) + (size_t)row * padded;
+    auto store = [&](int pl, int i, const uint4& v) {  // group i of the row
+        uint4* const stage = out + pl * plane + (i & ~7);
+        const int j = (i >> 2) & 1, q = i & 3;
+        if (ORDER == SMEM_ORDER) {
+            stage[stage_chunk(j, q)] = v;
+        } else {
+            reinterpret_cast<uint2*>(stage)[stage_piece(j, q, 0)] = make_uint2(v.x, v.y);
+            reinterpret_cast<uint2*>(stage)[stage_piece(j, q, 1)] = make_uint2(v.z, v.w);
+        }
+    };
+    auto convert = [&](int i, const RowGroup<PLANES>& v) {
+        v.convert(scale.x, [&](int pl, const uint4& o) { store(pl, i, o); });
     };
 #pragma unroll
     for (int u = 0; u < KEEP; u++)
         if (t + u * CONVERT_THREADS < groups) convert(t + u * CONVERT_THREADS, keep[u]);
-    for (int i = t + KEEP * CONVERT_THREADS; i < groups; i += CONVERT_THREADS) convert(i, load(i));
+    for (int i = t + KEEP * CONVERT_THREADS; i < groups; i += CONVERT_THREADS) {
+        g.load(src, i);
+        convert(i, g);
+    }
     if (t < padded - groups)  // the block that K lacks of its last stage
 #pragma unroll
-        for (int pl = 0; pl < PLANES; pl++) out[pl * plane + (groups & ~7) + stage_chunk(1, t)] = make_uint4(0u, 0u, 0u, 0u);
-    if (t == 0) unscale[row] = __uint_as_float((uint32_t)(127 - shift) << 23);
+        for (int pl = 0; pl < PLANES; pl++) store(pl, groups + t, make_uint4(0u, 0u, 0u, 0u));
+    if (t == 0) unscale[row] = scale.y;
 }
 
 // ---------------------------------------------------------------- epilogue pieces (one lane = one weight row)
 // r[j] = accumulator of (token m0 + j, weight row n).  Rows of y are ldy floats apart; a warp writes 32
-// consecutive floats of one token row per store.  m0 is a multiple of 32, so the row scales load as float4.
-__device__ __forceinline__ void store_chunk(float* __restrict__ y, int64_t ldy, int64_t col0, const float* unscale,
-                                            const uint32_t (&r)[32], int m0, int m, int n, int rows) {
+// consecutive floats of one token row per store.  m0 is a multiple of N, so the row scales load as float4.
+template <int N> __device__ __forceinline__ void store_chunk(float* __restrict__ y, int64_t ldy, int64_t col0, const float* unscale,
+                                            const uint32_t (&r)[N], int m0, int m, int n, int rows) {
     if (n >= rows || m0 >= m) return;
     float* yp = y + (int64_t)m0 * ldy + col0 + n;
-    if (m0 + 32 <= m) {
-        float sc[32];
+    if (m0 + N <= m) {
+        float sc[N];
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
+        for (int i = 0; i < N / 4; i++) {
             const float4 v = reinterpret_cast<const float4*>(unscale + m0)[i];
             sc[4 * i] = v.x, sc[4 * i + 1] = v.y, sc[4 * i + 2] = v.z, sc[4 * i + 3] = v.w;
         }
 #pragma unroll
-        for (int j = 0; j < 32; j++) yp[(int64_t)j * ldy] = __uint_as_float(r[j]) * sc[j];
+        for (int j = 0; j < N; j++) yp[(int64_t)j * ldy] = __uint_as_float(r[j]) * sc[j];
     } else {
 #pragma unroll
-        for (int j = 0; j < 32; j++)
+        for (int j = 0; j < N; j++)
             if (m0 + j < m) yp[(int64_t)j * ldy] = __uint_as_float(r[j]) * unscale[m0 + j];
     }
 }
 // A stream-K piece holds four tokens of a weight row in 16 bytes, [tokens / 4][128 rows]: a warp moves 512 contiguous
 // bytes per access, eight accesses per 32 tokens (one float at a time the owner's tail read its pieces at a third of the
 // speed: 8 - 11 us after the last MMA for 256 KB).
-__device__ __forceinline__ void write_piece_chunk(float* __restrict__ piece, const uint32_t (&r)[32], int tok, int row) {
+template <int N> __device__ __forceinline__ void write_piece_chunk(float* __restrict__ piece, const uint32_t (&r)[N], int tok, int row) {
     uint4* pp = reinterpret_cast<uint4*>(piece) + (size_t)(tok >> 2) * GEMM_BN + row;
 #pragma unroll
-    for (int j = 0; j < 8; j++) __stcg(pp + j * GEMM_BN, make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]));
+    for (int j = 0; j < N / 4; j++) __stcg(pp + j * GEMM_BN, make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]));
 }
-__device__ __forceinline__ void load_piece_chunk(const float* __restrict__ piece, float4 (&v)[8], int tok, int row) {
+template <int Q> __device__ __forceinline__ void load_piece_chunk(const float* __restrict__ piece, float4 (&v)[Q], int tok, int row) {
     const float4* pp = reinterpret_cast<const float4*>(piece) + (size_t)(tok >> 2) * GEMM_BN + row;
 #pragma unroll
-    for (int j = 0; j < 8; j++) v[j] = __ldcg(pp + j * GEMM_BN);
+    for (int j = 0; j < Q; j++) v[j] = __ldcg(pp + j * GEMM_BN);
 }
-__device__ __forceinline__ void add_piece_chunk(uint32_t (&r)[32], const float4 (&v)[8]) {
+template <int N> __device__ __forceinline__ void add_piece_chunk(uint32_t (&r)[N], const float4 (&v)[N / 4]) {
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
+    for (int j = 0; j < N / 4; j++) {
         r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + v[j].x);
         r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + v[j].y);
         r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + v[j].z);
@@ -478,7 +556,7 @@ __device__ __forceinline__ float byte_of(uint32_t w, uint32_t sel, float d, floa
 // What a lane holds of 8 + 8 rows x 128 k of a weight tile: for row half h (rows g = lane / 4 and g + 8) the words of
 // its element group (8 q .. 8 q + 7, q = lane & 3) in the four 32-k blocks, and those blocks' scales.  load() reads
 // them straight from global memory (16-byte pieces, the layout is fragment-ordered); pair<SUB>() converts blocks
-// 2 SUB and 2 SUB + 1 to fp16, one 16-byte chunk of the stage's row each, pair2<SUB>() to two fp16 per weight.
+// 2 SUB and 2 SUB + 1 to fp16, one 16-byte chunk of the stage's row each.
 template <int QT> struct DequantRegs;
 
 template <> struct DequantRegs<WF_QTYPE_Q4_0> {
@@ -493,12 +571,6 @@ template <> struct DequantRegs<WF_QTYPE_Q4_0> {
         const __half2 sx = as_half2(__byte_perm(s, s, 0x1010u)), sy = as_half2(__byte_perm(s, s, 0x3232u));
         o0 = word_to_half8_q4_0(w0, sx);
         o1 = word_to_half8_q4_0(w1, sy);
-    }
-    template <int SUB> __device__ __forceinline__ void pair2(uint4& h0, uint4& h1, uint4& l0, uint4& l1) const {
-        const uint32_t w0 = SUB ? c.z : c.x, w1 = SUB ? c.w : c.y, s = SUB ? sc.y : sc.x;
-        const __half2 sx = as_half2(__byte_perm(s, s, 0x1010u)), sy = as_half2(__byte_perm(s, s, 0x3232u));
-        word_to_half8x2_q4_0(w0, sx, h0, l0);
-        word_to_half8x2_q4_0(w1, sy, h1, l1);
     }
 };
 
@@ -518,13 +590,6 @@ template <> struct DequantRegs<WF_QTYPE_Q4_1> {
         o0 = word_to_half8(w0, s.x, m.x);
         o1 = word_to_half8(w1, s.y, m.y);
     }
-    template <int SUB> __device__ __forceinline__ void pair2(uint4& h0, uint4& h1, uint4& l0, uint4& l1) const {
-        const uint32_t w0 = SUB ? c.z : c.x, w1 = SUB ? c.w : c.y;
-        const float2 s = __half22float2(as_half2(SUB ? sc.y : sc.x));
-        const float2 m = __half22float2(as_half2(SUB ? mn.y : mn.x));
-        word_to_half8x2(w0, s.x, m.x, h0, l0);
-        word_to_half8x2(w1, s.y, m.y, h1, l1);
-    }
 };
 
 template <> struct DequantRegs<WF_QTYPE_Q8_0> {
@@ -540,12 +605,6 @@ template <> struct DequantRegs<WF_QTYPE_Q8_0> {
         const __half2 sx = as_half2(__byte_perm(s, s, 0x1010u)), sy = as_half2(__byte_perm(s, s, 0x3232u));
         o0 = words_to_half8_q8(h0, l0, sx);
         o1 = words_to_half8_q8(h1, l1, sy);
-    }
-    template <int SUB> __device__ __forceinline__ void pair2(uint4& r0, uint4& r1, uint4& e0, uint4& e1) const {
-        const uint32_t h0 = SUB ? ch.z : ch.x, h1 = SUB ? ch.w : ch.y, l0 = SUB ? cl.z : cl.x, l1 = SUB ? cl.w : cl.y, s = SUB ? sc.y : sc.x;
-        const __half2 sx = as_half2(__byte_perm(s, s, 0x1010u)), sy = as_half2(__byte_perm(s, s, 0x3232u));
-        words_to_half8x2_q8(h0, l0, sx, r0, e0);
-        words_to_half8x2_q8(h1, l1, sy, r1, e1);
     }
 };
 
@@ -568,13 +627,70 @@ template <> struct DequantRegs<WF_QTYPE_Q4_K> {  // one half (plane kb & 1) of a
         o0 = word_to_half8(w0, byte_of(scw, first, d.x, nd), byte_of(mnw, first, -d.y, nm));
         o1 = word_to_half8(w1, byte_of(scw, second, d.x, nd), byte_of(mnw, second, -d.y, nm));
     }
-    template <int SUB> __device__ __forceinline__ void pair2(uint4& h0, uint4& h1, uint4& l0, uint4& l1) const {
+};
+
+// The same of one stage alone, blocks 2 sub and 2 sub + 1, which pair2() converts to two fp16 per weight.
+template <int QT> struct DequantHalf;
+
+template <> struct DequantHalf<WF_QTYPE_Q4_0> {
+    uint2 c;
+    uint32_t sc;
+    __device__ __forceinline__ void load(const uint8_t* tile, int, int sub, int lane, int h) {
+        c = __ldg(reinterpret_cast<const uint2*>(tile + h * 512 + lane * 16 + sub * 8));
+        sc = __ldg(reinterpret_cast<const uint32_t*>(tile + Tile<WF_QTYPE_Q4_0>::SCALE_OFF + (lane >> 2) * 16 + h * 8 + sub * 4));
+    }
+    __device__ __forceinline__ void pair2(uint4& h0, uint4& h1, uint4& l0, uint4& l1) const {
+        word_to_half8x2_q4_0(c.x, as_half2(__byte_perm(sc, sc, 0x1010u)), h0, l0);
+        word_to_half8x2_q4_0(c.y, as_half2(__byte_perm(sc, sc, 0x3232u)), h1, l1);
+    }
+};
+
+template <> struct DequantHalf<WF_QTYPE_Q4_1> {
+    uint2 c;
+    uint32_t sc, mn;
+    __device__ __forceinline__ void load(const uint8_t* tile, int, int sub, int lane, int h) {
+        using T = Tile<WF_QTYPE_Q4_1>;
+        c = __ldg(reinterpret_cast<const uint2*>(tile + h * 512 + lane * 16 + sub * 8));
+        sc = __ldg(reinterpret_cast<const uint32_t*>(tile + T::SCALE_OFF + (lane >> 2) * 16 + h * 8 + sub * 4));
+        mn = __ldg(reinterpret_cast<const uint32_t*>(tile + T::MIN_OFF + (lane >> 2) * 16 + h * 8 + sub * 4));
+    }
+    __device__ __forceinline__ void pair2(uint4& h0, uint4& h1, uint4& l0, uint4& l1) const {
+        const float2 s = __half22float2(as_half2(sc)), m = __half22float2(as_half2(mn));
+        word_to_half8x2(c.x, s.x, m.x, h0, l0);
+        word_to_half8x2(c.y, s.y, m.y, h1, l1);
+    }
+};
+
+template <> struct DequantHalf<WF_QTYPE_Q8_0> {
+    uint2 ch, cl;
+    uint32_t sc;
+    __device__ __forceinline__ void load(const uint8_t* tile, int, int sub, int lane, int h) {
+        ch = __ldg(reinterpret_cast<const uint2*>(tile + h * 512 + lane * 16 + sub * 8));
+        cl = __ldg(reinterpret_cast<const uint2*>(tile + PLANE_BYTES + h * 512 + lane * 16 + sub * 8));
+        sc = __ldg(reinterpret_cast<const uint32_t*>(tile + Tile<WF_QTYPE_Q8_0>::SCALE_OFF + (lane >> 2) * 16 + h * 8 + sub * 4));
+    }
+    __device__ __forceinline__ void pair2(uint4& h0, uint4& h1, uint4& l0, uint4& l1) const {
+        words_to_half8x2_q8(ch.x, cl.x, as_half2(__byte_perm(sc, sc, 0x1010u)), h0, l0);
+        words_to_half8x2_q8(ch.y, cl.y, as_half2(__byte_perm(sc, sc, 0x3232u)), h1, l1);
+    }
+};
+
+template <> struct DequantHalf<WF_QTYPE_Q4_K> {
+    uint2 c;
+    uint32_t dd, scw, mnw;  // (d, dmin); 8-bit scales / mins of the stage's two sub-blocks
+    __device__ __forceinline__ void load(const uint8_t* tile, int plane, int sub, int lane, int h) {
+        using T = Tile<WF_QTYPE_Q4_K>;
+        const int g = lane >> 2;
+        c = __ldg(reinterpret_cast<const uint2*>(tile + plane * PLANE_BYTES + h * 512 + lane * 16 + sub * 8));
+        dd = __ldg(reinterpret_cast<const uint32_t*>(tile + T::D_OFF + g * 8 + h * 4));
+        scw = __ldg(reinterpret_cast<const uint16_t*>(tile + T::SC_OFF + g * 16 + h * 8 + plane * 4 + sub * 2));
+        mnw = __ldg(reinterpret_cast<const uint16_t*>(tile + T::MN_OFF + g * 16 + h * 8 + plane * 4 + sub * 2));
+    }
+    __device__ __forceinline__ void pair2(uint4& h0, uint4& h1, uint4& l0, uint4& l1) const {
         const float2 d = __half22float2(as_half2(dd));
         const float nd = -8388608.f * d.x, nm = 8388608.f * d.y;
-        const uint32_t w0 = SUB ? c.z : c.x, w1 = SUB ? c.w : c.y;
-        const uint32_t first = 0x7540u + 2 * SUB, second = first + 1;
-        word_to_half8x2(w0, byte_of(scw, first, d.x, nd), byte_of(mnw, first, -d.y, nm), h0, l0);
-        word_to_half8x2(w1, byte_of(scw, second, d.x, nd), byte_of(mnw, second, -d.y, nm), h1, l1);
+        word_to_half8x2(c.x, byte_of(scw, 0x7540u, d.x, nd), byte_of(mnw, 0x7540u, -d.y, nm), h0, l0);
+        word_to_half8x2(c.y, byte_of(scw, 0x7541u, d.x, nd), byte_of(mnw, 0x7541u, -d.y, nm), h1, l1);
     }
 };
 

@@ -273,7 +273,7 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
         stage_bytes = (size_t)split_stage_bytes(planes, p.bm);
         exchange = (size_t)split_exchange_bytes(p.bm, cluster);
     }
-    p.stages = (int)std::min<size_t>((GEMM_SMEM_LIMIT - 1024 - exchange) / stage_bytes, 8);
+    p.stages = (int)std::min<size_t>((GEMM_SMEM_LIMIT - 1024 - exchange) / stage_bytes, pair || f32 ? 8 : split_a_stages(1, p.bm));
     // A = fp16 weights, B = fp16 activations, D = fp32; both operands K-major
     p.idesc = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(p.bm >> 3) << 17) | ((uint32_t)((pair ? 2 * GEMM_BN : GEMM_BN) >> 4) << 24);
 

@@ -487,31 +487,31 @@ __device__ __forceinline__ void word_to_half8x2_q4_0(uint32_t w, __half2 s2, uin
     two(c.k[1], m1032, hi.z, lo.z);
     two(c.h[1], m72, hi.w, lo.w);
 }
-// Q8_0: s * (16 (hi - 8) + lo): the integer is exact in fp16 (|q| <= 128), one rounding in the product.
+// Q8_0: s * (16 (hi - 8) + lo): fma(16, 1024 + hi, -17536) = 16 hi - 1152 and the sum with 1024 + lo are exact in fp16, one rounding in
+// the product.
+__device__ __forceinline__ __half2 q8_pair(uint32_t hi, uint32_t lo, __half2 off) { return __hadd2(__hfma2(__float2half2_rn(16.f), as_half2(hi), off), as_half2(lo)); }
 __device__ __forceinline__ uint4 words_to_half8_q8(uint32_t wh, uint32_t wl, __half2 s2) {
     const Codes8 h = unpack8(wh), l = unpack8(wl);
-    const __half2 m1032 = __float2half2_rn(-1032.f), m72 = __float2half2_rn(-72.f);
-    const __half2 m1024 = __float2half2_rn(-1024.f), m64 = __float2half2_rn(-64.f), sixteen = __float2half2_rn(16.f);
+    const __half2 ok = __float2half2_rn(-17536.f), oh = __float2half2_rn(-1216.f);
     uint4 o;
-    o.x = as_u32(__hmul2(__hfma2(sixteen, __hadd2(as_half2(h.k[0]), m1032), __hadd2(as_half2(l.k[0]), m1024)), s2));
-    o.y = as_u32(__hmul2(__hfma2(sixteen, __hadd2(as_half2(h.h[0]), m72), __hadd2(as_half2(l.h[0]), m64)), s2));
-    o.z = as_u32(__hmul2(__hfma2(sixteen, __hadd2(as_half2(h.k[1]), m1032), __hadd2(as_half2(l.k[1]), m1024)), s2));
-    o.w = as_u32(__hmul2(__hfma2(sixteen, __hadd2(as_half2(h.h[1]), m72), __hadd2(as_half2(l.h[1]), m64)), s2));
+    o.x = as_u32(__hmul2(q8_pair(h.k[0], l.k[0], ok), s2));
+    o.y = as_u32(__hmul2(q8_pair(h.h[0], l.h[0], oh), s2));
+    o.z = as_u32(__hmul2(q8_pair(h.k[1], l.k[1], ok), s2));
+    o.w = as_u32(__hmul2(q8_pair(h.h[1], l.h[1], oh), s2));
     return o;
 }
 __device__ __forceinline__ void words_to_half8x2_q8(uint32_t wh, uint32_t wl, __half2 s2, uint4& hi, uint4& lo) {
     const Codes8 h = unpack8(wh), l = unpack8(wl);
-    const __half2 m1032 = __float2half2_rn(-1032.f), m72 = __float2half2_rn(-72.f);
-    const __half2 m1024 = __float2half2_rn(-1024.f), m64 = __float2half2_rn(-64.f), sixteen = __float2half2_rn(16.f);
-    auto two = [&](uint32_t ch, uint32_t cl, __half2 oh, __half2 ol, uint32_t& a, uint32_t& b) {
-        const __half2 q = __hfma2(sixteen, __hadd2(as_half2(ch), oh), __hadd2(as_half2(cl), ol)), r = __hmul2(q, s2);
+    const __half2 ok = __float2half2_rn(-17536.f), oh = __float2half2_rn(-1216.f);
+    auto two = [&](__half2 q, uint32_t& a, uint32_t& b) {
+        const __half2 r = __hmul2(q, s2);
         a = as_u32(r);
         b = as_u32(__hfma2(q, s2, __hneg2(r)));
     };
-    two(h.k[0], l.k[0], m1032, m1024, hi.x, lo.x);
-    two(h.h[0], l.h[0], m72, m64, hi.y, lo.y);
-    two(h.k[1], l.k[1], m1032, m1024, hi.z, lo.z);
-    two(h.h[1], l.h[1], m72, m64, hi.w, lo.w);
+    two(q8_pair(h.k[0], l.k[0], ok), hi.x, lo.x);
+    two(q8_pair(h.h[0], l.h[0], oh), hi.y, lo.y);
+    two(q8_pair(h.k[1], l.k[1], ok), hi.z, lo.z);
+    two(q8_pair(h.h[1], l.h[1], oh), hi.w, lo.w);
 }
 // Q4_K: a * code + b in fp32 (a = d * sc and b = -dmin * m are exact in fp32), rounded once to fp16.
 __device__ __forceinline__ uint32_t pack_half2(float a, float b) {

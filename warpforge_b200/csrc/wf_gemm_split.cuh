@@ -7,7 +7,7 @@
 // CTA sends each token of its accumulator to the rank that finishes it, by asynchronous stores straight into that CTA's
 // shared memory which count themselves on its barrier; each rank adds its tokens' S parts in rank order (deterministic)
 // and stores them.  No CTA has more to finish than another, and nothing goes through L2.
-// Measured, 64 tokens, Q4_0 [4096 x 4096]: 10.5 us a call (16.8 as stream-K shares); 33 tokens of Q4_1 [1000 x 1024]: 6.4 us.
+// Measured, 64 tokens, Q4_0 [4096 x 4096]: 9.3 us a call (16.8 as stream-K shares); 33 tokens of Q4_1 [1000 x 1024]: 6.2 us.
 //
 // A lies in TMEM, not in shared memory: the weights' fragment order is that of a 16x256b store, so a dequantizing lane's registers go
 // there as they are, without addresses, bank conflicts or a proxy fence; the tensor core keeps its pace at any token count
@@ -22,7 +22,13 @@
 //   warps 4-7   epilogue (TMEM lane quarter = warp % 4): accumulator -> the ranks' exchange buffers -> y
 //   warps 2,3,8-21  dequantization: quantized tiles from global memory -> fp16 rows of A in TMEM, in two sets of eight warps
 // TMEM: the accumulators (double buffered, so a tile is put together while the next one is computed), behind them the ring of
-// A stages.  A stage is 64 k.
+// A stages.
+// Stages.  bf16 tokens: 128 k of weights and activations together, four of them, so that the MMA warp has one barrier to wait for and
+// one commit per 128 k.  With stages of 64 k and barriers of their own for weights and activations the kernel took 664 cycles
+// per 128 k even with dequantization left out, whatever the number of tokens: the MMA warp's waits (75 - 90 cycles each,
+// though nothing had to be waited for) and commits, between the instructions of the five warps that share its scheduler (33 tokens,
+// Q4_0 [16384 x 2048] 11.8 -> 9.6 us a call, [4096 x 4096] 9.3 -> 8.1, Q5_0 [5003 x 2784] 77 tokens 11.7 -> 10.8).  fp32
+// tokens, whose MMAs take 960 cycles per 64 k: 64 k, weights and activations apart.
 // Every wait is bounded; on expiry the CTA sets a status bit, stops issuing work and still frees its TMEM.  Warps leave their
 // loops on their own, so there is no barrier between some of them: they meet on mbarriers, whose waits are bounded, and
 // all together at the end.
@@ -44,9 +50,9 @@ constexpr int SPLIT_FLUSH = 4;  // units of 128 k the accumulators of a PIECES 2
 constexpr int SPLIT_SETS = 2;   // sets of GEMM_DEQUANT_WARPS
 constexpr int SPLIT_THREADS = (6 + SPLIT_SETS * GEMM_DEQUANT_WARPS) * 32;
 
-inline __host__ __device__ int split_stage_bytes(int planes, int bm) { return planes * bm * 128; }  // of activations
-// Of weights, an even number: 8, or 2 - 6 for fp32 tokens.
-inline __host__ __device__ int split_a_stages(int pieces, int bm) { return min((512 - 2 * pieces * bm) / (32 * pieces), SPLIT_MAX_STAGES) & ~1; }
+inline __host__ __device__ int split_stage_bytes(int planes, int bm) { return (planes == 1 ? 2 : planes) * bm * 128; }  // of activations
+// Stages of weights that TMEM has room for: 4 of 128 k, or 2 - 6 of 64 k for fp32 tokens, an even number.
+inline __host__ __device__ int split_a_stages(int pieces, int bm) { return pieces == 1 ? 4 : min((512 - 4 * bm) / 64, SPLIT_MAX_STAGES) & ~1; }
 // exchange buffer: [S][groups of four tokens a rank finishes][128 rows] float4, where there are several ranks | token scales [4
 // epilogue warps][128]
 inline __host__ __device__ int split_groups(int bm, int ranks) { return (bm / 4 + ranks - 1) / ranks; }
@@ -60,7 +66,9 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
     constexpr int ACCS = PIECES;
     constexpr int FLUSH = PIECES == 1 ? 1 << 30 : SPLIT_FLUSH;
     constexpr int KBW = Tile<QT>::K / GEMM_BK;  // units per weight k-tile
-    constexpr uint32_t A_COLS = 32 * PIECES;    // TMEM columns of an A stage
+    constexpr uint32_t A_COLS = 64;             // TMEM columns of an A stage: two spans of 64 k, or both pieces of one
+    constexpr bool JOINT = PIECES == 1;         // weights and activations share stages and barriers (b_full, b_empty)
+    constexpr int SPANS = JOINT ? 2 : 1;        // of 64 k per stage
     // The two sets of dequantization warps take units by turns (bf16), or a stage each of every unit (fp32: there may be no more than two
     // stages, and a set that came back to one only after the other set's turn could not tell by the barrier's parity whether that
     // turn is over).
@@ -69,19 +77,19 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
     constexpr int DEPTH = 2;  // units a dequantization warp holds: one is converted while the other loads
     constexpr int COLS = PIECES == 1 ? 32 : 16; // that an epilogue warp takes at a time
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint64_t* b_full = reinterpret_cast<uint64_t*>(smem);        // [8] activations landed
+    uint64_t* b_full = reinterpret_cast<uint64_t*>(smem);        // [8] activations landed (JOINT: and weights dequantized)
     uint64_t* b_empty = b_full + SPLIT_MAX_STAGES;               // [8] read by the MMAs
-    uint64_t* a_full = b_empty + SPLIT_MAX_STAGES;               // [8] weights dequantized
-    uint64_t* a_empty = a_full + SPLIT_MAX_STAGES;               // [8] read by the MMAs
-    uint64_t* acc_full = a_empty + SPLIT_MAX_STAGES;             // [2]
+    uint64_t* a_full = JOINT ? b_full : b_empty + SPLIT_MAX_STAGES;    // [8] weights dequantized
+    uint64_t* a_empty = JOINT ? b_empty : a_full + SPLIT_MAX_STAGES;   // [8] read by the MMAs
+    uint64_t* acc_full = b_full + 4 * SPLIT_MAX_STAGES;          // [2]
     uint64_t* acc_empty = acc_full + 2;                          // [2]
     uint64_t* ex_full = acc_empty + 2;                           // the parts of this rank's tokens have arrived
     uint64_t* ex_empty = ex_full + 1;                            // every rank has read its exchange buffer
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ex_empty + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const uint32_t span_bytes = (uint32_t)p.bm * 128;  // 64 k of bm tokens
-    const uint32_t stage_bytes = PLANES * span_bytes;
-    const int stages = p.stages, a_stages = split_a_stages(PIECES, p.bm), S = p.ranks;
+    const uint32_t stage_bytes = (JOINT ? 2 : PLANES) * span_bytes;
+    const int stages = p.stages, a_stages = JOINT ? stages : split_a_stages(PIECES, p.bm), S = p.ranks;
     uint8_t* stage0 = smem + 1024;
     float4* ex = reinterpret_cast<float4*>(stage0 + (size_t)stages * stage_bytes);
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -134,7 +142,7 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
             prefetch_tensormap(&xmap);
             *abort_flag = 0;
         }
-        g_mbar_init(b_full + lane, lane >> 3 == 2 ? GEMM_DEQUANT_WARPS : 1);  // all four rings
+        g_mbar_init(b_full + lane, lane >> 3 == 2 ? GEMM_DEQUANT_WARPS : JOINT && lane < 8 ? GEMM_DEQUANT_WARPS + 1 : 1);  // the rings
         // acc_full, acc_empty (the four epilogue warps), ex_full, ex_empty
         if (lane < 6) g_mbar_init(acc_full + lane, lane == 2 || lane == 3 ? 4 : lane == 5 ? 4 * S : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -167,13 +175,18 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
             for (int tile = cluster; tile < tiles && !*abort_flag; tile += clusters) {
                 const int tok0 = (tile % p.m_tiles) * p.bm;
                 if (tile != cluster) last_tile(tile);
-                for (int st = 2 * kb0; st < 2 * kb1; st++, at.advance(stages)) {
+                for (int st = 2 * kb0; st < 2 * kb1; st += SPANS, at.advance(stages)) {
                     const int s = at.s;
                     if (!g_mbar_wait(&b_empty[s], at.phase ^ 1)) { fail(); break; }
                     uint8_t* b_stage = stage0 + (size_t)s * stage_bytes;
-                    g_mbar_expect_tx(&b_full[s], PLANES * span_bytes);
+                    g_mbar_expect_tx(&b_full[s], stage_bytes);
+                    if (JOINT) {
+                        tma_load_2d(b_stage, &xmap, st * 64, tok0, &b_full[s]);
+                        tma_load_2d(b_stage + span_bytes, &xmap, st * 64 + 64, tok0, &b_full[s]);
+                    } else {
 #pragma unroll
-                    for (int pl = 0; pl < PLANES; pl++) tma_load_2d(b_stage + pl * span_bytes, &xmap, st * 64, pl * p.m + tok0, &b_full[s]);
+                        for (int pl = 0; pl < PLANES; pl++) tma_load_2d(b_stage + pl * span_bytes, &xmap, st * 64, pl * p.m + tok0, &b_full[s]);
+                    }
                 }
             }
         }
@@ -192,26 +205,28 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
                 if (local >= 2 && !g_mbar_wait(&acc_empty[buf], ((local >> 1) - 1) & 1)) { fail(); ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(buf * ACCS * p.bm), e_tmem = d_tmem + (uint32_t)p.bm;
-                for (int st = 2 * g0; st < 2 * g1; st++) {
+                for (int st = 2 * g0; st < 2 * g1; st += SPANS) {
                     const int s = at.s;
-                    if (!g_mbar_wait(&b_full[s], at.phase) || !g_mbar_wait(&a_full[a_at.s], a_at.phase)) { fail(); ok = false; break; }
+                    if (!g_mbar_wait(&b_full[s], at.phase) || (!JOINT && !g_mbar_wait(&a_full[a_at.s], a_at.phase))) { fail(); ok = false; break; }
                     tc_fence_after();
                     const uint64_t bd = b_desc0 + (uint64_t)((uint32_t)s * stage_bytes >> 4);
-                    const uint32_t hi = a_tmem + (uint32_t)a_at.s * A_COLS, lo = hi + 32;
+                    const uint32_t hi = a_tmem + (uint32_t)(JOINT ? s : a_at.s) * A_COLS, lo = hi + 32;
                     const uint32_t acc = (uint32_t)(st - 2 * g0);
                     tc_mma_span_ts(d_tmem, hi, bd, p.idesc, acc, issue);
-                    if (PIECES == 2) {
+                    if (JOINT) {
+                        tc_mma_span_ts(d_tmem, lo, bd + span, p.idesc, 1u, issue);
+                    } else {
                         tc_mma_span_ts(e_tmem, lo, bd, p.idesc, acc, issue);
                         tc_mma_span_ts(e_tmem, hi, bd + span, p.idesc, 1u, issue);
                         tc_mma_span_ts(e_tmem, lo, bd + span, p.idesc, 1u, issue);
                         tc_mma_span_ts(e_tmem, hi, bd + 2 * span, p.idesc, 1u, issue);
                     }
-                    if (issue) {  // frees both stages when these MMAs have read them
-                        tc_commit(&a_empty[a_at.s]);
+                    if (issue) {  // frees the stages when these MMAs have read them
+                        if (!JOINT) tc_commit(&a_empty[a_at.s]);
                         tc_commit(&b_empty[s]);
                     }
                     at.advance(stages);
-                    a_at.advance(a_stages);
+                    if (!JOINT) a_at.advance(a_stages);
                 }
                 if (ok && issue) tc_commit(&acc_full[buf]);
                 g0 = g1;
@@ -320,20 +335,23 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
         }
     } else {
         // ------------------------------------------------ dequant warps
-        // One step: convert registers loaded earlier (still in registers), wait for the stage, store it and hand it over.  Converting
-        // before the wait keeps the arithmetic off the path between "the MMAs have released the stage" and "the stage is
-        // full again".
+        // One step: convert registers loaded earlier (still in registers; the first of two spans), wait for the stage, store it and hand
+        // it over.  Converting before the wait keeps arithmetic off the path between "the MMAs have released the stage" and "the
+        // stage is full again".
         const uint32_t a_mine = a_tmem + ((uint32_t)(dq * 16) << 16);
         StageCursor at;
         bool lapped = false;  // from the second lap on a wait is bounded by what earlier kernels let this one do
         auto advance = [&]() { lapped |= at.advance(a_stages); };
-        auto finish_step = [&](const Regs (&regs)[2], auto sub) {
-            uint4 out[2][2 * PIECES];
+        auto convert = [&](const Regs (&regs)[2], auto sub, uint4 (&out)[2][2 * PIECES]) {
 #pragma unroll
             for (int hh = 0; hh < 2; hh++) {
-                if constexpr (PIECES == 1) regs[hh].template pair<decltype(sub)::value>(out[hh][0], out[hh][1]);
+                if constexpr (JOINT) regs[hh].template pair<decltype(sub)::value>(out[hh][0], out[hh][1]);
                 else regs[hh].pair2(out[hh][0], out[hh][1], out[hh][2], out[hh][3]);
             }
+        };
+        auto finish_step = [&](const Regs (&regs)[2]) {
+            uint4 out[2][2 * PIECES];
+            convert(regs, std::integral_constant<int, 0>{}, out);
             if (lapped) {
                 asm volatile("griddepcontrol.wait;" ::: "memory");
                 lapped = false;
@@ -343,8 +361,14 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
                 return false;
             }
             tc_fence_after();
-#pragma unroll
-            for (int i = 0; i < PIECES; i++) tmem_st_span(a_mine + (uint32_t)at.s * A_COLS + 32 * i, out[0][2 * i], out[0][2 * i + 1], out[1][2 * i], out[1][2 * i + 1]);
+            const uint32_t to = a_mine + (uint32_t)at.s * A_COLS;
+            tmem_st_span(to, out[0][0], out[0][1], out[1][0], out[1][1]);
+            if constexpr (JOINT) {
+                convert(regs, std::integral_constant<int, 1>{}, out);
+                tmem_st_span(to + 32, out[0][0], out[0][1], out[1][0], out[1][1]);
+            } else {
+                tmem_st_span(to + 32, out[0][2], out[0][3], out[1][2], out[1][3]);
+            }
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
@@ -352,17 +376,16 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
             advance();
             return true;
         };
-        for (int i = 0; i < (PIECES == 1 ? 2 * set : set); i++) advance();
+        if (set > 0) advance();
         bool ok = true;
         for (int u = unit0; u < units && ok && !*abort_flag; u += TURN * DEPTH) {
 #pragma unroll
             for (int d = 0; d < DEPTH; d++) {
                 if (u + d * TURN >= units) break;
-                ok = finish_step(r[d], std::integral_constant<int, 0>{});
-                if (PIECES == 1 && ok) ok = finish_step(r[d], std::integral_constant<int, 1>{});
+                ok = finish_step(r[d]);
                 if (!ok) break;
                 load_next(r[d]);
-                for (int i = 0; i < (PIECES == 1 ? 2 : 1); i++) advance();  // over the other set's stages
+                advance();  // over the other set's stage
             }
         }
     }

@@ -58,6 +58,24 @@ def test_bf16_tokens(backend, oracle, name, rows, k, m):
     assert np.linalg.norm(d) <= 3e-4 * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("name", ["q4_0", "q8_0", "q4_k"])
+@pytest.mark.parametrize("rows,k,m", [
+    (7100, 3104, 1030),  # halves of 256 tokens, rows that the conversion's short form holds
+    (4700, 8224, 520),   # the same, the long form and more than it holds (Q4_0: clusters of two)
+    (5100, 4128, 1000),  # Q8_0, Q4_K: tiles of 512 tokens
+])
+def test_pairs_of_ctas(backend, oracle, name, rows, k, m):
+    """Sizes from which the cost functions take the CTA pairs, ragged in rows, K and tokens."""
+    from warpforge_b200.backend import Tensor
+
+    if name == "q4_k":
+        k = k // 256 * 256
+    bits = Q.synth_activation_bf16(m, k, rows + m)
+    got, want = _run(backend, oracle, name, rows, k, Q.bf16_bits_to_float(bits), Tensor.from_bf16_bits(bits))
+    assert np.max(np.abs(got - want)) <= 1e-3 * np.max(np.abs(want))
+    assert np.linalg.norm(got - want) <= 3e-4 * np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("name,f32", [("q4_0", False), ("q8_0", False), ("q4_k", False), ("q4_1", True), ("q8_0", True), ("q4_k", True)])
 @pytest.mark.parametrize("rows,k,tokens", [
     (20600, 128, (40,)),  # more tiles than clusters of one unit each: the sets of dequantizing warps take tiles by turns

@@ -107,35 +107,47 @@ static cudaError_t gemm_launch_one(Kernel kernel, const GemmParams& p, const CUt
     return cudaLaunchKernelEx(&cfg, kernel, p, map);
 }
 
-// What a call costs in us by either kernel, fitted to measurements on one B200 (weights from HBM, calls back to back): 6 - 8 us
-// of conversion, launch and start; a cost per unit of 128 k on the busiest CTA or pair; the parts put together.
-//   us by the fit / measured: split, bf16, [4096 x 4096]: 33 tokens (4 ranks) 13 / 12.4, 100 tokens 15 / 15.6; [11008 x 4096],
-//   128 tokens (3 ranks) 30 / 28; [16000 x 1024], 400 tokens: 1 rank 31 / 30, 2 ranks 53 / 64.
-//   pair: [4096 x 4096] 256 tokens 25 / 23, 512 tokens 38 / 35; [11008 x 4096] 256 tokens 31 / 32; [600 x 6976] 2000 tokens 47 / 47.5.
-static double split_cost(int qt, int64_t rounds, int units, int ranks, int bm, bool f32) {
-    const double b = bm / 128.0, unit = f32 ? 0.95 + 0.9 * b : (qt == WF_QTYPE_Q4_0 ? 0.6 : qt == WF_QTYPE_Q8_0 ? 0.8 : 0.7) + 0.12 * b;
-    const double together = ranks == 1 ? 0.5 + 0.5 * b : (f32 ? 0.5 + 4.0 * b : 1.0 + 3.0 * b);
-    return 6.0 + (double)rounds * (units * unit + together);
+// What a call costs in us by either kernel, fitted to measurements on one B200 (weights from HBM, calls back to back): 2200 calls of the
+// split kernel (11 - 2048 tokens, weights from [600 x 6976] to [14336 x 8192], every number of ranks, token tiles of 64, 96 and
+// 128), 220 of the pair kernel.  Conversion, launch and start; a cost per unit of 128 k on the busiest CTA or pair, where the slower
+// of dequantization and MMAs counts; the parts put together.  The fits are off by 9 % and 6 % (one standard deviation); what
+// they choose takes 1.5 % more time on average than the best of the settings measured, 14 % at worst, while the choices of the
+// constants before, made for A in shared memory, took 9 %, up to 60 %: 300 - 512 tokens of [4096 x 4096], pairs 28 us, clusters of one 18;
+// [11008 x 4096] Q4_K 128 tokens, 31.5 and 24.  80 calls and layers of 33 - 2048 tokens drawn at random: 0.936 x the time, worst
+// 1.05 ([528 x 5728], 162 tokens).
+static double split_cost(int qt, int64_t rounds, int units, int ranks, int bm, int64_t m, bool f32) {
+    const double b = bm / 128.0, t = (double)m / 256;
+    if (f32) {
+        const double dequant = qt == WF_QTYPE_Q4_0 ? 0.76 : qt == WF_QTYPE_Q4_1 ? 0.98 : qt == WF_QTYPE_Q8_0 ? 0.92 : 1.07;
+        const double unit = std::max(dequant, 0.56 + 1.12 * b);
+        return ranks == 1 ? 3.5 + 1.6 * t + (double)rounds * units * unit : 5.0 + 4.3 * t + (double)rounds * (units * unit + 0.6 * b);
+    }
+    const double dequant = qt == WF_QTYPE_Q4_0 ? 0.37 : qt == WF_QTYPE_Q4_1 ? 0.42 : qt == WF_QTYPE_Q8_0 ? 0.52 : 0.53;
+    const double unit = std::max(dequant, 0.07 + 0.35 * b);
+    return ranks == 1 ? 2.5 + 0.7 * t + (double)rounds * (units * unit + 1.3 + 0.25 * b) : 3.8 + 1.5 * t + (double)rounds * (units * unit + 3.6 * b);
 }
 // share: units of the busiest pair; a tile of U units is put together from the pieces of U / share pairs
-static double pair_cost(int64_t share, int k_blocks, int halves) {
-    return 8.0 + (double)share * (halves == 2 ? 1.5 : 1.0) + (double)((k_blocks + share - 1) / share) * (halves == 2 ? 4.5 : 2.2);
+static double pair_cost(int qt, int64_t share, int k_blocks, int halves, int64_t m) {
+    const double t = 11.3 + 3.5 * (double)m / 1024, pieces = (double)k_blocks / (double)share;
+    if (halves == 2) return t + 1.6 + (double)share * 1.7 + pieces * 1.6;
+    return t + (double)share * (qt == WF_QTYPE_Q4_0 || qt == WF_QTYPE_Q4_1 ? 0.83 : 0.96) + pieces * 1.1;
 }
+// Where two ways are close, the one that the fits know better: smaller token tiles and clusters instead of pairs have to promise as much.
+constexpr double SMALLER_TILES_GAIN = 0.92, CLUSTERS_GAIN = 0.95;
 
 // CTAs per tile of the split kernel, the cheapest by split_cost.
-static int split_ranks(const GemmDevice& d, int qt, int64_t tiles, int k_blocks, int bm, bool f32, int* clusters, double* cost) {
+static int split_ranks(const GemmDevice& d, int qt, int64_t tiles, int k_blocks, int bm, int64_t m, bool f32, double* cost) {
     int best = 1;
     *cost = 1e30;
     for (int n = 1; n <= SPLIT_MAX_RANKS && n <= k_blocks; n++) {
         if (d.clusters[n] < 1) continue;
         const int64_t rounds = (tiles + d.clusters[n] - 1) / d.clusters[n];
-        const double t = split_cost(qt, rounds, (k_blocks + n - 1) / n, n, bm, f32);
+        const double t = split_cost(qt, rounds, (k_blocks + n - 1) / n, n, bm, m, f32);
         if (t < *cost) {
             *cost = t;
             best = n;
         }
     }
-    *clusters = (int)std::min<int64_t>(d.clusters[best], tiles);
     return best;
 }
 
@@ -223,16 +235,24 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     // Clusters on tiles of 128 rows x up to 128 tokens.  Token tiles are of one size, in steps of 32 where there are several (the
     // epilogue works on 32 tokens at a time and must not reach into a neighbour); fp32: 96, so that two stages and the
     // exchange buffer fit.
-    const int most = f32 ? 96 : SPLIT_MAX_TOKENS;
-    const int64_t token_tiles = (call.m + most - 1) / most, grain = token_tiles > 1 ? 32 : 16;
-    p.bm = (int)(((call.m + token_tiles - 1) / token_tiles + grain - 1) / grain * grain);
     p.n_tiles = (int)((w.g.rows + GEMM_BN - 1) / GEMM_BN);
-    p.m_tiles = (int)((call.m + p.bm - 1) / p.bm);
     // the last 128-row block may reach past the padded row-tiles: the weight buffer must cover it
     if ((int64_t)p.n_tiles * (GEMM_BN / 16) > w.g.rt_alloc)
         return set_error(c, WF_ERR_SHAPE, "weight buffer does not cover the last 128-row block");
-    double cost = 0;
-    p.ranks = split_ranks(*dev, qt, (int64_t)p.n_tiles * p.m_tiles, p.k_blocks, p.bm, f32, &clusters, &cost);
+    double cost = 1e30;
+    for (int most = f32 ? 96 : SPLIT_MAX_TOKENS; most >= (f32 ? 96 : 64); most -= 32) {  // smaller tiles where they fill the device better
+        const int64_t token_tiles = (call.m + most - 1) / most, grain = token_tiles > 1 ? 32 : 16;
+        const int bm = (int)(((call.m + token_tiles - 1) / token_tiles + grain - 1) / grain * grain);
+        const int m_tiles = (int)((call.m + bm - 1) / bm);
+        double t = 0;
+        const int ranks = split_ranks(*dev, qt, (int64_t)p.n_tiles * m_tiles, p.k_blocks, bm, call.m, f32, &t);
+        if (t >= SMALLER_TILES_GAIN * cost) continue;
+        cost = t;
+        p.bm = bm;
+        p.m_tiles = m_tiles;
+        p.ranks = ranks;
+    }
+    clusters = (int)std::min<int64_t>(dev->clusters[p.ranks], (int64_t)p.n_tiles * p.m_tiles);
     // Pairs of CTAs on tiles of 256 rows x 512 or 256 tokens, stream-K shares.  A tile of U units shared by n pairs costs about U / n
     // units plus n - 1 pieces added by its owner, a piece costing about two units: no share is shorter than sqrt(2 U)
     // units, which bounds n for weights with few tiles.
@@ -245,7 +265,7 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     for (int halves = 1; halves <= 2 && !f32 && call.m > 64 && dev->pairs > 0; halves++) {
         const int64_t u = (int64_t)pair_n * ((call.m + halves * 256 - 1) / (halves * 256)) * p.k_blocks;
         const int n = (int)std::min<int64_t>(dev->pairs, std::max<int64_t>(1, u / min_units));
-        const double t = pair_cost((u + n - 1) / n, p.k_blocks, halves);
+        const double t = CLUSTERS_GAIN * pair_cost(qt, (u + n - 1) / n, p.k_blocks, halves, call.m);
         if (t >= cost) continue;
         cost = t;
         pair = true;

@@ -286,12 +286,16 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     } else {
         cluster = p.ranks;
         grid = clusters * cluster;
+        // The conversion of fp32 rows takes more registers than a GEMM's CTA leaves, so it waits on idle SMs and keeps the next GEMM's
+        // clusters from them.  Few rows are worth it: 14 shapes of 11 - 32 tokens 0.95 x (worst 1.02), 26 of 40 - 256 tokens 1.03 x
+        // (worst 1.14).
+        p.early = !f32 || call.m <= 32;
         p.unit_q = p.k_blocks / p.ranks;
         p.unit_r = p.k_blocks % p.ranks;
         p.tile_q = p.n_tiles * p.m_tiles / clusters;
         p.tile_r = p.n_tiles * p.m_tiles % clusters;
         stage_bytes = (size_t)split_stage_bytes(planes, p.bm);
-        exchange = (size_t)split_exchange_bytes(p.bm, cluster);
+        exchange = (size_t)split_exchange_bytes(f32 ? 2 : 1, p.bm, cluster);
     }
     p.stages = (int)std::min<size_t>((GEMM_SMEM_LIMIT - 1024 - exchange) / stage_bytes, pair || f32 ? 8 : split_a_stages(1, p.bm));
     // A = fp16 weights, B = fp16 activations, D = fp32; both operands K-major

@@ -32,6 +32,7 @@ struct GemmParams {
     int stages;
     int halves;          // pair kernel: 256-token halves of a token tile, 1 or 2
     int ranks;           // split kernel: CTAs of a cluster, which share a tile's K
+    int early;           // split kernel: let the next kernel be placed while this one runs
     uint32_t idesc;
     // pair kernel, stream-K: the (tile, k-block) units form one sequence, pair b owns units [b*q + min(b,r), ...)
     // split kernel: rank b owns those k-blocks of every tile, cluster c takes tile_q tiles, one more below tile_r

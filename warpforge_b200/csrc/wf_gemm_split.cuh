@@ -54,9 +54,11 @@ inline __host__ __device__ int split_stage_bytes(int planes, int bm) { return (p
 // Stages of weights that TMEM has room for: 4 of 128 k, or 2 - 6 of 64 k for fp32 tokens, an even number.
 inline __host__ __device__ int split_a_stages(int pieces, int bm) { return pieces == 1 ? 4 : min((512 - 4 * bm) / 64, SPLIT_MAX_STAGES) & ~1; }
 // exchange buffer: [S][groups of four tokens a rank finishes][128 rows] float4, where there are several ranks | token scales [4
-// epilogue warps][128]
+// epilogue warps][128] | fp32 tokens: sums of the groups of units so far, [groups of four tokens][128 rows] float4
 inline __host__ __device__ int split_groups(int bm, int ranks) { return (bm / 4 + ranks - 1) / ranks; }
-inline __host__ __device__ int split_exchange_bytes(int bm, int ranks) { return (ranks == 1 ? 0 : ranks * split_groups(bm, ranks) * GEMM_BN * 16) + 4 * SPLIT_MAX_TOKENS * 4; }
+inline __host__ __device__ int split_exchange_bytes(int pieces, int bm, int ranks) {
+    return (ranks == 1 ? 0 : ranks * split_groups(bm, ranks) * GEMM_BN * 16) + 4 * SPLIT_MAX_TOKENS * 4 + (pieces == 1 ? 0 : bm * GEMM_BN * 4);
+}
 
 // smem: [0, 1024) barriers, tmem slot | stages of activations, 1024-byte aligned | exchange buffer
 // Registers: 80 a thread, what the hardware has for 24 warps; 22 are launched, and what is left is room for four warps of the next call's
@@ -165,9 +167,9 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
             // The next call's conversion waits beside this kernel, and the next GEMM takes each SM as it becomes free (a call of
             // [5003 x 2784], 77 tokens, Q4_0: 12.7 -> 11.6 us; 64 tokens of [4096 x 4096], 12.7 -> 11.3).  Placed when the CTA
             // begins its last tile: a conversion that waits beside longer delays clusters of several tiles ([11008 x 4096], 128
-            // tokens, two tiles each: 27.6 us without, 28.9 placed at the start, 27.8 here).  fp32 tokens: 93 -> 98.
+            // tokens, two tiles each: 27.6 us without, 28.9 placed at the start, 27.8 here).  p.early: where it pays (gemm_launch).
             auto last_tile = [&](int tile) {
-                if (PIECES == 1 && tile + clusters >= tiles) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+                if (p.early && tile + clusters >= tiles) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             };
             last_tile(cluster);
             asm volatile("griddepcontrol.wait;" ::: "memory");  // the fp16 activations
@@ -244,7 +246,8 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
         // a copy for each warp, so that it shares nothing with the others (in registers they cost up to 5 %)
         float* const scale = reinterpret_cast<float*>(ex + (S == 1 ? 0 : (size_t)S * per * GEMM_BN)) + quarter * SPLIT_MAX_TOKENS;
         int local = 0, round = 0;
-        float* sums = p.partial + (size_t)blockIdx.x * SPLIT_MAX_TOKENS * GEMM_BN;
+        // (in global memory each 16 tokens waited for the L2 behind the last MMA: 38 shapes 0.98 x, Q8_0 [3000 x 6016] 96 tokens 23.7 -> 22.4 us)
+        float4* const sums = ex + (S == 1 ? 0 : (size_t)S * per * GEMM_BN) + 4 * SPLIT_MAX_TOKENS / 4 + row;
         asm volatile("griddepcontrol.wait;" ::: "memory");  // the row scales; no bounded wait before
         bool ok = true;
         for (int tile = cluster; tile < tiles && ok && !*abort_flag; tile += clusters, round++) {
@@ -272,11 +275,14 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
                     tmem_ld_accs(taddr + (uint32_t)c, p.bm, v);
                     if (PIECES == 2 && g0 > kb0) {  // what earlier groups of the tile came to
                         float4 e[COLS / 4];
-                        load_piece_chunk(sums, e, c, row);
+#pragma unroll
+                        for (int j = 0; j < COLS / 4; j++) e[j] = sums[((c >> 2) + j) * GEMM_BN];
                         add_piece_chunk(v, e);
                     }
                     if (PIECES == 2 && !last) {
-                        write_piece_chunk(sums, v, c, row);
+#pragma unroll
+                        for (int j = 0; j < COLS / 4; j++)
+                            sums[((c >> 2) + j) * GEMM_BN] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
                     } else if (S == 1) {
                         store_chunk(p.y, p.ldy, p.col0, scale - tok0, v, tok0 + c, p.m, n, p.rows);
                     } else {

@@ -111,7 +111,7 @@ struct GemvScratch {
     // tensor-core GEMM
     std::shared_ptr<uint8_t> d_x16;         // fp16 copy of the activations
     int64_t x16_bytes = 0;
-    std::shared_ptr<float> d_gemm_partial;  // [sm_count][512][128] pieces of tiles cut by a share boundary
+    std::shared_ptr<float> d_gemm_partial;  // [sm_count][256][128] pieces of tiles cut by a share boundary
     std::shared_ptr<unsigned int> d_gemm_ready;  // [sm_count][4] generation whose piece is complete, per 32-row quarter; then {generation, CTAs out}
 };
 // cudaMalloc for everything that a context allocates: where memory is short, its kept tile buffers go first.

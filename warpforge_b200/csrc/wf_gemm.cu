@@ -1,13 +1,13 @@
 // Prefill GEMM: y[m, rows] = x[m, K] . W[rows, K]^T for many tokens, W in the tiled quantized
 // layout of wf_layout.cuh, on the 5th-generation tensor cores:
 //
-//   D[weight rows x tokens] (fp32, in TMEM) += A[rows x 16] (fp16, smem) * B[16 x tokens] (fp16, smem)
+//   D[weight rows x tokens] (fp32, in TMEM) += A[rows x 16] (fp16, in TMEM) * B[16 x tokens] (fp16, smem)
 //
 // A call is two kernels: convert_rows_kernel rewrites the activations as fp16 times a power of two per row, and one of
-//   gemm_pair_kernel   (wf_gemm_pair.cuh)   pairs of CTAs on tiles of 256 rows x 512 tokens, stream-K
+//   gemm_pair_kernel   (wf_gemm_pair.cuh)   pairs of CTAs on tiles of 256 rows x up to 256 tokens, stream-K
 //   gemm_split_kernel  (wf_gemm_split.cuh)  clusters of CTAs that split the K of a tile of 128 rows x up to 128 tokens;
 //                                           also the kernel of fp32 activations
-// dequantizes the weights into shared memory and multiplies.  The launch side and the choice between them are here.
+// dequantizes the weights into TMEM and multiplies.  The launch side and the choice between them are here.
 //
 // bf16 activations: weights are rounded once to fp16 (relative 2^-12) after the exact fp32 dequantization; products
 // and sums are fp32 in the tensor core.  Replaces the host transpose + batch_matmul_f32 of
@@ -53,10 +53,10 @@ struct GemmDevice {
     int pairs = 0;
     int clusters[SPLIT_MAX_RANKS + 1] = {};
 };
-template <class Kernel> static cudaError_t max_clusters(Kernel kernel, int threads, int size, int* out) {
+template <class Kernel> static cudaError_t max_clusters(Kernel kernel, int size, int* out) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)size);
-    cfg.blockDim = dim3((unsigned)threads);
+    cfg.blockDim = dim3(GEMM_THREADS);
     cfg.dynamicSmemBytes = GEMM_SMEM_LIMIT;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -76,9 +76,9 @@ template <int QT> static cudaError_t gemm_prepare(int device, GemmDevice** out) 
     cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel<QT, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_split_kernel<QT, 2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
-    if (e == cudaSuccess) e = max_clusters(gemm_pair_kernel<QT>, GEMM_THREADS, 2, &d.pairs);
+    if (e == cudaSuccess) e = max_clusters(gemm_pair_kernel<QT>, 2, &d.pairs);
     for (int n = 1; n <= SPLIT_MAX_RANKS && e == cudaSuccess; n++) {
-        e = max_clusters(gemm_split_kernel<QT, 1, 1>, SPLIT_THREADS, n, &d.clusters[n]);
+        e = max_clusters(gemm_split_kernel<QT, 1, 1>, n, &d.clusters[n]);
         // one fewer than the device says: a cluster that does not find its place in the first wave costs a whole round
         if (n >= 3 && d.clusters[n] > 16) d.clusters[n]--;
     }
@@ -87,13 +87,13 @@ template <int QT> static cudaError_t gemm_prepare(int device, GemmDevice** out) 
 }
 
 template <class Kernel>
-static cudaError_t gemm_launch_one(Kernel kernel, const GemmParams& p, const CUtensorMap& map, int threads, int grid, int cluster, size_t smem, cudaStream_t s) {
+static cudaError_t gemm_launch_one(Kernel kernel, const GemmParams& p, const CUtensorMap& map, int grid, int cluster, size_t smem, cudaStream_t s) {
     // Programmatic stream serialization: this kernel may start while the conversion of the activations (the previous launch
     // of the stream) is still running; what reads the conversion's output waits with griddepcontrol.wait, the rest
     // (barrier set-up, TMEM allocation, the first weight loads and conversions) runs under it.
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)threads);
+    cfg.blockDim = dim3(GEMM_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
@@ -109,12 +109,11 @@ static cudaError_t gemm_launch_one(Kernel kernel, const GemmParams& p, const CUt
 
 // What a call costs in us by either kernel, fitted to measurements on one B200 (weights from HBM, calls back to back): 2200 calls of the
 // split kernel (11 - 2048 tokens, weights from [600 x 6976] to [14336 x 8192], every number of ranks, token tiles of 64, 96 and
-// 128), 220 of the pair kernel.  Conversion, launch and start; a cost per unit of 128 k on the busiest CTA or pair, where the slower
-// of dequantization and MMAs counts; the parts put together.  The fits are off by 9 % and 6 % (one standard deviation); what
-// they choose takes 1.5 % more time on average than the best of the settings measured, 14 % at worst, while the choices of the
-// constants before, made for A in shared memory, took 9 %, up to 60 %: 300 - 512 tokens of [4096 x 4096], pairs 28 us, clusters of one 18;
-// [11008 x 4096] Q4_K 128 tokens, 31.5 and 24.  80 calls and layers of 33 - 2048 tokens drawn at random: 0.936 x the time, worst
-// 1.05 ([528 x 5728], 162 tokens).
+// 128), 61 shapes of the pair kernel.  Conversion, launch and start; a cost per unit of 128 k on the busiest CTA or pair, where the
+// slower of dequantization and MMAs counts; the parts put together.  The fits are off by 9 % and 4 % (one standard deviation).  The
+// constants before, made for A in shared memory, chose settings 9 % from the best, up to 60 %: 300 - 512 tokens of [4096 x 4096],
+// pairs 28 us, clusters of one 18; [11008 x 4096] Q4_K 128 tokens, 31.5 and 24.  With these, 85 calls and layers of 33 - 2048 tokens
+// drawn at random took 0.936 x the time, worst 1.05 (Q5_0 [528 x 5728], 162 tokens).
 static double split_cost(int qt, int64_t rounds, int units, int ranks, int bm, int64_t m, bool f32) {
     const double b = bm / 128.0, t = (double)m / 256;
     if (f32) {
@@ -127,13 +126,12 @@ static double split_cost(int qt, int64_t rounds, int units, int ranks, int bm, i
     return ranks == 1 ? 2.5 + 0.7 * t + (double)rounds * (units * unit + 1.3 + 0.25 * b) : 3.8 + 1.5 * t + (double)rounds * (units * unit + 3.6 * b);
 }
 // share: units of the busiest pair; a tile of U units is put together from the pieces of U / share pairs
-static double pair_cost(int qt, int64_t share, int k_blocks, int halves, int64_t m) {
-    const double t = 11.3 + 3.5 * (double)m / 1024, pieces = (double)k_blocks / (double)share;
-    if (halves == 2) return t + 1.6 + (double)share * 1.7 + pieces * 1.6;
-    return t + (double)share * (qt == WF_QTYPE_Q4_0 || qt == WF_QTYPE_Q4_1 ? 0.83 : 0.96) + pieces * 1.1;
+static double pair_cost(int qt, int64_t share, int k_blocks, int bm, int64_t m) {
+    const double b = bm / 256.0, dequant = qt == WF_QTYPE_Q4_0 ? 0.45 : qt == WF_QTYPE_Q4_1 ? 0.5 : qt == WF_QTYPE_Q8_0 ? 0.62 : 0.6;
+    return 14.4 + 2.0 * (double)m / 1024 + (double)share * std::max(dequant, 0.79 * b) + 1.6 * b * (double)k_blocks / (double)share;
 }
 // Where two ways are close, the one that the fits know better: smaller token tiles and clusters instead of pairs have to promise as much.
-constexpr double SMALLER_TILES_GAIN = 0.92, CLUSTERS_GAIN = 0.95;
+constexpr double SMALLER_TILES_GAIN = 0.92, CLUSTERS_GAIN = 0.97;
 
 // CTAs per tile of the split kernel, the cheapest by split_cost.
 static int split_ranks(const GemmDevice& d, int qt, int64_t tiles, int k_blocks, int bm, int64_t m, bool f32, double* cost) {
@@ -253,36 +251,26 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
         p.ranks = ranks;
     }
     clusters = (int)std::min<int64_t>(dev->clusters[p.ranks], (int64_t)p.n_tiles * p.m_tiles);
-    // Pairs of CTAs on tiles of 256 rows x 512 or 256 tokens, stream-K shares.  A tile of U units shared by n pairs costs about U / n
-    // units plus n - 1 pieces added by its owner, a piece costing about two units: no share is shorter than sqrt(2 U)
-    // units, which bounds n for weights with few tiles.
-    const int pair_n = (int)((w.g.rows + 2 * GEMM_BN - 1) / (2 * GEMM_BN));
+    // Pairs of CTAs on tiles of 256 rows x up to 256 tokens (of one size, in steps of 32), stream-K shares.  A tile of U units shared by n
+    // pairs costs about U / n units plus n - 1 pieces added by its owner, a piece costing about two units: no share is shorter
+    // than sqrt(2 U) units, which bounds n for weights with few tiles.
+    const int pair_n = (int)((w.g.rows + 2 * GEMM_BN - 1) / (2 * GEMM_BN)), pair_m = (int)((call.m + PAIR_TOKENS - 1) / PAIR_TOKENS);
+    const int pair_bm = (int)(((call.m + pair_m - 1) / pair_m + 31) / 32 * 32);
     int min_units = 1;
     while ((int64_t)min_units * min_units < 2 * p.k_blocks) min_units++;
-    int64_t units = 0;
-    int workers = 0;
-    bool pair = false;
-    for (int halves = 1; halves <= 2 && !f32 && call.m > 64 && dev->pairs > 0; halves++) {
-        const int64_t u = (int64_t)pair_n * ((call.m + halves * 256 - 1) / (halves * 256)) * p.k_blocks;
-        const int n = (int)std::min<int64_t>(dev->pairs, std::max<int64_t>(1, u / min_units));
-        const double t = CLUSTERS_GAIN * pair_cost(qt, (u + n - 1) / n, p.k_blocks, halves, call.m);
-        if (t >= cost) continue;
-        cost = t;
-        pair = true;
-        p.halves = halves;
-        units = u;
-        workers = n;
-    }
+    const int64_t units = (int64_t)pair_n * pair_m * p.k_blocks;
+    const int workers = (int)std::min<int64_t>(dev->pairs, std::max<int64_t>(1, units / min_units));
+    const bool pair = !f32 && call.m > 64 && dev->pairs > 0 && CLUSTERS_GAIN * pair_cost(qt, (units + workers - 1) / workers, p.k_blocks, pair_bm, call.m) < cost;
     if (std::max(units, (int64_t)p.n_tiles * p.m_tiles * p.k_blocks) >= (1LL << 30)) return set_error(c, WF_ERR_TOO_LARGE, "GEMM has too many tile steps");
     if (pair) {
-        p.bm = 256;
+        p.bm = pair_bm;
         p.n_tiles = pair_n;
-        p.m_tiles = (int)((call.m + p.halves * 256 - 1) / (p.halves * 256));
+        p.m_tiles = pair_m;
         p.unit_q = (int)(units / workers);
         p.unit_r = (int)(units % workers);
         cluster = 2;
         grid = 2 * workers;
-        stage_bytes = (size_t)pair_stage_bytes(p.halves);
+        stage_bytes = PAIR_STAGE;
     } else {
         cluster = p.ranks;
         grid = clusters * cluster;
@@ -297,7 +285,7 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
         stage_bytes = (size_t)split_stage_bytes(planes, p.bm);
         exchange = (size_t)split_exchange_bytes(f32 ? 2 : 1, p.bm, cluster);
     }
-    p.stages = (int)std::min<size_t>((GEMM_SMEM_LIMIT - 1024 - exchange) / stage_bytes, pair || f32 ? 8 : split_a_stages(1, p.bm));
+    p.stages = (int)std::min<size_t>((GEMM_SMEM_LIMIT - 1024 - exchange) / stage_bytes, pair ? PAIR_STAGES : f32 ? 8 : split_a_stages(1, p.bm));
     // A = fp16 weights, B = fp16 activations, D = fp32; both operands K-major
     p.idesc = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(p.bm >> 3) << 17) | ((uint32_t)((pair ? 2 * GEMM_BN : GEMM_BN) >> 4) << 24);
 
@@ -320,7 +308,7 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     CUtensorMap map;
     const cuuint64_t dims[2] = {(cuuint64_t)kx, (cuuint64_t)(call.m * planes)};
     const cuuint64_t strides[1] = {(cuuint64_t)kx * 2};
-    const cuuint32_t box[2] = {64, (cuuint32_t)(pair ? 128 : p.bm)};
+    const cuuint32_t box[2] = {64, (cuuint32_t)(pair ? p.bm / 2 : p.bm)};
     const cuuint32_t estr[2] = {1, 1};
     CUresult r = encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x16, dims, strides, box, estr,
                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -337,19 +325,18 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         const bool alone = pair && w.g.k > CONVERT_KEEP_SHORT * CONVERT_THREADS * 8;
-        const auto convert = f32     ? convert_rows_kernel<3, 2, TMEM_ORDER>
-                             : !pair ? convert_rows_kernel<1, CONVERT_KEEP_SHORT, TMEM_ORDER>
-                             : alone ? convert_rows_kernel<1, CONVERT_KEEP_LONG, SMEM_ORDER>
-                                     : convert_rows_kernel<1, CONVERT_KEEP_SHORT, SMEM_ORDER>;
+        const auto convert = f32     ? convert_rows_kernel<3, 2>
+                             : alone ? convert_rows_kernel<1, CONVERT_KEEP_LONG>
+                                     : convert_rows_kernel<1, CONVERT_KEEP_SHORT>;
         WF_CUDA(c, cudaLaunchKernelEx(&cfg, convert, call.d_x, x16, unscale, (int)call.m, (int)w.g.k));
     }
     c->launches++;
-    const size_t smem = 1024 + (size_t)p.stages * stage_bytes + exchange;
+    const size_t smem = pair ? PAIR_SMEM : 1024 + (size_t)p.stages * stage_bytes + exchange;
     auto launch = [&](auto tag) {
         constexpr int QT = decltype(tag)::value;
-        return pair  ? gemm_launch_one(gemm_pair_kernel<QT>, p, map, GEMM_THREADS, grid, cluster, smem, s)
-               : f32 ? gemm_launch_one(gemm_split_kernel<QT, 2, 3>, p, map, SPLIT_THREADS, grid, cluster, smem, s)
-                     : gemm_launch_one(gemm_split_kernel<QT, 1, 1>, p, map, SPLIT_THREADS, grid, cluster, smem, s);
+        return pair  ? gemm_launch_one(gemm_pair_kernel<QT>, p, map, grid, cluster, smem, s)
+               : f32 ? gemm_launch_one(gemm_split_kernel<QT, 2, 3>, p, map, grid, cluster, smem, s)
+                     : gemm_launch_one(gemm_split_kernel<QT, 1, 1>, p, map, grid, cluster, smem, s);
     };
     const cudaError_t e = qt == WF_QTYPE_Q4_0   ? launch(std::integral_constant<int, WF_QTYPE_Q4_0>{})
                           : qt == WF_QTYPE_Q4_1 ? launch(std::integral_constant<int, WF_QTYPE_Q4_1>{})

@@ -11,12 +11,13 @@
 namespace wf {
 
 constexpr int GEMM_BN = 128;             // weight rows per CTA and tile (UMMA M per CTA)
-constexpr int GEMM_BK = 128;             // k per unit of the work split: two stages of 64 k
-constexpr int GEMM_DEQUANT_WARPS = 8;    // a set: a 16-row weight tile each (A in shared memory, sixteen of eight rows: 3 - 14 % slower)
-constexpr int GEMM_THREADS = (6 + GEMM_DEQUANT_WARPS) * 32;  // TMA, MMA, 4 epilogue, dequant warps
+constexpr int GEMM_BK = 128;             // k per unit of the work split
+constexpr int GEMM_DEQUANT_WARPS = 8;    // of a set: a 16-row weight tile each
+constexpr int GEMM_SETS = 2;             // sets, which take units by turns
+constexpr int GEMM_THREADS = (6 + GEMM_SETS * GEMM_DEQUANT_WARPS) * 32;  // TMA, MMA, 4 epilogue, dequantization warps
 constexpr int GEMM_WAIT_SPINS = 1 << 20;    // of an mbarrier wait, which suspends the thread for microseconds per try
 constexpr int GEMM_POLL_SPINS = 1 << 22;    // of a poll of global memory
-constexpr int GEMM_PIECE_TOKENS = 512;   // tokens a stream-K piece can hold
+constexpr int GEMM_PIECE_TOKENS = 256;   // tokens a stream-K piece can hold
 
 struct GemmParams {
     const uint8_t* tiles;
@@ -27,10 +28,9 @@ struct GemmParams {
     int rows, kt_w;      // kt_w: weight k-tiles per row-tile stripe (tile_k of the format)
     int rt_last;         // last row-tile in the weight buffer
     int m;               // tokens
-    int bm;              // tokens per MMA (UMMA N: multiple of 16, <= 256)
+    int bm;              // tokens of a tile (UMMA N: multiple of 16, pairs of 32, <= 256)
     int n_tiles, m_tiles, k_blocks;  // k_blocks = ceil(k / 128)
-    int stages;
-    int halves;          // pair kernel: 256-token halves of a token tile, 1 or 2
+    int stages;          // split kernel
     int ranks;           // split kernel: CTAs of a cluster, which share a tile's K
     int early;           // split kernel: let the next kernel be placed while this one runs
     uint32_t idesc;
@@ -122,46 +122,32 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(void* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(g_smem_u32(bar)) : "memory");
 }
-// One 64-k span of a tile: four MMAs of 16 k, 32 bytes (two descriptor units) apart in the swizzled rows.  Issued by the
-// thread whose `issue` is non-zero; the whole warp comes here with the same operands, which therefore sit in uniform
-// registers.  (Issued from a branch of one lane, every operand had to be moved there, and at about 200 cycles per MMA
+// One 64-k span of a tile: four MMAs of 16 k, A in TMEM (eight columns each), B 32 bytes (two descriptor units) apart in the swizzled
+// rows.  Issued by the thread whose `issue` is non-zero; the whole warp comes here with the same operands, which therefore sit in
+// uniform registers.  (Issued from a branch of one lane, every operand had to be moved there, and at about 200 cycles per MMA
 // the issuing thread, not the tensor core with its 128, set the pace.)  accumulate: 0 = the first MMA starts from zero.
-template <int GROUP> __device__ __forceinline__ void tc_mma_span(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t issue) {
-#define WF_MMA_SPAN(G)                                                                    \
+// With A in TMEM the tensor core reads only B from shared memory, and keeps its pace for any N from 32 on (cycles per MMA of 128 rows x 16 k, A in shared memory / in TMEM, measured: N = 16: 39 / 11, 48: 44 / 24,
+// 96: 56 / 48, 128: 64 / 64).
+template <int GROUP> __device__ __forceinline__ void tc_mma_span(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t issue) {
+#define WF_MMA_SPAN(G)                                                                 \
     asm volatile(                                                                         \
-        "{\n\t.reg .pred p, e, t;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"               \
-        "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"        \
-        "add.s64 a1, %1, 2;\n\tadd.s64 a2, %1, 4;\n\tadd.s64 a3, %1, 6;\n\t"               \
-        "add.s64 b1, %2, 2;\n\tadd.s64 b2, %2, 4;\n\tadd.s64 b3, %2, 6;\n\t"               \
-        "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], %1, %2, %3, p;\n\t"              \
-        "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], a1, b1, %3, t;\n\t"              \
-        "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], a2, b2, %3, t;\n\t"              \
-        "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], a3, b3, %3, t;\n\t}" ::"r"(d_tmem), \
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue)                   \
+        "{\n\t.reg .pred p, e, t;\n\t.reg .b32 a1, a2, a3;\n\t.reg .b64 b1, b2, b3;\n\t"  \
+        "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"      \
+        "add.s32 a1, %1, 8;\n\tadd.s32 a2, %1, 16;\n\tadd.s32 a3, %1, 24;\n\t"            \
+        "add.s64 b1, %2, 2;\n\tadd.s64 b2, %2, 4;\n\tadd.s64 b3, %2, 6;\n\t"              \
+        "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], [%1], %2, %3, p;\n\t"           \
+        "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], [a1], b1, %3, t;\n\t"           \
+        "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], [a2], b2, %3, t;\n\t"           \
+        "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], [a3], b3, %3, t;\n\t}" ::"r"(d_tmem), \
+        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue)                  \
         : "memory")
     if (GROUP == 1) WF_MMA_SPAN("1");
     else WF_MMA_SPAN("2");
 #undef WF_MMA_SPAN
 }
-// The same with A in TMEM (cta_group::1): 16 k are eight columns there.  The tensor core then reads only B from shared memory, and keeps
-// its pace for any N from 32 on (cycles per MMA of 128 rows x 16 k, A in shared memory / in TMEM, measured: N = 16: 39 / 11, 48: 44 / 24,
-// 96: 56 / 48, 128: 64 / 64).
-__device__ __forceinline__ void tc_mma_span_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t issue) {
-    asm volatile(
-        "{\n\t.reg .pred p, e, t;\n\t.reg .b32 a1, a2, a3;\n\t.reg .b64 b1, b2, b3;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
-        "add.s32 a1, %1, 8;\n\tadd.s32 a2, %1, 16;\n\tadd.s32 a3, %1, 24;\n\t"
-        "add.s64 b1, %2, 2;\n\tadd.s64 b2, %2, 4;\n\tadd.s64 b3, %2, 6;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, t;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, t;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue)
-        : "memory");
-}
 // 16 rows x 64 k of fp16 into 16 lanes x 32 columns of TMEM.  A lane holds rows g = lane / 4 (r0) and g + 8 (r1), of either 32-k block the
 // eight elements 8 q .. 8 q + 7 (q = lane % 4): of each 16-byte piece the first half goes into the columns of one MMA, the
-// second into those of the next (order of k: stage_piece).
+// second into those of the next (order of k: span_piece).
 __device__ __forceinline__ void tmem_st_span(uint32_t taddr, const uint4& r0b0, const uint4& r0b1, const uint4& r1b0, const uint4& r1b1) {
     asm volatile(
         "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
@@ -239,16 +225,11 @@ __device__ __forceinline__ void tmem_ld_accs(uint32_t taddr, int bm, uint32_t (&
     for (int j = 0; j < 16; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(e[j]));
 }
 
-// ---------------------------------------------------------------- the order of k inside a stage
-// A stage row is 64 k = eight 16-byte chunks; group q (eight k) of 32-k block j lies in chunk 2 q + j, in the weights' rows and
-// the activations' alike (the sum does not care).  A lane stores group q of both blocks of a row; a 16-byte shared-memory
-// store is served eight lanes at a time, two neighbouring rows x four groups of one block, which under the 128-byte
-// swizzle meet eight different chunks this way.  With the blocks one after the other they met four, a two-way conflict.
-__host__ __device__ inline int stage_chunk(int j, int q) { return 2 * q + j; }
-// Where the weights go to TMEM (tmem_st_span), elements 8 q + 4 h .. + 3 of block j are the q-th quarter of the 16 k of MMA 2 j + h: as
-// 8-byte pieces of a stage row, piece 4 (2 j + h) + q.
-__host__ __device__ inline int stage_piece(int j, int q, int h) { return 4 * (2 * j + h) + q; }
-enum RowOrder { SMEM_ORDER, TMEM_ORDER };
+// ---------------------------------------------------------------- the order of k inside a span
+// 64 k are four MMAs of 16.  What tmem_st_span does with the weights makes elements 8 q + 4 h .. + 3 of 32-k block j the q-th quarter of
+// the 16 k of MMA 2 j + h, so a row of activations has them, as 8-byte pieces of its 128 bytes, at piece 4 (2 j + h) + q (the sum
+// does not care).
+__host__ __device__ inline int span_piece(int j, int q, int h) { return 4 * (2 * j + h) + q; }
 
 // ---------------------------------------------------------------- activations to fp16
 // x16 = fp16(x * 2^s) with s chosen so that the largest magnitude of the row lands in [2^14, 2^15), or 126
@@ -256,7 +237,7 @@ enum RowOrder { SMEM_ORDER, TMEM_ORDER };
 //   bf16 (PLANES 1): exact whenever the scaled value is a normal fp16.
 //   fp32 (PLANES 3): v = hi + mid + lo, each the fp16 nearest to what is left: exact down to 2^-39 of the largest
 //   (below that, what fp32 rounding leaves of a sum that the largest takes part in).
-// Rows are padded to whole stages of 64 k (zeros) and lie in the stages' order of k.
+// Rows are padded to whole spans of 64 k (zeros) and lie in the spans' order of k.
 template <int PLANES> struct RowGroup {  // eight elements of a row
     uint4 a, b;                          // b: fp32 only
     __device__ __forceinline__ void load(const void* row, int i) {
@@ -324,7 +305,7 @@ __device__ __forceinline__ float2 row_scale(int emax) {
 constexpr int CONVERT_THREADS = 256;
 constexpr int CONVERT_KEEP_SHORT = 2;  // rows of 4096 (bf16)
 constexpr int CONVERT_KEEP_LONG = 4;   // rows of 8192
-template <int PLANES, int KEEP, RowOrder ORDER>
+template <int PLANES, int KEEP>
 __global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 && KEEP == CONVERT_KEEP_SHORT ? 8 : 5) convert_rows_kernel(const void* x, __half* __restrict__ x16, float* __restrict__ unscale,
                                                                        int m, int k) {
     __shared__ int s_max[CONVERT_THREADS / 32];
@@ -369,14 +350,10 @@ __global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 && KEEP == CONVER
     const float2 scale = row_scale(emax);
     uint4* out = reinterpret_cast<uint4*>(x16) + (size_t)row * padded;
     auto store = [&](int pl, int i, const uint4& v) {  // group i of the row
-        uint4* const stage = out + pl * plane + (i & ~7);
+        uint2* const span = reinterpret_cast<uint2*>(out + pl * plane + (i & ~7));
         const int j = (i >> 2) & 1, q = i & 3;
-        if (ORDER == SMEM_ORDER) {
-            stage[stage_chunk(j, q)] = v;
-        } else {
-            reinterpret_cast<uint2*>(stage)[stage_piece(j, q, 0)] = make_uint2(v.x, v.y);
-            reinterpret_cast<uint2*>(stage)[stage_piece(j, q, 1)] = make_uint2(v.z, v.w);
-        }
+        span[span_piece(j, q, 0)] = make_uint2(v.x, v.y);
+        span[span_piece(j, q, 1)] = make_uint2(v.z, v.w);
     };
     auto convert = [&](int i, const RowGroup<PLANES>& v) {
         v.convert(scale.x, [&](int pl, const uint4& o) { store(pl, i, o); });

@@ -11,7 +11,7 @@
 //
 // A lies in TMEM, not in shared memory: the weights' fragment order is that of a 16x256b store, so a dequantizing lane's registers go
 // there as they are, without addresses, bank conflicts or a proxy fence; the tensor core keeps its pace at any token count
-// (tc_mma_span_ts), and shared memory is left to the activations, which for fp32 tokens bounded the kernel (416 KB per 128 k and
+// (tc_mma_span), and shared memory is left to the activations, which for fp32 tokens bounded the kernel (416 KB per 128 k and
 // 96 tokens, 3250 cycles, where the products take 1900).  Two sets of eight dequantizing warps instead of one.  us a call,
 // with A in shared memory and eight warps / so: Q4_0 [16384 x 2048] 128 tokens 16.4 / 13.1, Q8_0 [4096 x 11008] 96 tokens 28.7 /
 // 25.0, Q4_1 [11008 x 4096] 96 fp32 tokens 44.4 / 39.0.
@@ -47,8 +47,6 @@ namespace wf {
 
 constexpr int SPLIT_MAX_STAGES = 8, SPLIT_MAX_RANKS = 8, SPLIT_MAX_TOKENS = 128;
 constexpr int SPLIT_FLUSH = 4;  // units of 128 k the accumulators of a PIECES 2 kernel take before they are drained
-constexpr int SPLIT_SETS = 2;   // sets of GEMM_DEQUANT_WARPS
-constexpr int SPLIT_THREADS = (6 + SPLIT_SETS * GEMM_DEQUANT_WARPS) * 32;
 
 inline __host__ __device__ int split_stage_bytes(int planes, int bm) { return (planes == 1 ? 2 : planes) * bm * 128; }  // of activations
 // Stages of weights that TMEM has room for: 4 of 128 k, or 2 - 6 of 64 k for fp32 tokens, an even number.
@@ -74,7 +72,7 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
     // The two sets of dequantization warps take units by turns (bf16), or a stage each of every unit (fp32: there may be no more than two
     // stages, and a set that came back to one only after the other set's turn could not tell by the barrier's parity whether that
     // turn is over).
-    constexpr int TURN = PIECES == 1 ? SPLIT_SETS : 1;
+    constexpr int TURN = PIECES == 1 ? GEMM_SETS : 1;
     using Regs = std::conditional_t<PIECES == 1, DequantRegs<QT>, DequantHalf<QT>>;
     constexpr int DEPTH = 2;  // units a dequantization warp holds: one is converted while the other loads
     constexpr int COLS = PIECES == 1 ? 32 : 16; // that an epilogue warp takes at a time
@@ -214,14 +212,14 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
                     const uint64_t bd = b_desc0 + (uint64_t)((uint32_t)s * stage_bytes >> 4);
                     const uint32_t hi = a_tmem + (uint32_t)(JOINT ? s : a_at.s) * A_COLS, lo = hi + 32;
                     const uint32_t acc = (uint32_t)(st - 2 * g0);
-                    tc_mma_span_ts(d_tmem, hi, bd, p.idesc, acc, issue);
+                    tc_mma_span<1>(d_tmem, hi, bd, p.idesc, acc, issue);
                     if (JOINT) {
-                        tc_mma_span_ts(d_tmem, lo, bd + span, p.idesc, 1u, issue);
+                        tc_mma_span<1>(d_tmem, lo, bd + span, p.idesc, 1u, issue);
                     } else {
-                        tc_mma_span_ts(e_tmem, lo, bd, p.idesc, acc, issue);
-                        tc_mma_span_ts(e_tmem, hi, bd + span, p.idesc, 1u, issue);
-                        tc_mma_span_ts(e_tmem, lo, bd + span, p.idesc, 1u, issue);
-                        tc_mma_span_ts(e_tmem, hi, bd + 2 * span, p.idesc, 1u, issue);
+                        tc_mma_span<1>(e_tmem, lo, bd, p.idesc, acc, issue);
+                        tc_mma_span<1>(e_tmem, hi, bd + span, p.idesc, 1u, issue);
+                        tc_mma_span<1>(e_tmem, lo, bd + span, p.idesc, 1u, issue);
+                        tc_mma_span<1>(e_tmem, hi, bd + 2 * span, p.idesc, 1u, issue);
                     }
                     if (issue) {  // frees the stages when these MMAs have read them
                         if (!JOINT) tc_commit(&a_empty[a_at.s]);

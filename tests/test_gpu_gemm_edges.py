@@ -1,6 +1,5 @@
-"""The tensor-core kernels at the edges of their tiles: CTA pairs (256 rows x 512 or 256 tokens; the cost function takes them
-from 65 tokens on where there are tiles enough) and K-splitting clusters (128 rows x 128 tokens; ranks with no tokens of their own to finish, several tiles per
-cluster), K that ends inside a stage of 64, and fp32 tokens.
+"""The tensor-core kernels at the edges of their tiles: K-splitting clusters (128 rows x 128 tokens; ranks with no tokens of their own to finish, several tiles per
+cluster, clusters of one), CTA pairs (256 rows x up to 256 tokens; the cost function takes them where there are tiles enough), K that ends inside a span of 64, and fp32 tokens.
 
 bf16 tokens: the bars of test_gpu_gemm.py.  fp32 tokens: products are exact to 2^-22 and an accumulator takes at most 32
 steps between two drains, each cutting the partial sum off at its 24th bit: 32 x 2^-23 = 3.8e-6 of the result at
@@ -41,10 +40,10 @@ def _run(backend, oracle, name, rows, k, x, tensor):
 
 @pytest.mark.parametrize("name", sorted(QT))
 @pytest.mark.parametrize("rows,k,m", [
-    (130, 352, 33), (1000, 1120, 80), (700, 5152, 77), (2500, 672, 128),  # clusters; K ends inside a stage
-    (3000, 544, 129), (3072, 1024, 257), (2900, 288, 513), (1600, 2080, 1100),  # pairs; 129 tokens: one half, 257: the next begins
+    (130, 352, 33), (1000, 1120, 80), (700, 5152, 77), (2500, 672, 128),  # clusters; K ends inside a span
+    (3000, 544, 129), (3072, 1024, 257), (2900, 288, 513), (1600, 2080, 1100),  # clusters of one, on several token tiles of 64 to 128
     (300, 800, 300), (128, 4128, 600),  # few tiles: clusters on several token tiles
-    (2900, 4096, 300), (2900, 4128, 129), (2900, 8192, 130), (2900, 8224, 300),  # pairs; K at the ends of what the conversion's two forms hold
+    (2900, 4096, 300), (2900, 4128, 129), (2900, 8192, 130), (2900, 8224, 300),  # K at the ends of what the conversion holds of a row
 ])
 def test_bf16_tokens(backend, oracle, name, rows, k, m):
     from warpforge_b200.backend import Tensor
@@ -60,9 +59,10 @@ def test_bf16_tokens(backend, oracle, name, rows, k, m):
 
 @pytest.mark.parametrize("name", ["q4_0", "q8_0", "q4_k"])
 @pytest.mark.parametrize("rows,k,m", [
-    (7100, 3104, 1030),  # halves of 256 tokens, rows that the conversion's short form holds
-    (4700, 8224, 520),   # the same, the long form and more than it holds (Q4_0: clusters of two)
-    (5100, 4128, 1000),  # Q8_0, Q4_K: tiles of 512 tokens
+    (7100, 3104, 1030),  # tiles of 224 tokens, rows that the conversion's short form holds
+    (4700, 8224, 520),   # 192 tokens, the long form and more than it holds
+    (5100, 4128, 1000),  # 256 tokens
+    (3600, 8224, 300),   # 160 tokens; few tiles, each cut several times
 ])
 def test_pairs_of_ctas(backend, oracle, name, rows, k, m):
     """Sizes from which the cost functions take the CTA pairs, ragged in rows, K and tokens."""

@@ -243,7 +243,8 @@ __global__ void __launch_bounds__(768, 1) gemm_pair_kernel(const GemmParams p, c
             }
             tc_fence_before();  // the accumulator has been read: the MMA issuer may overwrite it
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_rank(g_smem_u32(acc_empty), 0));
+            // nobody waits for the last segment's word, which could come after the leader has left
+            if (lane == 0 && u + g.kb1 - g.kb0 < u1) mbar_arrive_cluster(map_to_rank(g_smem_u32(acc_empty), 0));
             for (int c = 0; c < cols; c += PAIR_COLS) {  // a lane reads what it wrote
                 uint32_t v[PAIR_COLS];
 #pragma unroll

@@ -59,8 +59,7 @@ inline __host__ __device__ int split_exchange_bytes(int pieces, int bm, int rank
 }
 
 // smem: [0, 1024) barriers, tmem slot | stages of activations, 1024-byte aligned | exchange buffer
-// Registers: 80 a thread, what the hardware has for 24 warps; 22 are launched, and what is left is room for four warps of the next call's
-// conversion.
+// Registers: 80 a thread, what the hardware has for 24 warps (it counts in fours); 22 are launched.
 template <int QT, int PIECES, int PLANES>
 __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap) {
     constexpr int ACCS = PIECES;
@@ -162,9 +161,9 @@ __global__ void __launch_bounds__(768, 1) gemm_split_kernel(const GemmParams p, 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer (activations)
         if (lane == 0) {
-            // The next call's conversion waits beside this kernel, and the next GEMM takes each SM as it becomes free (a call of
+            // The next call's conversion waits on SMs that are idle meanwhile, and the next GEMM takes each SM as it becomes free (a call of
             // [5003 x 2784], 77 tokens, Q4_0: 12.7 -> 11.6 us; 64 tokens of [4096 x 4096], 12.7 -> 11.3).  Placed when the CTA
-            // begins its last tile: a conversion that waits beside longer delays clusters of several tiles ([11008 x 4096], 128
+            // begins its last tile: a conversion that waits longer delays clusters of several tiles ([11008 x 4096], 128
             // tokens, two tiles each: 27.6 us without, 28.9 placed at the start, 27.8 here).  p.early: where it pays (gemm_launch).
             auto last_tile = [&](int tile) {
                 if (p.early && tile + clusters >= tiles) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

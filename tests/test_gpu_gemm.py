@@ -1,5 +1,5 @@
 """GPU parity of the tensor-core prefill GEMM (more than 8 bf16 tokens), through the C ABI,
-against the CPU oracle.  The GEMM rounds each dequantized weight once to fp16 (relative 2^-12)
+against the CPU oracle.  The GEMM rounds each dequantized weight once to fp16 (at most 2^-11)
 and accumulates exact products in fp32, so the bars are: max|d| / max|y| <= 1e-3 (the stated
 tolerance) and rms(d) / rms(y) <= 3e-4; the elementwise 1e-3*|y| rule cannot hold for outputs
 that cancel to nearly zero with any 16-bit weight operand and is reported, not asserted."""
@@ -72,6 +72,33 @@ def test_gemm_wide_dynamic_range_rows(backend, oracle):
         else:
             _check(got[r:r + 1], want[r:r + 1])
     w.close()
+
+
+def test_q4_1_minima_far_below_their_scales(backend, oracle):
+    """scale * code + min is rounded once.  Rows of codes 0 have weights that are their minima, which fp16 holds: y is exact but for
+    the sums (positive terms, of which an accumulation of 16 k cuts the sum and its terms at the 24th bit: 2 * 2^-23 each), though the
+    scales are 2^6 to 2^12 times as large.  Other rows: 2^-11 of each product on top.  A block with an Inf for a scale and no
+    code 0 gives Inf."""
+    rows, k, m = 200, 544, 40
+    rng = np.random.default_rng(41)
+    blocks = Q.synth_q4_1(rows, k, 41).reshape(rows, -1, 20).copy()
+    d = rng.uniform(0.5, 1.0, blocks.shape[:2]).astype(np.float16)
+    blocks[:, :, 0:2] = d[..., None].view(np.uint8)
+    blocks[:, :, 2:4] = (d * 2.0 ** -rng.integers(6, 13, d.shape) * rng.uniform(0.5, 1.0, d.shape)).astype(np.float16)[..., None].view(np.uint8)
+    blocks[:100, :, 4:] = 0
+    blocks[150, 3, 0:2] = np.frombuffer(np.float16(np.inf).tobytes(), np.uint8)
+    blocks[150, 3, 4:] |= 0x11
+    blocks = blocks.reshape(rows, -1)
+    xb = Q.float_to_bf16_bits(rng.uniform(0.5, 1.5, (m, k)).astype(np.float32)).reshape(m, k)
+    w = backend.upload_weight(Q.QuantizationType.Q4_1, blocks, rows, k)
+    got = _gemm(backend, w, xb).astype(np.float64)
+    w.close()
+    want = Q.bf16_bits_to_float(xb).reshape(m, k).astype(np.float64) @ oracle.dequant(O.Q4_1, blocks, rows * k).reshape(rows, k).astype(np.float64).T
+    assert np.all(got[:, 150] == np.inf) and np.all(want[:, 150] == np.inf)
+    got, want = np.delete(got, 150, 1), np.delete(want, 150, 1)
+    sums = 2 * (k / 16) * 2.0 ** -23
+    assert np.all(np.abs(got - want)[:, :100] <= sums * want[:, :100])
+    assert np.all(np.abs(got - want)[:, 100:] <= (sums + 2.0 ** -11) * want[:, 100:])
 
 
 def test_config3_q4k_prefill_sampled_rows(backend, oracle):

@@ -9,7 +9,7 @@
 //                                           also the kernel of fp32 activations
 // dequantizes the weights into TMEM and multiplies.  The launch side and the choice between them are here.
 //
-// bf16 activations: weights are rounded once to fp16 (relative 2^-12) after the exact fp32 dequantization; products
+// bf16 activations: weights are rounded once to fp16 (at most 2^-11 of a weight) after the exact fp32 dequantization; products
 // and sums are fp32 in the tensor core.  Replaces the host transpose + batch_matmul_f32 of
 // warpforge-backend-nvidia/src/main/java/io/surfworks/warpforge/backend/nvidia/ops/DotGeneralKernel.java:169-298.
 #include "wf_gather_route.h"

@@ -491,10 +491,9 @@ __device__ __forceinline__ void words_to_half8x2_q8(uint32_t wh, uint32_t wl, __
     two(q8_pair(h.k[1], l.k[1], ok), hi.z, lo.z);
     two(q8_pair(h.h[1], l.h[1], oh), hi.w, lo.w);
 }
-// Q4_1 and Q4_K: a product of two fp16 plus an fp32 in fp32, rounded once to fp16.  The mixed-precision fma takes the unpacked codes as
-// they are: three operations a pair, where widening first took five (Q4_1: 26 -> 18 operations per eight weights, Q4_K 26 -> 22).  Measured, 33 -
-// 2048 tokens: Q4_1 0.985 x the time (512 tokens of [4096 x 4096] 22.7 -> 21.5 us; worst 1.058, 64 tokens of [11008 x 4096]), Q4_K 0.990 x
-// (128 tokens of [11008 x 4096] 22.8 -> 22.3).
+// Q4_1 and Q4_K: a product of two fp16 plus an fp32 in fp32, rounded once to fp16.  The mixed-precision fma takes the codes as fp16:
+// three operations a pair, where widening first took five (Q4_1 and Q4_K 26 -> 22 operations per eight weights; 33 - 2048 tokens of Q4_K
+// 0.990 x the time).
 __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
     __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
@@ -508,11 +507,13 @@ __device__ __forceinline__ uint32_t fma_pair(uint32_t h2, uint32_t s, float c) {
         : "r"(h2), "r"(s), "f"(c));
     return pack_half2(x, y);
 }
-// Q4_1: scale * code + min; the unpacked values carry 1024 / 64
+// Q4_1: scale * code + min.  The 1024 or 64 that the unpacked code carries is taken off in fp16, exactly; taken off as a multiple of the
+// scale inside the min, it cost up to 2^-14 of the scale, which a min of 2^-8 of the scale shows in its sixth bit, and made
+// every weight of a block whose scale is Inf a NaN ([11008 x 4096], 33 tokens: 17.6 us so, 17.2 now; [8192 x 8192], 1024: 105.7, 105.5).
 __device__ __forceinline__ uint4 word_to_half8_q4_1(uint32_t w, uint32_t s, float m) {
     const Codes8 c = unpack8(w);
-    const float sf = __low2float(as_half2(s)), bk = fmaf(-1024.f, sf, m), bh = fmaf(-64.f, sf, m);
-    return make_uint4(fma_pair(c.k[0], s, bk), fma_pair(c.h[0], s, bh), fma_pair(c.k[1], s, bk), fma_pair(c.h[1], s, bh));
+    auto code = [](uint32_t v, float off) { return as_u32(__hadd2(as_half2(v), __float2half2_rn(off))); };
+    return make_uint4(fma_pair(code(c.k[0], -1024.f), s, m), fma_pair(code(c.h[0], -64.f), s, m), fma_pair(code(c.k[1], -1024.f), s, m), fma_pair(code(c.h[1], -64.f), s, m));
 }
 // Q4_K: d * (sc * code) + b, b = -dmin * m: sc * code, at most 945, is exact in fp16
 __device__ __forceinline__ uint4 word_to_half8_q4_k(uint32_t w, __half2 sc, uint32_t d, float b) {

@@ -74,6 +74,32 @@ def test_gemm_wide_dynamic_range_rows(backend, oracle):
     w.close()
 
 
+@pytest.mark.parametrize("name", sorted(QT))
+@pytest.mark.parametrize("f32", [False, True])
+def test_every_weight_by_itself(backend, oracle, name, f32):
+    """Tokens with a single 1: y is each weight as the tensor core got it, rounded once to fp16, or for fp32 tokens as two fp16 (22 bits).
+    Q8_0 with every byte there is, -128 included."""
+    from warpforge_b200.backend import DotGeneralOp, LINEAR_DIMS, Tensor
+
+    qt, oq = QT[name]
+    rows, k = 272, 512
+    blocks = Q.synth_weight(qt, rows, k, 71)
+    if name == "q8_0":
+        blocks = blocks.reshape(rows, -1, 34).copy()
+        blocks[:, :, 2:] = np.random.default_rng(71).integers(0, 256, blocks[:, :, 2:].shape)
+        blocks = blocks.reshape(rows, -1)
+    w = backend.upload_weight(qt, blocks, rows, k)
+    x = np.eye(k, dtype=np.float32)
+    t = Tensor.from_float_array(x) if f32 else Tensor.from_bf16_bits(Q.float_to_bf16_bits(x).reshape(k, k))
+    got = backend.execute(DotGeneralOp(LINEAR_DIMS, (k, rows)), [t, w])[0].data.T
+    w.close()
+    want = oracle.dequant(oq, blocks, rows * k).reshape(rows, k)
+    if f32:
+        assert np.all(np.abs(got.astype(np.float64) - want) <= 2.0 ** -22 * np.abs(want))
+    else:
+        assert np.array_equal(got, want.astype(np.float16).astype(np.float32))
+
+
 def test_q4_1_minima_far_below_their_scales(backend, oracle):
     """scale * code + min is rounded once.  Rows of codes 0 have weights that are their minima, which fp16 holds: y is exact but for
     the sums (positive terms, of which an accumulation of 16 k cuts the sum and its terms at the 24th bit: 2 * 2^-23 each), though the

@@ -121,7 +121,7 @@ static double split_cost(int qt, int64_t rounds, int units, int ranks, int bm, i
         const double unit = std::max(dequant, 0.56 + 1.12 * b);
         return ranks == 1 ? 3.5 + 1.6 * t + (double)rounds * units * unit : 5.0 + 4.3 * t + (double)rounds * (units * unit + 0.6 * b);
     }
-    const double dequant = qt == WF_QTYPE_Q4_0 ? 0.37 : qt == WF_QTYPE_Q4_1 ? 0.42 : qt == WF_QTYPE_Q8_0 ? 0.52 : 0.53;
+    const double dequant = qt == WF_QTYPE_Q4_0 ? 0.37 : qt == WF_QTYPE_Q4_1 ? 0.42 : qt == WF_QTYPE_Q8_0 ? 0.45 : 0.53;
     const double unit = std::max(dequant, 0.07 + 0.35 * b);
     return ranks == 1 ? 2.5 + 0.7 * t + (double)rounds * (units * unit + 1.3 + 0.25 * b) : 3.8 + 1.5 * t + (double)rounds * (units * unit + 3.6 * b);
 }

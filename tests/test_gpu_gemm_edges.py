@@ -76,6 +76,31 @@ def test_pairs_of_ctas(backend, oracle, name, rows, k, m):
     assert np.linalg.norm(got - want) <= 3e-4 * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("name,rows,k,m", [  # weights of 37 MB and more, 132 MB read again
+    ("q8_0", 6000, 6016, 1200),  # one whole tile a pair, then 29 of 47 units
+    ("q5_0", 6000, 6016, 2000),  # two
+    ("q4_k", 8100, 7936, 1100),  # one; the rest is more than a tile a pair
+    ("q4_0", 8190, 8224, 1030),
+    ("q4_1", 7700, 8000, 1100),
+])
+def test_pairs_that_take_whole_tiles_first(backend, oracle, name, rows, k, m):
+    """Three rows of every 128, all tokens."""
+    from warpforge_b200.backend import DotGeneralOp, LINEAR_DIMS, Tensor
+
+    qt = Q.QuantizationType[name.upper()]
+    blocks = Q.synth_weight(qt, rows, k, rows + m)
+    bits = Q.synth_activation_bf16(m, k, rows + m)
+    w = backend.upload_weight(qt, blocks, rows, k)
+    got = [backend.execute(DotGeneralOp(LINEAR_DIMS, (m, rows)), [Tensor.from_bf16_bits(bits), w])[0].data for _ in range(2)]
+    w.close()
+    assert np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
+    sample = np.unique(np.concatenate([np.arange(0, rows, 128), np.minimum(np.arange(127, rows + 127, 128), rows - 1), np.arange(rows // 128) * 128 + 61]))
+    want = Q.bf16_bits_to_float(bits).reshape(m, k).astype(np.float64) @ oracle.dequant(QT[name], blocks[sample], len(sample) * k).reshape(-1, k).astype(np.float64).T
+    d = got[0][:, sample] - want
+    assert np.max(np.abs(d)) <= 1e-3 * np.max(np.abs(want))
+    assert np.linalg.norm(d) <= 3e-4 * np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("name,f32", [("q4_0", False), ("q8_0", False), ("q4_k", False), ("q4_1", True), ("q8_0", True), ("q4_k", True)])
 @pytest.mark.parametrize("rows,k,tokens", [
     (20600, 128, (40,)),  # more tiles than clusters of one unit each: the sets of dequantizing warps take tiles by turns

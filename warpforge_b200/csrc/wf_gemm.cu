@@ -75,8 +75,12 @@ template <int QT> static cudaError_t gemm_prepare(int device, GemmDevice** out) 
     if (d.ready) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel<QT, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_split_kernel<QT, 2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
-    if (e == cudaSuccess) e = max_clusters(gemm_pair_kernel<QT>, 2, &d.pairs);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<QT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<QT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_LIMIT);
+    if (e == cudaSuccess) e = max_clusters(gemm_pair_kernel<QT, false>, 2, &d.pairs);
+    int waved = 0;
+    if (e == cudaSuccess) e = max_clusters(gemm_pair_kernel<QT, true>, 2, &waved);
+    d.pairs = std::min(d.pairs, waved);
     for (int n = 1; n <= SPLIT_MAX_RANKS && e == cudaSuccess; n++) {
         e = max_clusters(gemm_split_kernel<QT, 1, 1>, n, &d.clusters[n]);
         // one fewer than the device says: a cluster that does not find its place in the first wave costs a whole round
@@ -132,6 +136,22 @@ static double pair_cost(int qt, int64_t share, int k_blocks, int bm, int64_t m) 
 }
 // Where two ways are close, the one that the fits know better: smaller token tiles and clusters instead of pairs have to promise as much.
 constexpr double SMALLER_TILES_GAIN = 0.92, CLUSTERS_GAIN = 0.97;
+
+// Whole tiles that each pair takes before the units of the rest are dealt.  A weight is read once per token tile, and where its tiles lie in
+// shares one behind the other, the pairs that read the same rows do so at different times: what does not stay in the L2 comes from
+// memory each time (Q8_0 [8192 x 8192], 2000 tokens, 8 token tiles: 570 MB; 194 with waves, whose neighbours walk the same rows in step).
+// The pieces of the rest meet at the very end then, and nothing hides that: it has to be 24 units a pair.  us without / with waves:
+//   a larger weight: Q8_0 [8192 x 8192] 2048 tokens 236 / 209, 1024 tokens 115 / 110, 768 tokens (19 units left) 89.4 / 89.8, [28672 x 4096]
+//   600 tokens 136 / 121, [12288 x 4096] 1024 tokens 86.5 / 85, Q4_0 [8192 x 8192] 2048 tokens (37.7 MB) 202 / 196
+//   less of it, or less read again: Q8_0 [8192 x 4096] 1024 tokens (35.7 MB) 62.1 / 62.5, Q4_K [14336 x 4096] 1024 tokens (34 MB) 94 / 95,
+//   Q8_0 [20000 x 2048] 1024 tokens (131 MB read again) 77.7 / 79.3
+constexpr int64_t WAVES_WEIGHT_BYTES = 37000000, WAVES_BYTES_AGAIN = 132000000, WAVES_REST_UNITS = 24;
+static int64_t pair_waves(int64_t tiles, int64_t workers, int k_blocks, int token_tiles, int64_t weight_bytes) {
+    if (weight_bytes < WAVES_WEIGHT_BYTES || (token_tiles - 1) * weight_bytes < WAVES_BYTES_AGAIN) return 0;
+    int64_t waves = tiles / workers;
+    while (waves > 0 && (tiles - waves * workers) * k_blocks < WAVES_REST_UNITS * workers) waves--;
+    return waves;
+}
 
 // CTAs per tile of the split kernel, the cheapest by split_cost.
 static int split_ranks(const GemmDevice& d, int qt, int64_t tiles, int k_blocks, int bm, int64_t m, bool f32, double* cost) {
@@ -266,8 +286,10 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
         p.bm = pair_bm;
         p.n_tiles = pair_n;
         p.m_tiles = pair_m;
-        p.unit_q = (int)(units / workers);
-        p.unit_r = (int)(units % workers);
+        p.waves = (int)pair_waves((int64_t)pair_n * pair_m, workers, p.k_blocks, pair_m, w.g.bytes());
+        const int64_t rest = units - (int64_t)p.waves * workers * p.k_blocks;
+        p.unit_q = (int)(rest / workers);
+        p.unit_r = (int)(rest % workers);
         cluster = 2;
         grid = 2 * workers;
         stage_bytes = PAIR_STAGE;
@@ -334,7 +356,7 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     const size_t smem = pair ? PAIR_SMEM : 1024 + (size_t)p.stages * stage_bytes + exchange;
     auto launch = [&](auto tag) {
         constexpr int QT = decltype(tag)::value;
-        return pair  ? gemm_launch_one(gemm_pair_kernel<QT>, p, map, grid, cluster, smem, s)
+        return pair  ? gemm_launch_one(p.waves > 0 ? gemm_pair_kernel<QT, true> : gemm_pair_kernel<QT, false>, p, map, grid, cluster, smem, s)
                : f32 ? gemm_launch_one(gemm_split_kernel<QT, 2, 3>, p, map, grid, cluster, smem, s)
                      : gemm_launch_one(gemm_split_kernel<QT, 1, 1>, p, map, grid, cluster, smem, s);
     };

@@ -34,9 +34,9 @@ struct GemmParams {
     int ranks;           // split kernel: CTAs of a cluster, which share a tile's K
     int early;           // split kernel: let the next kernel be placed while this one runs
     uint32_t idesc;
-    // pair kernel, stream-K: the (tile, k-block) units form one sequence, pair b owns units [b*q + min(b,r), ...)
+    // pair kernel: `waves` whole tiles a pair, then stream-K: the (tile, k-block) units behind form one sequence, pair b owns [b*q + min(b,r), ...)
     // split kernel: rank b owns those k-blocks of every tile, cluster c takes tile_q tiles, one more below tile_r
-    int unit_q, unit_r, tile_q, tile_r;
+    int unit_q, unit_r, tile_q, tile_r, waves;
     float* partial;        // [ctas][GEMM_PIECE_TOKENS][128] fp32: a CTA's piece of a tile that begins in an earlier pair
     unsigned int* ready;   // [ctas][4] generation whose piece (per 32-row quarter) is complete in `partial`
     unsigned int* gen;     // [0] generations completed so far, [1] CTAs that have left the current launch: the kernel

@@ -8,8 +8,8 @@
 // 1500 cycles per 128 k and 256 tokens.)  What bounds it now: in long loops the power cap; in one call, 4 us until the first MMA, 3 - 6
 // us behind the last one.
 // us a call, tiles of 512 or 256 tokens with A in shared memory / this: Q4_0 [11008 x 4096] 2048 tokens 150 / 139, Q4_K [14336 x 4096]
-// 512 tokens 56 / 54, 700 tokens 85 / 76, [3584 x 8192] 1024 tokens 63 / 57, Q8_0 [8192 x 8192] 300 tokens 61 / 52, 1024
-// tokens 112 / 116.
+// 512 tokens 56 / 54, 700 tokens 85 / 76, [3584 x 8192] 1024 tokens 63 / 57, Q8_0 [8192 x 8192] 1024 tokens
+// 110 / 109, 2000 tokens 210 / 202.
 //
 // Warp roles in each CTA (704 threads):
 //   warp 0      TMA producer: this CTA's half of a tile's tokens, two spans of 64 k a stage, 128-byte swizzle
@@ -21,8 +21,9 @@
 // for its TMA arrive on it.  Everything the MMAs release (`s_empty`, `acc_full`) is committed to both CTAs by multicast.
 //
 // Work split ("stream-K"): all (tile, k-block) units form one sequence in tile order, cut into equal contiguous shares,
-// one per pair, so every SM does the same number of MMA steps whatever the tile count.  A tile cut by a share boundary is
-// finished by the pair that holds its first k-block: the pairs holding the rest reach their piece first (it is the
+// one per pair, so every SM does the same number of MMA steps whatever the tile count.  Where the weight is larger than what the L2 keeps, each
+// pair takes whole tiles first, in step with its neighbours (pair_waves), and the units of what is left are dealt.  A tile cut by a share boundary is
+// finished by the pair that holds its first k-block: the pairs holding the rest reach their piece before that (it is the
 // head of their share), write it to a scratch buffer and publish the launch number; the owner reaches the tile last,
 // when all its warps are free: twelve of them (three per TMEM lane quarter) add the pieces in pair order
 // (deterministic) and write y.  Both CTAs of a pair walk the same units, and each hands over and finishes its own rows.
@@ -40,32 +41,59 @@ constexpr int PAIR_STAGES = 3;                           // of activations, and 
 constexpr int PAIR_SPILL = PAIR_TOKENS * GEMM_BN * 4;    // 128 KB: a segment's sums on their way to memory
 constexpr size_t PAIR_SMEM = 1024 + (size_t)PAIR_STAGES * PAIR_STAGE + PAIR_SPILL;
 
-// A pair's share of the unit sequence, cut into segments: a segment is a run of k-blocks of one tile.
+// A pair's units: with WAVES those of p.waves whole tiles (tile w * pairs + pair) first, then its share of the units of the tiles behind the
+// waves.  One counter runs over them: it has the number among those units in the share, [v0, v1), and begins waves * k_blocks below v0.
+// They are walked in segments: a segment is a run of k-blocks of one tile.
+__device__ __forceinline__ int share_begin(const GemmParams& p, int pair) { return pair * p.unit_q + min(pair, p.unit_r); }
 struct GemmSegment {
     int tile, kb0, kb1;  // k-blocks [kb0, kb1) of `tile`
 };
-__device__ __forceinline__ void pair_units(const GemmParams& p, int pair, int& u0, int& u1) {
-    u0 = pair * p.unit_q + min(pair, p.unit_r);
-    u1 = u0 + p.unit_q + (pair < p.unit_r ? 1 : 0);
-}
-// the segment that starts at unit u (u < u1)
-__device__ __forceinline__ GemmSegment segment_at(const GemmParams& p, int u, int u1) {
+// the segment that starts at unit u (u < u1) of this pair, whose counter began at u0
+template <bool WAVES> __device__ __forceinline__ GemmSegment segment_at(const GemmParams& p, int u, int u0, int u1) {
     GemmSegment g;
+    if (WAVES && u - u0 < p.waves * p.k_blocks) {
+        g.tile = (u - u0) / p.k_blocks * (int)(gridDim.x >> 1) + (int)(blockIdx.x >> 1);
+        g.kb0 = 0;
+        g.kb1 = p.k_blocks;
+        return g;
+    }
     g.tile = u / p.k_blocks;
     g.kb0 = u - g.tile * p.k_blocks;
     g.kb1 = min(p.k_blocks, g.kb0 + (u1 - u));
+    if (WAVES) g.tile += p.waves * (int)(gridDim.x >> 1);
     return g;
 }
 
 // Where a dequant warp's loads stand in the pair's units: they run a few units ahead of the conversions.  rank: which 128 of
 // the tile's 256 rows; dq: 16-row tile of the 128.
-template <int QT, int KBW> struct GemmLoadWalk {
+template <int QT, int KBW, bool WAVES> struct GemmLoadWalk {
     const GemmParams& p;
-    int u, u1, tile, kb, row0;
+    int u, u1, tile, kb, row0, waves;  // waves: whole tiles to come, with the present one
     const uint8_t* row = nullptr;
-    __device__ __forceinline__ GemmLoadWalk(const GemmParams& p_, int first, int u1_, int rank, int dq)
-        : p(p_), u(first), u1(u1_), tile(first / p_.k_blocks), kb(first - tile * p_.k_blocks), row0(rank * (GEMM_BN / 16) + dq) {
+    __device__ __forceinline__ GemmLoadWalk(const GemmParams& p_, int u0, int u1_, int set, int rank, int dq)
+        : p(p_), u(u0 + set), u1(u1_), row0(rank * (GEMM_BN / 16) + dq), waves(WAVES ? p_.waves : 0) {
+        if (WAVES) {
+            tile = (int)(blockIdx.x >> 1);
+            kb = set;
+            if (kb >= p.k_blocks) advance();
+        } else {
+            tile = u / p.k_blocks;
+            kb = u - tile * p.k_blocks;
+        }
         set_row();
+    }
+    __device__ __forceinline__ void advance() {  // to the tile that kb lies in
+        for (; kb >= p.k_blocks; kb -= p.k_blocks) {
+            if (!WAVES || waves == 0) {
+                tile++;
+            } else if (--waves > 0) {
+                tile += (int)(gridDim.x >> 1);
+            } else {
+                const int v0 = share_begin(p, (int)(blockIdx.x >> 1)), t = v0 / p.k_blocks;
+                tile = p.waves * (int)(gridDim.x >> 1) + t;
+                kb += v0 - t * p.k_blocks;
+            }
+        }
     }
     __device__ __forceinline__ void set_row() {  // rows behind the buffer's last tile are computed and never stored
         const int64_t rt = min((int64_t)(tile / p.m_tiles) * (2 * GEMM_BN / 16) + row0, (int64_t)p.rt_last);
@@ -79,7 +107,7 @@ template <int QT, int KBW> struct GemmLoadWalk {
         u += GEMM_SETS;
         kb += GEMM_SETS;
         if (kb < p.k_blocks) return;
-        for (; kb >= p.k_blocks; kb -= p.k_blocks) tile++;
+        advance();
         set_row();
     }
 };
@@ -99,7 +127,7 @@ __device__ __forceinline__ void tc_commit_pair(void* bar) {
 }
 
 // smem: [0, 1024) barriers + tmem slot | stages, 1024-byte aligned
-template <int QT>
+template <int QT, bool WAVES>
 __global__ void __launch_bounds__(768, 1) gemm_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);           // [4] leader: both CTAs' operands of the stage are in place
@@ -116,8 +144,7 @@ __global__ void __launch_bounds__(768, 1) gemm_pair_kernel(const GemmParams p, c
     const uint32_t rank = cluster_rank();
     const bool leader = rank == 0;
     const int pair = (int)(blockIdx.x >> 1), pairs = (int)(gridDim.x >> 1);
-    int u0, u1;
-    pair_units(p, pair, u0, u1);
+    const int v0 = share_begin(p, pair), u0 = v0 - (WAVES ? p.waves * p.k_blocks : 0), u1 = share_begin(p, pair + 1);
     constexpr int KBW = Tile<QT>::K / GEMM_BK;  // units per weight k-tile
 
     // Dequantization warps: the first weights are requested before all set-up; which warp takes what: see the cluster kernel.
@@ -126,7 +153,7 @@ __global__ void __launch_bounds__(768, 1) gemm_pair_kernel(const GemmParams p, c
     const int set = nth >> 1, dq = 2 * (warp & 3) + (nth & 1);
     constexpr int DEPTH = 2;  // units a warp holds: one is converted while the other loads
     DequantRegs<QT> r[DEPTH][2];
-    GemmLoadWalk<QT, KBW> walk(p, u0 + set, u1, (int)rank, dq);
+    GemmLoadWalk<QT, KBW, WAVES> walk(p, u0, u1, set, (int)rank, dq);
     if (dequant) {
 #pragma unroll
         for (int d = 0; d < DEPTH; d++) walk.next(r[d], lane);
@@ -157,7 +184,7 @@ __global__ void __launch_bounds__(768, 1) gemm_pair_kernel(const GemmParams p, c
             asm volatile("griddepcontrol.wait;" ::: "memory");  // the fp16 activations
             StageCursor at;
             for (int u = u0; u < u1 && !*abort_flag;) {
-                const GemmSegment g = segment_at(p, u, u1);
+                const GemmSegment g = segment_at<WAVES>(p, u, u0, u1);
                 const int tok0 = (g.tile % p.m_tiles) * p.bm + (int)rank * (p.bm >> 1);
                 for (int kb = g.kb0; kb < g.kb1; kb++, at.advance(PAIR_STAGES)) {
                     const int s = at.s;
@@ -180,7 +207,7 @@ __global__ void __launch_bounds__(768, 1) gemm_pair_kernel(const GemmParams p, c
             StageCursor at;
             int local = 0;
             for (int u = u0; u < u1 && !*abort_flag; local++) {
-                const GemmSegment g = segment_at(p, u, u1);
+                const GemmSegment g = segment_at<WAVES>(p, u, u0, u1);
                 bool ok = true;
                 // the epilogues must have read the segment before this one
                 if (local > 0 && !g_mbar_wait(acc_empty, (local - 1) & 1)) { fail(); break; }
@@ -224,7 +251,7 @@ __global__ void __launch_bounds__(768, 1) gemm_pair_kernel(const GemmParams p, c
         float* mine = p.partial + (size_t)blockIdx.x * GEMM_PIECE_TOKENS * GEMM_BN;
         uint4* const spill = reinterpret_cast<uint4*>(stage0 + PAIR_STAGES * PAIR_STAGE) + row;  // [tokens / 4][128 rows]
         for (int u = u0; u < u1 && !*abort_flag; local++) {
-            const GemmSegment g = segment_at(p, u, u1);
+            const GemmSegment g = segment_at<WAVES>(p, u, u0, u1);
             const int nt = g.tile / p.m_tiles, mt = g.tile % p.m_tiles;
             const int n = nt * (2 * GEMM_BN) + (int)rank * GEMM_BN + row;
             const bool starts = g.kb0 == 0, ends = g.kb1 == p.k_blocks;
@@ -313,12 +340,12 @@ __global__ void __launch_bounds__(768, 1) gemm_pair_kernel(const GemmParams p, c
     // following pairs: the last segment of the share.  Twelve warps (three per TMEM lane quarter) add the pieces of
     // this CTA's rows in pair order and write y.
     __syncwarp();
-    if (u0 < u1 && warp < 12) {
+    if (v0 < u1 && warp < 12) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         unsigned int launch_gen = ld_acquire_u32(p.gen) + 1u;
         if (launch_gen == 0u) launch_gen = 1u;
-        const int tile = (u1 - 1) / p.k_blocks;
-        const int kb0 = max(u0, tile * p.k_blocks) - tile * p.k_blocks, kb1 = u1 - tile * p.k_blocks;
+        const int t = (u1 - 1) / p.k_blocks, tile = t + (WAVES ? p.waves * pairs : 0);  // t: among the tiles behind the waves
+        const int kb0 = max(v0, t * p.k_blocks) - t * p.k_blocks, kb1 = u1 - t * p.k_blocks;
         if (kb0 == 0 && kb1 < p.k_blocks) {
             const int quarter = warp & 3, slice = warp >> 2;
             const int row = quarter * 32 + lane;
@@ -326,11 +353,9 @@ __global__ void __launch_bounds__(768, 1) gemm_pair_kernel(const GemmParams p, c
             const int n = nt * (2 * GEMM_BN) + (int)rank * GEMM_BN + row;
             int last_pair = pair;
             bool ok = !*abort_flag;
-            const int tile_end = (tile + 1) * p.k_blocks;
+            const int tile_end = (t + 1) * p.k_blocks;
             for (int c = pair + 1; c < pairs && ok; c++) {
-                int c0, c1;
-                pair_units(p, c, c0, c1);
-                if (c0 >= tile_end) break;
+                if (share_begin(p, c) >= tile_end) break;
                 last_pair = c;  // no share is empty
                 int spins = 0;
                 while (ld_acquire_u32(p.ready + (2 * c + (int)rank) * 4 + quarter) != launch_gen && ++spins < GEMM_POLL_SPINS) __nanosleep(64);
@@ -347,15 +372,15 @@ __global__ void __launch_bounds__(768, 1) gemm_pair_kernel(const GemmParams p, c
             auto fetch = [&](int cc, int ci) { load_piece_chunk(p.partial + (size_t)(2 * cc + (int)rank) * GEMM_PIECE_TOKENS * GEMM_BN, v, ci * PAIR_COLS, row); };
             if (ok && slice < chunks) fetch(pair + 1, slice);  // the next pair always holds a piece
             for (int ci = slice; ci < chunks && ok; ci += 3) {
-                uint32_t t[PAIR_COLS];
-                tmem_ld16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ci * PAIR_COLS), t);
-                add_piece_chunk(t, v);
+                uint32_t a[PAIR_COLS];
+                tmem_ld16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ci * PAIR_COLS), a);
+                add_piece_chunk(a, v);
                 for (int cc = pair + 2; cc <= last_pair; cc++) {  // pieces in pair order
                     fetch(cc, ci);
-                    add_piece_chunk(t, v);
+                    add_piece_chunk(a, v);
                 }
                 if (ci + 3 < chunks) fetch(pair + 1, ci + 3);  // under the stores of this one
-                store_chunk(p.y, p.ldy, p.col0, p.row_unscale, t, mt * p.bm + ci * PAIR_COLS, p.m, n, p.rows);
+                store_chunk(p.y, p.ldy, p.col0, p.row_unscale, a, mt * p.bm + ci * PAIR_COLS, p.m, n, p.rows);
             }
         }
     }

@@ -372,6 +372,12 @@ int wf_plan_several_tokens(int qtype, int64_t rows, int64_t k, int cols, int x_i
  * bring the sums of their slices together in clusters of at most eight CTAs, and a change from clusters to one slice costs the launch
  * behind.  slices = 0 throughout: a launch fits neither way, and the program runs as one persistent kernel. */
 int wf_plan_program(int qtype, int n, const int64_t* rows, const int64_t* k, int tokens, int sm_count, int* slices, int* k_tiles_per_slice);
+/* How wf_qlinear would run `tokens` rows (33 and more of bf16, 11 and more of fp32) on a [rows x k] weight of type qtype on the context's
+ * device: pairs = 1, pairs of CTAs on tiles of 256 rows, stream-K; 0, clusters on tiles of 128 rows that split K.  Tokens of a tile,
+ * CTAs of a cluster (2 for pairs), how many clusters or pairs there are, and the whole tiles that a pair takes before the units of
+ * the rest are dealt. */
+int wf_plan_many_tokens(int64_t ctx, int qtype, int64_t rows, int64_t k, int64_t tokens, int x_is_f32, int* pairs, int* tile_tokens,
+                        int* ctas, int* groups, int* waves);
 
 #ifdef __cplusplus
 }

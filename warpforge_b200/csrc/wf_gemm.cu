@@ -169,6 +169,66 @@ static int split_ranks(const GemmDevice& d, int qt, int64_t tiles, int k_blocks,
     return best;
 }
 
+// How a call is cut: which kernel, its tiles, and what share of them a CTA or pair has.
+struct GemmChoice {
+    bool pair;
+    int bm, n_tiles, m_tiles, k_blocks;
+    int cluster;      // CTAs of a cluster (the ranks that split K), 2 for pairs
+    int groups;       // clusters or pairs
+    int waves;        // pairs: whole tiles that each takes first
+    int64_t rest;     // pairs: units behind the waves
+    bool too_large;
+};
+static GemmChoice gemm_choose(const GemmDevice& d, const WeightGeom& g, int64_t m, bool f32) {
+    GemmChoice c{};
+    c.k_blocks = (int)((g.k + GEMM_BK - 1) / GEMM_BK);
+    // Clusters on tiles of 128 rows x up to 128 tokens.  Token tiles are of one size, in steps of 32 where there are several (the
+    // epilogue works on 32 tokens at a time and must not reach into a neighbour); fp32: 96, so that two stages and the
+    // exchange buffer fit.
+    c.n_tiles = (int)((g.rows + GEMM_BN - 1) / GEMM_BN);
+    double cost = 1e30;
+    for (int most = f32 ? 96 : SPLIT_MAX_TOKENS; most >= (f32 ? 96 : 64); most -= 32) {  // smaller tiles where they fill the device better
+        const int64_t token_tiles = (m + most - 1) / most, grain = token_tiles > 1 ? 32 : 16;
+        const int bm = (int)(((m + token_tiles - 1) / token_tiles + grain - 1) / grain * grain);
+        const int m_tiles = (int)((m + bm - 1) / bm);
+        double t = 0;
+        const int ranks = split_ranks(d, g.qtype, (int64_t)c.n_tiles * m_tiles, c.k_blocks, bm, m, f32, &t);
+        if (t >= SMALLER_TILES_GAIN * cost) continue;
+        cost = t;
+        c.bm = bm;
+        c.m_tiles = m_tiles;
+        c.cluster = ranks;
+    }
+    c.groups = (int)std::min<int64_t>(d.clusters[c.cluster], (int64_t)c.n_tiles * c.m_tiles);
+    // Pairs of CTAs on tiles of 256 rows x up to 256 tokens (of one size, in steps of 32), stream-K shares.  A tile of U units shared by n
+    // pairs costs about U / n units plus n - 1 pieces added by its owner, a piece costing about two units: no share is shorter
+    // than sqrt(2 U) units, which bounds n for weights with few tiles.
+    const int pair_n = (int)((g.rows + 2 * GEMM_BN - 1) / (2 * GEMM_BN)), pair_m = (int)((m + PAIR_TOKENS - 1) / PAIR_TOKENS);
+    const int pair_bm = (int)(((m + pair_m - 1) / pair_m + 31) / 32 * 32);
+    int min_units = 1;
+    while ((int64_t)min_units * min_units < 2 * c.k_blocks) min_units++;
+    const int64_t units = (int64_t)pair_n * pair_m * c.k_blocks;
+    const int workers = (int)std::min<int64_t>(d.pairs, std::max<int64_t>(1, units / min_units));
+    c.too_large = std::max(units, (int64_t)c.n_tiles * c.m_tiles * c.k_blocks) >= (1LL << 30);
+    c.pair = !f32 && m > 64 && d.pairs > 0 && CLUSTERS_GAIN * pair_cost(g.qtype, (units + workers - 1) / workers, c.k_blocks, pair_bm, m) < cost;
+    if (c.pair) {
+        c.bm = pair_bm;
+        c.n_tiles = pair_n;
+        c.m_tiles = pair_m;
+        c.cluster = 2;
+        c.groups = workers;
+        c.waves = (int)pair_waves((int64_t)pair_n * pair_m, workers, c.k_blocks, pair_m, g.bytes());
+        c.rest = units - (int64_t)c.waves * workers * c.k_blocks;
+    }
+    return c;
+}
+static cudaError_t gemm_device(int qt, int device, GemmDevice** out) {
+    return qt == WF_QTYPE_Q4_0   ? gemm_prepare<WF_QTYPE_Q4_0>(device, out)
+           : qt == WF_QTYPE_Q4_1 ? gemm_prepare<WF_QTYPE_Q4_1>(device, out)
+           : qt == WF_QTYPE_Q8_0 ? gemm_prepare<WF_QTYPE_Q8_0>(device, out)
+                                 : gemm_prepare<WF_QTYPE_Q4_K>(device, out);
+}
+
 // The stream's scratch, grown on demand.
 static int gemm_scratch(Context* c, cudaStream_t s, GemvScratch& sc, int64_t x16_bytes) {
     if (x16_bytes > sc.x16_bytes) {
@@ -230,12 +290,15 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     const int planes = f32 ? 3 : 1;
     GemmDevice* dev = nullptr;
     {
-        const cudaError_t e = qt == WF_QTYPE_Q4_0   ? gemm_prepare<WF_QTYPE_Q4_0>(c->device, &dev)
-                              : qt == WF_QTYPE_Q4_1 ? gemm_prepare<WF_QTYPE_Q4_1>(c->device, &dev)
-                              : qt == WF_QTYPE_Q8_0 ? gemm_prepare<WF_QTYPE_Q8_0>(c->device, &dev)
-                                                    : gemm_prepare<WF_QTYPE_Q4_K>(c->device, &dev);
+        const cudaError_t e = gemm_device(qt, c->device, &dev);
         if (e != cudaSuccess) return cuda_status(c, e, "gemm attributes");
     }
+    // the last 128-row block may reach past the padded row-tiles: the weight buffer must cover it
+    if ((w.g.rows + GEMM_BN - 1) / GEMM_BN * (GEMM_BN / 16) > w.g.rt_alloc)
+        return set_error(c, WF_ERR_SHAPE, "weight buffer does not cover the last 128-row block");
+    const GemmChoice ch = gemm_choose(*dev, w.g, call.m, f32);
+    if (ch.too_large) return set_error(c, WF_ERR_TOO_LARGE, "GEMM has too many tile steps");
+    const bool pair = ch.pair;
     GemmParams p{};
     p.tiles = w.d_tiles;
     p.y = call.d_y;
@@ -246,64 +309,27 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
     p.kt_w = (int)w.g.kt;
     p.rt_last = (int)w.g.rt_alloc - 1;
     p.m = (int)call.m;
-    p.k_blocks = (int)((w.g.k + GEMM_BK - 1) / GEMM_BK);
-
-    int grid, cluster, clusters = 0;
+    p.k_blocks = ch.k_blocks;
+    p.bm = ch.bm;
+    p.n_tiles = ch.n_tiles;
+    p.m_tiles = ch.m_tiles;
+    const int cluster = ch.cluster, grid = ch.groups * ch.cluster;
     size_t stage_bytes, exchange = 0;
-    // Clusters on tiles of 128 rows x up to 128 tokens.  Token tiles are of one size, in steps of 32 where there are several (the
-    // epilogue works on 32 tokens at a time and must not reach into a neighbour); fp32: 96, so that two stages and the
-    // exchange buffer fit.
-    p.n_tiles = (int)((w.g.rows + GEMM_BN - 1) / GEMM_BN);
-    // the last 128-row block may reach past the padded row-tiles: the weight buffer must cover it
-    if ((int64_t)p.n_tiles * (GEMM_BN / 16) > w.g.rt_alloc)
-        return set_error(c, WF_ERR_SHAPE, "weight buffer does not cover the last 128-row block");
-    double cost = 1e30;
-    for (int most = f32 ? 96 : SPLIT_MAX_TOKENS; most >= (f32 ? 96 : 64); most -= 32) {  // smaller tiles where they fill the device better
-        const int64_t token_tiles = (call.m + most - 1) / most, grain = token_tiles > 1 ? 32 : 16;
-        const int bm = (int)(((call.m + token_tiles - 1) / token_tiles + grain - 1) / grain * grain);
-        const int m_tiles = (int)((call.m + bm - 1) / bm);
-        double t = 0;
-        const int ranks = split_ranks(*dev, qt, (int64_t)p.n_tiles * m_tiles, p.k_blocks, bm, call.m, f32, &t);
-        if (t >= SMALLER_TILES_GAIN * cost) continue;
-        cost = t;
-        p.bm = bm;
-        p.m_tiles = m_tiles;
-        p.ranks = ranks;
-    }
-    clusters = (int)std::min<int64_t>(dev->clusters[p.ranks], (int64_t)p.n_tiles * p.m_tiles);
-    // Pairs of CTAs on tiles of 256 rows x up to 256 tokens (of one size, in steps of 32), stream-K shares.  A tile of U units shared by n
-    // pairs costs about U / n units plus n - 1 pieces added by its owner, a piece costing about two units: no share is shorter
-    // than sqrt(2 U) units, which bounds n for weights with few tiles.
-    const int pair_n = (int)((w.g.rows + 2 * GEMM_BN - 1) / (2 * GEMM_BN)), pair_m = (int)((call.m + PAIR_TOKENS - 1) / PAIR_TOKENS);
-    const int pair_bm = (int)(((call.m + pair_m - 1) / pair_m + 31) / 32 * 32);
-    int min_units = 1;
-    while ((int64_t)min_units * min_units < 2 * p.k_blocks) min_units++;
-    const int64_t units = (int64_t)pair_n * pair_m * p.k_blocks;
-    const int workers = (int)std::min<int64_t>(dev->pairs, std::max<int64_t>(1, units / min_units));
-    const bool pair = !f32 && call.m > 64 && dev->pairs > 0 && CLUSTERS_GAIN * pair_cost(qt, (units + workers - 1) / workers, p.k_blocks, pair_bm, call.m) < cost;
-    if (std::max(units, (int64_t)p.n_tiles * p.m_tiles * p.k_blocks) >= (1LL << 30)) return set_error(c, WF_ERR_TOO_LARGE, "GEMM has too many tile steps");
     if (pair) {
-        p.bm = pair_bm;
-        p.n_tiles = pair_n;
-        p.m_tiles = pair_m;
-        p.waves = (int)pair_waves((int64_t)pair_n * pair_m, workers, p.k_blocks, pair_m, w.g.bytes());
-        const int64_t rest = units - (int64_t)p.waves * workers * p.k_blocks;
-        p.unit_q = (int)(rest / workers);
-        p.unit_r = (int)(rest % workers);
-        cluster = 2;
-        grid = 2 * workers;
+        p.waves = ch.waves;
+        p.unit_q = (int)(ch.rest / ch.groups);
+        p.unit_r = (int)(ch.rest % ch.groups);
         stage_bytes = PAIR_STAGE;
     } else {
-        cluster = p.ranks;
-        grid = clusters * cluster;
+        p.ranks = ch.cluster;
         // The conversion of fp32 rows takes more registers than a GEMM's CTA leaves, so it waits on idle SMs and keeps the next GEMM's
         // clusters from them.  Few rows are worth it: 14 shapes of 11 - 32 tokens 0.95 x (worst 1.02), 26 of 40 - 256 tokens 1.03 x
         // (worst 1.14).
         p.early = !f32 || call.m <= 32;
         p.unit_q = p.k_blocks / p.ranks;
         p.unit_r = p.k_blocks % p.ranks;
-        p.tile_q = p.n_tiles * p.m_tiles / clusters;
-        p.tile_r = p.n_tiles * p.m_tiles % clusters;
+        p.tile_q = p.n_tiles * p.m_tiles / ch.groups;
+        p.tile_r = p.n_tiles * p.m_tiles % ch.groups;
         stage_bytes = (size_t)split_stage_bytes(planes, p.bm);
         exchange = (size_t)split_exchange_bytes(f32 ? 2 : 1, p.bm, cluster);
     }
@@ -370,3 +396,34 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
 }
 
 }  // namespace wf
+
+extern "C" int wf_plan_many_tokens(int64_t ctx, int qtype, int64_t rows, int64_t k, int64_t tokens, int x_is_f32, int* pairs, int* tile_tokens,
+                                   int* ctas, int* groups, int* waves) {
+    using namespace wf;
+    Context* c = get_context(ctx);
+    if (!c) return WF_ERR_INVALID_HANDLE;
+    ScopedLock lk(c);
+    if (!lk.ok) return WF_ERR_BUSY;
+    WF_CUDA(c, cudaSetDevice(c->device));
+    WeightGeom g{};
+    g.qtype = device_qtype(qtype);
+    if (g.qtype != WF_QTYPE_Q4_0 && g.qtype != WF_QTYPE_Q4_1 && g.qtype != WF_QTYPE_Q8_0 && g.qtype != WF_QTYPE_Q4_K) return WF_ERR_UNSUPPORTED_TYPE;
+    if (rows < 1 || k < 1 || k % block_k(qtype) || !many_tokens(x_is_f32 != 0, tokens) || !pairs || !tile_tokens || !ctas || !groups || !waves)
+        return WF_ERR_INVALID_ARGUMENT;
+    g.rows = rows;
+    g.k = k;
+    g.rt = (rows + TILE_ROWS - 1) / TILE_ROWS;
+    g.kt = (k + tile_k(g.qtype) - 1) / tile_k(g.qtype);
+    g.rt_alloc = (g.rt + 7) / 8 * 8;
+    GemmDevice* dev = nullptr;
+    const cudaError_t e = gemm_device(g.qtype, c->device, &dev);
+    if (e != cudaSuccess) return cuda_status(c, e, "gemm attributes");
+    const GemmChoice ch = gemm_choose(*dev, g, tokens, x_is_f32 != 0);
+    if (ch.too_large) return WF_ERR_TOO_LARGE;
+    *pairs = ch.pair ? 1 : 0;
+    *tile_tokens = ch.bm;
+    *ctas = ch.cluster;
+    *groups = ch.groups;
+    *waves = ch.waves;
+    return WF_OK;
+}

@@ -4,6 +4,9 @@ cluster, clusters of one), CTA pairs (256 rows x up to 256 tokens; the cost func
 bf16 tokens: the bars of test_gpu_gemm.py.  fp32 tokens: products are exact to 2^-22 and an accumulator takes at most 32
 steps between two drains, each cutting the partial sum off at its 24th bit: 32 x 2^-23 = 3.8e-6 of the result at
 the very most, in the 2-norm against float64."""
+import collections
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -36,6 +39,16 @@ def _run(backend, oracle, name, rows, k, x, tensor):
     assert np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
     wf = oracle.dequant(QT[name], blocks, rows * k).reshape(rows, k).astype(np.float64)
     return got[0], x.astype(np.float64) @ wf.T
+
+
+Plan = collections.namedtuple("Plan", "pairs tokens ctas groups waves")
+
+
+def _plan(backend, name, rows, k, m, f32=False):
+    ctx = backend.cuda_context
+    v = [ctypes.c_int() for _ in Plan._fields]
+    ctx._ck("plan", ctx._lib.wf_plan_many_tokens(ctx.handle, Q.QuantizationType[name.upper()].ggml_type, rows, k, m, int(f32), *map(ctypes.byref, v)))
+    return Plan(*(x.value for x in v))
 
 
 @pytest.mark.parametrize("name", sorted(QT))
@@ -74,6 +87,16 @@ def test_pairs_of_ctas(backend, oracle, name, rows, k, m):
     got, want = _run(backend, oracle, name, rows, k, Q.bf16_bits_to_float(bits), Tensor.from_bf16_bits(bits))
     assert np.max(np.abs(got - want)) <= 1e-3 * np.max(np.abs(want))
     assert np.linalg.norm(got - want) <= 3e-4 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("name,rows,k,m,pairs", [  # us by clusters of one / by pairs
+    ("q4_k", 8192, 8192, 256, 1),  # 42.7 / 40.2
+    ("q4_1", 9000, 6976, 700, 1),  # 91.8 / 75.7
+    ("q8_0", 5003, 2784, 512, 0),  # 25.0 / 28.7
+    ("q4_0", 4096, 4096, 512, 0),  # 18.6 / 28
+])
+def test_choice_of_the_kernel(backend, name, rows, k, m, pairs):
+    assert _plan(backend, name, rows, k, m).pairs == pairs
 
 
 @pytest.mark.parametrize("name,rows,k,m", [  # weights of 37 MB and more, 132 MB read again

@@ -114,10 +114,11 @@ static cudaError_t gemm_launch_one(Kernel kernel, const GemmParams& p, const CUt
 // What a call costs in us by either kernel, fitted to measurements on one B200 (weights from HBM, calls back to back): 2200 calls of the
 // split kernel (11 - 2048 tokens, weights from [600 x 6976] to [14336 x 8192], every number of ranks, token tiles of 64, 96 and
 // 128), 61 shapes of the pair kernel.  Conversion, launch and start; a cost per unit of 128 k on the busiest CTA or pair, where the
-// slower of dequantization and MMAs counts; the parts put together.  The fits are off by 9 % and 4 % (one standard deviation).  The
-// constants before, made for A in shared memory, chose settings 9 % from the best, up to 60 %: 300 - 512 tokens of [4096 x 4096],
-// pairs 28 us, clusters of one 18; [11008 x 4096] Q4_K 128 tokens, 31.5 and 24.  With these, 85 calls and layers of 33 - 2048 tokens
-// drawn at random took 0.936 x the time, worst 1.05 (Q5_0 [528 x 5728], 162 tokens).
+// slower of dequantization and MMAs counts; the parts put together.  The fits are off by 9 % and 5 % (one standard deviation); of 495 calls
+// of 40 - 2048 tokens the choice is 1.7 % off the best of the settings that promise most.
+// Clusters of one, more than 32 units: the clock sinks and the weights come from memory, up to 0.56 us a unit at K = 8192 (without
+// that term Q4_K [8192 x 8192] 256 tokens went to them, 42.7 us, pairs 40.2, three weights in turn 136 and 123; Q4_1 [9000 x 6976] 700
+// tokens 91.8 and 75.7).
 static double split_cost(int qt, int64_t rounds, int units, int ranks, int bm, int64_t m, bool f32) {
     const double b = bm / 128.0, t = (double)m / 256;
     if (f32) {
@@ -125,9 +126,10 @@ static double split_cost(int qt, int64_t rounds, int units, int ranks, int bm, i
         const double unit = std::max(dequant, 0.56 + 1.12 * b);
         return ranks == 1 ? 3.5 + 1.6 * t + (double)rounds * units * unit : 5.0 + 4.3 * t + (double)rounds * (units * unit + 0.6 * b);
     }
-    const double dequant = qt == WF_QTYPE_Q4_0 ? 0.37 : qt == WF_QTYPE_Q4_1 ? 0.42 : qt == WF_QTYPE_Q8_0 ? 0.45 : 0.53;
+    const double dequant = qt == WF_QTYPE_Q4_0 ? 0.37 : qt == WF_QTYPE_Q4_1 ? 0.42 : qt == WF_QTYPE_Q8_0 ? 0.44 : 0.53;
     const double unit = std::max(dequant, 0.07 + 0.35 * b);
-    return ranks == 1 ? 2.5 + 0.7 * t + (double)rounds * (units * unit + 1.3 + 0.25 * b) : 3.8 + 1.5 * t + (double)rounds * (units * unit + 3.6 * b);
+    if (ranks == 1) return 2.5 + 0.7 * t + (double)rounds * (units * (unit + 0.0008 * std::max(0, units - 32)) + 1.3 + 0.25 * b);
+    return 3.8 + 1.5 * t + (double)rounds * (units * unit + 3.6 * b);
 }
 // share: units of the busiest pair; a tile of U units is put together from the pieces of U / share pairs
 static double pair_cost(int qt, int64_t share, int k_blocks, int bm, int64_t m) {

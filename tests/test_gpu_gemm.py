@@ -41,7 +41,7 @@ def _check(got, want):
 @pytest.mark.parametrize("name", ["q4_0", "q8_0", "q4_k", "q4_1", "q5_0"])
 @pytest.mark.parametrize("rows,k,m", [(128, 256, 16), (256, 1024, 64), (1000, 2048, 300), (136, 512, 9), (4096, 4096, 33),
                                       (256, 1024, 513), (384, 1280, 700), (2048, 512, 1024),
-                                      # enough tiles for the token tiles of 2 x 256: a last tile with one half, rows not a multiple of 128
+                                      # more tiles than clusters of one, a last token tile of one token, rows not a multiple of 128
                                       (4800, 256, 513), (4864, 512, 700)])
 def test_gemm_matches_oracle(backend, oracle, name, rows, k, m):
     qt, oq = QT[name]
@@ -151,34 +151,48 @@ def test_config3_q4k_prefill_sampled_rows(backend, oracle):
     w.close()
 
 
-def test_gemm_recorded_in_a_graph_replays_with_new_activations(oracle):
-    """A many-token wf_qlinear recorded once into a CUDA graph and replayed with different activations: the pieces of
-    tiles shared between CTAs are matched by a generation the kernel counts itself, so a replay can never take a
-    previous replay's piece for its own."""
+@pytest.mark.parametrize("rows,k,m,pairs", [(1000, 2048, 64, 0), (784, 11008, 1319, 1)])
+def test_gemm_recorded_in_a_graph_replays_with_new_activations(oracle, rows, k, m, pairs):
+    """A many-token wf_qlinear recorded once into a CUDA graph and replayed with different activations.  Pairs of CTAs, here about three to a
+    tile: the pieces of a tile are matched by a generation that the kernel counts itself, so a replay never takes a piece of an
+    earlier replay, or of the calls that ran between the replays, for its own."""
+    import ctypes
+
     from warpforge_b200 import _native as N
     from warpforge_b200.backend import CudaContext, QuantizedWeight
 
     ctx = CudaContext(0)
     lib = ctx._lib
     try:
-        rows, k, m = 1000, 2048, 64  # 8 row tiles x 16 k-steps over 148 CTAs: every tile is shared by several CTAs
+        plan = [ctypes.c_int() for _ in range(5)]
+        ctx._ck("plan", lib.wf_plan_many_tokens(ctx.handle, Q.QuantizationType.Q4_K.ggml_type, rows, k, m, 0, *map(ctypes.byref, plan)))
+        assert plan[0].value == pairs
+        if pairs:
+            assert plan[3].value > 2 * -(-rows // 256) * -(-m // plan[1].value)  # pairs, tiles
         blocks = Q.synth_q4_k(rows, k, 91)
         w = QuantizedWeight(ctx, Q.QuantizationType.Q4_K, blocks, rows, k)
+        wf = oracle.dequant(O.Q4_K, blocks, rows * k).reshape(rows, k).astype(np.float64)
         xs = [Q.synth_activation_bf16(m, k, 91 + i) for i in range(4)]
-        dx, dy = ctx.allocate(xs[0].nbytes), ctx.allocate(m * rows * 4)
+        dx, dy, between = ctx.allocate(xs[0].nbytes), ctx.allocate(m * rows * 4), ctx.allocate(m * rows * 4)
+        run = lambda y: ctx._ck("wf_qlinear", lib.wf_qlinear(ctx.handle, w.handle, dx, N.WF_DTYPE_BF16, 1, m, y, 1, 0))  # noqa: E731
         ctx.copy_to_device(dx, xs[0])
-        ctx._ck("wf_qlinear", lib.wf_qlinear(ctx.handle, w.handle, dx, N.WF_DTYPE_BF16, 1, m, dy, 1, 0))  # eager: allocates scratch
+        run(dy)  # eager: allocates scratch
         ctx.synchronize()
         ctx.graph_begin()
-        ctx._ck("wf_qlinear", lib.wf_qlinear(ctx.handle, w.handle, dx, N.WF_DTYPE_BF16, 1, m, dy, 1, 0))
+        run(dy)
         g = ctx.graph_end()
         got = np.empty((m, rows), np.float32)
-        for x in xs[1:]:
+        for n, x in enumerate(xs[1:]):
+            want = Q.bf16_bits_to_float(x).reshape(m, k).astype(np.float64) @ wf.T
             ctx.copy_to_device(dx, x)
-            ctx.graph_launch(g)
+            for _ in range(n):
+                run(between)
+            for _ in range(2):
+                ctx.graph_launch(g)
             ctx.synchronize()
-            ctx.copy_to_host(got, dy)
-            _check(got, oracle.qlinear(O.Q4_K, blocks, rows, k, Q.bf16_bits_to_float(x), nthreads=oracle.max_threads()))
+            for y in [dy] + [between] * (n > 0):
+                ctx.copy_to_host(got, y)
+                _check(got, want)
         ctx.graph_destroy(g)
         w.close()
     finally:

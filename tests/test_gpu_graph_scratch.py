@@ -11,8 +11,9 @@ from warpforge_b200 import quant as Q
 
 pytestmark = pytest.mark.gpu
 
-CASES = [  # (rows, k, tokens): both GEMM kernels, fp32 tokens, sums that go through memory, one token cut between CTAs
-    (1000, 1120, 64, False), (3072, 1024, 512, False), (640, 1024, 96, True), (700, 27008, 31, False), (4096, 11008, 1, False)]
+PAIRS = (784, 11168, 1319, False)
+CASES = [  # (rows, k, tokens): clusters, several token tiles, pairs of CTAs, fp32 tokens, sums that go through memory, one token cut between CTAs
+    (1000, 1120, 64, False), (3072, 1024, 512, False), PAIRS, (640, 1024, 96, True), (700, 27008, 31, False), (4096, 11008, 1, False)]
 
 
 def _setup(ctx, rows, k, m, f32):
@@ -47,6 +48,10 @@ def test_stream_destroyed(rows, k, m, f32):
 
     ctx = CudaContext(0)
     try:
+        if (rows, k, m, f32) == PAIRS:  # whose pieces lie in the stream's scratch
+            plan = [ctypes.c_int() for _ in range(5)]
+            ctx._ck("plan", ctx._lib.wf_plan_many_tokens(ctx.handle, Q.QuantizationType.Q4_0.ggml_type, rows, k, m, 0, *map(ctypes.byref, plan)))
+            assert plan[0].value == 1
         w, dx, dy, call = _setup(ctx, rows, k, m, f32)
         s = ctx.create_stream()
         call(s)  # the scratch of the stream

@@ -374,10 +374,10 @@ int gemm_launch(Context* c, const GemvCall& call, cudaStream_t s) {
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        const bool alone = pair && w.g.k > CONVERT_KEEP_SHORT * CONVERT_THREADS * 8;
-        const auto convert = f32     ? convert_rows_kernel<3, 2>
-                             : alone ? convert_rows_kernel<1, CONVERT_KEEP_LONG>
-                                     : convert_rows_kernel<1, CONVERT_KEEP_SHORT>;
+        const bool longer = w.g.k > CONVERT_KEEP_SHORT * CONVERT_THREADS * 8;
+        const auto convert = f32      ? convert_rows_kernel<3, 2>
+                             : longer ? convert_rows_kernel<1, CONVERT_KEEP_LONG>
+                                      : convert_rows_kernel<1, CONVERT_KEEP_SHORT>;
         WF_CUDA(c, cudaLaunchKernelEx(&cfg, convert, call.d_x, x16, unscale, (int)call.m, (int)w.g.k));
     }
     c->launches++;

@@ -298,13 +298,14 @@ __device__ __forceinline__ float2 row_scale(int emax) {
 // not kept: converting inside the GEMM, every rank's warps their share of the rows, with tags to wait for: what a warp does for a
 // row and then for the tags is a chain of trips to the L2, 4 us longer until the first MMA (77 tokens of [5003 x 2784]: 12.7 ->
 // 14.4 us a call, 64 of [1000 x 1024]: 6.8 -> 9.8).
-// KEEP: groups a thread keeps between the scan and the conversion; what is left of a longer row is read again.  Before the cluster GEMM
-// and for rows of 4096 it takes 32 registers a thread.  The pair GEMM triggers nothing early, so before it rows of more than
-// 4096 elements are held whole, in 48 registers ([4096 x 8192], Q4_0, 1024 tokens: 65.9 -> 64.5 us a call, 512 tokens: 40.2 ->
-// 39.3; rows that the smaller form holds gain nothing: [11008 x 4096], 2048 tokens, 143.9 against 145.1).
+// KEEP: groups a thread keeps between the scan and the conversion; what is left of a longer row is read again.  Rows of up to 4096 elements:
+// two, held to 32 registers a thread, so that eight rows and not five lie on an SM (with 46, us a call: Q4_K [1000 x 1024] 700 tokens 8.9 ->
+// 10.4, [2048 x 2048] 128 tokens 8.5 -> 9.5, Q4_1 [4096 x 1024] 300 tokens 8.6 -> 9.3; 66 calls 0.996 x).  Longer rows: four, in 48 registers,
+// whichever GEMM follows (155 calls of 33 - 700 tokens, K = 4608 - 11008, 0.952 x, worst 1.014: Q8_0 [1024 x 8192] 128 tokens 13.8 -> 11.4,
+// Q4_0 [4096 x 11008] 96 tokens 19.9 -> 17.6).
 constexpr int CONVERT_THREADS = 256;
-constexpr int CONVERT_KEEP_SHORT = 2;  // rows of 4096 (bf16)
-constexpr int CONVERT_KEEP_LONG = 4;   // rows of 8192
+constexpr int CONVERT_KEEP_SHORT = 2;  // rows of up to 4096 (bf16)
+constexpr int CONVERT_KEEP_LONG = 4;   // up to 8192 held whole
 template <int PLANES, int KEEP>
 __global__ void __launch_bounds__(CONVERT_THREADS, PLANES == 1 && KEEP == CONVERT_KEEP_SHORT ? 8 : 5) convert_rows_kernel(const void* x, __half* __restrict__ x16, float* __restrict__ unscale,
                                                                        int m, int k) {

@@ -98,8 +98,10 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
-// Arrives on a barrier of another CTA of the cluster (its address there: map_to_rank).  Default semantics (release at CTA scope): the operands handed over were put in place by the async-proxy fence and the
-// CTA's own barriers; `.release.cluster` costs a fence that waits for the thread's loads in flight, 0.9 us per stage.
+// Arrives on a barrier of another CTA of the cluster (its address there: map_to_rank).  Default semantics (release at CTA scope): weights that
+// are handed over lie in the sender's TMEM, where tcgen05.wait::st has seen them arrive, and the fences before_thread_sync in front of the arrive
+// and after_thread_sync behind the wait put the MMAs behind them; a TMA's data has landed when its own barrier says so; an exchange buffer that is given
+// back has been read into registers.  `.release.cluster` costs a fence that waits for the thread's loads in flight, 0.9 us per stage.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }

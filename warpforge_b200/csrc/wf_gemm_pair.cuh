@@ -3,7 +3,7 @@
 //
 // A pair computes 256 weight rows x up to 256 tokens: one tcgen05.mma of M = 256 spans both SMs, each SM holding its own 128 rows of A
 // (dequantized weights, fp16, in TMEM behind the accumulator), HALF of the tokens of B and its own 128 accumulator rows.
-// With A in TMEM the MMAs keep the tensor core's pace: 1000 cycles per 128 k and 256 tokens, 64 bytes of shared memory a
+// With A in TMEM the MMAs keep the tensor core's pace, 1024 cycles per 128 k and 256 tokens, and take 64 bytes of shared memory a
 // cycle of the 128 it can.  (A in shared memory, tiles of 512 tokens with eight dequantization warps: 109 bytes a cycle, 1300 -
 // 1500 cycles per 128 k and 256 tokens.)  What bounds it now: in long loops the power cap; in one call, 4 us until the first MMA, 3 - 6
 // us behind the last one.
@@ -126,13 +126,13 @@ __device__ __forceinline__ void tc_commit_pair(void* bar) {
                  : "memory");
 }
 
-// smem: [0, 1024) barriers + tmem slot | stages, 1024-byte aligned
+// smem: [0, 1024) barriers + tmem slot | PAIR_STAGES stages, 1024-byte aligned | a segment's sums, PAIR_SPILL
 template <int QT, bool WAVES>
 __global__ void __launch_bounds__(768, 1) gemm_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem);           // [4] leader: both CTAs' operands of the stage are in place
-    uint64_t* b_full = full + PAIR_STAGES;                        // [4] rank 1: its own TMA data has landed
-    uint64_t* s_empty = b_full + PAIR_STAGES;                     // [4] stage consumed by the MMAs
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem);           // [3] leader: both CTAs' operands of the stage are in place
+    uint64_t* b_full = full + PAIR_STAGES;                        // [3] rank 1: its own TMA data has landed
+    uint64_t* s_empty = b_full + PAIR_STAGES;                     // [3] stage consumed by the MMAs
     uint64_t* acc_full = s_empty + PAIR_STAGES;                   // the accumulator holds a segment
     uint64_t* acc_empty = acc_full + 1;                           // leader: the epilogues of both CTAs have read it
     uint64_t* tail_full = acc_empty + 1;                          // the accumulator of the tile shared with the following pairs
